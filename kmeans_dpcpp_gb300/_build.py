@@ -39,6 +39,7 @@ CU_SOURCES = [
     "kernels_util.cu",
     "kernels_lloyd.cu",
     "kernels_reloc.cu",
+    "kernels_step.cu",
     "kernels_mixed.cu",
     "driver.cu",
     "capi.cu",
@@ -47,7 +48,8 @@ CU_SOURCES = [
     "serve.cu",
     "init.cu",
 ]
-HEADERS = ["km_common.cuh", "km_kernels.cuh", "km_fit.cuh", "km_mixed.cuh", "km_batch.cuh"]
+HEADERS = ["km_common.cuh", "km_kernels.cuh", "km_fit.cuh", "km_mixed.cuh", "km_batch.cuh",
+           "km_step.cuh", "km_dist.cuh"]
 
 
 def _digest(paths, extra=""):

@@ -112,7 +112,7 @@ template <typename T, typename I>
 int reduce_centroids(const T *sz_cp, const T *c_cp, T *out_sz, T *out_c, I *list, I *n_empty,
                      int64_t P, int64_t d, int64_t k, cudaStream_t s) {
     CHECK_DIMS(P, d, k);
-    return launch_reduce_centroids<T, I, T>(sz_cp, c_cp, out_sz, out_c, list, n_empty, P, d, k,
+    return launch_reduce_centroids<T, I>(sz_cp, c_cp, out_sz, out_c, list, n_empty, P, d, k,
                                              s);
 }
 
@@ -124,7 +124,7 @@ int compute_threshold(const T *data, int64_t n, int64_t topk, T *thr, cudaStream
                   (long long)topk, (long long)n);
     Scratch sc;
     KMC_TRY(sc.alloc(threshold_scratch_bytes(), s));
-    return launch_threshold<T>(data, n, nullptr, topk, thr, sc.ptr, s);
+    return launch_threshold<T>(data, n, topk, thr, sc.ptr, s);
 }
 
 template <typename T, typename I>
@@ -135,7 +135,7 @@ int select_far(int64_t n_sel, const T *dist, const T *thr, I *sel, I *n_gt, I *n
     KMC_CHECK_ARG(n_sel <= n, "Argument `n_select` is too large");
     Scratch sc;
     KMC_TRY(sc.alloc(select_scratch_bytes(n_sel), s));
-    return launch_select<T, I>(nullptr, n_sel, dist, thr, sel, n_gt, n_eq, n, sc.ptr, n_sel, s);
+    return launch_select<T, I>(n_sel, dist, thr, sel, n_gt, n_eq, n, sc.ptr, s);
 }
 
 template <typename T, typename I>
@@ -157,12 +157,11 @@ int relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *
     T *thr = reinterpret_cast<T *>(b + o_thr);
     I *cnt = reinterpret_cast<I *>(b + o_cnt);
     I *sel = reinterpret_cast<I *>(b + o_sel);
-    KMC_TRY(launch_threshold<T>(sq_dist, n, nullptr, n_empty, thr, b + o_tsc, s));
+    KMC_TRY(launch_threshold<T>(sq_dist, n, n_empty, thr, b + o_tsc, s));
     KMC_TRY(launch_fill<I>(cnt, I(0), 1, s));
     KMC_TRY(launch_fill<I>(cnt + 1, I(1), 1, s));
-    KMC_TRY(launch_select<T, I>(nullptr, n_empty, sq_dist, thr, sel, cnt, cnt + 1, n, b + o_ssc,
-                                n_empty, s));
-    return launch_relocate<T, I>(nullptr, n_empty, X, w, labels, sel, cnt, list, C, sizes,
+    KMC_TRY(launch_select<T, I>(n_empty, sq_dist, thr, sel, cnt, cnt + 1, n, b + o_ssc, s));
+    return launch_relocate<T, I>(n_empty, X, w, labels, sel, cnt, list, C, sizes,
                                  inertia, n, d, k, s);
 }
 
@@ -452,7 +451,7 @@ int kmc_fit_step(kmc_fit_t fit, int64_t n_iterations) {
     kmc::Range range("kmc.fit_step");
     KMC_FIT_CHECK(fit);
     KMC_CHECK_ARG(n_iterations >= 0, "n_iterations must be non-negative");
-    for (int64_t t = 0; t < n_iterations; ++t) KMC_TRY(fit->impl->enqueue_iteration());
+    for (int64_t t = 0; t < n_iterations; ++t) KMC_TRY(fit->impl->enqueue_iteration(true));
     return KMC_OK;
 }
 int kmc_fit_run(kmc_fit_t fit) {

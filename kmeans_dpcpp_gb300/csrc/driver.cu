@@ -8,14 +8,14 @@
 //   swap -> ++n_iter;   while (n_iter < max_iter && shift_sum > tol).
 //
 // Here every kernel of an iteration is guarded by a device-resident loop
-// state: the loop-control kernel sets `done` once the reference's condition
-// fails, after which the remaining enqueued kernels return immediately.  The
-// relocation kernels are gated by the device value of n_empty.  The host
-// therefore enqueues iterations in batches and reads the state once per batch
-// instead of twice per iteration.  Centroid buffers do not ping-pong: new
-// centroids are copied back into the current buffer after the shift test, so
-// one iteration body works for every iteration (and can be captured once
-// into a CUDA graph).  The convergence total and the final inertia are summed
+// state: the end of an iteration (km_step.cuh) sets `done` once the
+// reference's condition fails, after which the remaining enqueued kernels
+// return immediately, and pauses the loop when a cluster is empty, until the
+// host has launched the relocation.  The host therefore enqueues iterations in batches and reads the
+// state once per batch instead of twice per iteration.  Centroid buffers do
+// not ping-pong: new centroids overwrite the current buffer at the end of an
+// iteration, so one iteration body works for every iteration (and can be
+// captured once into a CUDA graph).  The convergence total and the final inertia are summed
 // in float64.
 #include <algorithm>
 #include <cstdarg>
@@ -53,20 +53,19 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
         return o;
     };
     const size_t o_state = take(sizeof(LoopState));
+    const size_t o_ctl = take(sizeof(StepCtl));
+    const size_t o_scp = take(sizeof(double) * P * d * k);
+    const size_t o_zcp = take(sizeof(double) * P * k);
     const size_t o_hn = take(sizeof(T) * k);
+    const size_t o_prev = take(sizeof(T) * d * k);
+    const size_t o_sums = take(sizeof(T) * d * k);
     const size_t o_sizes = take(sizeof(T) * k);
     const size_t o_shifts = take(sizeof(T) * k);
     const size_t o_sq = take(sizeof(T) * n);
-    const size_t o_scp = take(sizeof(double) * P * d * k);
-    const size_t o_zcp = take(sizeof(double) * P * k);
-    const size_t o_list = take(sizeof(I) * (k + 1));
-    const size_t o_sel = take(sizeof(I) * (n + 2));
-    const size_t o_gate = take(sizeof(int64_t));
-    const size_t o_thr = take(sizeof(T));
+    const size_t o_list = take(sizeof(int64_t) * k);
+    const size_t o_rel = take(sizeof(int64_t) * 3 * k);
     const size_t o_part = take(sizeof(double) * sum_partials_size());
     const size_t o_dsum = take(sizeof(double) * 2);
-    const size_t o_tsc = take(threshold_scratch_bytes());
-    const size_t o_ssc = take(select_scratch_bytes(k));
     KMC_TRY(ws.alloc(off, p.stream));
     // the plain kernels' centroid-tile width for this (d, k, dtype)
     if (uses_private_copies()) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
@@ -83,22 +82,23 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     }
     char *b = ws.as<char>();
     state = reinterpret_cast<LoopState *>(b + o_state);
+    ctl = reinterpret_cast<StepCtl *>(b + o_ctl);
+    sums_cp = reinterpret_cast<double *>(b + o_scp);
+    sizes_cp = reinterpret_cast<double *>(b + o_zcp);
     hn = reinterpret_cast<T *>(b + o_hn);
+    prev = reinterpret_cast<T *>(b + o_prev);
+    sums = reinterpret_cast<T *>(b + o_sums);
     sizes = reinterpret_cast<T *>(b + o_sizes);
     shifts = reinterpret_cast<T *>(b + o_shifts);
     sq_dist = reinterpret_cast<T *>(b + o_sq);
-    sums_cp = reinterpret_cast<double *>(b + o_scp);
-    sizes_cp = reinterpret_cast<double *>(b + o_zcp);
-    empty_list = reinterpret_cast<I *>(b + o_list);
-    n_empty = empty_list + k;
-    selected = reinterpret_cast<I *>(b + o_sel);
-    counters = selected + n;
-    gate = reinterpret_cast<int64_t *>(b + o_gate);
-    threshold = reinterpret_cast<T *>(b + o_thr);
+    empty_list = reinterpret_cast<int64_t *>(b + o_list);
+    reloc = reinterpret_cast<int64_t *>(b + o_rel);
     partials = reinterpret_cast<double *>(b + o_part);
     dsum = reinterpret_cast<double *>(b + o_dsum);
-    thr_scratch = b + o_tsc;
-    sel_scratch = b + o_ssc;
+    // the control block and the private copies start at zero; each iteration
+    // leaves them so
+    KMC_CUDA_TRY(cudaMemsetAsync(ctl, 0, uses_private_copies() ? o_hn - o_ctl : o_scp - o_ctl,
+                                 p.stream));
 
     LoopState h{};
     h.done = 0;
@@ -115,24 +115,13 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
 }
 
 template <typename T, typename I>
-int PlainFit<T, I>::enqueue_iteration() {
+int PlainFit<T, I>::enqueue_iteration(bool relocate) {
     const FitParams<T, I> &p = prm;
     const int64_t n = p.n, d = p.d, k = p.k;
     cudaStream_t s = p.stream;
-    T *cur = p.centroids;       // this_centroids_t
-    T *nxt = p.new_centroids;   // new_centroids_t
-    const int64_t thr_launches = 1 + 2 * (sizeof(T) == 4 ? 4 : 8);
-    const T *xv = nullptr;
-    int64_t xfs = 0, xss = 0;
-    x_view(&xv, &xfs, &xss);
     // kmeans_lloyd_driver.hpp:86-111
-    KMC_TRY(launch_half_norm<T>(cur, hn, d, k, s, state));
-    const bool copies = uses_private_copies();
-    if (copies) {
-        KMC_TRY(launch_fill<double>(sums_cp, 0.0, P * d * k, s, state));
-        KMC_TRY(launch_fill<double>(sizes_cp, 0.0, P * k, s, state));
-    }
-    KMC_TRY(launch_fill<I>(n_empty, I(0), 1, s, state));
+    int64_t begin_launches = 0, step_launches = 0, finish_launches = 0;
+    KMC_TRY(begin_step(&begin_launches));
     // kmeans_lloyd_driver.hpp:124-143
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (profiling) {
@@ -140,42 +129,42 @@ int PlainFit<T, I>::enqueue_iteration() {
         KMC_CUDA_TRY(cudaEventCreate(&e1));
         KMC_CUDA_TRY(cudaEventRecord(e0, s));
     }
-    int64_t step_launches = 0;
-    KMC_TRY(step_assign_and_accumulate(cur, &step_launches));
+    KMC_TRY(step_assign_and_accumulate(p.centroids, &step_launches));
     if (profiling) {
         KMC_CUDA_TRY(cudaEventRecord(e1, s));
         phase_events.emplace_back(e0, e1);
     }
-    // kmeans_lloyd_driver.hpp:155-170
-    KMC_TRY(reduce_step(nxt));
-    int64_t verbose_launches = 0;
+    // kmeans_lloyd_driver.hpp:155-170, 317-353
+    KMC_TRY(finish_step(&finish_launches));
+    launches += begin_launches + step_launches + finish_launches;
     if (p.verbose) {
-        // kmeans_lloyd_driver.hpp:179-197: inertia of the *undivided* sums.
-        KMC_TRY(launch_inertia<T, I>(xv, p.w, nxt, p.labels, sq_dist, n, d, k, s, state, nullptr,
-                                     xfs, xss));
-        KMC_TRY(launch_sum_f64<T>(sq_dist, n, partials, dsum, s, state));
-        verbose_launches = 3;
+        // kmeans_lloyd_driver.hpp:179-197: inertia of the *undivided* sums
+        // (before a relocation moves any)
+        const T *xv = nullptr;
+        int64_t xfs = 0, xss = 0;
+        x_view(&xv, &xfs, &xss);
+        KMC_TRY(launch_inertia<T, I>(xv, p.w, sums, p.labels, sq_dist, n, d, k, s, xfs, xss));
+        KMC_TRY(launch_sum_f64<T>(sq_dist, n, partials, dsum, s));
+        launches += 3;
     }
-    // kmeans_lloyd_driver.hpp:217-312, gated on the device value of n_empty.
-    KMC_TRY(launch_gate_from_count<I>(n_empty, gate, s, state));
-    KMC_TRY(launch_inertia<T, I>(xv, nullptr, cur, p.labels, sq_dist, n, d, k, s, state, gate,
-                                 xfs, xss));
-    KMC_TRY(launch_threshold<T>(sq_dist, n, gate, 0, threshold, thr_scratch, s, state));
-    KMC_TRY(launch_fill<I>(counters, I(0), 1, s, state));
-    KMC_TRY(launch_fill<I>(counters + 1, I(1), 1, s, state));
-    KMC_TRY(launch_select<T, I>(gate, 0, sq_dist, threshold, selected, counters, counters + 1, n,
-                                sel_scratch, k, s, state));
-    KMC_TRY(launch_relocate<T, I>(gate, 0, xv, p.w, p.labels, selected, counters, empty_list,
-                                  nxt, sizes, sq_dist, n, d, k, s, state, xfs, xss));
-    // kmeans_lloyd_driver.hpp:317-353
-    KMC_TRY(launch_divide_and_shift<T>(cur, nxt, sizes, shifts, d, k, s, state));
-    KMC_TRY(launch_loop_control<T>(shifts, k, state, s));
-    KMC_CUDA_TRY(cudaMemcpyAsync(cur, nxt, sizeof(T) * d * k, cudaMemcpyDeviceToDevice, s));
-    // 4 (norm, fills) + step + 2 (reduce) + gate + inertia + threshold + 2 fills
-    // + 4 (select) + relocate + divide/shift + control
-    launches += (copies ? 4 : 2) + step_launches + 2 + verbose_launches + 1 + 1 + thr_launches + 2 +
-                select_launches(k) + 1 + 1 + 1;
+    if (relocate) KMC_TRY(enqueue_relocation());
     ++issued;
+    return KMC_OK;
+}
+
+// kmeans_lloyd_driver.hpp:217-312, of an iteration that left clusters empty
+template <typename T, typename I>
+int PlainFit<T, I>::enqueue_relocation() {
+    const FitParams<T, I> &p = prm;
+    const T *xv = nullptr;
+    int64_t xfs = 0, xss = 0, crs = 0;
+    x_view(&xv, &xfs, &xss);
+    const T *cr = c_rows(&crs);
+    const RelocArgs<T, I> ra{p.centroids, p.new_centroids, prev, sums, sizes, shifts, empty_list,
+                             reloc, reloc + p.k, reloc + 2 * p.k, xv, p.w, p.labels, sq_dist, p.n,
+                             p.d, p.k, xfs, xss, cr, crs, wait_clocks(), state, ctl};
+    KMC_TRY((launch_relocation<T, I>(ra, p.stream)));
+    ++launches;
     return KMC_OK;
 }
 
@@ -202,18 +191,27 @@ int PlainFit<T, I>::run(int64_t max_batch) {
     LoopState h{};
     KMC_TRY(read_state(h));
     int64_t batch = 1;
-    while (!h.done && issued < p.max_iter) {
-        int64_t m = p.verbose ? 1 : std::min<int64_t>(batch, p.max_iter - issued);
+    while (h.done == kPaused || (!h.done && h.n_iter < p.max_iter)) {
+        // an iteration that left clusters empty paused the loop; the rest of
+        // its batch did nothing
+        if (h.done == kPaused) {
+            KMC_TRY(enqueue_relocation());
+            batch = 1;
+        }
+        const int64_t left = p.max_iter - h.n_iter - (h.done == kPaused ? 1 : 0);
+        int64_t m = p.verbose ? 1 : std::min<int64_t>(batch, left);
+        if (p.verbose && h.done == kPaused) m = 0;
         if (max_batch > 0) m = std::min<int64_t>(m, max_batch);
-        for (int64_t t = 0; t < m; ++t) KMC_TRY(enqueue_iteration());
+        const bool fresh = h.done != kPaused;
+        for (int64_t t = 0; t < m; ++t) KMC_TRY(enqueue_iteration(false));
         KMC_TRY(read_state(h));
-        if (p.verbose && p.print_fn != nullptr && h.n_iter > 0) {
+        if (p.verbose && p.print_fn != nullptr && fresh) {
             double tot = 0.0;
             KMC_CUDA_TRY(cudaMemcpy(&tot, dsum, sizeof(double), cudaMemcpyDeviceToHost));
             char line[128];
             // kmeans_lloyd_driver.hpp:199-204
-            snprintf(line, sizeof(line), "Iteration: %lld Inertia: %.9g", (long long)(h.n_iter - 1),
-                     (double)(T)tot);
+            snprintf(line, sizeof(line), "Iteration: %lld Inertia: %.9g",
+                     (long long)(h.done == kPaused ? h.n_iter : h.n_iter - 1), (double)(T)tot);
             p.print_fn(line, p.print_ctx);
         }
         if (batch < 64) batch *= 2;
@@ -228,13 +226,13 @@ int PlainFit<T, I>::finalize_enqueue(LoopState *state_out, double *inertia_out) 
     cudaStream_t s = p.stream;
     // kmeans_lloyd_driver.hpp:360-418: final assignment and inertia against
     // the final centroids.
-    KMC_TRY(launch_half_norm<T>(p.centroids, hn, d, k, s));
     KMC_TRY(final_assignment());
     const T *xv = nullptr;
-    int64_t xfs = 0, xss = 0;
+    int64_t xfs = 0, xss = 0, crs = 0;
     x_view(&xv, &xfs, &xss);
-    KMC_TRY(launch_inertia<T, I>(xv, p.w, p.centroids, p.labels, sq_dist, n, d, k, s, nullptr,
-                                 nullptr, xfs, xss));
+    const T *cr = c_rows(&crs);
+    KMC_TRY(launch_inertia<T, I>(xv, p.w, p.centroids, p.labels, sq_dist, n, d, k, s, xfs, xss, cr,
+                                 crs));
     KMC_TRY(launch_sum_f64<T>(sq_dist, n, partials, dsum, s));
     launches += 5;
     if (p.new_centroids != p.centroids && d * k > 0)
@@ -259,15 +257,16 @@ int PlainFit<T, I>::finalize(int64_t *n_iter_out, double *inertia_out) {
 }
 
 template <typename T, typename I>
-int PlainFit<T, I>::reduce_step(T *nxt) {
+int PlainFit<T, I>::finish_step(int64_t *n_launches) {
     const FitParams<T, I> &p = prm;
-    return launch_reduce_centroids<T, I, double>(sizes_cp, sums_cp, sizes, nxt, empty_list,
-                                                 n_empty, P, p.d, p.k, p.stream, state);
+    const PlainSums src{sums_cp, sizes_cp, p.d * p.k, p.k, P};
+    return launch_reduce_and_finish<T>(src, P, finish_args(), n_launches, p.stream);
 }
 
 template <typename T, typename I>
 int PlainFit<T, I>::final_assignment() {
     const FitParams<T, I> &p = prm;
+    KMC_TRY(launch_half_norm<T>(p.centroids, hn, p.d, p.k, p.stream));
     return launch_assignment<T, I>(p.X, p.centroids, hn, p.labels, p.n, p.d, p.k, p.stream,
                                    nullptr, tile_variant);
 }

@@ -79,6 +79,7 @@
 #include "km_batch.cuh"
 #include "km_fit.cuh"
 #include "km_mixed.cuh"
+#include "km_step.cuh"
 
 namespace kmc {
 
@@ -108,6 +109,12 @@ struct MixedConsts {
     unsigned int wmax_bits;  // max |w| (fp32 bits; fixed-point sums only)
     int fx_shift;            // w x and w are summed as the integers w x 2^fx_shift, w 2^fx_shift
     int fx_ok;               // the fixed-point sums may be used (finite bounds)
+    // per pass, cleared by the preparation's last CTA
+    int acc_dirty;                  // fixed-point fits: a term went to the float64 copies
+    unsigned prep_ticket;
+    unsigned hmax_bits;             // max |hn_j| (fp32 bits)
+    unsigned long long c2max_bits;  // max ||c_j||^2, max of its operands' rounding
+    unsigned long long dc2max_bits; // errors' squared norms, scaled (fp64 bits)
 };
 
 // Order-independent totals of the fixed-point sums (d <= 32): element e
@@ -123,6 +130,7 @@ struct FxAcc {
     unsigned long long *lo;
     int64_t stride;  // elements per copy
     int copies;
+    int *dirty;      // set when a term went to the float64 copies instead
     // the copy of block b
     __device__ __forceinline__ FxAcc copy_of(unsigned b) const {
         FxAcc r = *this;
@@ -153,6 +161,7 @@ __device__ __forceinline__ void add_packed_row(const FxAcc &fx, double *acc64, i
         const int pk = fx.xq[i * ds + j];
         if (pk == 1) {
             const float v = j < d4 ? __fmul_rn(xrow[i * d4 + j], wv) : wv;
+            *reinterpret_cast<volatile int *>(fx.dirty) = 1;
             atomicAdd(j < d4 ? acc64 + c * d4 + j : acc64 + k_pad * d4 + c, (double)v);
         } else if (pk != 0) {
             fx_add(fx, j < d4 ? c * d4 + j : k * d4 + c,
@@ -444,6 +453,7 @@ __device__ __noinline__ void rare_terms(const MixedArgs &a, double *acc64, int64
         for (int j = c0; j < c0 + nc; ++j) {
             if (stage[r * ds + j] != 1) continue;
             const float w = a.w[i0 + r];
+            *reinterpret_cast<volatile int *>(a.fx.dirty) = 1;
             if (j < d4) {
                 const float v = __fmul_rn(a.xrow[(i0 + r) * d4 + j], w);
                 if (v != 0.f) atomicAdd(acc64 + (int64_t)c * d4 + j, (double)v);
@@ -1227,151 +1237,163 @@ __device__ __forceinline__ float max16() {
     return BF16 ? 3.3895313892515355e38f : 65504.f;
 }
 
-// Centroid image (rows j < k_pad, zero padding), the half-norm block and the
-// per-centroid norms ||c_j|| and ||round16(c_j sigma) - c_j sigma|| / sigma
-// (both rounded up).  Row j of the half-norm block holds (h0, h1, h2) with
+// Preparation of a pass: half norms (sequential fma over the features, as the
+// reference's), the centroid image (rows j < k_pad, zero padding) with its
+// half-norm block, the row-major fp32 centroids, the constants of the error
+// bound, and a cleared recheck count.  Row j of the half-norm block holds
+// (h0, h1, h2) with
 //   c0 h0 + c1 h1 + c2 h2 = -sigma^2 hn_j   (c = norm_coef)
 // up to sigma^2 |hn_j| u^3 (u = 2^-11 fp16, 2^-8 bf16; plus 2^-35 for fp16
 // subnormal parts): h0 is the rounded leading part and each following part
 // the rounded remainder, formed exactly in fp64.  A value that would leave the
 // operand range is clamped and raises consts->overflow, which disables
 // certification for the pass (every sample is then re-evaluated exactly).
+//
+// One launch instead of five (half norms, image, bound constants and two
+// resets: 27 us at k = 1024, all latency): a CTA takes the 8 rows of one
+// swizzle atom, G = 8 nkb (rounded up to a power of two) lanes per row, lane
+// qc of a row its features 8 qc .. 8 qc + 7; the float64 operations (2 per
+// clock and SM) are kept to the squared norms, the square roots to the last
+// CTA, which turns the maxima over all rows into the bound's constants.
+constexpr int kPrepRows = 8;
+
 template <int BF16>
-__global__ void c_image_kernel(const float *C, const float *hn, int64_t d, int64_t k,
-                               int64_t k_pad, int nkb, MixedConsts *c, uint8_t *img, float *cn2,
-                               float *dcn, float *ct, int64_t d4, const LoopState *guard) {
+__global__ void __launch_bounds__(256) mixed_prep_kernel(
+    const float *C, int64_t d, int64_t k, int64_t k_pad, int nkb, MixedConsts *c, uint8_t *img,
+    float *hn, float *ct, int64_t d4, int *n_flagged, const LoopState *guard) {
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
+    __shared__ float cs[64 * 4 * (kPrepRows + 1)];
+    __shared__ double q_sh[2][kPrepRows];
+    __shared__ float h_sh[kPrepRows];
+    const int tid = threadIdx.x, G = (int)blockDim.x / kPrepRows;
+    const int64_t j0 = (int64_t)blockIdx.x * kPrepRows;
     const float sigma = c->sigma;
     const double s2 = (double)sigma * (double)sigma;
     const float lim = max16<BF16>();
     bool ovf = false;
-    // One thread per (centroid row j, 8-feature chunk): G = 8 nkb rounded up
-    // to a power of two consecutive lanes hold one row, the ones past its 8 nkb
-    // chunks idle (k_pad G is a multiple of 32, so every warp is either
-    // entirely inside the range or entirely past it, and a row's lanes never
-    // straddle two warps).
-    const int G = (nkb <= 1) ? 8 : (nkb == 2 ? 16 : 32);
-    const int64_t total = k_pad * G;
-    for (int64_t tt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; tt < total;
-         tt += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = tt / G;
-        const int qc = (int)(tt % G), kb = qc >> 3, ch = qc & 7;
-        const bool lane_used = kb < nkb;
-        const int64_t f0 = (int64_t)kb * 64 + ch * 8;
-        double q2 = 0.0, qd = 0.0;
+    if (blockIdx.x == 0 && tid == 0) *n_flagged = 0;
+    for (int e = tid; e < nkb * 64 * kPrepRows; e += (int)blockDim.x) {
+        const int f = e / kPrepRows, r = e % kPrepRows;
+        cs[f * (kPrepRows + 1) + r] = (f < d && j0 + r < k) ? C[f * k + j0 + r] : 0.f;
+    }
+    __syncthreads();
+    const int r = tid / G, qc = tid % G, kb = qc >> 3, ch = qc & 7;
+    const int64_t j = j0 + r;
+    const int f0 = qc * 8;
+    double q2 = 0.0, qd = 0.0;
+    if (kb < nkb) {
         float v[8], xr[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const int64_t f = f0 + e;
-            const float x = (lane_used && j < k && f < d) ? C[f * k + j] : 0.f;
+            const float x = cs[(f0 + e) * (kPrepRows + 1) + r];
             q2 += (double)x * (double)x;
             float sv = x * sigma;
             if (!(fabsf(sv) <= lim)) {
                 ovf = true;
                 sv = (sv > 0.f) ? lim : ((sv < 0.f) ? -lim : 0.f);
             }
-            const double dv = (double)round16<BF16>(sv) - (double)sv;
+            const double dv = (double)(round16<BF16>(sv) - sv);  // exact in fp32
             qd += dv * dv;
             v[e] = sv;
             xr[e] = x;
         }
-        if (lane_used) {
-            // d4 is a multiple of 4 and f0 of 8: whole float4 stores
-            float4 *cdst = reinterpret_cast<float4 *>(ct + j * d4 + f0);
-            if (f0 < d4) cdst[0] = make_float4(xr[0], xr[1], xr[2], xr[3]);
-            if (f0 + 4 < d4) cdst[1] = make_float4(xr[4], xr[5], xr[6], xr[7]);
-            uint4 pk;
-            pk.x = pack2<BF16>(v[0], v[1]);
-            pk.y = pack2<BF16>(v[2], v[3]);
-            pk.z = pack2<BF16>(v[4], v[5]);
-            pk.w = pack2<BF16>(v[6], v[7]);
-            *reinterpret_cast<uint4 *>(img + (size_t)kb * k_pad * 128 +
-                                       sw128_offset((uint32_t)j, (uint32_t)ch * 8)) = pk;
-        }
-        // the row's squared norms over its G chunk lanes
-        for (int o = G >> 1; o > 0; o >>= 1) {
-            q2 += __shfl_xor_sync(0xffffffffu, q2, o);
-            qd += __shfl_xor_sync(0xffffffffu, qd, o);
-        }
-        if (qc != 0) continue;
-        float h0 = 0.f, h1 = 0.f, h2 = 0.f;
+        // d4 is a multiple of 4 and f0 of 8: whole float4 stores
+        float4 *cdst = reinterpret_cast<float4 *>(ct + j * d4 + f0);
+        if (f0 < d4) cdst[0] = make_float4(xr[0], xr[1], xr[2], xr[3]);
+        if (f0 + 4 < d4) cdst[1] = make_float4(xr[4], xr[5], xr[6], xr[7]);
+        uint4 pk;
+        pk.x = pack2<BF16>(v[0], v[1]);
+        pk.y = pack2<BF16>(v[2], v[3]);
+        pk.z = pack2<BF16>(v[4], v[5]);
+        pk.w = pack2<BF16>(v[6], v[7]);
+        *reinterpret_cast<uint4 *>(img + (size_t)kb * k_pad * 128 +
+                                   sw128_offset((uint32_t)j, (uint32_t)ch * 8)) = pk;
+    }
+    // the row's squared norms over its G lanes
+    for (int o = G >> 1; o > 0; o >>= 1) {
+        q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+        qd += __shfl_xor_sync(0xffffffffu, qd, o);
+    }
+    if (qc == 0) {
+        float h = 0.f, h0 = 0.f, h1 = 0.f, h2 = 0.f;
         if (j < k) {
-            const double H = (double)hn[j] * s2;
+#pragma unroll 8
+            for (int f = 0; f < (int)d; ++f) {
+                const float x = cs[f * (kPrepRows + 1) + r];
+                h = __fmaf_rn(x, x, h);
+            }
+            h = h / 2.f;
+            hn[j] = h;
+            const double H = (double)h * s2;
+            // the coefficients are powers of two: exact reciprocals
             const double c0 = -(double)norm_coef(BF16, 0), c1 = -(double)norm_coef(BF16, 1),
                          c2 = -(double)norm_coef(BF16, 2);
-            h0 = round16<BF16>((float)(H / c0));
+            h0 = round16<BF16>((float)(H * (1.0 / c0)));
             if (!(fabsf(h0) <= lim)) {
                 ovf = true;
                 h0 = (H > 0.0) ? lim : -lim;
             }
             const double r1 = H - c0 * (double)h0;
-            h1 = round16<BF16>((float)(r1 / c1));
+            h1 = round16<BF16>((float)(r1 * (1.0 / c1)));
             const double r2 = r1 - c1 * (double)h1;
-            h2 = round16<BF16>((float)(r2 / c2));
+            h2 = round16<BF16>((float)(r2 * (1.0 / c2)));
             if (!(fabsf(h1) <= lim) || !(fabsf(h2) <= lim)) {
                 ovf = true;
                 h1 = 0.f;
                 h2 = 0.f;
             }
-            cn2[j] = __double2float_ru(sqrt(q2) * (1.0 + 1e-12));
-            dcn[j] = __double2float_ru(sqrt(qd) / (double)sigma * (1.0 + 1e-12));
         }
         uint8_t *nb = img + (size_t)nkb * k_pad * 128;
         uint4 p0 = make_uint4(pack2<BF16>(h0, h1), pack2<BF16>(h2, 0.f), 0u, 0u);
         *reinterpret_cast<uint4 *>(nb + sw32_offset((uint32_t)j, 0)) = p0;
         *reinterpret_cast<uint4 *>(nb + sw32_offset((uint32_t)j, 8)) = make_uint4(0u, 0u, 0u, 0u);
+        // NaN norms never raise a maximum
+        q_sh[0][r] = q2 == q2 ? q2 : 0.0;
+        q_sh[1][r] = qd == qd ? qd : 0.0;
+        h_sh[r] = h == h ? fabsf(h) : 0.f;
     }
     if (ovf) atomicOr(&c->overflow, 1);
-}
-
-// Per-iteration bound constants (one block), in the scaled units of the
-// scores (sigma^2).  Resets the overflow flag raised by c_image_kernel.
-__global__ void bound_kernel(const float *cn2, const float *dcn, const float *hn, int64_t d,
-                             int64_t k, int bf16, MixedConsts *c, const LoopState *guard) {
-    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
-    __shared__ float sh[3][32];
-    float m2 = 0.f, m1 = 0.f, mh = 0.f;
-    for (int64_t j = threadIdx.x; j < k; j += blockDim.x) {
-        m2 = fmaxf(m2, cn2[j]);
-        m1 = fmaxf(m1, dcn[j]);
-        mh = fmaxf(mh, fabsf(hn[j]));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-        mh = fmaxf(mh, __shfl_xor_sync(0xffffffffu, mh, o));
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        sh[0][wid] = m2;
-        sh[1][wid] = m1;
-        sh[2][wid] = mh;
-    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            m2 = fmaxf(m2, sh[0][w]);
-            m1 = fmaxf(m1, sh[1][w]);
-            mh = fmaxf(mh, sh[2][w]);
+    if (tid == 0) {
+        double m2 = 0.0, md = 0.0;
+        float mh = 0.f;
+        for (int q = 0; q < kPrepRows; ++q) {
+            m2 = fmax(m2, q_sh[0][q]);
+            md = fmax(md, q_sh[1][q]);
+            mh = fmaxf(mh, h_sh[q]);
         }
-        const double sigma = (double)c->sigma, s2 = sigma * sigma;
-        const double u = bf16 ? 0x1p-8 : 0x1p-11;
-        const double cmax = (double)m2, dcmax = (double)m1;
-        // bf16 subnormal inputs may be flushed by the tensor cores (fp16
-        // subnormals are part of the measured rounding errors)
-        const double flush = bf16 ? 0x1p-126 * sqrt((double)d) * (1 + u) : 0.0;
-        const double alpha =
-            dcmax + 0x1p-16 * (cmax + dcmax) + (double)(d + 4) * 0x1p-23 * cmax + flush;
-        const double beta1 = (cmax + dcmax) * (1 + 0x1p-16);
-        const double hfloor = (bf16 ? 0x1p-126 : 0x1p-34) / s2;
-        const double beta0 =
-            (double)mh * (u * u * u + 0x1p-16 + 0x1p-23) + hfloor + flush * cmax;
-        c->alpha = __double2float_ru(alpha * s2 * (1 + 1e-6));
-        c->beta1 = __double2float_ru(beta1 * s2 * (1 + 1e-6));
-        c->beta0 = c->overflow ? pos_inf<float>()
-                               : __double2float_ru(beta0 * s2 * (1 + 1e-6) + 1e-37);
-        c->overflow = 0;
+        // non-negative: ordered like their bits
+        atomicMax(&c->c2max_bits, (unsigned long long)__double_as_longlong(m2));
+        atomicMax(&c->dc2max_bits, (unsigned long long)__double_as_longlong(md));
+        atomicMax(&c->hmax_bits, __float_as_uint(mh));
     }
+    if (!last_cta(&c->prep_ticket) || tid != 0) return;
+    volatile MixedConsts *vc = c;
+    const double u = BF16 ? 0x1p-8 : 0x1p-11;
+    const double m2 = __longlong_as_double((long long)vc->c2max_bits);
+    const double md = __longlong_as_double((long long)vc->dc2max_bits);
+    const double mh = (double)__uint_as_float(vc->hmax_bits);
+    const int over = vc->overflow;
+    const double cmax = (double)__double2float_ru(sqrt(m2) * (1.0 + 1e-12));
+    const double dcmax = (double)__double2float_ru(sqrt(md) / (double)sigma * (1.0 + 1e-12));
+    // bf16 subnormal inputs may be flushed by the tensor cores (fp16
+    // subnormals are part of the measured rounding errors)
+    const double flush = BF16 ? 0x1p-126 * sqrt((double)d) * (1 + u) : 0.0;
+    const double alpha =
+        dcmax + 0x1p-16 * (cmax + dcmax) + (double)(d + 4) * 0x1p-23 * cmax + flush;
+    const double beta1 = (cmax + dcmax) * (1 + 0x1p-16);
+    const double hfloor = (BF16 ? 0x1p-126 : 0x1p-34) / s2;
+    const double beta0 = mh * (u * u * u + 0x1p-16 + 0x1p-23) + hfloor + flush * cmax;
+    c->alpha = __double2float_ru(alpha * s2 * (1 + 1e-6));
+    c->beta1 = __double2float_ru(beta1 * s2 * (1 + 1e-6));
+    c->beta0 =
+        over ? pos_inf<float>() : __double2float_ru(beta0 * s2 * (1 + 1e-6) + 1e-37);
+    c->overflow = 0;
+    c->acc_dirty = 0;
+    c->c2max_bits = 0ull;
+    c->dc2max_bits = 0ull;
+    c->hmax_bits = 0u;
+    c->prep_ticket = 0u;
 }
 
 // Exact fp32 re-evaluation of samples whose margin did not certify them: the
@@ -1405,8 +1427,13 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
     const int *flagged, const int *n_flagged, int64_t n, int64_t d, int64_t k, int64_t d4,
     void *labels, int label64, int update, int acc_f64, float *sums32, double *acc64,
     int64_t k_pad, int n_copies, const LoopState *guard, int passes, int64_t pass_cols, FxAcc fx,
-    const MixedConsts *consts) {
+    const MixedConsts *consts, long long *stats) {
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // the fit's statistics: samples rechecked in this pass, and in total
+        stats[0] = *n_flagged;
+        stats[1] += *n_flagged;
+    }
     constexpr int kWarps = kRecheckThreads / 32;
     const bool use_fx = fx.xq != nullptr && consts->fx_ok;
     fx = fx.copy_of(blockIdx.x);
@@ -1642,75 +1669,89 @@ __global__ void __launch_bounds__(256) combine_kernel(
     }
 }
 
-// Per-CTA copies of the cluster-major sums (fp32 or fp64) -> (d, k) centroid
-// sums and sizes in dataT: copies added in index order in fp64, rounded once.
+// The sums of an iteration (km_step.cuh): the fixed-point totals (exact to one
+// rounding), then the cluster-major float copies ([copy][k_pad d4 + k_pad]),
+// each copy zeroed once read.  With fixed-point totals the float64 copies hold
+// anything only when a kernel set acc_dirty (`always`: the assignment's own
+// float64 reductions use them).
 template <typename A>
-__global__ void km_to_dk_kernel(const A *copies, int n_copies, float *out_c, float *out_sizes,
-                                int64_t d, int64_t k, int64_t k_pad, int64_t d4, FxAcc fx,
-                                const MixedConsts *consts, const LoopState *guard) {
-    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
-    const int64_t cs = k_pad * d4 + k_pad;
-    // consecutive threads read consecutive words of every copy
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < k * d4 + k;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const bool is_size = e >= k * d4;
-        const int64_t off = is_size ? k_pad * d4 + (e - k * d4) : e;
-        const int64_t j = e / d4, f = e % d4;
-        if (!is_size && f >= d) continue;
-        // the integer totals (exact to one rounding), then the copies added
-        // in index order; loads issued eight ahead of the adds
-        double acc = 0.0;
-        if (fx.hi != nullptr && consts->fx_ok) {
-            long long h = 0;
-            unsigned long long l = 0;
-            for (int c = 0; c < fx.copies; ++c) {
-                h += fx.hi[(int64_t)c * fx.stride + e];
-                l += fx.lo[(int64_t)c * fx.stride + e];
+struct MixedSums {
+    A *copies;
+    int n_copies, always;
+    int64_t k, k_pad, d4;
+    FxAcc fx;
+    MixedConsts *consts;
+    struct Part {
+        double v;
+        long long hi;
+        unsigned long long lo;
+    };
+    // cluster-major, the sizes last
+    __device__ __forceinline__ void at(int64_t e, int64_t d, int64_t *f, int64_t *j) const {
+        if (e < k * d) {
+            *j = e / d;
+            *f = e - *j * d;
+        } else {
+            *f = d;
+            *j = e - k * d;
+        }
+    }
+    __device__ __forceinline__ Part load(int64_t f, int64_t j, int64_t d, int g, int groups) const {
+        Part p = zero();
+        const bool use_fx = fx.hi != nullptr && consts->fx_ok;
+        if (use_fx) {
+            const int64_t e = f < d ? j * d4 + f : k * d4 + j;
+            for (int c = g; c < fx.copies; c += 4 * groups) {
+                long long h[4];
+                unsigned long long l[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool in = c + u * groups < fx.copies;
+                    h[u] = in ? fx.hi[(c + u * groups) * fx.stride + e] : 0;
+                    l[u] = in ? fx.lo[(c + u * groups) * fx.stride + e] : 0ull;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (c + u * groups < fx.copies) {
+                        fx.hi[(c + u * groups) * fx.stride + e] = 0;
+                        fx.lo[(c + u * groups) * fx.stride + e] = 0ull;
+                    }
+                    p.hi += h[u];
+                    p.lo += l[u];
+                }
             }
-            acc = ((double)h * 4294967296.0 + (double)l) * (1.0 / (double)pow2f(consts->fx_shift));
         }
-        int c = 0;
-        for (; c + 8 <= n_copies; c += 8) {
-            A v[8];
+        if (!use_fx || always || consts->acc_dirty) {
+            A *q = copies + (f < d ? j * d4 + f : k_pad * d4 + j);
+            const int64_t stride = k_pad * d4 + k_pad;
+            for (int c = g; c < n_copies; c += 8 * groups) {
+                A v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = copies[(int64_t)(c + u) * cs + off];
+                for (int u = 0; u < 8; ++u)
+                    v[u] = c + u * groups < n_copies ? q[(c + u * groups) * stride] : A(0);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) acc += (double)v[u];
+                for (int u = 0; u < 8; ++u)
+                    if (c + u * groups < n_copies) q[(c + u * groups) * stride] = A(0);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (c + u * groups < n_copies) p.v += (double)v[u];
+            }
         }
-        for (; c < n_copies; ++c) acc += (double)copies[(int64_t)c * cs + off];
-        if (is_size)
-            out_sizes[e - k * d4] = (float)acc;
-        else
-            out_c[f * k + j] = (float)acc;
+        return p;
     }
-}
-
-__global__ void reset_kernel(float *sums32, double *acc64, int64_t count, int acc_f64,
-                             int *n_flagged, FxAcc fx, int64_t fx_count, const LoopState *guard) {
-    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        if (acc_f64)
-            acc64[e] = 0.0;
-        else
-            sums32[e] = 0.f;
+    static __device__ __forceinline__ Part zero() { return Part{0.0, 0, 0ull}; }
+    static __device__ __forceinline__ void add(Part &a, const Part &b) {
+        a.v += b.v;
+        a.hi += b.hi;
+        a.lo += b.lo;
     }
-    if (fx.hi != nullptr)
-        for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-             e < fx_count * fx.copies; e += (int64_t)gridDim.x * blockDim.x) {
-            fx.hi[e] = 0;
-            fx.lo[e] = 0ull;
-        }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n_flagged = 0;
-}
-
-// Copies the flagged count of this pass into the per-fit statistics.
-__global__ void stats_kernel(const int *n_flagged, long long *last, long long *total,
-                             const LoopState *guard) {
-    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
-    *last = *n_flagged;
-    *total += *n_flagged;
-}
+    __device__ __forceinline__ double value(const Part &p) const {
+        if (fx.hi == nullptr || !consts->fx_ok) return p.v;
+        return ((double)p.hi * 4294967296.0 + (double)p.lo) *
+                   (1.0 / (double)pow2f(consts->fx_shift)) + p.v;
+    }
+    __device__ __forceinline__ void done() const {}
+};
 
 using MixedKernel = void (*)(MixedArgs);
 
@@ -1861,9 +1902,9 @@ int tune_mixed_variant(int64_t d, int64_t k, int form, bool large, const std::ve
         tl_force_mixed_variant = -1;
         if (rc != KMC_OK) continue;
         float ms = 0.f;
-        rc = fit->enqueue_iteration();
+        rc = fit->enqueue_iteration(true);
         if (rc == KMC_OK) rc = cudaEventRecord(e0, s) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
-        for (int it = 0; it < 4 && rc == KMC_OK; ++it) rc = fit->enqueue_iteration();
+        for (int it = 0; it < 4 && rc == KMC_OK; ++it) rc = fit->enqueue_iteration(true);
         if (rc == KMC_OK) rc = cudaEventRecord(e1, s) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
         if (rc == KMC_OK) rc = cudaEventSynchronize(e1) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
         if (rc == KMC_OK) rc = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
@@ -1896,7 +1937,6 @@ struct MixedFit : PlainFit<float, I> {
     float *sums32 = nullptr;
     double *acc64 = nullptr;
     int n_copies = 1;  // private copies of the cluster sums (one per CTA)
-    float *cn2 = nullptr, *dcn = nullptr;
     MixedConsts *consts = nullptr;
     uint4 *cand = nullptr;
     int *flagged = nullptr, *n_flagged = nullptr, *err_dev = nullptr;
@@ -1934,8 +1974,9 @@ struct MixedFit : PlainFit<float, I> {
     // its variant has them, the recheck and the column passes' combine.
     bool fx_on = false;
     FxAcc fx_acc() const {
-        return fx_on ? FxAcc{xq, fxhi, fxlo, this->prm.k * d4 + this->prm.k, n_copies}
-                     : FxAcc{nullptr, nullptr, nullptr, 0, 1};
+        return fx_on ? FxAcc{xq, fxhi, fxlo, this->prm.k * d4 + this->prm.k, n_copies,
+                             &consts->acc_dirty}
+                     : FxAcc{nullptr, nullptr, nullptr, 0, 1, &consts->acc_dirty};
     }
 
     static bool supported(int64_t d, int64_t k) {
@@ -2026,9 +2067,9 @@ struct MixedFit : PlainFit<float, I> {
         const size_t o_ndx = take(sizeof(float) * p.n);
         // Small sums get private copies, one per CTA of the assignment for
         // large n: their few addresses would otherwise serialise the
-        // reductions of all SMs.  Every iteration zeroes and reduces every
-        // copy, so small fits get one copy per eight tiles instead (a
-        // 50K-sample fit spent more time there than in its assignment).
+        // reductions of all SMs.  Every iteration reduces every copy, so
+        // small fits get one copy per eight tiles instead (a 50K-sample fit
+        // spent more time there than in its assignment).
         // Large sums (c3-sized, 266 KB) stay single: per-CTA copies would
         // crowd L2 for less contention than they remove.
         n_copies = (k_pad * d4 <= 32768)
@@ -2043,8 +2084,6 @@ struct MixedFit : PlainFit<float, I> {
         const size_t o_fx = take(fx_on ? 2 * sizeof(long long) * (size_t)n_copies *
                                                  (size_t)(p.k * d4 + p.k)
                                            : 16);
-        const size_t o_cn2 = take(sizeof(float) * p.k);
-        const size_t o_dcn = take(sizeof(float) * p.k);
         const size_t o_cst = take(sizeof(MixedConsts));
         // candidate masks (and best scores) of every column pass
         const size_t o_cand = take(sizeof(uint4) * (size_t)p.n * passes);
@@ -2067,8 +2106,6 @@ struct MixedFit : PlainFit<float, I> {
             fxhi = reinterpret_cast<long long *>(b + o_fx);
             fxlo = reinterpret_cast<unsigned long long *>(fxhi + n_copies * (p.k * d4 + p.k));
         }
-        cn2 = reinterpret_cast<float *>(b + o_cn2);
-        dcn = reinterpret_cast<float *>(b + o_dcn);
         consts = reinterpret_cast<MixedConsts *>(b + o_cst);
         cand = reinterpret_cast<uint4 *>(b + o_cand);
         pmax = reinterpret_cast<float *>(b + o_pmax);
@@ -2077,6 +2114,11 @@ struct MixedFit : PlainFit<float, I> {
         err_dev = n_flagged + 1;
         stats = reinterpret_cast<long long *>(b + o_st);
         KMC_CUDA_TRY(cudaMemsetAsync(consts, 0, sizeof(MixedConsts), s));
+        if (p.w != nullptr) {
+            // the sums start at zero; each iteration's end leaves them so
+            KMC_CUDA_TRY(cudaMemsetAsync(b + o_s32, 0, o_xf - o_s32, s));
+            KMC_CUDA_TRY(cudaMemsetAsync(b + o_fx, 0, o_cst - o_fx, s));
+        }
         KMC_CUDA_TRY(cudaMemsetAsync(n_flagged, 0, sizeof(int) * 4, s));
         KMC_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(long long) * 2, s));
         // one-time conversion of X (charged to the fit, reported separately)
@@ -2116,30 +2158,30 @@ struct MixedFit : PlainFit<float, I> {
         return KMC_OK;
     }
 
+    // the preparation is part of the assignment pass
+    int begin_step(int64_t *n_launches) override {
+        *n_launches = 0;
+        return KMC_OK;
+    }
+    long long wait_clocks() const override { return wait_limit; }
+    const float *c_rows(int64_t *stride) const override {
+        *stride = d4;
+        return ct;
+    }
+
     int centroid_prep(const float *cur, const LoopState *guard) {
         const FitParams<float, I> &p = this->prm;
-        cudaStream_t s = p.stream;
-        const int64_t lanes = k_pad * (nkb <= 1 ? 8 : (nkb == 2 ? 16 : 32));  // c_image's G
-        if (bf16)
-            c_image_kernel<1><<<grid1d(lanes, 128, 4096), 128, 0, s>>>(
-                cur, this->hn, p.d, p.k, k_pad, nkb, consts, cimg, cn2, dcn, ct, d4, guard);
-        else
-            c_image_kernel<0><<<grid1d(lanes, 128, 4096), 128, 0, s>>>(
-                cur, this->hn, p.d, p.k, k_pad, nkb, consts, cimg, cn2, dcn, ct, d4, guard);
-        KMC_TRY(check_launch("c_image"));
-        bound_kernel<<<1, 1024, 0, s>>>(cn2, dcn, this->hn, p.d, p.k, bf16, consts, guard);
-        return check_launch("bound");
+        const int lanes = nkb <= 1 ? 8 : (nkb == 2 ? 16 : 32);
+        auto kern = bf16 ? mixed_prep_kernel<1> : mixed_prep_kernel<0>;
+        kern<<<(unsigned)(k_pad / kPrepRows), lanes * kPrepRows, 0, p.stream>>>(
+            cur, p.d, p.k, k_pad, nkb, consts, cimg, this->hn, ct, d4, n_flagged, guard);
+        return check_launch("mixed_prep");
     }
 
     int assign_pass(const float *cur, int update, const LoopState *guard) {
         const FitParams<float, I> &p = this->prm;
         cudaStream_t s = p.stream;
         KMC_TRY(centroid_prep(cur, guard));
-        const int64_t csz = (int64_t)n_copies * (k_pad * d4 + k_pad);
-        reset_kernel<<<grid1d(csz, 256, 4096), 256, 0, s>>>(sums32, acc64, csz, acc_f64,
-                                                           n_flagged, fx_acc(), p.k * d4 + p.k,
-                                                           guard);
-        KMC_TRY(check_launch("mixed_reset"));
         MixedArgs a;
         a.ximg = ximg;
         a.cimg = cimg;
@@ -2217,31 +2259,29 @@ struct MixedFit : PlainFit<float, I> {
         recheck_kernel<<<(unsigned)rgrid, kRecheckThreads, 0, s>>>(
             xrow, ct, this->hn, p.w, cand, flagged, n_flagged, p.n, p.d, p.k, d4, p.labels,
             a.label64, update, acc_f64, sums32, acc64, k_pad, n_copies, guard, passes, pass_cols,
-            fx_acc(), consts);
-        KMC_TRY(check_launch("mixed_recheck"));
-        stats_kernel<<<1, 1, 0, s>>>(n_flagged, stats, stats + 1, guard);
-        return check_launch("mixed_stats");
+            fx_acc(), consts, stats);
+        return check_launch("mixed_recheck");
     }
 
     int step_assign_and_accumulate(const float *cur, int64_t *n_launches) override {
-        *n_launches = 6 + (passes > 1 ? passes : 0);
+        *n_launches = 3 + (passes > 1 ? passes : 0);
         return assign_pass(cur, 1, this->state);
     }
 
-    int reduce_step(float *nxt) override {
+    int finish_step(int64_t *n_launches) override {
         const FitParams<float, I> &p = this->prm;
-        cudaStream_t s = p.stream;
-        if (acc_f64)
-            km_to_dk_kernel<double><<<grid1d(p.k * d4 + p.k, 256, 4096), 256, 0, s>>>(
-                acc64, n_copies, nxt, this->sizes, p.d, p.k, k_pad, d4, fx_acc(), consts,
-                this->state);
-        else
-            km_to_dk_kernel<float><<<grid1d(p.k * d4 + p.k, 256, 4096), 256, 0, s>>>(
-                sums32, n_copies, nxt, this->sizes, p.d, p.k, k_pad, d4,
-                FxAcc{nullptr, nullptr, nullptr, 0, 1}, consts, this->state);
-        KMC_TRY(check_launch("km_to_dk"));
-        return launch_empty_list<float, I>(this->sizes, this->empty_list, this->n_empty, p.k, s,
-                                           this->state);
+        if (acc_f64) {
+            // the assignment of a one-pass fit without shared-memory sums
+            // reduces into the float64 copies itself
+            const MixedSums<double> src{acc64, n_copies, passes == 1 && own_k == 0 ? 1 : 0,
+                                        p.k, k_pad, d4, fx_acc(), consts};
+            return launch_reduce_and_finish<float>(src, n_copies, this->finish_args(), n_launches,
+                                                   p.stream);
+        }
+        const MixedSums<float> src{sums32, n_copies, 1, p.k, k_pad, d4,
+                                   FxAcc{nullptr, nullptr, nullptr, 0, 1, nullptr}, consts};
+        return launch_reduce_and_finish<float>(src, n_copies, this->finish_args(), n_launches,
+                                               p.stream);
     }
 
     int final_assignment() override { return assign_pass(this->prm.centroids, 0, nullptr); }

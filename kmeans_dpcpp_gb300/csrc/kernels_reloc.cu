@@ -19,10 +19,6 @@ namespace kmc {
 
 namespace {
 
-__device__ __forceinline__ bool stopped(const LoopState *g) {
-    return g != nullptr && *reinterpret_cast<const volatile int *>(&g->done) != 0;
-}
-
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
@@ -65,13 +61,10 @@ struct SelectState {
     long long pad;
 };
 
-__global__ void threshold_init_kernel(SelectState *st, const int64_t *topk_dev,
-                                      int64_t topk_host, int64_t n, const LoopState *guard) {
+__global__ void threshold_init_kernel(SelectState *st, int64_t topk, int64_t n) {
     int t = threadIdx.x;
     st->hist[t] = 0ull;
     if (t == 0) {
-        int64_t topk = (topk_dev != nullptr) ? *topk_dev : topk_host;
-        if (stopped(guard)) topk = 0;
         if (topk > n) topk = n;
         st->active = (topk > 0) ? 1 : 0;
         st->rank = (topk > 0) ? (unsigned long long)(topk - 1) : 0ull;
@@ -144,7 +137,6 @@ struct SelHeader {
     long long need_eq;
     long long sorted;  // 1: gt elements are ranked, 0: written in index order
     long long n_sel;
-    long long active;
     long long n_total;
 };
 
@@ -182,10 +174,8 @@ __device__ __forceinline__ void block_range(int64_t n, int64_t &b0, int64_t &b1)
 }
 
 template <typename T>
-__global__ void select_count_kernel(const T *dist, const T *thr, int64_t n, SelLayout L,
-                                    const int64_t *gate, const LoopState *guard) {
+__global__ void select_count_kernel(const T *dist, const T *thr, int64_t n, SelLayout L) {
     __shared__ long long sg[32], se[32];
-    if (stopped(guard) || (gate != nullptr && *gate == 0)) return;
     int64_t b0, b1;
     block_range(n, b0, b1);
     const T th = *thr;
@@ -216,26 +206,43 @@ __global__ void select_count_kernel(const T *dist, const T *thr, int64_t n, SelL
     }
 }
 
+// One CTA of kSelGrid threads: exclusive sums over the counting CTAs (512
+// dependent loads by one thread took 27 us or more).
 template <typename I>
-__global__ void select_scan_kernel(SelLayout L, const int64_t *n_sel_dev, int64_t n_sel_host,
-                                   I *n_gt, I *n_eq, int64_t n_total, const int64_t *gate,
-                                   const LoopState *guard) {
-    if (threadIdx.x != 0) return;
-    SelHeader *h = L.hdr;
-    if (stopped(guard) || (gate != nullptr && *gate == 0)) {
-        h->active = 0;
-        return;
+__global__ void __launch_bounds__(kSelGrid) select_scan_kernel(SelLayout L, int64_t n_selected,
+                                                               I *n_gt, I *n_eq,
+                                                               int64_t n_total) {
+    __shared__ long long wg[32], we[32];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const long long g = L.cnt_gt[t], e = L.cnt_eq[t];
+    long long ig = g, ie = e;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long a = __shfl_up_sync(0xffffffffu, ig, o);
+        const long long b = __shfl_up_sync(0xffffffffu, ie, o);
+        if (lane >= o) {
+            ig += a;
+            ie += b;
+        }
     }
+    if (lane == 31) {
+        wg[wid] = ig;
+        we[wid] = ie;
+    }
+    __syncthreads();
     long long sg = 0, se = 0;
-    for (int b = 0; b < kSelGrid; ++b) {
-        long long g = L.cnt_gt[b], e = L.cnt_eq[b];
-        L.cnt_gt[b] = sg;
-        L.cnt_eq[b] = se;
-        sg += g;
-        se += e;
+    for (int q = 0; q < kSelGrid / 32; ++q) {
+        if (q < wid) {
+            ig += wg[q];
+            ie += we[q];
+        }
+        sg += wg[q];
+        se += we[q];
     }
-    long long n_sel = (n_sel_dev != nullptr) ? (long long)*n_sel_dev : (long long)n_sel_host;
-    h->active = 1;
+    L.cnt_gt[t] = ig - g;
+    L.cnt_eq[t] = ie - e;
+    if (t != 0) return;
+    SelHeader *h = L.hdr;
+    const long long n_sel = (long long)n_selected;
     h->n_sel = n_sel;
     h->n_total = n_total;
     h->total_gt = sg;
@@ -256,7 +263,6 @@ __global__ void select_write_kernel(const T *dist, const T *thr, int64_t n, SelL
     __shared__ int wg[32], we[32];
     __shared__ long long base_g, base_e;
     const SelHeader *h = L.hdr;
-    if (h->active == 0) return;
     int64_t b0, b1;
     block_range(n, b0, b1);
     const T th = *thr;
@@ -318,7 +324,7 @@ __global__ void select_write_kernel(const T *dist, const T *thr, int64_t n, SelL
 template <typename T, typename I>
 __global__ void select_rank_kernel(const T *dist, SelLayout L, I *selected) {
     const SelHeader *h = L.hdr;
-    if (h->active == 0 || h->sorted == 0) return;
+    if (h->sorted == 0) return;
     const long long m = h->total_gt;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m;
          e += (long long)gridDim.x * blockDim.x) {
@@ -366,7 +372,7 @@ __device__ __forceinline__ long long count_before(const T *dist, const long long
 template <typename T>
 __global__ void select_merge_kernel(const T *dist, SelLayout L, int pass) {
     const SelHeader *h = L.hdr;
-    if (h->active == 0 || h->sorted == 0) return;
+    if (h->sorted == 0) return;
     const long long m = h->total_gt, len = 1ll << pass;
     if (len >= m) return;
     const long long *src = (pass & 1) ? L.gt_tmp : L.gt_list;
@@ -392,7 +398,7 @@ __global__ void select_merge_kernel(const T *dist, SelLayout L, int pass) {
 template <typename T, typename I>
 __global__ void select_place_kernel(SelLayout L, I *selected) {
     const SelHeader *h = L.hdr;
-    if (h->active == 0 || h->sorted == 0) return;
+    if (h->sorted == 0) return;
     const long long m = h->total_gt;
     int passes = 0;
     while ((1ll << passes) < m) ++passes;
@@ -406,14 +412,9 @@ __global__ void select_place_kernel(SelLayout L, I *selected) {
 
 // relocate_empty_clusters_kernel, src/util_kernels.hpp:302-390.
 template <typename T, typename I>
-__global__ void relocate_kernel(const int64_t *n_empty_dev, int64_t n_empty_host, const T *X,
-                                const T *w, const I *labels, const I *selected, const I *n_gt,
-                                const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
-                                int64_t d, int64_t k, const LoopState *guard, int64_t fs,
-                                int64_t ss) {
-    if (stopped(guard)) return;
-    int64_t n_empty = (n_empty_dev != nullptr) ? *n_empty_dev : n_empty_host;
-    if (n_empty <= 0) return;
+__global__ void relocate_kernel(int64_t n_empty, const T *X, const T *w, const I *labels,
+                                const I *selected, const I *n_gt, const I *empty_list, T *sums,
+                                T *sizes, T *inertia, int64_t n, int64_t d, int64_t k) {
     const int64_t gt = (int64_t)*n_gt;
     // Samples available: the gt ones plus the eq ones written at the back.
     if (n_empty > n) n_empty = n;
@@ -429,7 +430,7 @@ __global__ void relocate_kernel(const int64_t *n_empty_dev, int64_t n_empty_host
         // caller-supplied indices: never dereference out of range
         if (old < 0 || old >= k || cl < 0 || cl >= k) continue;
         T wv = w[s];
-        T xw = mul_rn(X[f * fs + s * ss], wv);  // rounded product, as in the reference
+        T xw = mul_rn(X[f * n + s], wv);  // rounded product, as in the reference
         sums[f * k + old] -= xw;
         sums[f * k + cl] = xw;
         if (f == 0) {
@@ -440,20 +441,15 @@ __global__ void relocate_kernel(const int64_t *n_empty_dev, int64_t n_empty_host
     }
 }
 
-template <typename I>
-__global__ void gate_kernel(const I *n_empty, int64_t *gate, const LoopState *guard) {
-    if (threadIdx.x == 0) *gate = stopped(guard) ? 0 : (int64_t)*n_empty;
-}
-
 }  // namespace
 
 size_t threshold_scratch_bytes() { return align256(sizeof(SelectState)); }
 
 template <typename T>
-int launch_threshold(const T *data, int64_t n, const int64_t *topk_dev, int64_t topk_host,
-                     T *threshold, void *scratch, cudaStream_t s, const LoopState *guard) {
+int launch_threshold(const T *data, int64_t n, int64_t topk, T *threshold, void *scratch,
+                     cudaStream_t s) {
     SelectState *st = static_cast<SelectState *>(scratch);
-    threshold_init_kernel<<<1, 256, 0, s>>>(st, topk_dev, topk_host, n, guard);
+    threshold_init_kernel<<<1, 256, 0, s>>>(st, topk, n);
     KMC_TRY(check_launch("threshold_init"));
     int64_t g = ceil_div<int64_t>(n, 1024);
     int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, (int64_t)num_sms() * 4));
@@ -472,23 +468,13 @@ size_t select_scratch_bytes(int64_t max_selected) {
     return align256(256 + 2 * sizeof(long long) * kSelGrid + sizeof(long long) * m * lists);
 }
 
-int64_t select_launches(int64_t max_selected) {
-    if (max_selected <= kRankAllPairs) return 4;
-    int64_t passes = 0;
-    while ((int64_t(1) << passes) < max_selected) ++passes;
-    return 3 + passes + 1;
-}
-
 template <typename T, typename I>
-int launch_select(const int64_t *n_selected_dev, int64_t n_selected_host, const T *dist,
-                  const T *threshold, I *selected, I *n_gt, I *n_eq, int64_t n, void *scratch,
-                  int64_t max_selected, cudaStream_t s, const LoopState *guard) {
+int launch_select(int64_t max_selected, const T *dist, const T *threshold, I *selected, I *n_gt,
+                  I *n_eq, int64_t n, void *scratch, cudaStream_t s) {
     SelLayout L = sel_layout(scratch, max_selected);
-    const int64_t *gate = n_selected_dev;
-    select_count_kernel<T><<<kSelGrid, kSelBlock, 0, s>>>(dist, threshold, n, L, gate, guard);
+    select_count_kernel<T><<<kSelGrid, kSelBlock, 0, s>>>(dist, threshold, n, L);
     KMC_TRY(check_launch("select_count"));
-    select_scan_kernel<I><<<1, 32, 0, s>>>(L, n_selected_dev, n_selected_host, n_gt, n_eq, n,
-                                           gate, guard);
+    select_scan_kernel<I><<<1, kSelGrid, 0, s>>>(L, max_selected, n_gt, n_eq, n);
     KMC_TRY(check_launch("select_scan"));
     select_write_kernel<T, I><<<kSelGrid, kSelBlock, 0, s>>>(dist, threshold, n, L, selected);
     KMC_TRY(check_launch("select_write"));
@@ -509,45 +495,28 @@ int launch_select(const int64_t *n_selected_dev, int64_t n_selected_host, const 
 }
 
 template <typename T, typename I>
-int launch_relocate(const int64_t *n_empty_dev, int64_t n_empty_host, const T *X, const T *w,
-                    const I *labels, const I *selected, const I *n_gt, const I *empty_list,
-                    T *sums, T *sizes, T *inertia, int64_t n, int64_t d, int64_t k,
-                    cudaStream_t s, const LoopState *guard, int64_t x_fstride,
-                    int64_t x_sstride) {
+int launch_relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *selected,
+                    const I *n_gt, const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
+                    int64_t d, int64_t k, cudaStream_t s) {
     int grid = (int)ceil_div<int64_t>(std::max<int64_t>(d, 1), 128);
-    const int64_t fs = x_fstride > 0 ? x_fstride : n, ss = x_fstride > 0 ? x_sstride : 1;
-    relocate_kernel<T, I><<<grid, 128, 0, s>>>(n_empty_dev, n_empty_host, X, w, labels, selected,
-                                               n_gt, empty_list, sums, sizes, inertia, n, d, k,
-                                               guard, fs, ss);
+    relocate_kernel<T, I><<<grid, 128, 0, s>>>(n_empty, X, w, labels, selected, n_gt, empty_list,
+                                               sums, sizes, inertia, n, d, k);
     return check_launch("relocate");
 }
 
-template <typename I>
-int launch_gate_from_count(const I *n_empty, int64_t *gate, cudaStream_t s,
-                           const LoopState *guard) {
-    gate_kernel<I><<<1, 32, 0, s>>>(n_empty, gate, guard);
-    return check_launch("relocation_gate");
-}
-
-template int launch_threshold<float>(const float *, int64_t, const int64_t *, int64_t, float *,
-                                     void *, cudaStream_t, const LoopState *);
-template int launch_threshold<double>(const double *, int64_t, const int64_t *, int64_t,
-                                      double *, void *, cudaStream_t, const LoopState *);
+template int launch_threshold<float>(const float *, int64_t, int64_t, float *, void *,
+                                     cudaStream_t);
+template int launch_threshold<double>(const double *, int64_t, int64_t, double *, void *,
+                                      cudaStream_t);
 #define KMC_INST_RELOC(T, I)                                                                  \
-    template int launch_select<T, I>(const int64_t *, int64_t, const T *, const T *, I *, I *, \
-                                     I *, int64_t, void *, int64_t, cudaStream_t,             \
-                                     const LoopState *);                                      \
-    template int launch_relocate<T, I>(const int64_t *, int64_t, const T *, const T *,        \
-                                       const I *, const I *, const I *, const I *, T *, T *,  \
-                                       T *, int64_t, int64_t, int64_t, cudaStream_t,          \
-                                       const LoopState *, int64_t, int64_t);
+    template int launch_select<T, I>(int64_t, const T *, const T *, I *, I *, I *, int64_t,   \
+                                     void *, cudaStream_t);                                   \
+    template int launch_relocate<T, I>(int64_t, const T *, const T *, const I *, const I *,   \
+                                       const I *, const I *, T *, T *, T *, int64_t, int64_t, \
+                                       int64_t, cudaStream_t);
 KMC_INST_RELOC(float, int32_t)
 KMC_INST_RELOC(float, int64_t)
 KMC_INST_RELOC(double, int32_t)
 KMC_INST_RELOC(double, int64_t)
-template int launch_gate_from_count<int32_t>(const int32_t *, int64_t *, cudaStream_t,
-                                             const LoopState *);
-template int launch_gate_from_count<int64_t>(const int64_t *, int64_t *, cudaStream_t,
-                                             const LoopState *);
 
 }  // namespace kmc

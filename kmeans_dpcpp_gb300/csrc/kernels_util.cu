@@ -5,6 +5,7 @@
 // Arithmetic order follows the SYCL kernels cited on each function: sums over
 // features run sequentially f = 0..d-1 with a fused multiply-add, exactly as
 // `acc += a * b` is contracted by the reference's device compiler.
+#include "km_dist.cuh"
 #include "km_kernels.cuh"
 
 namespace kmc {
@@ -39,8 +40,17 @@ __global__ void half_norm_kernel(const T *C, T *out, int64_t d, int64_t k,
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= k) return;
     T acc = T(0);
-    for (int64_t f = 0; f < d; ++f) {
-        T v = C[f * k + j];
+    // eight features' loads in flight before the sequential chain
+    int64_t f = 0;
+    for (; f + 8 <= d; f += 8) {
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = C[(f + u) * k + j];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc = fma_t(v[u], v[u], acc);
+    }
+    for (; f < d; ++f) {
+        const T v = C[f * k + j];
         acc = fma_t(v, v, acc);
     }
     out[j] = acc / T(2);
@@ -48,23 +58,19 @@ __global__ void half_norm_kernel(const T *C, T *out, int64_t d, int64_t k,
 
 // reduce_centroid_data_kernel, src/util_kernels.hpp:87-161, part 1: sums of
 // the private copies in copy order 0..P-1 (sums and sizes).
-// A is the accumulator type of the copies (dataT for the public API, float64
-// inside the driver); the result is rounded once to dataT.
-template <typename T, typename A>
-__global__ void reduce_copies_kernel(const A *sizes_cp, const A *cent_cp, T *out_sizes,
-                                     T *out_cent, int64_t P, int64_t d, int64_t k,
-                                     const LoopState *guard) {
-    if (stopped(guard)) return;
+template <typename T>
+__global__ void reduce_copies_kernel(const T *sizes_cp, const T *cent_cp, T *out_sizes,
+                                     T *out_cent, int64_t P, int64_t d, int64_t k) {
     int64_t dk = d * k;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < dk + k;
          e += (int64_t)gridDim.x * blockDim.x) {
         // copies added in index order; loads issued eight ahead of the adds
-        const A *src = (e < dk) ? cent_cp + e : sizes_cp + (e - dk);
+        const T *src = (e < dk) ? cent_cp + e : sizes_cp + (e - dk);
         const int64_t stride = (e < dk) ? dk : k;
-        A s = A(0);
+        T s = T(0);
         int64_t p = 0;
         for (; p + 8 <= P; p += 8) {
-            A v[8];
+            T v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) v[u] = src[(p + u) * stride];
 #pragma unroll
@@ -72,9 +78,9 @@ __global__ void reduce_copies_kernel(const A *sizes_cp, const A *cent_cp, T *out
         }
         for (; p < P; ++p) s += src[p * stride];
         if (e < dk)
-            out_cent[e] = (T)s;
+            out_cent[e] = s;
         else
-            out_sizes[e - dk] = (T)s;
+            out_sizes[e - dk] = s;
     }
 }
 
@@ -83,9 +89,7 @@ __global__ void reduce_copies_kernel(const A *sizes_cp, const A *cent_cp, T *out
 // here the list is built in ascending cluster order by one block, starting
 // at the counter's current value.
 template <typename T, typename I>
-__global__ void empty_list_kernel(const T *sizes, I *list, I *n_empty, int64_t k,
-                                  const LoopState *guard) {
-    if (stopped(guard)) return;
+__global__ void empty_list_kernel(const T *sizes, I *list, I *n_empty, int64_t k) {
     __shared__ int warp_counts[32];
     __shared__ long long base_sh;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -127,42 +131,6 @@ __global__ void shifts_kernel(const T *old_c, const T *new_c, T *out, int64_t d,
     out[j] = acc;
 }
 
-// Driver fusion of broadcast_division_kernel (util_kernels.hpp:9-41) and the
-// shift kernel above: same per-element operations, one pass over (d, k).
-template <typename T>
-__global__ void divide_and_shift_kernel(const T *__restrict__ old_c, T *__restrict__ new_c,
-                                        const T *__restrict__ sizes, T *__restrict__ shifts,
-                                        int64_t d, int64_t k, const LoopState *guard) {
-    if (stopped(guard)) return;
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    T sz = sizes[j];
-    T acc = T(0);
-    // features in groups of 8: the group's loads are all in flight before
-    // its divisions and the (sequential, as the reference's) fma chain
-    constexpr int kG = 8;
-    for (int64_t f0 = 0; f0 < d; f0 += kG) {
-        T nv[kG], ov[kG];
-#pragma unroll
-        for (int e = 0; e < kG; ++e) {
-            const int64_t f = f0 + e;
-            nv[e] = (f < d) ? new_c[f * k + j] : T(0);
-            ov[e] = (f < d) ? old_c[f * k + j] : T(0);
-        }
-#pragma unroll
-        for (int e = 0; e < kG; ++e) {
-            const int64_t f = f0 + e;
-            if (f < d) {
-                T c = nv[e] / sz;
-                new_c[f * k + j] = c;
-                T diff = ov[e] - c;
-                acc = fma_t(diff, diff, acc);
-            }
-        }
-    }
-    shifts[j] = acc;
-}
-
 // Fixed-order block reduction of doubles (deterministic for a given grid).
 __device__ double block_sum(double v, double *sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -178,33 +146,11 @@ __device__ double block_sum(double v, double *sh) {
     return r;  // valid in thread 0
 }
 
-// Loop control of driver_lloyd (src/kmeans_lloyd_driver.hpp:83, 343-353):
-// the total shift (float64 here) is compared with tol in dataT, n_iter += 1.
-template <typename T>
-__global__ void loop_control_kernel(const T *shifts, int64_t k, LoopState *st) {
-    __shared__ double sh[32];
-    if (*reinterpret_cast<volatile int *>(&st->done)) return;
-    double acc = 0.0;
-    for (int64_t j = threadIdx.x; j < k; j += blockDim.x) acc += (double)shifts[j];
-    double tot = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-        st->last_shift = tot;
-        st->n_iter += 1;
-        T shift_t = (T)tot;
-        T tol_t = (T)st->tol;
-        bool go_on = (st->n_iter < st->max_iter) && (shift_t > tol_t);
-        if (!go_on) st->done = 1;
-    }
-}
-
 // compute_inertia_kernel / compute_uniform_weight_inertia_kernel,
 // src/compute_inertia.hpp:11-99.  w == nullptr gives the unit-weight form.
 template <typename T, typename I>
 __global__ void inertia_kernel(const T *X, const T *w, const T *C, const I *labels, T *out,
-                               int64_t n, int64_t d, int64_t k, const LoopState *guard,
-                               const int64_t *gate, int64_t fs, int64_t ss) {
-    if (stopped(guard)) return;
-    if (gate != nullptr && *gate == 0) return;
+                               int64_t n, int64_t d, int64_t k, int64_t fs, int64_t ss) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         int64_t c = (int64_t)labels[i];
@@ -212,12 +158,35 @@ __global__ void inertia_kernel(const T *X, const T *w, const T *C, const I *labe
             out[i] = pos_inf<T>();
             continue;
         }
-        T acc = T(0);
-        for (int64_t f = 0; f < d; ++f) {
-            T diff = X[f * fs + i * ss] - C[f * k + c];
-            acc = fma_t(diff, diff, acc);
-        }
+        const T acc = sq_dist_cols<T>(X, fs, ss, C, d, k, i, c);
         out[i] = (w != nullptr) ? mul_rn(acc, w[i]) : acc;
+    }
+}
+
+// The same for row-major samples and centroids (zero-padded to a multiple of
+// four features).  Bound by reading X once: 10M x 64 took 2.97 ms with a thread
+// per row reading X and the (d, k) centroids 4 bytes at a time.
+constexpr int kInertiaThreads = 256;
+template <typename I>
+__global__ void __launch_bounds__(kInertiaThreads)
+    inertia_rows_kernel(const float *X, int64_t ss, const float *w, const float *C, int64_t cs,
+                        const I *labels, float *out, int64_t n, int64_t d, int64_t k) {
+    extern __shared__ float tiles[];
+    const int lane = threadIdx.x & 31;
+    float *tile = tiles + (threadIdx.x >> 5) * kDistTile;
+    for (int64_t i0 = blockIdx.x * (int64_t)kInertiaThreads; i0 < n;
+         i0 += (int64_t)gridDim.x * kInertiaThreads) {
+        const int64_t i = i0 + threadIdx.x;
+        const int64_t c = i < n ? (int64_t)labels[i] : -1;
+        const bool ok = c >= 0 && c < k;
+        float v = pos_inf<float>();
+        if (d > kRowVec) {
+            const float r = sq_dist_warp(X, ss, C, cs, d, i - lane, ok ? c : -1, tile);
+            if (ok) v = r;
+        } else if (ok) {
+            v = sq_dist_row(X + i * ss, C + c * cs, d);
+        }
+        if (i < n) out[i] = ok && w != nullptr ? mul_rn(v, w[i]) : v;
     }
 }
 
@@ -225,10 +194,8 @@ constexpr int kSumGrid = 1024;
 constexpr int kSumBlock = 256;
 
 template <typename T>
-__global__ void sum_stage1_kernel(const T *data, int64_t n, double *partials,
-                                  const LoopState *guard) {
+__global__ void sum_stage1_kernel(const T *data, int64_t n, double *partials) {
     __shared__ double sh[32];
-    if (stopped(guard)) return;
     double acc = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -237,10 +204,8 @@ __global__ void sum_stage1_kernel(const T *data, int64_t n, double *partials,
     if (threadIdx.x == 0) partials[blockIdx.x] = r;
 }
 
-__global__ void sum_stage2_kernel(const double *partials, int count, double *out,
-                                  const LoopState *guard) {
+__global__ void sum_stage2_kernel(const double *partials, int count, double *out) {
     __shared__ double sh[32];
-    if (stopped(guard)) return;
     double acc = 0.0;
     for (int i = threadIdx.x; i < count; i += blockDim.x) acc += partials[i];
     double r = block_sum(acc, sh);
@@ -248,8 +213,7 @@ __global__ void sum_stage2_kernel(const double *partials, int count, double *out
 }
 
 template <typename T>
-__global__ void fill_kernel(T *p, T v, int64_t count, const LoopState *guard) {
-    if (stopped(guard)) return;
+__global__ void fill_kernel(T *p, T v, int64_t count) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count;
          e += (int64_t)gridDim.x * blockDim.x)
         p[e] = v;
@@ -279,23 +243,15 @@ int launch_half_norm(const T *C, T *out, int64_t d, int64_t k, cudaStream_t s,
     return check_launch("half_l2_norm");
 }
 
-template <typename T, typename I, typename A>
-int launch_reduce_centroids(const A *sizes_cp, const A *cent_cp, T *out_sizes, T *out_cent,
-                            I *empty_list, I *n_empty, int64_t P, int64_t d, int64_t k,
-                            cudaStream_t s, const LoopState *guard) {
-    if (k == 0) return KMC_OK;
-    reduce_copies_kernel<T, A><<<grid_for(d * k + k, 256, 8192), 256, 0, s>>>(
-        sizes_cp, cent_cp, out_sizes, out_cent, P, d, k, guard);
-    KMC_TRY(check_launch("reduce_centroids_data"));
-    empty_list_kernel<T, I><<<1, 1024, 0, s>>>(out_sizes, empty_list, n_empty, k, guard);
-    return check_launch("empty_clusters_list");
-}
-
 template <typename T, typename I>
-int launch_empty_list(const T *sizes, I *list, I *n_empty, int64_t k, cudaStream_t s,
-                      const LoopState *guard) {
+int launch_reduce_centroids(const T *sizes_cp, const T *cent_cp, T *out_sizes, T *out_cent,
+                            I *empty_list, I *n_empty, int64_t P, int64_t d, int64_t k,
+                            cudaStream_t s) {
     if (k == 0) return KMC_OK;
-    empty_list_kernel<T, I><<<1, 1024, 0, s>>>(sizes, list, n_empty, k, guard);
+    reduce_copies_kernel<T><<<grid_for(d * k + k, 256, 8192), 256, 0, s>>>(
+        sizes_cp, cent_cp, out_sizes, out_cent, P, d, k);
+    KMC_TRY(check_launch("reduce_centroids_data"));
+    empty_list_kernel<T, I><<<1, 1024, 0, s>>>(out_sizes, empty_list, n_empty, k);
     return check_launch("empty_clusters_list");
 }
 
@@ -307,47 +263,40 @@ int launch_shifts(const T *old_c, const T *new_c, T *out, int64_t d, int64_t k,
     return check_launch("centroid_shifts");
 }
 
-template <typename T>
-int launch_divide_and_shift(const T *old_c, T *new_c, const T *sizes, T *shifts, int64_t d,
-                            int64_t k, cudaStream_t s, const LoopState *guard) {
-    if (k == 0) return KMC_OK;
-    divide_and_shift_kernel<T><<<grid_for(k, 128, 1 << 20), 128, 0, s>>>(old_c, new_c, sizes,
-                                                                         shifts, d, k, guard);
-    return check_launch("divide_and_shift");
-}
-
-template <typename T>
-int launch_loop_control(const T *shifts, int64_t k, LoopState *state, cudaStream_t s) {
-    loop_control_kernel<T><<<1, 1024, 0, s>>>(shifts, k, state);
-    return check_launch("loop_control");
-}
-
 template <typename T, typename I>
 int launch_inertia(const T *X, const T *w, const T *C, const I *labels, T *out, int64_t n,
-                   int64_t d, int64_t k, cudaStream_t s, const LoopState *guard,
-                   const int64_t *gate, int64_t x_fstride, int64_t x_sstride) {
+                   int64_t d, int64_t k, cudaStream_t s, int64_t x_fstride, int64_t x_sstride,
+                   const T *c_rows, int64_t c_stride) {
     if (n == 0) return KMC_OK;
     const int64_t fs = x_fstride > 0 ? x_fstride : n, ss = x_fstride > 0 ? x_sstride : 1;
-    inertia_kernel<T, I><<<grid_for(n, 256, 16384), 256, 0, s>>>(X, w, C, labels, out, n, d, k,
-                                                                 guard, gate, fs, ss);
+    if constexpr (sizeof(T) == 4) {
+        if (c_rows != nullptr && fs == 1) {
+            const size_t smem =
+                d > kRowVec ? sizeof(float) * kDistTile * (kInertiaThreads / 32) : 0;
+            inertia_rows_kernel<I><<<grid_for(n, kInertiaThreads, num_sms() * 16), kInertiaThreads,
+                                     smem, s>>>(X, ss, w, c_rows, c_stride, labels, out, n, d, k);
+            return check_launch("compute_inertia_rows");
+        }
+    }
+    inertia_kernel<T, I><<<grid_for(n, 256, 16384), 256, 0, s>>>(X, w, C, labels, out, n, d, k, fs,
+                                                                 ss);
     return check_launch("compute_inertia");
 }
 
 int64_t sum_partials_size() { return kSumGrid; }
 
 template <typename T>
-int launch_sum_f64(const T *data, int64_t n, double *partials, double *out, cudaStream_t s,
-                   const LoopState *guard) {
-    sum_stage1_kernel<T><<<kSumGrid, kSumBlock, 0, s>>>(data, n, partials, guard);
+int launch_sum_f64(const T *data, int64_t n, double *partials, double *out, cudaStream_t s) {
+    sum_stage1_kernel<T><<<kSumGrid, kSumBlock, 0, s>>>(data, n, partials);
     KMC_TRY(check_launch("sum_stage1"));
-    sum_stage2_kernel<<<1, 1024, 0, s>>>(partials, kSumGrid, out, guard);
+    sum_stage2_kernel<<<1, 1024, 0, s>>>(partials, kSumGrid, out);
     return check_launch("sum_stage2");
 }
 
 template <typename T>
-int launch_fill(T *p, T v, int64_t count, cudaStream_t s, const LoopState *guard) {
+int launch_fill(T *p, T v, int64_t count, cudaStream_t s) {
     if (count == 0) return KMC_OK;
-    fill_kernel<T><<<grid_for(count, 256, 8192), 256, 0, s>>>(p, v, count, guard);
+    fill_kernel<T><<<grid_for(count, 256, 8192), 256, 0, s>>>(p, v, count);
     return check_launch("fill");
 }
 
@@ -356,33 +305,20 @@ int launch_fill(T *p, T v, int64_t count, cudaStream_t s, const LoopState *guard
     template int launch_half_norm<T>(const T *, T *, int64_t, int64_t, cudaStream_t,          \
                                      const LoopState *);                                      \
     template int launch_shifts<T>(const T *, const T *, T *, int64_t, int64_t, cudaStream_t); \
-    template int launch_divide_and_shift<T>(const T *, T *, const T *, T *, int64_t, int64_t, \
-                                            cudaStream_t, const LoopState *);                 \
-    template int launch_loop_control<T>(const T *, int64_t, LoopState *, cudaStream_t);       \
-    template int launch_sum_f64<T>(const T *, int64_t, double *, double *, cudaStream_t,      \
-                                   const LoopState *);                                        \
-    template int launch_fill<T>(T *, T, int64_t, cudaStream_t, const LoopState *);
+    template int launch_sum_f64<T>(const T *, int64_t, double *, double *, cudaStream_t);     \
+    template int launch_fill<T>(T *, T, int64_t, cudaStream_t);
 
 #define KMC_INST_TI(T, I)                                                                     \
-    template int launch_reduce_centroids<T, I, T>(const T *, const T *, T *, T *, I *, I *,   \
-                                                  int64_t, int64_t, int64_t, cudaStream_t,    \
-                                                  const LoopState *);                         \
-    template int launch_empty_list<T, I>(const T *, I *, I *, int64_t, cudaStream_t,          \
-                                         const LoopState *);                                  \
+    template int launch_reduce_centroids<T, I>(const T *, const T *, T *, T *, I *, I *,      \
+                                               int64_t, int64_t, int64_t, cudaStream_t);      \
     template int launch_inertia<T, I>(const T *, const T *, const T *, const I *, T *,        \
-                                      int64_t, int64_t, int64_t, cudaStream_t,                \
-                                      const LoopState *, const int64_t *, int64_t, int64_t);
+                                      int64_t, int64_t, int64_t, cudaStream_t, int64_t,       \
+                                      int64_t, const T *, int64_t);
 
 KMC_INST_T(float)
 KMC_INST_T(double)
-template int launch_fill<int32_t>(int32_t *, int32_t, int64_t, cudaStream_t, const LoopState *);
-template int launch_fill<int64_t>(int64_t *, int64_t, int64_t, cudaStream_t, const LoopState *);
-template int launch_reduce_centroids<float, int32_t, double>(
-    const double *, const double *, float *, float *, int32_t *, int32_t *, int64_t, int64_t,
-    int64_t, cudaStream_t, const LoopState *);
-template int launch_reduce_centroids<float, int64_t, double>(
-    const double *, const double *, float *, float *, int64_t *, int64_t *, int64_t, int64_t,
-    int64_t, cudaStream_t, const LoopState *);
+template int launch_fill<int32_t>(int32_t *, int32_t, int64_t, cudaStream_t);
+template int launch_fill<int64_t>(int64_t *, int64_t, int64_t, cudaStream_t);
 KMC_INST_TI(float, int32_t)
 KMC_INST_TI(float, int64_t)
 KMC_INST_TI(double, int32_t)

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "km_kernels.cuh"
+#include "km_step.cuh"
 
 namespace kmc {
 
@@ -53,8 +54,11 @@ struct FitBase {
     // Enqueue iterations until the loop stops (batches of at most max_batch
     // iterations between host checks; <= 0 means unbounded growth).
     virtual int run(int64_t max_batch) = 0;
-    // Enqueue exactly one iteration (no host synchronisation).
-    virtual int enqueue_iteration() = 0;
+    // Enqueue exactly one iteration (no host synchronisation).  An iteration
+    // that leaves clusters empty pauses the loop (km_step.cuh) until
+    // enqueue_relocation; with `relocate` that is enqueued too.
+    virtual int enqueue_iteration(bool relocate) = 0;
+    virtual int enqueue_relocation() = 0;
     virtual int read_state(LoopState &out) = 0;
     // Device copy of the loop state (read by every kernel of an iteration).
     virtual const LoopState *device_state() const = 0;
@@ -93,13 +97,11 @@ struct PlainFit : FitBase {
     int64_t P = 1;  // private copies used internally
     Scratch ws;
     LoopState *state = nullptr;
-    T *hn = nullptr, *sizes = nullptr, *shifts = nullptr, *sq_dist = nullptr;
-    double *sums_cp = nullptr, *sizes_cp = nullptr;  // float64 accumulators
-    T *threshold = nullptr;
-    I *empty_list = nullptr, *n_empty = nullptr, *selected = nullptr, *counters = nullptr;
-    int64_t *gate = nullptr;
+    StepCtl *ctl = nullptr;
+    T *hn = nullptr, *prev = nullptr, *sums = nullptr, *sizes = nullptr, *shifts = nullptr, *sq_dist = nullptr;
+    double *sums_cp = nullptr, *sizes_cp = nullptr;  // float64 accumulators, zero between steps
+    int64_t *empty_list = nullptr, *reloc = nullptr;  // (k); relocation lists (3 k)
     double *partials = nullptr, *dsum = nullptr;
-    void *thr_scratch = nullptr, *sel_scratch = nullptr;
     int64_t issued = 0;
     int host_done = 0;
     int tile_variant = 0;  // autotuned centroid-tile width of the plain kernels
@@ -112,7 +114,8 @@ struct PlainFit : FitBase {
     }
 
     int init(const FitParams<T, I> &p);
-    int enqueue_iteration() override;
+    int enqueue_iteration(bool relocate) override;
+    int enqueue_relocation() override;
     int read_state(LoopState &out) override;
     int run(int64_t max_batch) override;
     int finalize(int64_t *n_iter_out, double *inertia_out) override;
@@ -123,9 +126,21 @@ struct PlainFit : FitBase {
     virtual int step_assign_and_accumulate(const T *cur, int64_t *n_launches);
     // Labels against the final centroids (kmeans_lloyd_driver.hpp:372-386).
     virtual int final_assignment();
-    // Private copies -> new centroid sums, sizes and the empty-cluster list
-    // (kmeans_lloyd_driver.hpp:155-170).
-    virtual int reduce_step(T *nxt);
+    // Cluster sums -> next centroids, shifts, stop rule (km_step.cuh).
+    virtual int finish_step(int64_t *n_launches);
+    FinishArgs<T> finish_args() const {
+        const FitParams<T, I> &p = prm;
+        return FinishArgs<T>{p.centroids, p.new_centroids, prev, sums, sizes, shifts, empty_list,
+                             p.d, p.k, 1, state, ctl};
+    }
+    // Limit (SM clocks) of the waits of a relocation's grid barriers.
+    virtual long long wait_clocks() const { return 4000000000LL; }
+    // Half norms of the current centroids, where the form's own preparation
+    // does not make them.
+    virtual int begin_step(int64_t *n_launches) {
+        *n_launches = 1;
+        return launch_half_norm<T>(prm.centroids, hn, prm.d, prm.k, prm.stream, state);
+    }
     // Whether the step accumulates into the driver's float64 private copies
     // (the mixed forms keep their own sums).
     virtual bool uses_private_copies() const { return true; }
@@ -138,6 +153,12 @@ struct PlainFit : FitBase {
         *x = prm.X;
         *fs = prm.n;
         *ss = 1;
+    }
+    // Row-major copy of the last assignment's centroids beside a row-major view,
+    // or null.
+    virtual const T *c_rows(int64_t *stride) const {
+        *stride = 0;
+        return nullptr;
     }
 };
 

@@ -1,4 +1,4 @@
-// Host-side launchers for every kernel of the engine.  Each launcher returns a
+// Host-side launchers of the engine's kernels.  Each launcher returns a
 // KMC_* status.  `guard`, when non-null, points to the device-resident loop
 // state of the Lloyd driver: guarded kernels return immediately once the loop
 // has stopped, so the driver can enqueue iterations ahead of the convergence
@@ -12,7 +12,7 @@ namespace kmc {
 // Device-resident control block of one Lloyd fit (see driver.cu).
 struct LoopState {
     int done;              // 1 once the loop stopped (max_iter or shift <= tol)
-    int relocations;       // number of iterations that relocated clusters
+    int pad0;
     long long n_iter;      // iterations executed
     long long max_iter;
     double tol;            // tol rounded to dataT, widened back to double
@@ -25,8 +25,8 @@ struct LoopState {
 // A kernel of the fit gave up a device-side wait (it then stopped the loop).
 inline int check_device_error(const LoopState &s) {
     if (s.err != 0) {
-        set_error("a tensor-core kernel of this fit gave up a device-side wait after its time "
-                  "limit; the loop was stopped and its results are not valid");
+        set_error("a kernel of this fit gave up a device-side wait after its time limit; the loop "
+                  "was stopped and its results are not valid");
         return KMC_ERR_DEVICE_TIMEOUT;
     }
     return KMC_OK;
@@ -86,40 +86,31 @@ int launch_broadcast_divide(T *X, const T *y, int64_t rows, int64_t cols, cudaSt
 template <typename T>
 int launch_half_norm(const T *C, T *out, int64_t d, int64_t k, cudaStream_t s,
                      const LoopState *guard = nullptr);
-// A: accumulator type of the private copies (dataT or double).
-template <typename T, typename I, typename A>
-int launch_reduce_centroids(const A *sizes_cp, const A *cent_cp, T *out_sizes, T *out_cent,
-                            I *empty_list, I *n_empty, int64_t P, int64_t d, int64_t k,
-                            cudaStream_t s, const LoopState *guard = nullptr);
-// Empty-cluster list in ascending order, appended from *n_empty.
+// Private copies -> sums, sizes and the empty-cluster list (ascending,
+// appended from *n_empty).
 template <typename T, typename I>
-int launch_empty_list(const T *sizes, I *list, I *n_empty, int64_t k, cudaStream_t s,
-                      const LoopState *guard = nullptr);
+int launch_reduce_centroids(const T *sizes_cp, const T *cent_cp, T *out_sizes, T *out_cent,
+                            I *empty_list, I *n_empty, int64_t P, int64_t d, int64_t k,
+                            cudaStream_t s);
 template <typename T>
 int launch_shifts(const T *old_c, const T *new_c, T *out, int64_t d, int64_t k,
                   cudaStream_t s);
-// new_c /= sizes (per cluster), then shifts[j] = sum_f (old_c - new_c)^2.
-template <typename T>
-int launch_divide_and_shift(const T *old_c, T *new_c, const T *sizes, T *shifts, int64_t d,
-                            int64_t k, cudaStream_t s, const LoopState *guard);
-// Loop control: float64 total of shifts, n_iter += 1, convergence test.
-template <typename T>
-int launch_loop_control(const T *shifts, int64_t k, LoopState *state, cudaStream_t s);
 // w == nullptr selects the unit-weight variant.  X is feature-major (d, n)
 // unless x_fstride > 0: then element (f, i) is X[f * x_fstride + i * x_sstride]
-// (a row-major copy has x_fstride = 1, x_sstride = its row length).
+// (a row-major copy has x_fstride = 1, x_sstride = its row length).  c_rows: a
+// row-major copy of C, rows of c_stride floats zero-padded to a multiple of
+// four like those of X (x_fstride = 1), or null.
 template <typename T, typename I>
 int launch_inertia(const T *X, const T *w, const T *C, const I *labels, T *out, int64_t n,
-                   int64_t d, int64_t k, cudaStream_t s, const LoopState *guard = nullptr,
-                   const int64_t *gate = nullptr, int64_t x_fstride = 0, int64_t x_sstride = 1);
+                   int64_t d, int64_t k, cudaStream_t s, int64_t x_fstride = 0,
+                   int64_t x_sstride = 1, const T *c_rows = nullptr, int64_t c_stride = 0);
 // Deterministic float64 sum of n values into *out (device).  `partials` must
 // hold sum_partials_size() doubles.
 int64_t sum_partials_size();
 template <typename T>
-int launch_sum_f64(const T *data, int64_t n, double *partials, double *out, cudaStream_t s,
-                   const LoopState *guard = nullptr);
+int launch_sum_f64(const T *data, int64_t n, double *partials, double *out, cudaStream_t s);
 template <typename T>
-int launch_fill(T *p, T v, int64_t count, cudaStream_t s, const LoopState *guard = nullptr);
+int launch_fill(T *p, T v, int64_t count, cudaStream_t s);
 
 // ---- kernels_lloyd.cu : SIMT tiled distance kernels (exact FP32/FP64) ----
 // variant: centroid-tile width of the autotuner (0: 16 x the default micro-
@@ -149,32 +140,22 @@ template <typename T>
 int launch_distances(const T *X, const T *C, T *out, int64_t n, int64_t d, int64_t k,
                      cudaStream_t s);
 
-// ---- kernels_reloc.cu : threshold (radix select), selection, relocation ----
+// ---- kernels_reloc.cu : threshold (radix select), selection, relocation of
+// the reference-shaped calls and the batched engine (a fit's own iterations
+// relocate in kernels_step.cu) ----
 // Scratch bytes needed by launch_threshold for n samples.
 size_t threshold_scratch_bytes();
 template <typename T>
-int launch_threshold(const T *data, int64_t n, const int64_t *topk_dev, int64_t topk_host,
-                     T *threshold, void *scratch, cudaStream_t s,
-                     const LoopState *guard = nullptr);
-// Scratch for launch_select; max_selected bounds n_selected.
-size_t select_scratch_bytes(int64_t max_selected);
-// Kernels launch_select enqueues for a given max_selected.
-int64_t select_launches(int64_t max_selected);
-// `scratch` holds select_scratch_bytes(max_selected) bytes; n_selected (on the
-// device or the host) is at most max_selected.
+int launch_threshold(const T *data, int64_t n, int64_t topk, T *threshold, void *scratch,
+                     cudaStream_t s);
+// Scratch for launch_select of n_selected samples.
+size_t select_scratch_bytes(int64_t n_selected);
 template <typename T, typename I>
-int launch_select(const int64_t *n_selected_dev, int64_t n_selected_host, const T *dist,
-                  const T *threshold, I *selected, I *n_gt, I *n_eq, int64_t n, void *scratch,
-                  int64_t max_selected, cudaStream_t s, const LoopState *guard = nullptr);
+int launch_select(int64_t n_selected, const T *dist, const T *threshold, I *selected, I *n_gt,
+                  I *n_eq, int64_t n, void *scratch, cudaStream_t s);
 template <typename T, typename I>
-int launch_relocate(const int64_t *n_empty_dev, int64_t n_empty_host, const T *X, const T *w,
-                    const I *labels, const I *selected, const I *n_gt, const I *empty_list,
-                    T *sums, T *sizes, T *inertia, int64_t n, int64_t d, int64_t k,
-                    cudaStream_t s, const LoopState *guard = nullptr, int64_t x_fstride = 0,
-                    int64_t x_sstride = 1);
-// Copies *n_empty (indT) into an int64 device scalar (0 when the loop stopped).
-template <typename I>
-int launch_gate_from_count(const I *n_empty, int64_t *gate, cudaStream_t s,
-                           const LoopState *guard);
+int launch_relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *selected,
+                    const I *n_gt, const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
+                    int64_t d, int64_t k, cudaStream_t s);
 
 }  // namespace kmc

@@ -113,8 +113,8 @@ extern "C" int kmc_select_samples_far_from_centroid_noalloc_f32_i32(
                   "static selection scratch is too small");
     void *scratch = nullptr;
     KMC_TRY(scratch_for_current_device(&scratch));
-    return launch_select<float, int32_t>(nullptr, n_selected, distance_to_centroid, threshold,
+    return launch_select<float, int32_t>(n_selected, distance_to_centroid, threshold,
                                          selected_samples_idx, n_selected_gt_threshold,
-                                         n_selected_eq_threshold, n_samples, scratch, n_selected,
+                                         n_selected_eq_threshold, n_samples, scratch,
                                          reinterpret_cast<cudaStream_t>(stream));
 }

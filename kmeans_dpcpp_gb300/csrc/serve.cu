@@ -374,13 +374,12 @@ struct BatchEngine {
         int32_t *counters = sm.selected + h.n;
         KMC_TRY(launch_inertia<float, int32_t>(h.X, nullptr, h.C, h.labels, sm.sq_dist, h.n, h.d,
                                                h.k, s));
-        KMC_TRY(launch_threshold<float>(sm.sq_dist, h.n, nullptr, m, sm.thr, sm.thr_scratch, s));
+        KMC_TRY(launch_threshold<float>(sm.sq_dist, h.n, m, sm.thr, sm.thr_scratch, s));
         KMC_TRY(launch_fill<int32_t>(counters, 0, 1, s));
         KMC_TRY(launch_fill<int32_t>(counters + 1, 1, 1, s));
-        KMC_TRY(launch_select<float, int32_t>(nullptr, m, sm.sq_dist, sm.thr, sm.selected,
-                                              counters, counters + 1, h.n, sm.sel_scratch, h.k,
-                                              s));
-        KMC_TRY(launch_relocate<float, int32_t>(nullptr, m, h.X, h.w, h.labels, sm.selected,
+        KMC_TRY(launch_select<float, int32_t>(m, sm.sq_dist, sm.thr, sm.selected, counters,
+                                              counters + 1, h.n, sm.sel_scratch, s));
+        KMC_TRY(launch_relocate<float, int32_t>(m, h.X, h.w, h.labels, sm.selected,
                                                 counters, sm.empty_list, sm.Cn, sm.sizes,
                                                 sm.sq_dist, h.n, h.d, h.k, s));
         ++relocations;
@@ -546,7 +545,7 @@ constexpr int kItersPerVisit = 4;
 int capture_iteration(Active &a) {
     cudaGraph_t g = nullptr;
     KMC_CUDA_TRY(cudaStreamBeginCapture(a.st, cudaStreamCaptureModeRelaxed));
-    int rc = a.fit->enqueue_iteration();
+    int rc = a.fit->enqueue_iteration(false);
     if (rc == KMC_OK) {
         const cudaError_t e = cudaMemcpyAsync(a.hstate, a.fit->device_state(), sizeof(LoopState),
                                               cudaMemcpyDeviceToHost, a.st);
@@ -924,7 +923,10 @@ struct Server {
                     retire(KMC_REQ_DONE, KMC_OK);
                 continue;
             }
-            if (a.iter_graph == nullptr || hs->done) {
+            // a paused loop relocates its empty clusters and goes on
+            const bool paused = hs->done == kPaused;
+            if (paused) KMC_TRY(a.fit->enqueue_relocation());
+            if (a.iter_graph == nullptr || (hs->done && !paused)) {
                 KMC_TRY(a.fit->finalize_enqueue(a.hstate, a.hinertia));
                 a.final_enqueued = true;
             } else {
