@@ -40,6 +40,11 @@ CU_SOURCES = [
     "kernels_lloyd.cu",
     "kernels_reloc.cu",
     "kernels_step.cu",
+    "reg_f32d.cu",
+    "reg_f32f.cu",
+    "reg_f64.cu",
+    "reg_dist.cu",
+    "sums64.cu",
     "kernels_mixed.cu",
     "driver.cu",
     "capi.cu",
@@ -49,7 +54,8 @@ CU_SOURCES = [
     "init.cu",
 ]
 HEADERS = ["km_common.cuh", "km_kernels.cuh", "km_fit.cuh", "km_mixed.cuh", "km_batch.cuh",
-           "km_step.cuh", "km_dist.cuh"]
+           "km_step.cuh", "km_dist.cuh", "km_reg.cuh",
+           "km_reg_kernel.cuh"]
 
 
 def _digest(paths, extra=""):
@@ -86,7 +92,7 @@ def _compile_cu(src):
 def build_library(verbose=False):
     """Compile the CUDA sources and link libkmeans_gb300.so (sm_103a)."""
     srcs = [s for s in CU_SOURCES if os.path.exists(os.path.join(CSRC, s))]
-    with _cf.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with _cf.ThreadPoolExecutor(max_workers=min(os.cpu_count() or 8, len(srcs))) as ex:
         objs = list(ex.map(_compile_cu, srcs))
     tag = _digest(objs)
     stamp = os.path.join(BUILD_DIR, "lib.stamp")

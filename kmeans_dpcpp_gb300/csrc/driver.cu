@@ -32,19 +32,24 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     prm = p;
     const int64_t n = p.n, d = p.d, k = p.k;
     KMC_CHECK_ARG(n >= 0 && d >= 0 && k >= 0, "negative array dimension");
-    // Small sums get one float64 copy per CTA of the fused step (two CTAs
-    // per SM), filled with fire-and-forget global reductions; shared-memory
-    // float64 atomics would be compare-and-swap loops on the critical path.
-    // float64 samples get a copy per CTA up to 256 MiB of copies: each CTA
-    // then sums its samples in a fixed order (bit-reproducible centroids).
+    // Small sums get one float64 copy per CTA of the fused step, filled with
+    // fire-and-forget global reductions; shared-memory float64 atomics would
+    // be compare-and-swap loops on the critical path.  float64 samples are
+    // summed in a fixed order (bit-reproducible centroids): by sums64.cu, or by
+    // the fused tiles with a copy per CTA up to 256 MiB of copies.
+    split64 = sizeof(T) == 8 && reg::fits(d) && sums64_fits(d, k);
     if (!uses_private_copies()) {
         P = 1;
+    } else if (split64) {
+        P = sums64_copies(n, d, k);
     } else if (sizeof(T) == 8) {
         const int64_t per_copy = 8 * (d + 1) * std::max<int64_t>(k, 1);
         P = std::max<int64_t>(1, std::min<int64_t>(2 * (int64_t)num_sms(),
                                                    (int64_t(256) << 20) / per_copy));
+    } else if ((d + 1) * k <= 8192) {
+        P = (reg::fits(d) ? 1 : 2) * (int64_t)num_sms();
     } else {
-        P = ((d + 1) * k <= 8192) ? 2 * (int64_t)num_sms() : 1;
+        P = 1;
     }
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -67,8 +72,8 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     const size_t o_part = take(sizeof(double) * sum_partials_size());
     const size_t o_dsum = take(sizeof(double) * 2);
     KMC_TRY(ws.alloc(off, p.stream));
-    // the plain kernels' centroid-tile width for this (d, k, dtype)
-    if (uses_private_copies()) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
+    // the tile kernels' width for this (d, k, dtype), where they are used
+    if (uses_private_copies() && !reg::fits(d)) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
     if (p.x_rowmajor && !reads_rowmajor()) {
         KMC_TRY(xt.alloc(sizeof(T) * (size_t)n * (size_t)d, p.stream));
         if (sizeof(T) == 4)
@@ -172,6 +177,15 @@ template <typename T, typename I>
 int PlainFit<T, I>::step_assign_and_accumulate(const T *cur, int64_t *n_launches) {
     const FitParams<T, I> &p = prm;
     *n_launches = 1;
+    if constexpr (sizeof(T) == 8) {
+        if (split64) {
+            *n_launches = 2;
+            KMC_TRY((launch_assignment<T, I>(p.X, cur, hn, p.labels, p.n, p.d, p.k, p.stream,
+                                             state)));
+            return launch_sums64<I>(p.X, p.w, p.labels, sums_cp, sizes_cp, p.n, p.d, p.k, P,
+                                    p.stream, state);
+        }
+    }
     return launch_fused_step<T, I, double>(p.X, p.w, cur, hn, p.labels, sums_cp, sizes_cp, p.n,
                                            p.d, p.k, P, p.stream, state, tile_variant);
 }

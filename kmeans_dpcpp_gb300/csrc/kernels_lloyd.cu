@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "km_kernels.cuh"
+#include "km_reg.cuh"
 
 namespace kmc {
 
@@ -396,9 +397,17 @@ int launch_tile(TileArgs<T, I, A> args, cudaStream_t s) {
 
 }  // namespace
 
+// Up to 64 features the samples fit the registers of the threads (km_reg.cuh);
+// the tiles of this file take the rest, and float64 sums in shared memory of
+// few private copies.
 template <typename T, typename I>
 int launch_assignment(const T *X, const T *C, const T *hn, I *labels, int64_t n, int64_t d,
                       int64_t k, cudaStream_t s, const LoopState *guard, int variant) {
+    if (reg::fits(d)) {
+        const reg::Args<T, double> r{X, nullptr, C, hn, labels, sizeof(I) == 8, nullptr, nullptr,
+                                     nullptr, n, d, k, 1, guard};
+        return reg::launch_labels<T, double>(r, s);
+    }
     TileArgs<T, I> a{X, nullptr, C, hn, labels, nullptr, nullptr, nullptr, n, d, k, 1, 0, 0,
                      guard};
     if (variant == 1) return launch_tile<T, I, MODE_ASSIGN, T, variant_tn<T>(1)>(a, s);
@@ -406,10 +415,12 @@ int launch_assignment(const T *X, const T *C, const T *hn, I *labels, int64_t n,
     return launch_tile<T, I, MODE_ASSIGN>(a, s);
 }
 
+namespace {
+
 template <typename T, typename I, typename A>
-int launch_fused_step(const T *X, const T *w, const T *C, const T *hn, I *labels, A *sums_cp,
-                      A *sizes_cp, int64_t n, int64_t d, int64_t k, int64_t P, cudaStream_t s,
-                      const LoopState *guard, int variant) {
+int launch_tile_step(const T *X, const T *w, const T *C, const T *hn, I *labels, A *sums_cp,
+                     A *sizes_cp, int64_t n, int64_t d, int64_t k, int64_t P, cudaStream_t s,
+                     const LoopState *guard, int variant) {
     // float64 sums of float samples with one copy per CTA go straight to
     // global memory (native reductions); otherwise small sums are privatised
     // in shared memory (float64 samples: ordered plain updates, no atomics)
@@ -425,9 +436,35 @@ int launch_fused_step(const T *X, const T *w, const T *C, const T *hn, I *labels
     return launch_tile<T, I, MODE_FUSED, A>(a, s);
 }
 
+}  // namespace
+
+template <typename T, typename I, typename A>
+int launch_fused_step(const T *X, const T *w, const T *C, const T *hn, I *labels, A *sums_cp,
+                      A *sizes_cp, int64_t n, int64_t d, int64_t k, int64_t P, cudaStream_t s,
+                      const LoopState *guard, int variant) {
+    if constexpr (sizeof(T) == 4) {
+        // float sums keep a copy per CTA: with fewer copies the tiles' partial
+        // sums in shared memory round less
+        if (reg::fits(d) && (sizeof(A) == 8 || P >= num_sms())) {
+            const reg::Args<T, A> r{X, w, C, hn, labels, sizeof(I) == 8, sums_cp, sizes_cp, nullptr,
+                                    n, d, k, P, guard};
+            return reg::launch_labels<T, A>(r, s);
+        }
+    }
+    return launch_tile_step<T, I, A>(X, w, C, hn, labels, sums_cp, sizes_cp, n, d, k, P, s, guard,
+                                     variant);
+}
+
 template <typename T>
 int launch_distances(const T *X, const T *C, T *out, int64_t n, int64_t d, int64_t k,
                      cudaStream_t s) {
+    if constexpr (sizeof(T) == 4) {
+        if (reg::fits(d)) {
+            const reg::Args<float, float> r{X, nullptr, C, nullptr, nullptr, 0, nullptr, nullptr,
+                                            out, n, d, k, 1, nullptr};
+            return reg::launch_dist(r, s);
+        }
+    }
     TileArgs<T, int32_t> a{X, nullptr, C, nullptr, nullptr, nullptr, nullptr, out,
                            n, d, k, 1, 0, 0, nullptr};
     return launch_tile<T, int32_t, MODE_DIST>(a, s);
@@ -489,8 +526,8 @@ int tune_fit_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
             rc = launch_fill<double>(sums, 0.0, d * k + k, s);
             if (rc == KMC_OK) rc = cudaEventRecord(e0, s) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
             if (rc == KMC_OK)
-                rc = launch_fused_step<T, int32_t, double>(X, w, C, hn, lab, sums, sums + d * k,
-                                                           n, d, k, 1, s, nullptr, v);
+                rc = launch_tile_step<T, int32_t, double>(X, w, C, hn, lab, sums, sums + d * k,
+                                                          n, d, k, 1, s, nullptr, v);
             if (rc == KMC_OK) rc = cudaEventRecord(e1, s) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
             if (rc == KMC_OK) rc = cudaEventSynchronize(e1) == cudaSuccess ? KMC_OK : KMC_ERR_CUDA;
             float ms = 0.f;

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "km_kernels.cuh"
+#include "km_reg.cuh"
 #include "km_step.cuh"
 
 namespace kmc {
@@ -104,6 +105,7 @@ struct PlainFit : FitBase {
     double *partials = nullptr, *dsum = nullptr;
     int64_t issued = 0;
     int host_done = 0;
+    bool split64 = false;  // float64 samples: labels, then sums (sums64.cu)
     int tile_variant = 0;  // autotuned centroid-tile width of the plain kernels
     Scratch xt;  // feature-major copy of a row-major X (forms that need one)
 

@@ -1,0 +1,83 @@
+// Assignment, fused step and distances of up to 64 features with the samples
+// in registers.
+//
+// A thread holds S samples (S x DP registers, DP = features rounded up to a
+// multiple of 4, the rest zero) and walks the centroids, which the CTA keeps
+// in shared memory: every lane of a warp reads the same centroid, so one
+// 16-byte shared-memory read feeds 4 S (2 S for pairs, below) fused
+// multiply-adds of all 32 lanes, nothing is exchanged between threads, and
+// warps never wait for one another.  The 128 x 128 tiles of tile_kernel
+// (kernels_lloyd.cu) spend as long on staging, barriers and the argmin over 16
+// threads as on the products when there are few features.
+//
+// Each score keeps the reference's arithmetic (sequential fma over f = 0..d-1,
+// hn - dot, strict < over ascending centroids; src/device_functions.hpp:
+// 106-162).  Padded features add 0 * 0, which leaves every sum as it is.
+//
+// Up to 32 features two samples share an instruction (fma.rn.f32x2: the same
+// rounding per half, one issue slot for two products; the FMA pipe, not the
+// issue slots, is then the bound).  Both halves need the same centroid value,
+// so shared memory holds each value twice; beyond 32 features that would
+// saturate the shared-memory port, and single fmas are used.
+#pragma once
+
+#include "km_kernels.cuh"
+
+namespace kmc {
+namespace reg {
+
+constexpr int kMaxFeatures = 64;
+constexpr size_t kSmemBytes = 220 * 1024;
+
+constexpr int MODE_LABELS = 0, MODE_DIST = 1;
+
+__host__ __device__ constexpr bool paired(int DP, int mode) { return DP <= 32 || mode == MODE_DIST; }
+__host__ __device__ constexpr int samples_per_thread(int DP) { return DP <= 32 ? 4 : 2; }
+__host__ __device__ constexpr int max_threads(int DP) { return DP <= 16 ? 512 : 384; }
+// Floats per centroid in shared memory: a multiple of 4 that is 4 mod 8, so
+// that staging 8 centroids x 4 features writes 32 different banks.
+__host__ __device__ constexpr int row_floats(int DP, int mode) {
+    const int w = paired(DP, mode) ? 2 * DP : DP;
+    return (w % 8 == 4) ? w : w + 4;
+}
+// Centroids held at once.
+__host__ __device__ constexpr int chunk_rows(int DP, int mode) {
+    return (int)(kSmemBytes / sizeof(float)) / (row_floats(DP, mode) + 1);
+}
+
+template <typename T, typename A>
+struct Args {
+    const T *X;   // (d, n)
+    const T *w;   // (n), with sums
+    const T *C;   // (d, k)
+    const T *hn;  // (k)
+    void *labels;
+    int label64;
+    A *sums, *sizes;  // private copies ([P][d k], [P][k]); null: labels only
+    T *dist;          // MODE_DIST: (k, n)
+    int64_t n, d, k, P;
+    const LoopState *guard;
+};
+
+// f32 input, A = float or double sums, and float64 input (labels only); one
+// launcher per feature class, defined in reg_*.cu.
+template <typename T, typename A>
+int launch_labels(const Args<T, A> &a, cudaStream_t s);
+int launch_dist(const Args<float, float> &a, cudaStream_t s);
+
+// Whether the shapes are taken (the callers' rule adds what they measured).
+inline bool fits(int64_t d) { return d >= 1 && d <= kMaxFeatures; }
+
+}  // namespace reg
+
+// ---- sums64.cu: float64 cluster sums of float64 samples, given the labels ----
+// Whether a CTA can hold its own copies of the sums.
+bool sums64_fits(int64_t d, int64_t k);
+// Number of private copies written ([copies][d k] then sizes [copies][k]).
+int64_t sums64_copies(int64_t n, int64_t d, int64_t k);
+template <typename I>
+int launch_sums64(const double *X, const double *w, const I *labels, double *sums, double *sizes,
+                  int64_t n, int64_t d, int64_t k, int64_t copies, cudaStream_t s,
+                  const LoopState *guard);
+
+}  // namespace kmc
