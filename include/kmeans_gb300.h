@@ -609,8 +609,9 @@ int kmc_batch_remove(kmc_batch_t batch, int64_t instance);
 int kmc_batch_stats(kmc_batch_t batch, int64_t *steps_out, int64_t *graph_builds_out,
                     int64_t *relocations_out);
 int kmc_batch_destroy(kmc_batch_t batch);
-/* Tile autotuner: centroid-window variant (0: 32, 1: 64, 2: 128 columns) the
- * batched assignment uses for (d, k, float32); measured once, cached. */
+/* Tile autotuner: centroid columns per step (0: 16, 1: 32, 2: 64; for more
+ * features than a panel takes 32, 64, 128) the batched assignment uses for
+ * (d, k, float32); measured once, cached. */
 int kmc_tile_variant(int64_t n_features, int64_t n_clusters, kmc_stream_t stream,
                      int *variant_out);
 /* Seeded synthetic Gaussian blobs written on the device, X_t (d, n). */

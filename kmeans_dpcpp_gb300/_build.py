@@ -44,6 +44,10 @@ CU_SOURCES = [
     "reg_f32f.cu",
     "reg_f64.cu",
     "reg_dist.cu",
+    "panel_f32d.cu",
+    "panel_f32f.cu",
+    "panel_f64.cu",
+    "panel_dist.cu",
     "sums64.cu",
     "kernels_mixed.cu",
     "driver.cu",
@@ -55,7 +59,7 @@ CU_SOURCES = [
 ]
 HEADERS = ["km_common.cuh", "km_kernels.cuh", "km_fit.cuh", "km_mixed.cuh", "km_batch.cuh",
            "km_step.cuh", "km_dist.cuh", "km_reg.cuh",
-           "km_reg_kernel.cuh"]
+           "km_reg_kernel.cuh", "km_panel.cuh", "km_panel_kernel.cuh"]
 
 
 def _digest(paths, extra=""):

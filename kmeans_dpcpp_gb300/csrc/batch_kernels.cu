@@ -5,22 +5,25 @@
 //   batch_prep    one CTA per instance: half norms of its centroids
 //                 (src/util_kernels.hpp:47-82 order), zeroed float64 sums,
 //                 reset work-queue counters
-//   batch_assign  persistent CTAs pop (instance, run of 128-sample tiles)
-//                 items from a device work queue.  Each (sample, centroid)
+//   batch_panel   persistent CTAs pop (instance, run of 128-sample tiles)
+//                 items from a device work queue and walk them in panels of 32
+//                 samples per warp (km_panel.cuh).  Each (sample, centroid)
 //                 pair gets the plain form's arithmetic -- sequential FMA dot
 //                 over f = 0..d-1, D = hn - dot, strict < over ascending j
 //                 (src/device_functions.hpp:106-162) -- so labels equal a
 //                 single fit's bit for bit.  Fitting instances add w*x into
-//                 float64 sums, privatised per item in shared memory when the
-//                 instance's k*(d+1) doubles fit in 72 KB.  Three kernels
-//                 differ in the centroid window (32, 64 or 128 columns per
-//                 pass); the autotuner picks one per (d, k)
+//                 float64 copies of the sums.  Three kernels differ in the
+//                 centroids per thread (16, 32 or 64 columns per step); the
+//                 autotuner picks one per (d, k)
+//   batch_assign  the same for instances of more features than a panel takes,
+//                 in 128-sample tiles (centroid windows of 32, 64 or 128)
 //   batch_reduce  one CTA per fitting instance: sums rounded once to float32,
 //                 sizes, ascending empty-cluster list
 //                 (src/util_kernels.hpp:87-161)
 //   batch_update  one CTA per fitting instance: divide, per-cluster shifts,
 //                 float64 total, the driver's stop rule
 //                 (src/kmeans_lloyd_driver.hpp:317-353), copy-back
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
@@ -32,6 +35,7 @@
 #include <sys/stat.h>
 
 #include "km_batch.cuh"
+#include "km_panel_kernel.cuh"
 
 namespace kmc {
 
@@ -60,7 +64,7 @@ __device__ double block_sum_b(double v, double *sh) {
 }
 
 __global__ void batch_prep_kernel(BInst *tab, const int *idx, int count, int *counters) {
-    if (blockIdx.x == 0 && threadIdx.x < 2 * kBatchVariants) counters[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < kBatchCounters) counters[threadIdx.x] = 0;
     if ((int)blockIdx.x >= count) return;
     BInst &in = tab[idx[blockIdx.x]];
     const int d = in.d, k = in.k;
@@ -130,6 +134,7 @@ __global__ void __launch_bounds__(kThreadsB, 2)
         if (it >= n_items) break;
         const BItem item = items[it];
         const BInst &in = tab[item.inst];
+        if (panel::fits(in.d, DIST ? panel::MODE_DIST : panel::MODE_LABELS)) continue;
         const float *X = in.X, *C = in.C, *hn = in.hn, *w = in.w;
         int32_t *labels = in.labels;
         const int64_t n = in.n;
@@ -306,6 +311,44 @@ __global__ void __launch_bounds__(kThreadsB, 2)
     }
 }
 
+// The same items for instances whose samples fit panels (km_panel.cuh): the
+// CTA takes an item, its warps the item's panels of 32 samples; TN centroids
+// per thread, so 8 TN columns per step.
+template <int TN, int DIST>
+__global__ void __launch_bounds__(32 * panel::kMaxWarps, 1)
+    batch_panel_kernel(const BInst *tab, const BItem *items, int n_items, int *counter) {
+    extern __shared__ __align__(16) float psmem[];
+    __shared__ int item_sh;
+    constexpr int mode = DIST ? panel::MODE_DIST : panel::MODE_LABELS;
+    while (true) {
+        __syncthreads();  // the last item's shared memory is free
+        if (threadIdx.x == 0) item_sh = atomicAdd(counter, 1);
+        __syncthreads();
+        const int it = item_sh;
+        if (it >= n_items) break;
+        const BItem item = items[it];
+        const BInst &in = tab[item.inst];
+        const int warps = panel::warps_for(in.d, mode);
+        if (warps == 0) continue;  // batch_assign_kernel takes it
+        const int64_t copy = DIST ? 0 : (int64_t)(blockIdx.x % (unsigned)in.copies);
+        const int64_t dk = (int64_t)in.d * in.k;
+        // the copies lie one after another, each with its sizes
+        double *sums = in.mode == B_FIT ? in.sums + copy * (dk + in.k) : nullptr;
+        constexpr int64_t per_tile = kBatchTileM / panel::kRows;
+        const int64_t first = item.tile0 * per_tile, end = first + item.ntiles * per_tile;
+        if constexpr (DIST) {
+            const panel::Args<float, float> a{in.X, nullptr, in.C, nullptr, nullptr, 0, nullptr,
+                                              nullptr, in.dist, in.n, in.d, in.k, 1, nullptr};
+            panel::run_panels<TN, mode, float, float>(a, warps, first, end, warps, 0, psmem);
+        } else {
+            const panel::Args<float, double> a{in.X, in.w, in.C, in.hn, in.labels, 0, sums,
+                                               sums ? sums + dk : nullptr, nullptr, in.n, in.d,
+                                               in.k, 1, nullptr};
+            panel::run_panels<TN, mode, float, double>(a, warps, first, end, warps, 0, psmem);
+        }
+    }
+}
+
 __global__ void batch_reduce_kernel(BInst *tab, const int *idx, int count, int *n_empty_out) {
     if ((int)blockIdx.x >= count) return;
     BInst &in = tab[idx[blockIdx.x]];
@@ -479,9 +522,26 @@ int launch_assign_v(int variant, const BInst *tab, const BItem *items, int n_ite
     return check_launch("batch_assign");
 }
 
+template <int TN, int DIST>
+int prepare_panels() {
+    KMC_CUDA_TRY(cudaFuncSetAttribute(batch_panel_kernel<TN, DIST>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)panel::kSmemBytes));
+    return KMC_OK;
+}
+
+template <int TN, int DIST>
+int launch_panels(const BInst *tab, const BItem *items, int n_items, int *counter,
+                  cudaStream_t s) {
+    const int grid = std::min(n_items, num_sms());
+    batch_panel_kernel<TN, DIST><<<grid, 32 * panel::kMaxWarps, panel::kSmemBytes, s>>>(
+        tab, items, n_items, counter);
+    return check_launch("batch_panel");
+}
+
 std::mutex g_tune_mu;
-// autotuner choices by (d, power-of-two bucket of k, tag); tag "f32" is the
-// batched engine's centroid window, "fit-f32" / "fit-f64" the single-fit tile
+// autotuner choices by (d, power-of-two bucket of k, tag); tag "f32-panel" is
+// the batched engine's centroid window, "fit-f32" / "fit-f64" the single-fit tile
 std::map<std::tuple<int64_t, int64_t, std::string>, int> g_tune;
 bool g_tune_loaded = false;
 
@@ -529,16 +589,8 @@ void tune_store(int64_t d, int64_t k, const std::string &tag, int v) {
 
 }  // namespace
 
-int batch_variant_width(int v) { return v == 0 ? 32 : (v == 1 ? 64 : 128); }
-
 int batch_sum_copies(int64_t d, int64_t k) {
     return ((d + 1) * k * (int64_t)sizeof(double) <= (int64_t)kPrivBytes) ? kSumCopies : 1;
-}
-
-size_t batch_assign_smem(int v) {
-    const size_t b = v == 0 ? BTile<2>::base_bytes
-                            : (v == 1 ? BTile<4>::base_bytes : BTile<8>::base_bytes);
-    return b + kPrivBytes;
 }
 
 int launch_batch_prep(BInst *tab, const int *idx, int count, int *counters, cudaStream_t s) {
@@ -553,12 +605,32 @@ int prepare_batch_assign() {
     KMC_TRY((assign_shape<8, 0>(2, &sh)));
     KMC_TRY((assign_shape<2, 1>(0, &sh)));
     KMC_TRY((assign_shape<4, 1>(1, &sh)));
-    return assign_shape<8, 1>(2, &sh);
+    KMC_TRY((assign_shape<8, 1>(2, &sh)));
+    KMC_TRY((prepare_panels<2, 0>()));
+    KMC_TRY((prepare_panels<4, 0>()));
+    KMC_TRY((prepare_panels<8, 0>()));
+    KMC_TRY((prepare_panels<2, 1>()));
+    KMC_TRY((prepare_panels<4, 1>()));
+    return prepare_panels<8, 1>();
 }
 
-int launch_batch_assign(int variant, int dist, const BInst *tab, const BItem *items,
+bool batch_in_panels(int64_t d, int dist) {
+    return panel::fits(d, dist ? panel::MODE_DIST : panel::MODE_LABELS);
+}
+
+int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, const BItem *items,
                         int n_items, int *counter, cudaStream_t s) {
     if (n_items <= 0) return KMC_OK;
+    if (panels) {
+        if (dist) {
+            if (variant == 0) return launch_panels<2, 1>(tab, items, n_items, counter, s);
+            if (variant == 1) return launch_panels<4, 1>(tab, items, n_items, counter, s);
+            return launch_panels<8, 1>(tab, items, n_items, counter, s);
+        }
+        if (variant == 0) return launch_panels<2, 0>(tab, items, n_items, counter, s);
+        if (variant == 1) return launch_panels<4, 0>(tab, items, n_items, counter, s);
+        return launch_panels<8, 0>(tab, items, n_items, counter, s);
+    }
     if (dist) {
         if (variant == 0) return launch_assign_v<2, 1>(0, tab, items, n_items, counter, s);
         if (variant == 1) return launch_assign_v<4, 1>(1, tab, items, n_items, counter, s);
@@ -640,7 +712,8 @@ int tune_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
     // one measurement per (d, power-of-two bucket of k)
     int64_t k = 1;
     while (k < k_in) k <<= 1;
-    if (tune_lookup(d, k, "f32", variant) && *variant < kBatchVariants) return KMC_OK;
+    if (tune_lookup(d, k, "f32-panel", variant) && *variant < kBatchVariants) return KMC_OK;
+    KMC_TRY(prepare_batch_assign());
     // Time the three assign kernels on a synthetic fitting instance of this
     // (d, k): 256 tiles of 128 samples, blobs around k centres.
     const int64_t n = 256 * kBatchTileM;
@@ -691,7 +764,7 @@ int tune_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
         for (int rep = 0; rep < 3; ++rep) {
             KMC_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), s));
             KMC_CUDA_TRY(cudaEventRecord(e0, s));
-            KMC_TRY(launch_batch_assign(v, 0, tab, items, 64, cnt, s));
+            KMC_TRY(launch_batch_assign(v, 0, batch_in_panels(d, 0), tab, items, 64, cnt, s));
             KMC_CUDA_TRY(cudaEventRecord(e1, s));
             KMC_CUDA_TRY(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -706,7 +779,7 @@ int tune_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     KMC_CUDA_TRY(cudaStreamSynchronize(s));
-    tune_record(d, k, "f32", best);
+    tune_record(d, k, "f32-panel", best);
     *variant = best;
     return KMC_OK;
 }

@@ -37,7 +37,7 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     // be compare-and-swap loops on the critical path.  float64 samples are
     // summed in a fixed order (bit-reproducible centroids): by sums64.cu, or by
     // the fused tiles with a copy per CTA up to 256 MiB of copies.
-    split64 = sizeof(T) == 8 && reg::fits(d) && sums64_fits(d, k);
+    split64 = sizeof(T) == 8 && panel::fits(d) && sums64_fits(d, k);
     if (!uses_private_copies()) {
         P = 1;
     } else if (split64) {
@@ -47,7 +47,7 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
         P = std::max<int64_t>(1, std::min<int64_t>(2 * (int64_t)num_sms(),
                                                    (int64_t(256) << 20) / per_copy));
     } else if ((d + 1) * k <= 8192) {
-        P = (reg::fits(d) ? 1 : 2) * (int64_t)num_sms();
+        P = (panel::fits(d) ? 1 : 2) * (int64_t)num_sms();
     } else {
         P = 1;
     }
@@ -73,7 +73,7 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     const size_t o_dsum = take(sizeof(double) * 2);
     KMC_TRY(ws.alloc(off, p.stream));
     // the tile kernels' width for this (d, k, dtype), where they are used
-    if (uses_private_copies() && !reg::fits(d)) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
+    if (uses_private_copies() && !panel::fits(d)) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
     if (p.x_rowmajor && !reads_rowmajor()) {
         KMC_TRY(xt.alloc(sizeof(T) * (size_t)n * (size_t)d, p.stream));
         if (sizeof(T) == 4)

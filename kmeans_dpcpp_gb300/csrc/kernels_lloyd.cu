@@ -35,7 +35,7 @@
 #include <type_traits>
 
 #include "km_kernels.cuh"
-#include "km_reg.cuh"
+#include "km_panel.cuh"
 
 namespace kmc {
 
@@ -397,17 +397,30 @@ int launch_tile(TileArgs<T, I, A> args, cudaStream_t s) {
 
 }  // namespace
 
-// Up to 64 features the samples fit the registers of the threads (km_reg.cuh);
-// the tiles of this file take the rest, and float64 sums in shared memory of
-// few private copies.
+namespace {
+
+// Samples in registers (few centroids), or in panels; false: neither takes the
+// shape (the tiles of this file do).
+template <typename T, typename A>
+bool launch_warp_labels(const reg::Args<T, A> &r, cudaStream_t s, int *rc) {
+    if (reg::fits(r.d, r.k, reg::MODE_LABELS))
+        *rc = reg::launch_labels<T, A>(r, s);
+    else if (panel::fits(r.d))
+        *rc = panel::launch_labels<T, A>(r, s);
+    else
+        return false;
+    return true;
+}
+
+}  // namespace
+
 template <typename T, typename I>
 int launch_assignment(const T *X, const T *C, const T *hn, I *labels, int64_t n, int64_t d,
                       int64_t k, cudaStream_t s, const LoopState *guard, int variant) {
-    if (reg::fits(d)) {
-        const reg::Args<T, double> r{X, nullptr, C, hn, labels, sizeof(I) == 8, nullptr, nullptr,
-                                     nullptr, n, d, k, 1, guard};
-        return reg::launch_labels<T, double>(r, s);
-    }
+    const reg::Args<T, double> r{X, nullptr, C, hn, labels, sizeof(I) == 8, nullptr, nullptr,
+                                 nullptr, n, d, k, 1, guard};
+    int rc = KMC_OK;
+    if (launch_warp_labels<T, double>(r, s, &rc)) return rc;
     TileArgs<T, I> a{X, nullptr, C, hn, labels, nullptr, nullptr, nullptr, n, d, k, 1, 0, 0,
                      guard};
     if (variant == 1) return launch_tile<T, I, MODE_ASSIGN, T, variant_tn<T>(1)>(a, s);
@@ -445,10 +458,11 @@ int launch_fused_step(const T *X, const T *w, const T *C, const T *hn, I *labels
     if constexpr (sizeof(T) == 4) {
         // float sums keep a copy per CTA: with fewer copies the tiles' partial
         // sums in shared memory round less
-        if (reg::fits(d) && (sizeof(A) == 8 || P >= num_sms())) {
+        if (sizeof(A) == 8 || P >= num_sms()) {
             const reg::Args<T, A> r{X, w, C, hn, labels, sizeof(I) == 8, sums_cp, sizes_cp, nullptr,
                                     n, d, k, P, guard};
-            return reg::launch_labels<T, A>(r, s);
+            int rc = KMC_OK;
+            if (launch_warp_labels<T, A>(r, s, &rc)) return rc;
         }
     }
     return launch_tile_step<T, I, A>(X, w, C, hn, labels, sums_cp, sizes_cp, n, d, k, P, s, guard,
@@ -459,11 +473,10 @@ template <typename T>
 int launch_distances(const T *X, const T *C, T *out, int64_t n, int64_t d, int64_t k,
                      cudaStream_t s) {
     if constexpr (sizeof(T) == 4) {
-        if (reg::fits(d)) {
-            const reg::Args<float, float> r{X, nullptr, C, nullptr, nullptr, 0, nullptr, nullptr,
-                                            out, n, d, k, 1, nullptr};
-            return reg::launch_dist(r, s);
-        }
+        const reg::Args<float, float> r{X, nullptr, C, nullptr, nullptr, 0, nullptr, nullptr, out,
+                                        n, d, k, 1, nullptr};
+        if (reg::fits(d, k, reg::MODE_DIST)) return reg::launch_dist(r, s);
+        if (panel::fits(d, panel::MODE_DIST)) return panel::launch_dist(r, s);
     }
     TileArgs<T, int32_t> a{X, nullptr, C, nullptr, nullptr, nullptr, nullptr, out,
                            n, d, k, 1, 0, 0, nullptr};

@@ -31,7 +31,7 @@ struct BInst {
     long long n;
     int d, k;
     int mode;              // B_FIT or B_ASSIGN
-    int variant;           // centroid-window width: 0 -> 32, 1 -> 64, 2 -> 128
+    int variant;           // centroid columns per step: 0 -> 16, 1 -> 32, 2 -> 64 (panels)
     int copies;            // private copies of sums (CTA b adds into copy b % copies)
     LoopState st;          // done / n_iter / max_iter / tol / last_shift
 };
@@ -45,20 +45,22 @@ struct BItem {
 
 constexpr int kBatchVariants = 3;
 constexpr int kBatchTileM = 128;
+// work-queue counters: per (panels or wide instances, kind, variant)
+constexpr int kBatchCounters = 4 * kBatchVariants;
 
-int batch_variant_width(int v);
 // Private global copies of an instance's float64 sums: small sums get several
 // (their few addresses would serialise the reductions of many CTAs).
 int batch_sum_copies(int64_t d, int64_t k);
-// Dynamic shared memory of one assign CTA of variant v.
-size_t batch_assign_smem(int v);
 
 // ---- launchers (batch.cu) ----
 int launch_batch_prep(BInst *tab, const int *idx, int count, int *counters, cudaStream_t s);
 // Sets the assign kernels' shared-memory attributes (outside graph capture).
 int prepare_batch_assign();
 // dist != 0: the transform kernel (items of B_TRANSFORM instances only).
-int launch_batch_assign(int variant, int dist, const BInst *tab, const BItem *items,
+// panels: the kernel for instances whose features fit panels (it skips the
+// other items, as the other kernel skips these).
+bool batch_in_panels(int64_t d, int dist);
+int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, const BItem *items,
                         int n_items, int *counter, cudaStream_t s);
 int launch_batch_reduce(BInst *tab, const int *idx, int count, int *n_empty_out,
                         cudaStream_t s);

@@ -6,7 +6,7 @@
 #include <vector>
 
 #include "km_kernels.cuh"
-#include "km_reg.cuh"
+#include "km_panel.cuh"
 #include "km_step.cuh"
 
 namespace kmc {

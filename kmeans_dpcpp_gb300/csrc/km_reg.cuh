@@ -1,24 +1,25 @@
-// Assignment, fused step and distances of up to 64 features with the samples
-// in registers.
+// Labels, fused step and distances of up to 64 features and few centroids, with
+// the samples in registers.
 //
 // A thread holds S samples (S x DP registers, DP = features rounded up to a
 // multiple of 4, the rest zero) and walks the centroids, which the CTA keeps
-// in shared memory: every lane of a warp reads the same centroid, so one
-// 16-byte shared-memory read feeds 4 S (2 S for pairs, below) fused
-// multiply-adds of all 32 lanes, nothing is exchanged between threads, and
-// warps never wait for one another.  The 128 x 128 tiles of tile_kernel
-// (kernels_lloyd.cu) spend as long on staging, barriers and the argmin over 16
-// threads as on the products when there are few features.
+// in shared memory: every lane of a warp reads the same centroid, nothing is
+// exchanged between threads, and warps never wait for one another.  With few
+// centroids the samples' loads are what counts, and S x d of them are in
+// flight per thread; with more, the panels' micro-tiles (km_panel.cuh) use the
+// FMA pipe better (labels of 1M samples, registers against panels: 14 features
+// and 32 centroids 36 / 40 us, 64 and 20: 90 / 127 us, 8 and 8: 11 / 25 us,
+// 4 and 64: 27 / 35 us; but 16 and 1000: 859 / 630 us).
 //
 // Each score keeps the reference's arithmetic (sequential fma over f = 0..d-1,
 // hn - dot, strict < over ascending centroids; src/device_functions.hpp:
 // 106-162).  Padded features add 0 * 0, which leaves every sum as it is.
 //
 // Up to 32 features two samples share an instruction (fma.rn.f32x2: the same
-// rounding per half, one issue slot for two products; the FMA pipe, not the
-// issue slots, is then the bound).  Both halves need the same centroid value,
-// so shared memory holds each value twice; beyond 32 features that would
-// saturate the shared-memory port, and single fmas are used.
+// rounding per half, one issue slot for two products).  Both halves need the
+// same centroid value, so shared memory holds each value twice; beyond 32
+// features that would saturate the shared-memory port, and single fmas are
+// used.
 #pragma once
 
 #include "km_kernels.cuh"
@@ -65,8 +66,11 @@ template <typename T, typename A>
 int launch_labels(const Args<T, A> &a, cudaStream_t s);
 int launch_dist(const Args<float, float> &a, cudaStream_t s);
 
-// Whether the shapes are taken (the callers' rule adds what they measured).
-inline bool fits(int64_t d) { return d >= 1 && d <= kMaxFeatures; }
+// Up to this many centroids the registers are used for labels / distances.
+constexpr int64_t kFewLabels = 64, kFewDist = 32;
+inline bool fits(int64_t d, int64_t k, int mode) {
+    return d >= 1 && d <= kMaxFeatures && k <= (mode == MODE_DIST ? kFewDist : kFewLabels);
+}
 
 }  // namespace reg
 

@@ -1,0 +1,11 @@
+// Instances of km_panel.cuh: labels (and float64 sums) of float samples.
+#include "km_panel_kernel.cuh"
+
+namespace kmc {
+namespace panel {
+template <>
+int launch_labels<float, double>(const Args<float, double> &a, cudaStream_t s, int tn) {
+    return launch_any<MODE_LABELS, float, double>(a, s, tn);
+}
+}  // namespace panel
+}  // namespace kmc

@@ -179,7 +179,7 @@ struct BatchEngine {
         const size_t o_all = o_tab + align256(sizeof(BInst) * cap);
         const size_t o_fit = o_all + align256(sizeof(int) * cap);
         const size_t o_cnt = o_fit + align256(sizeof(int) * cap);
-        const size_t o_ne = o_cnt + align256(sizeof(int) * 2 * kBatchVariants);
+        const size_t o_ne = o_cnt + align256(sizeof(int) * kBatchCounters);
         const size_t o_dn = o_ne + align256(sizeof(int) * cap);
         KMC_TRY(dev.alloc(o_dn + align256(sizeof(int) * cap), s));
         char *b = dev.as<char>();
@@ -289,12 +289,15 @@ struct BatchEngine {
         all.clear();
         fits.clear();
         std::vector<BItem> items[2][kBatchVariants];
+        bool use[2][2][kBatchVariants] = {};  // [panels][kind][variant]
         for (int64_t q = 0; q < cap; ++q) {
             if (state[(size_t)q] != RUNNING) continue;
             const BInst &h = tab[(size_t)q];
             all.push_back((int)q);
             if (h.mode == B_FIT) fits.push_back((int)q);
             append_items((int)q, h.n, h.mode, h.variant, items);
+            const int kind = h.mode == B_TRANSFORM ? 1 : 0;
+            use[batch_in_panels(h.d, kind) ? 1 : 0][kind][h.variant] = true;
         }
         int64_t total = 0;
         for (int kind = 0; kind < 2; ++kind)
@@ -333,9 +336,12 @@ struct BatchEngine {
                 if (n_items[0][v] + n_items[1][v] == 0) continue;
                 KMC_CUDA_TRY(cudaStreamWaitEvent(side[v], ev_fork, 0));
                 for (int kind = 0; kind < 2; ++kind)
-                    KMC_TRY(launch_batch_assign(v, kind, tab_d, items_d + item_off[kind][v],
-                                                n_items[kind][v],
-                                                counters_d + kind * kBatchVariants + v, side[v]));
+                    for (int pn = 1; pn >= 0; --pn)
+                        if (use[pn][kind][v])
+                            KMC_TRY(launch_batch_assign(
+                                v, kind, pn != 0, tab_d, items_d + item_off[kind][v],
+                                n_items[kind][v],
+                                counters_d + (2 * pn + kind) * kBatchVariants + v, side[v]));
                 KMC_CUDA_TRY(cudaEventRecord(ev_join[v], side[v]));
                 KMC_CUDA_TRY(cudaStreamWaitEvent(s, ev_join[v], 0));
             }

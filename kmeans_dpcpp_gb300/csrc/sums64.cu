@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(32 * kSumsWarps, 1)
 }  // namespace
 
 bool sums64_fits(int64_t d, int64_t k) {
-    return d >= 1 && d <= reg::kMaxFeatures && warps_for(d, k) >= 1;
+    return d >= 1 && warps_for(d, k) >= 1;
 }
 
 int64_t sums64_copies(int64_t n, int64_t d, int64_t k) {

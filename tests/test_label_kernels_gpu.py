@@ -1,7 +1,7 @@
-"""The kernels that hold the samples in registers (up to 64 features) at the
-edges of their feature classes, of a warp's samples and of the centroids that
-shared memory holds at once, in every data type; beyond 64 features the tile
-kernels answer.  Labels, distances and (with integer data) sums must equal the
+"""The kernels that hold the samples in registers (few centroids) or in panels
+of shared memory, at the edges of their feature classes, of a warp's samples
+and of the centroids that shared memory holds at once, in every data type;
+beyond 148 features the tile kernels answer.  Labels, distances and (with integer data) sums must equal the
 oracle's exactly: the arithmetic per score is the same.
 
 Float64 labels come from float32 scores wherever those decide them, so they are
@@ -39,7 +39,9 @@ def _labels(X, C, hn=None, it="int64"):
 SHAPES = [(1, 1, 1), (31, 2, 2), (127, 4, 7), (129, 5, 33), (1000, 8, 16), (257, 9, 300), (513, 12, 5),
           (300, 13, 1700), (5000, 16, 127), (1025, 17, 64), (700, 20, 1), (333, 24, 40), (640, 28, 90),
           (2000, 32, 900), (400, 33, 20), (800, 40, 65), (150, 48, 3), (260, 56, 128), (4000, 64, 1000),
-          (500, 65, 30), (30_000, 14, 50)]
+          (500, 65, 30), (30_000, 14, 50), (70_001, 14, 100), (2500, 1, 65), (1111, 2, 66), (900, 3, 129),
+          (1300, 30, 191), (4000, 64, 1025), (700, 65, 64), (650, 99, 800), (330, 128, 33), (300, 148, 70),
+          (200, 149, 90), (150, 300, 17)]
 
 
 @pytest.mark.parametrize("n,d,k", SHAPES)
@@ -113,7 +115,7 @@ def test_float64_labels_with_given_half_norms(oracle, seed):
 
 
 @pytest.mark.parametrize("d,k", [(1, 3), (14, 127), (15, 40), (16, 200), (31, 20), (33, 300), (64, 64), (64, 400),
-                                 (14, 2000)])
+                                 (14, 2000), (100, 70), (128, 150), (148, 40), (160, 33)])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("it", ["int32", "int64"])
 def test_weighted_iterations_equal_the_oracles(oracle, d, k, dt, it):
@@ -136,7 +138,8 @@ def test_weighted_iterations_equal_the_oracles(oracle, d, k, dt, it):
     np.testing.assert_array_equal(lab.cpu().numpy(), lab_o)
 
 
-@pytest.mark.parametrize("d,k,copies", [(14, 16, 200), (14, 16, 3), (32, 256, 300), (64, 90, 152), (70, 30, 400)])
+@pytest.mark.parametrize("d,k,copies", [(14, 16, 200), (14, 16, 3), (32, 256, 300), (64, 90, 152), (70, 30, 400),
+                                        (100, 300, 160), (150, 20, 200)])
 def test_fused_step_with_many_and_few_copies(oracle, d, k, copies):
     import torch
 
