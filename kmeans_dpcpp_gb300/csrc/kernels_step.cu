@@ -111,10 +111,15 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
         } else if (ok) {
             v = sq_dist_cols<T>(a.X, a.fs, a.ss, a.prev, d, k, i, c);
         }
-        if (i < b1) {
-            a.sq_dist[i] = v;
-            atomicAdd(&h32[order_of(v) >> (8 * kDigits - 8)], 1u);
-        }
+        if (i < b1) a.sq_dist[i] = v;
+        // the leading digits of similar distances are the same few: lanes that
+        // share the first lane's digit count once
+        const unsigned digit = (unsigned)(order_of(v) >> (8 * kDigits - 8));
+        const unsigned in = __ballot_sync(0xffffffffu, i < b1);
+        const unsigned lead = __shfl_sync(0xffffffffu, digit, 0);
+        const unsigned same = __ballot_sync(0xffffffffu, digit == lead) & in;
+        if (lane == 0 && same != 0u) atomicAdd(&h32[lead], (unsigned)__popc(same));
+        if (i < b1 && digit != lead) atomicAdd(&h32[digit], 1u);
     }
     unsigned long long prefix = 0ull, rank = (unsigned long long)(m - 1);
     for (int p = 0; p < kDigits; ++p) {

@@ -48,14 +48,26 @@ __device__ __forceinline__ void copy_wait_all() {
 // Certification of float64 labels by float32 scores.  In units scaled by the
 // power of two sigma (largest |centroid coordinate| about 2^10), with u = 2^-24,
 // x and c rounded to float32 and the sequential float32 dot product:
-//   |score32 - score64| <= E_i = 1.002 u ((d + 3) ||x_i|| Cmax + 2 Hmax) + floor
+//   |score32 - score64| <= E_ij = 1.002 u ((d + 3) ||x_i|| ||c_j|| + 2 |hn_j|) + floor
 // (d + 2 roundings of the products and operands, one of the subtraction, one of
 // the half norm; the factor also covers the reference's own float64 rounding),
-// floor for subnormal operands and products.  A sample whose best score is more
-// than 2 E_i below the second best has the same winner in float64; any other
-// (also every NaN or infinite bound) is evaluated in float64 by its warp.
+// floor for subnormal operands and products.  With the maxima over j of the
+// norms this is a bound per sample.
+//
+// One centroid far from all others would spoil it for every sample.  Centroids
+// beyond `reach` (8 harmonic means of the norms) whose half norm is at least
+// 0.49 ||c_j||^2 are left out of the maxima for samples with ||x_i|| <= reach / 4:
+// their ||x_i|| ||c_j|| <= ||c_j||^2 / 4, so their scores are at least
+// 0.24 ||c_j||^2 and E_ij <= u (1.05 d + 7.3) score_ij, a relative error.
+//
+// A sample whose second best score exceeds its best by more than
+//   2 E_i + u (1.06 d + 8) (|best| + |second|)
+// has the same winner in float64; any other (also every NaN or infinite bound)
+// is evaluated in float64 by its warp.
 struct Bound {
-    float slope, base;  // E_i = slope ||x_i|| + base
+    float slope, base;            // E_i = slope ||x_i|| + base, centroids within reach
+    float slope_all, base_all;    // all centroids
+    float reach4, rel;            // reach / 4, u (1.06 d + 8)
 };
 
 // Samples (of the panel) and centroids (of the column block) of a thread.
@@ -181,7 +193,7 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
     int *labs = reinterpret_cast<int *>(smem + L.labs) + (idle ? 0 : warp) * kRows;
 
     float sigma = 1.f;
-    Bound bound{0.f, 0.f};
+    Bound bound{};
     auto block_max = [&](float v) {
         for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
         __syncthreads();
@@ -200,24 +212,56 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
         m = block_max(m);
         const int sh = min(100, max(-100, 10 - ((int)(__float_as_uint(m) >> 23) - 127)));
         if (m > 0.f && m < pos_inf<float>()) sigma = __uint_as_float((unsigned)(127 + sh) << 23);
-        float c2 = 0.f, h = 0.f;
-        for (int64_t j = tid; j < k; j += blockDim.x) {
+        // Norms twice: first the reach, then the maxima.  A float32 sum of
+        // squares is within (1 + u)^(d + 1) of the exact one.
+        auto norm = [&](int64_t j) {
             float q = 0.f;
             for (int f = 0; f < d; ++f) {
                 const float v = (float)a.C[(int64_t)f * k + j] * sigma;
                 q = __fmaf_rn(v, v, q);
             }
-            c2 = fmaxf(c2, q);
-            h = fmaxf(h, fabsf((float)((double)a.hn[j] * ((double)sigma * (double)sigma))));
+            return __fsqrt_rn(q);
+        };
+        float inv = 0.f;
+        for (int64_t j = tid; j < k; j += blockDim.x) inv += 1.f / norm(j);
+        for (int o = 16; o > 0; o >>= 1) inv += __shfl_xor_sync(0xffffffffu, inv, o);
+        __syncthreads();
+        if (lane == 0) red_sh[warp] = inv;
+        __syncthreads();
+        inv = 0.f;
+        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) inv += red_sh[q];
+        const float reach = 8.f * (float)k / inv;  // 0 when a norm is
+        float cn = 0.f, hn = 0.f, ca = 0.f, ha = 0.f, out_of_reach = 0.f;
+        for (int64_t j = tid; j < k; j += blockDim.x) {
+            const float c = norm(j);
+            const float h = (float)((double)a.hn[j] * ((double)sigma * (double)sigma));
+            ca = fmaxf(ca, c);
+            ha = fmaxf(ha, fabsf(h));
+            const bool far = c * (1.f - 0x1p-12f) > reach && h >= 0.4905f * c * c;
+            if (far) {
+                out_of_reach = 1.f;
+            } else {
+                cn = fmaxf(cn, c);
+                hn = fmaxf(hn, fabsf(h));
+            }
         }
-        c2 = block_max(c2);
-        h = block_max(h);
-        // a float32 sum of squares is within (1 + u)^(d + 1) of the exact one
-        const float cmax = __fadd_ru(__fsqrt_ru(__fmul_ru(c2, 1.f + 0x1p-14f)), 0x1p-60f);
+        out_of_reach = block_max(out_of_reach);
+        cn = block_max(cn);
+        hn = block_max(hn);
+        ca = block_max(ca);
+        ha = block_max(ha);
         const float tiny = sigma * 0x1p-145f;  // 16 sigma 2^-149: subnormal operands
-        bound.slope = __fadd_ru(__fmul_ru(1.002f * 0x1p-24f * (float)(d + 3), cmax), tiny);
-        bound.base = __fadd_ru(__fmul_ru(1.002f * 0x1p-23f, h),
-                               __fadd_ru(__fmul_ru(tiny, cmax), 0x1p-120f));
+        auto slope = [&](float c) {
+            c = __fadd_ru(__fmul_ru(c, 1.f + 0x1p-14f), 0x1p-60f);
+            return __fadd_ru(__fmul_ru(1.002f * 0x1p-24f * (float)(d + 3), c), tiny);
+        };
+        const float floor0 = __fadd_ru(__fmul_ru(tiny, __fmul_ru(ca, 1.01f)), 0x1p-120f);
+        bound.slope = slope(cn);
+        bound.base = __fadd_ru(__fmul_ru(1.002f * 0x1p-23f, hn), floor0);
+        bound.slope_all = slope(ca);
+        bound.base_all = __fadd_ru(__fmul_ru(1.002f * 0x1p-23f, ha), floor0);
+        bound.reach4 = 0.25f * reach;
+        bound.rel = out_of_reach > 0.f ? (1.06f * (float)d + 8.f) * 0x1p-24f : 0.f;
     }
 
     // Columns j0 .. j0 + kp - 1 (zero beyond k), in blocks of BN columns
@@ -395,8 +439,14 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
                 q = __fmaf_rn(v, v, q);
             }
             const float nx = __fadd_ru(__fsqrt_ru(__fmul_ru(q, 1.f + 0x1p-14f)), 0x1p-60f);
-            const float e2 = 2.f * __fadd_ru(__fmul_ru(nx, bound.slope), bound.base);
-            const bool sure = __fsub_rd(second[0], best[0]) > e2;
+            const bool near = nx <= bound.reach4;
+            const float e = near ? __fadd_ru(__fmul_ru(nx, bound.slope), bound.base)
+                                 : __fadd_ru(__fmul_ru(nx, bound.slope_all), bound.base_all);
+            float need = 2.f * e;
+            if (bound.rel > 0.f)
+                need = __fadd_ru(
+                    need, __fmul_ru(bound.rel, __fadd_ru(fabsf(best[0]), fabsf(second[0]))));
+            const bool sure = __fsub_rd(second[0], best[0]) > need;
             unsigned todo = __ballot_sync(0xffffffffu, !sure && i0 + row < n);
             while (todo != 0u) {
                 // one undecided sample at a time, the warp's lanes over its centroids

@@ -11,8 +11,9 @@
 // other lane touches: no atomics, no barriers, and the samples of a copy are
 // added in ascending order.  A warp's next 32 samples are copied in
 // asynchronously while it adds the current ones.  The copies of a CTA are
-// added in order into the CTA's copy in global memory.  2M x 14, k = 127: the
-// sums took most of 12.2 ms when one thread owned each cluster; 0.1 ms here.
+// added in order into the CTA's copy in global memory.  An iteration of 2M x 14,
+// k = 127 took 12.2 ms when the float64 tiles also added the sums, one thread
+// owning each cluster; labels and sums together take 0.5 ms now.
 #include <algorithm>
 
 #include "km_reg.cuh"
@@ -93,15 +94,29 @@ __global__ void __launch_bounds__(32 * kSumsWarps, 1)
         __syncwarp();
         const double *st = stage + (size_t)b * stage_doubles(d);
         const I *lb = lab + 32 * b;
-        // samples past n were staged as zeros with label 0: they add nothing
-        for (int q = 0; q < 32 / kUnits; ++q) {
-            const int s = half * 16 + q;
-            const double wv = st[d * kPitch + s];
-            double *row = mine + (int64_t)lb[s] * ds;
-            for (int f = f0; f < ds; f += HALF ? 16 : 32) {
-                double v = st[f * kPitch + s];
-                if (f < d && wv != 1.0) v = __dmul_rn(v, wv);  // rounded, as the reference
-                row[f] += v;
+        // Samples past n were staged as zeros with label 0: they add nothing.
+        // The next sample's operands are read ahead of this one's update; a
+        // weight of one is recognised by its bits (a float64 compare would
+        // cost as much as the addition).
+        constexpr int kStep = HALF ? 16 : 32, kMine = 32 / kUnits;
+        const int s0 = half * 16;
+        for (int f = f0; f < ds; f += kStep) {
+            const double *xf = st + f * kPitch + s0, *wf = st + d * kPitch + s0;
+            int64_t lab_n = lb[s0];
+            double x_n = xf[0], w_n = wf[0];
+#pragma unroll 4
+            for (int q = 0; q < kMine; ++q) {
+                double *to = mine + lab_n * ds + f;
+                const double wv = w_n;
+                double v = x_n;
+                if (q + 1 < kMine) {
+                    lab_n = lb[s0 + q + 1];
+                    x_n = xf[q + 1];
+                    w_n = wf[q + 1];
+                }
+                if (f < d && __double_as_longlong(wv) != 0x3ff0000000000000ll)
+                    v = __dmul_rn(v, wv);  // rounded, as the reference
+                *to += v;
             }
         }
         __syncwarp();  // the buffer is refilled two tiles later
