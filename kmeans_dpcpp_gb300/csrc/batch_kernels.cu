@@ -2,9 +2,8 @@
 // synthetic-data generator used by the serving loop, and the tile autotuner.
 //
 // Per engine step (every active instance advances one Lloyd iteration):
-//   batch_prep    one CTA per instance: half norms of its centroids
-//                 (src/util_kernels.hpp:47-82 order), zeroed float64 sums,
-//                 reset work-queue counters
+//   batch_prep    half norms of the centroids (src/util_kernels.hpp:47-82
+//                 order), reset work-queue counters
 //   batch_panel   persistent CTAs pop (instance, run of 128-sample tiles)
 //                 items from a device work queue and walk them in panels of 32
 //                 samples per warp (km_panel.cuh).  Each (sample, centroid)
@@ -17,12 +16,11 @@
 //                 autotuner picks one per (d, k)
 //   batch_assign  the same for instances of more features than a panel takes,
 //                 in 128-sample tiles (centroid windows of 32, 64 or 128)
-//   batch_reduce  one CTA per fitting instance: sums rounded once to float32,
-//                 sizes, ascending empty-cluster list
-//                 (src/util_kernels.hpp:87-161)
-//   batch_update  one CTA per fitting instance: divide, per-cluster shifts,
-//                 float64 total, the driver's stop rule
-//                 (src/kmeans_lloyd_driver.hpp:317-353), copy-back
+//   batch_reduce  sums rounded once to float32, sizes, ascending empty-cluster
+//                 list (src/util_kernels.hpp:87-161), the copies zeroed again
+//   batch_update  divide, per-cluster shifts, float64 total, the driver's stop
+//                 rule (src/kmeans_lloyd_driver.hpp:317-353), copy-back
+//                 (several CTAs per fitting instance in both)
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -36,6 +34,7 @@
 
 #include "km_batch.cuh"
 #include "km_panel_kernel.cuh"
+#include "km_step.cuh"
 
 namespace kmc {
 
@@ -47,40 +46,32 @@ constexpr int kTM = 8;
 constexpr size_t kPrivBytes = 72 * 1024;  // with the tiles: two CTAs per SM
 constexpr int kSumCopies = 48;            // global copies of small instances' sums
 
-// Deterministic block-wide float64 sum (same shape as the single-fit loop
-// control: warp shuffles, then warp 0 over the warp totals).
-__device__ double block_sum_b(double v, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (wid == 0) {
-        r = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-    }
-    __syncthreads();
-    return r;  // valid in thread 0
-}
+constexpr int kPrepThreads = 128;
 
-__global__ void batch_prep_kernel(BInst *tab, const int *idx, int count, int *counters) {
-    if (blockIdx.x == 0 && threadIdx.x < kBatchCounters) counters[threadIdx.x] = 0;
-    if ((int)blockIdx.x >= count) return;
-    BInst &in = tab[idx[blockIdx.x]];
-    const int d = in.d, k = in.k;
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-        float acc = 0.f;
-        for (int f = 0; f < d; ++f) {
-            const float v = in.C[(int64_t)f * k + j];
-            acc = __fmaf_rn(v, v, acc);
-        }
-        in.hn[j] = acc / 2.f;
+// Half norms, a thread per cluster (gridDim.x CTAs per instance).
+__global__ void __launch_bounds__(kPrepThreads)
+    batch_prep_kernel(BInst *tab, const int *idx, int count, int *counters) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kBatchCounters)
+        counters[threadIdx.x] = 0;
+    if ((int)blockIdx.y >= count) return;
+    BInst &in = tab[idx[blockIdx.y]];
+    const int d = in.d, k = in.k, j = blockIdx.x * kPrepThreads + threadIdx.x;
+    if (j >= k) return;
+    const float *C = in.C + j;
+    float acc = 0.f;
+    int f = 0;
+    for (; f + 8 <= d; f += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = C[(int64_t)(f + u) * k];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc = __fmaf_rn(v[u], v[u], acc);
     }
-    if (in.mode == B_FIT) {
-        const int64_t total = ((int64_t)d * k + k) * in.copies;
-        for (int64_t e = threadIdx.x; e < total; e += blockDim.x) in.sums[e] = 0.0;
-        if (threadIdx.x == 0) in.empty_list[k] = 0;
+    for (; f < d; ++f) {
+        const float v = C[(int64_t)f * k];
+        acc = __fmaf_rn(v, v, acc);
     }
+    in.hn[j] = acc / 2.f;
 }
 
 template <int HN>
@@ -349,91 +340,157 @@ __global__ void __launch_bounds__(32 * panel::kMaxWarps, 1)
     }
 }
 
-__global__ void batch_reduce_kernel(BInst *tab, const int *idx, int count, int *n_empty_out) {
-    if ((int)blockIdx.x >= count) return;
-    BInst &in = tab[idx[blockIdx.x]];
-    const int d = in.d, k = in.k;
-    const int64_t dk = (int64_t)d * k;
-    for (int64_t e = threadIdx.x; e < dk + k; e += blockDim.x) {
-        // copies added in index order; loads issued eight ahead of the adds
-        const double *src = in.sums + e;
-        double s = 0.0;
-        int c = 0;
-        for (; c + 8 <= in.copies; c += 8) {
-            double v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(c + u) * (dk + k)];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s += v[u];
-        }
-        for (; c < in.copies; ++c) s += src[(int64_t)c * (dk + k)];
-        if (e < dk)
-            in.Cn[e] = (float)s;
-        else
-            in.sizes[e - dk] = (float)s;
+// True in the CTA of an instance (gridDim.x of them) that finishes last.
+__device__ __forceinline__ bool last_of_instance(unsigned *ticket) {
+    __shared__ int last_sh;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last_sh = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+        if (last_sh) *ticket = 0u;
     }
     __syncthreads();
-    // ascending empty-cluster list
+    if (last_sh) __threadfence();
+    return last_sh != 0;
+}
+
+// Private copies -> float32 sums and sizes, the copies zeroed once read, and
+// the ascending empty-cluster list.  An instance gets gridDim.x CTAs; a CTA
+// takes 32 elements at a time, their copies shared by 16 threads (as in
+// reduce_sums_kernel).  One CTA per instance left most SMs idle and walked the
+// copies one latency after another: 124 us for 24 instances.
+constexpr int kBatchReduceThreads = kReduceLanes * kReduceGroups;
+
+__global__ void __launch_bounds__(kBatchReduceThreads)
+    batch_reduce_kernel(BInst *tab, const int *idx, int count, int *n_empty_out) {
+    if ((int)blockIdx.y >= count) return;
+    __shared__ double red[kReduceGroups][kReduceLanes];
     __shared__ int warp_counts[32];
-    __shared__ int base_sh;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    if (threadIdx.x == 0) base_sh = 0;
-    __syncthreads();
-    for (int j0 = 0; j0 < k; j0 += blockDim.x) {
+    BInst &in = tab[idx[blockIdx.y]];
+    const int d = in.d, k = in.k;
+    const int64_t dk = (int64_t)d * k, total = dk + k;
+    const int el = threadIdx.x % kReduceLanes, g = threadIdx.x / kReduceLanes;
+    if (in.copies == 1) {
+        for (int64_t e = blockIdx.x * (int64_t)kBatchReduceThreads + threadIdx.x; e < total;
+             e += (int64_t)gridDim.x * kBatchReduceThreads) {
+            const float v = (float)in.sums[e];
+            in.sums[e] = 0.0;
+            if (e < dk)
+                in.Cn[e] = v;
+            else
+                in.sizes[e - dk] = v;
+        }
+    } else {
+        for (int64_t e0 = blockIdx.x * (int64_t)kReduceLanes; e0 < total;
+             e0 += (int64_t)gridDim.x * kReduceLanes) {
+            const int64_t e = e0 + el;
+            double acc = 0.0;
+            if (e < total) {
+                for (int c = g; c < in.copies; c += 4 * kReduceGroups) {
+                    double v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        v[u] = c + u * kReduceGroups < in.copies
+                                   ? in.sums[(int64_t)(c + u * kReduceGroups) * total + e]
+                                   : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (c + u * kReduceGroups < in.copies) {
+                            in.sums[(int64_t)(c + u * kReduceGroups) * total + e] = 0.0;
+                            acc += v[u];
+                        }
+                }
+            }
+            red[g][el] = acc;
+            __syncthreads();
+            if (g == 0 && e < total) {
+#pragma unroll
+                for (int q = 1; q < kReduceGroups; ++q) acc += red[q][el];
+                if (e < dk)
+                    in.Cn[e] = (float)acc;
+                else
+                    in.sizes[e - dk] = (float)acc;
+            }
+            __syncthreads();
+        }
+    }
+    if (!last_of_instance(&in.tickets[0])) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = kBatchReduceThreads / 32;
+    int base = 0;
+    for (int j0 = 0; j0 < k; j0 += kBatchReduceThreads) {
         const int j = j0 + threadIdx.x;
-        const bool empty = (j < k) && (in.sizes[j] == 0.f);
+        const bool empty = (j < k) && (__ldcg(in.sizes + j) == 0.f);
         const unsigned ballot = __ballot_sync(0xffffffffu, empty);
         if (lane == 0) warp_counts[wid] = __popc(ballot);
         __syncthreads();
-        int before = 0, total = 0;
+        int before = 0, all = 0;
         for (int q = 0; q < nwarps; ++q) {
             if (q < wid) before += warp_counts[q];
-            total += warp_counts[q];
+            all += warp_counts[q];
         }
-        if (empty) {
-            const int pos = base_sh + before + __popc(ballot & ((1u << lane) - 1u));
-            if (pos >= 0 && pos < k) in.empty_list[pos] = j;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) base_sh += total;
+        if (empty) in.empty_list[base + before + __popc(ballot & ((1u << lane) - 1u))] = j;
+        base += all;
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        in.empty_list[k] = base_sh;
-        n_empty_out[blockIdx.x] = base_sh;
+        in.empty_list[k] = base;
+        in.n_empty = base;
+        n_empty_out[blockIdx.y] = base;
     }
 }
 
-__global__ void batch_update_kernel(BInst *tab, const int *idx, int count, int *done_out) {
-    if ((int)blockIdx.x >= count) return;
-    BInst &in = tab[idx[blockIdx.x]];
+// Division, shifts (kept in hn, which the next step recomputes) and, in the
+// instance's last CTA, the driver's stop rule.  A CTA takes 32 clusters.
+__global__ void __launch_bounds__(kFinishThreads)
+    batch_update_kernel(BInst *tab, const int *idx, int count, int *done_out, int relocated) {
+    if ((int)blockIdx.y >= count) return;
+    BInst &in = tab[idx[blockIdx.y]];
+    if (!relocated && in.n_empty != 0) return;  // the host relocates first
+    __shared__ float diff_sh[kFinishElems];
     __shared__ double sh[32];
-    const int d = in.d, k = in.k;
-    double part = 0.0;
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-        const float sz = in.sizes[j];
-        float acc = 0.f;
-        for (int f = 0; f < d; ++f) {
-            const int64_t e = (int64_t)f * k + j;
-            const float c = in.Cn[e] / sz;
-            in.Cn[e] = c;
-            const float diff = in.C[e] - c;
-            acc = __fmaf_rn(diff, diff, acc);
+    constexpr int kClusters = 32, kFeatures = kFinishElems / kClusters;
+    const int d = in.d, k = in.k, tid = threadIdx.x;
+    for (int j0 = blockIdx.x * kClusters; j0 < k; j0 += gridDim.x * kClusters) {
+        const int j = j0 + (tid & 31);
+        const float size = j < k ? in.sizes[j] : 1.f;
+        float shift = 0.f;
+        for (int f0 = 0; f0 < d; f0 += kFeatures) {
+            float s[kFinishOwn], old[kFinishOwn];
+#pragma unroll
+            for (int u = 0; u < kFinishOwn; ++u) {
+                const int f = f0 + (tid >> 5) + u * (kFinishThreads / 32);
+                s[u] = old[u] = 0.f;
+                if (f < d && j < k) {
+                    s[u] = in.Cn[(int64_t)f * k + j];
+                    old[u] = in.C[(int64_t)f * k + j];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kFinishOwn; ++u) {
+                const int fl = (tid >> 5) + u * (kFinishThreads / 32), f = f0 + fl;
+                if (f < d && j < k) {
+                    const float c = s[u] / size;
+                    in.Cn[(int64_t)f * k + j] = c;
+                    in.C[(int64_t)f * k + j] = c;
+                    diff_sh[fl * kClusters + (tid & 31)] = old[u] - c;
+                }
+            }
+            __syncthreads();
+            if (tid < 32 && j < k) {
+                const int fn = d - f0 < kFeatures ? d - f0 : kFeatures;
+#pragma unroll 8
+                for (int fl = 0; fl < fn; ++fl) {
+                    const float v = diff_sh[fl * kClusters + tid];
+                    shift = __fmaf_rn(v, v, shift);
+                }
+            }
+            __syncthreads();
         }
-        part += (double)acc;
+        if (tid < 32 && j < k) in.hn[j] = shift;
     }
-    const double tot = block_sum_b(part, sh);
-    if (threadIdx.x == 0) {
-        in.st.last_shift = tot;
-        in.st.n_iter += 1;
-        const float shift_t = (float)tot;
-        const float tol_t = (float)in.st.tol;
-        const bool go_on = (in.st.n_iter < in.st.max_iter) && (shift_t > tol_t);
-        if (!go_on) in.st.done = 1;
-        done_out[blockIdx.x] = in.st.done;
-    }
-    __syncthreads();
-    for (int64_t e = threadIdx.x; e < (int64_t)d * k; e += blockDim.x) in.C[e] = in.Cn[e];
+    if (!last_of_instance(&in.tickets[1])) return;
+    stop_rule<float>(in.hn, k, &in.st, sh);
+    if (tid == 0) done_out[blockIdx.y] = in.st.done;
 }
 
 // SplitMix64 output function (S. Vigna, public domain).
@@ -593,8 +650,11 @@ int batch_sum_copies(int64_t d, int64_t k) {
     return ((d + 1) * k * (int64_t)sizeof(double) <= (int64_t)kPrivBytes) ? kSumCopies : 1;
 }
 
-int launch_batch_prep(BInst *tab, const int *idx, int count, int *counters, cudaStream_t s) {
-    batch_prep_kernel<<<count > 0 ? count : 1, 256, 0, s>>>(tab, idx, count, counters);
+int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int *counters,
+                      cudaStream_t s) {
+    const dim3 grid((unsigned)std::max<int64_t>(1, ceil_div<int64_t>(max_k, kPrepThreads)),
+                    (unsigned)std::max(count, 1));
+    batch_prep_kernel<<<grid, kPrepThreads, 0, s>>>(tab, idx, count, counters);
     return check_launch("batch_prep");
 }
 
@@ -641,16 +701,28 @@ int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, co
     return launch_assign_v<8, 0>(2, tab, items, n_items, counter, s);
 }
 
-int launch_batch_reduce(BInst *tab, const int *idx, int count, int *n_empty_out,
-                        cudaStream_t s) {
+namespace {
+// CTAs per instance: enough for the largest, together about four per SM.
+unsigned ctas_per_instance(int64_t most, int count) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, 4 * (int64_t)num_sms() / count));
+}
+}  // namespace
+
+int launch_batch_reduce(BInst *tab, const int *idx, int count, int64_t max_elems,
+                        int *n_empty_out, cudaStream_t s) {
     if (count <= 0) return KMC_OK;
-    batch_reduce_kernel<<<count, 1024, 0, s>>>(tab, idx, count, n_empty_out);
+    const dim3 grid(ctas_per_instance(ceil_div<int64_t>(max_elems, 2 * kReduceLanes), count),
+                    (unsigned)count);
+    batch_reduce_kernel<<<grid, kBatchReduceThreads, 0, s>>>(tab, idx, count, n_empty_out);
     return check_launch("batch_reduce");
 }
 
-int launch_batch_update(BInst *tab, const int *idx, int count, int *done_out, cudaStream_t s) {
+int launch_batch_update(BInst *tab, const int *idx, int count, int64_t max_k, int *done_out,
+                        bool relocated, cudaStream_t s) {
     if (count <= 0) return KMC_OK;
-    batch_update_kernel<<<count, 1024, 0, s>>>(tab, idx, count, done_out);
+    const dim3 grid(ctas_per_instance(ceil_div<int64_t>(max_k, 32), count), (unsigned)count);
+    batch_update_kernel<<<grid, kFinishThreads, 0, s>>>(tab, idx, count, done_out,
+                                                        relocated ? 1 : 0);
     return check_launch("batch_update");
 }
 

@@ -33,6 +33,8 @@ struct BInst {
     int mode;              // B_FIT or B_ASSIGN
     int variant;           // centroid columns per step: 0 -> 16, 1 -> 32, 2 -> 64 (panels)
     int copies;            // private copies of sums (CTA b adds into copy b % copies)
+    int n_empty;           // empty clusters of this step
+    unsigned tickets[2];   // CTAs of batch_reduce / batch_update that are through
     LoopState st;          // done / n_iter / max_iter / tol / last_shift
 };
 
@@ -53,7 +55,8 @@ constexpr int kBatchCounters = 4 * kBatchVariants;
 int batch_sum_copies(int64_t d, int64_t k);
 
 // ---- launchers (batch.cu) ----
-int launch_batch_prep(BInst *tab, const int *idx, int count, int *counters, cudaStream_t s);
+int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int *counters,
+                      cudaStream_t s);
 // Sets the assign kernels' shared-memory attributes (outside graph capture).
 int prepare_batch_assign();
 // dist != 0: the transform kernel (items of B_TRANSFORM instances only).
@@ -62,9 +65,14 @@ int prepare_batch_assign();
 bool batch_in_panels(int64_t d, int dist);
 int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, const BItem *items,
                         int n_items, int *counter, cudaStream_t s);
-int launch_batch_reduce(BInst *tab, const int *idx, int count, int *n_empty_out,
-                        cudaStream_t s);
-int launch_batch_update(BInst *tab, const int *idx, int count, int *done_out, cudaStream_t s);
+// Copies -> sums, sizes and empty-cluster lists of the fits idx; max_elems,
+// max_k: the largest (d + 1) k and k among them.
+int launch_batch_reduce(BInst *tab, const int *idx, int count, int64_t max_elems,
+                        int *n_empty_out, cudaStream_t s);
+// Division, shifts and stop rule; fits with empty clusters are left alone
+// unless `relocated`.
+int launch_batch_update(BInst *tab, const int *idx, int count, int64_t max_k, int *done_out,
+                        bool relocated, cudaStream_t s);
 int launch_blobs(float *X, int64_t n, int64_t d, int64_t n_centers, float box_lo,
                  float box_hi, float std_lo, float std_hi, uint64_t seed, cudaStream_t s);
 int launch_gather_rows(const float *X, int64_t n, int64_t d, const int32_t *idx, int64_t k,

@@ -2,19 +2,19 @@
 // with their extern "C" entry points (include/kmeans_gb300.h).
 //
 // BatchEngine::step() advances every running instance by one iteration:
-//   graph A   batch_prep -> batch_assign (one launch per centroid-window
-//             variant in use, all fed from the device work queue) ->
-//             batch_reduce
-//   host      reads the empty-cluster counts of the fitting instances; those
-//             with empty clusters run the single-fit relocation chain
-//             (kmeans_lloyd_driver.hpp:217-312) on their own buffers
-//   graph B   batch_update (divide, shifts, stop rule, copy-back)
-//   host      reads the stop flags; finished fits get the driver's final pass
-//             (half norms, assignment, weighted inertia, float64 total,
-//             kmeans_lloyd_driver.hpp:360-418); predictions finish after
-//             their assignment
-// The two graphs are captured once per set of running instances and replayed
-// until an instance joins or leaves.
+//   graph     batch_prep -> batch_panel / batch_assign (one launch per
+//             centroid-window variant in use, all fed from the device work
+//             queue) -> batch_reduce -> batch_update (divide, shifts, stop
+//             rule, copy-back; instances with empty clusters are left alone)
+//   host      reads the empty-cluster counts and stop flags of the fitting
+//             instances; those with empty clusters run the relocation chain
+//             (kmeans_lloyd_driver.hpp:217-312) on their own buffers and then
+//             batch_update; finished fits get the driver's final pass (half
+//             norms, assignment, weighted inertia, float64 total,
+//             kmeans_lloyd_driver.hpp:360-418), side by side on three
+//             streams; predictions finish after their assignment
+// The graph is captured once per set of running instances and replayed until
+// an instance joins or leaves.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -137,16 +137,22 @@ struct BatchEngine {
     int n_items[2][kBatchVariants] = {{0, 0, 0}, {0, 0, 0}};
     int64_t item_off[2][kBatchVariants] = {{0, 0, 0}, {0, 0, 0}};
     bool dirty = true;
-    GraphExec gA, gB;
+    GraphExec graph;
+    int64_t max_k = 1, max_elems = 1;  // over the fitting instances
+    Scratch list_mem;                  // instances to update after a relocation
     int *host_i = nullptr;  // pinned: empty counts then done flags
+    LoopState *host_st = nullptr;  // pinned, per instance: final loop state
+    double *host_tot = nullptr;    // and inertia
     int64_t steps = 0, graph_builds = 0, relocations = 0;
 
     ~BatchEngine() {
         if (s) cudaStreamSynchronize(s);
         if (host_i) cudaFreeHost(host_i);
+        if (host_st) cudaFreeHost(host_st);
+        if (host_tot) cudaFreeHost(host_tot);
         // device memory is released (stream-ordered) before the stream goes
-        gA.reset();
-        gB.reset();
+        graph.reset();
+        list_mem.release();
         mem.clear();
         items_mem.release();
         dev.release();
@@ -190,6 +196,9 @@ struct BatchEngine {
         nempty_d = reinterpret_cast<int *>(b + o_ne);
         done_d = reinterpret_cast<int *>(b + o_dn);
         KMC_CUDA_TRY(cudaMallocHost(&host_i, sizeof(int) * 2 * cap));
+        KMC_CUDA_TRY(cudaMallocHost(&host_st, sizeof(LoopState) * cap));
+        KMC_CUDA_TRY(cudaMallocHost(&host_tot, sizeof(double) * cap));
+        KMC_TRY(list_mem.alloc(sizeof(int) * cap, s));
         tab.assign((size_t)cap, BInst{});
         state.assign((size_t)cap, FREE);
         mem.resize((size_t)cap);
@@ -243,6 +252,9 @@ struct BatchEngine {
         h.sizes = m->sizes;
         h.sums = m->sums;
         h.copies = mode == B_FIT ? batch_sum_copies(d, k) : 1;
+        // each step's reduction leaves the sums at zero again
+        if (mode == B_FIT)
+            KMC_CUDA_TRY(cudaMemsetAsync(m->sums, 0, sizeof(double) * (d * k + k) * h.copies, s));
         h.labels = labels;
         h.dist = dist;
         h.empty_list = m->empty_list;
@@ -265,7 +277,7 @@ struct BatchEngine {
         KMC_TRY(upload(q));
         dirty = true;
         *out = q;
-        if (h.st.done) KMC_TRY(finish_fit(q));
+        if (h.st.done) KMC_TRY(finish_fits({(int)q}));
         return KMC_OK;
     }
 
@@ -288,13 +300,20 @@ struct BatchEngine {
     int plan() {
         all.clear();
         fits.clear();
+        max_k = max_elems = 1;
+        int64_t all_k = 1;
         std::vector<BItem> items[2][kBatchVariants];
         bool use[2][2][kBatchVariants] = {};  // [panels][kind][variant]
         for (int64_t q = 0; q < cap; ++q) {
             if (state[(size_t)q] != RUNNING) continue;
             const BInst &h = tab[(size_t)q];
             all.push_back((int)q);
-            if (h.mode == B_FIT) fits.push_back((int)q);
+            all_k = std::max<int64_t>(all_k, h.k);
+            if (h.mode == B_FIT) {
+                fits.push_back((int)q);
+                max_k = std::max<int64_t>(max_k, h.k);
+                max_elems = std::max<int64_t>(max_elems, ((int64_t)h.d + 1) * h.k);
+            }
             append_items((int)q, h.n, h.mode, h.variant, items);
             const int kind = h.mode == B_TRANSFORM ? 1 : 0;
             use[batch_in_panels(h.d, kind) ? 1 : 0][kind][h.variant] = true;
@@ -327,8 +346,8 @@ struct BatchEngine {
         KMC_CUDA_TRY(cudaStreamSynchronize(s));
         // kernel attributes are set outside the capture
         KMC_TRY(prepare_batch_assign());
-        KMC_TRY(capture(&gA, [&]() -> int {
-            KMC_TRY(launch_batch_prep(tab_d, all_d, (int)all.size(), counters_d, s));
+        KMC_TRY(capture(&graph, [&]() -> int {
+            KMC_TRY(launch_batch_prep(tab_d, all_d, (int)all.size(), all_k, counters_d, s));
             KMC_CUDA_TRY(cudaEventRecord(ev_fork, s));
             // one branch per centroid-window variant: its assignment items,
             // then its transform items
@@ -345,10 +364,8 @@ struct BatchEngine {
                 KMC_CUDA_TRY(cudaEventRecord(ev_join[v], side[v]));
                 KMC_CUDA_TRY(cudaStreamWaitEvent(s, ev_join[v], 0));
             }
-            return launch_batch_reduce(tab_d, fit_d, (int)fits.size(), nempty_d, s);
-        }));
-        KMC_TRY(capture(&gB, [&]() -> int {
-            return launch_batch_update(tab_d, fit_d, (int)fits.size(), done_d, s);
+            KMC_TRY(launch_batch_reduce(tab_d, fit_d, (int)fits.size(), max_elems, nempty_d, s));
+            return launch_batch_update(tab_d, fit_d, (int)fits.size(), max_k, done_d, false, s);
         }));
         ++graph_builds;
         dirty = false;
@@ -393,23 +410,37 @@ struct BatchEngine {
     }
 
     // kmeans_lloyd_driver.hpp:360-418: labels and weighted inertia against
-    // the final centroids.
-    int finish_fit(int64_t q) {
-        const BInst &h = tab[(size_t)q];
-        SlotMem &sm = *mem[(size_t)q];
-        KMC_TRY(launch_half_norm<float>(h.C, sm.hn, h.d, h.k, s));
-        KMC_TRY(launch_assignment<float, int32_t>(h.X, h.C, sm.hn, h.labels, h.n, h.d, h.k, s));
-        KMC_TRY(launch_inertia<float, int32_t>(h.X, h.w, h.C, h.labels, sm.sq_dist, h.n, h.d,
-                                               h.k, s));
-        KMC_TRY(launch_sum_f64<float>(sm.sq_dist, h.n, sm.partials, sm.dsum, s));
-        LoopState st{};
-        double tot = 0.0;
-        KMC_CUDA_TRY(cudaMemcpyAsync(&st, &tab_d[q].st, sizeof(st), cudaMemcpyDeviceToHost, s));
-        KMC_CUDA_TRY(cudaMemcpyAsync(&tot, sm.dsum, sizeof(double), cudaMemcpyDeviceToHost, s));
+    // the final centroids.  The fits run side by side on the side streams.
+    int finish_fits(const std::vector<int> &done) {
+        if (done.empty()) return KMC_OK;
+        const int streams = (int)std::min<size_t>(kBatchVariants, done.size());
+        KMC_CUDA_TRY(cudaEventRecord(ev_fork, s));
+        for (int v = 0; v < streams; ++v) KMC_CUDA_TRY(cudaStreamWaitEvent(side[v], ev_fork, 0));
+        for (size_t t = 0; t < done.size(); ++t) {
+            const int q = done[t];
+            const BInst &h = tab[(size_t)q];
+            SlotMem &sm = *mem[(size_t)q];
+            cudaStream_t st = side[t % (size_t)streams];
+            KMC_TRY(launch_half_norm<float>(h.C, sm.hn, h.d, h.k, st));
+            KMC_TRY(launch_assignment<float, int32_t>(h.X, h.C, sm.hn, h.labels, h.n, h.d, h.k, st));
+            KMC_TRY(launch_inertia<float, int32_t>(h.X, h.w, h.C, h.labels, sm.sq_dist, h.n, h.d,
+                                                   h.k, st));
+            KMC_TRY(launch_sum_f64<float>(sm.sq_dist, h.n, sm.partials, sm.dsum, st));
+            KMC_CUDA_TRY(cudaMemcpyAsync(host_st + q, &tab_d[q].st, sizeof(LoopState),
+                                         cudaMemcpyDeviceToHost, st));
+            KMC_CUDA_TRY(cudaMemcpyAsync(host_tot + q, sm.dsum, sizeof(double),
+                                         cudaMemcpyDeviceToHost, st));
+        }
+        for (int v = 0; v < streams; ++v) {
+            KMC_CUDA_TRY(cudaEventRecord(ev_join[v], side[v]));
+            KMC_CUDA_TRY(cudaStreamWaitEvent(s, ev_join[v], 0));
+        }
         KMC_CUDA_TRY(cudaStreamSynchronize(s));
-        res_iter[(size_t)q] = st.n_iter;
-        res_inertia[(size_t)q] = tot;
-        state[(size_t)q] = FINISHED;
+        for (int q : done) {
+            res_iter[(size_t)q] = host_st[q].n_iter;
+            res_inertia[(size_t)q] = host_tot[q];
+            state[(size_t)q] = FINISHED;
+        }
         dirty = true;
         return KMC_OK;
     }
@@ -417,22 +448,38 @@ struct BatchEngine {
     int step(int64_t *n_active) {
         if (dirty) KMC_TRY(plan());
         if (!all.empty()) {
-            KMC_CUDA_TRY(cudaGraphLaunch(gA.exec, s));
+            KMC_CUDA_TRY(cudaGraphLaunch(graph.exec, s));
             const size_t nf = fits.size();
             if (nf > 0) {
                 KMC_CUDA_TRY(cudaMemcpyAsync(host_i, nempty_d, sizeof(int) * nf,
                                              cudaMemcpyDeviceToHost, s));
-                KMC_CUDA_TRY(cudaStreamSynchronize(s));
-                for (size_t t = 0; t < nf; ++t)
-                    if (host_i[t] > 0) KMC_TRY(relocate(fits[t], host_i[t]));
-                KMC_CUDA_TRY(cudaGraphLaunch(gB.exec, s));
                 KMC_CUDA_TRY(cudaMemcpyAsync(host_i + cap, done_d, sizeof(int) * nf,
                                              cudaMemcpyDeviceToHost, s));
             }
             KMC_CUDA_TRY(cudaStreamSynchronize(s));
-            ++steps;
+            // instances with empty clusters: relocation, then their update
+            std::vector<int> moved, slot;
             for (size_t t = 0; t < nf; ++t)
-                if (host_i[cap + t]) KMC_TRY(finish_fit(fits[t]));
+                if (host_i[t] > 0) {
+                    KMC_TRY(relocate(fits[t], host_i[t]));
+                    moved.push_back(fits[t]);
+                    slot.push_back((int)t);
+                }
+            if (!moved.empty()) {
+                KMC_CUDA_TRY(cudaMemcpyAsync(list_mem.ptr, moved.data(), sizeof(int) * moved.size(),
+                                             cudaMemcpyHostToDevice, s));
+                KMC_TRY(launch_batch_update(tab_d, list_mem.as<int>(), (int)moved.size(), max_k,
+                                            done_d, true, s));
+                KMC_CUDA_TRY(cudaMemcpyAsync(host_i, done_d, sizeof(int) * moved.size(),
+                                             cudaMemcpyDeviceToHost, s));
+                KMC_CUDA_TRY(cudaStreamSynchronize(s));
+                for (size_t t = 0; t < moved.size(); ++t) host_i[cap + slot[t]] = host_i[t];
+            }
+            ++steps;
+            std::vector<int> done;
+            for (size_t t = 0; t < nf; ++t)
+                if (host_i[cap + t]) done.push_back(fits[t]);
+            KMC_TRY(finish_fits(done));
             for (int q : all)
                 if (tab[(size_t)q].mode != B_FIT) {
                     state[(size_t)q] = FINISHED;
