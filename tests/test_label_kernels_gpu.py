@@ -161,3 +161,23 @@ def test_fused_step_with_many_and_few_copies(oracle, d, k, copies):
     # sums of multiples of 1/2 below 2^23: exact in float32
     np.testing.assert_array_equal(cc.sum(0).cpu().numpy(), sums_o)
     np.testing.assert_array_equal(sc.sum(0).cpu().numpy(), sizes_o)
+
+
+@pytest.mark.parametrize("copies", [1, 7, 8, 9, 16, 17, 130, 1000])
+@pytest.mark.parametrize("d,k", [(1, 1), (3, 11), (14, 33)])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_copies_of_any_number_are_reduced(copies, d, k, dt):
+    # small integers: exact sums in any order; cluster 0 stays empty
+    import torch
+
+    import kmeans_dpcpp_gb300 as kdp
+
+    rng = np.random.default_rng(copies + d + k)
+    cc, sc = rng.integers(-4, 5, (copies, d, k)).astype(dt), rng.integers(1, 4, (copies, k)).astype(dt)
+    sc[:, 0] = 0
+    out, sizes = _gpu(np.full((d, k), np.nan, dt)), _gpu(np.full(k, np.nan, dt))
+    empty, n_empty = torch.full((k,), -1, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    kdp.reduce_centroids_data(_gpu(sc), _gpu(cc), sizes, out, empty, n_empty, 128, None)[0].wait()
+    np.testing.assert_array_equal(out.cpu().numpy(), cc.sum(0))
+    np.testing.assert_array_equal(sizes.cpu().numpy(), sc.sum(0))
+    assert n_empty.item() == 1 and empty[0].item() == 0
