@@ -59,8 +59,7 @@
 //               when those sums do not fit shared memory,
 //               red.global.add.f64 per feature into the CTA's copy
 // Samples that fail certification are accumulated by the recheck kernel.
-// Waits poll mbarrier.test_wait (no suspension: with tensor-core kernels of
-// several streams at once, suspended waiters sometimes slept for seconds).
+// Waits poll mbarrier.test_wait.
 //
 // Every wait is bounded.  A wait that runs out raises the CTA's error flag;
 // the other roles see it and stop, the producer and the MMA issuer then wait
@@ -976,7 +975,12 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                 }
             }
             const int tb = tl & 1;
-            if (mbar_wait(&uempty[tb], (((uint32_t)tl >> 1) & 1u) ^ 1u, err, lim) && win) {
+            // Only the thread that hands the row over waits: its own arrival is
+            // part of the next phase, so the phase it waits for cannot be
+            // overtaken.  A loser's arrival is not: one that polled late saw
+            // the barrier two phases on, with the parity of the phase it
+            // waited for, and never passed.
+            if (win && mbar_wait(&uempty[tb], (((uint32_t)tl >> 1) & 1u) ^ 1u, err, lim)) {
                 lab_s[tb * kTileM + row] = code;
                 mbar_arrive(&ufull[tb]);
             }

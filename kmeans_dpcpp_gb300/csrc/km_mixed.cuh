@@ -42,13 +42,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
                  : "memory");
 }
 
-// Non-blocking test of the phase with the given parity.  The waits below poll
-// it with a short sleep between polls.  The suspending form
-// (mbarrier.try_wait with a suspend-time hint) is not used: with tensor-core
-// kernels of several streams running at once, a thread suspended in it
-// sometimes stayed asleep for seconds after the phase had completed (fits of
-// the request server gave up their waits after the 2 s limit; with polling
-// none did).
+// Non-blocking test of the phase with the given parity; the waits below poll
+// it.
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -63,8 +58,9 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
 
 // Waits for the phase with the given parity.  Returns false (and raises the
 // CTA error flag) after `limit` SM clocks, or as soon as another role has
-// raised the flag.  After a few polls the waiter sleeps ~0.1 us between
-// polls, so waiting warps leave the issue slots to the working ones.
+// raised the flag.  A thread may wait only for a phase that cannot be followed by
+// another one without its own arrival: two phases on, the parity is the same
+// again and a late poll would never pass.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *err,
                                           long long limit = kWaitClocks) {
     if (mbar_test(bar, parity)) return true;
