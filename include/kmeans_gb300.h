@@ -513,13 +513,12 @@ int kmc_fit_tile_variant(int64_t n_features, int64_t n_clusters, int dtype_bytes
                          kmc_stream_t stream, int *variant_out);
 int kmc_fit_set_tile_variant(kmc_fit_t fit, int variant);
 /* Mixed forms: the session's kernel variant, 10 * ring stages + f, where f = 4
- * or 2 is the fixed-point cluster sums with that many columns per update
- * thread and f = 0 the float reductions (-1 for a plain session).  The
+ * or 2 is the fixed-point cluster sums (up to 32 features) with that many rows
+ * in flight per lane and f = 0 any other (-1 for a plain session).  The
  * autotuner times the variants that fit shared memory on a synthetic fit once
  * per (n_features, power-of-two bucket of n_clusters, form, size class: at
  * least 32 128-sample tiles per SM or fewer), caches the fastest beside the
- * tile choices above (KMC_TUNE=0: the deepest ring with the widest
- * fixed-point sums).  Sessions of the request server use a cached choice or
+ * tile choices above (KMC_TUNE=0: the deepest ring, f = 2).  Sessions of the request server use a cached choice or
  * that default and never time variants on a request's path.  Every variant gives the same labels.
  * kmc_debug_force_mixed_variant forces a variant for the fits created
  * afterwards (a test hook; -1 restores the tuner; a variant that does not fit

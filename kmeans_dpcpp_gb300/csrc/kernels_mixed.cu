@@ -48,22 +48,16 @@
 // -inf (their half norm), so no score needs a test against k.  A pass without
 // sums over 4M x 64: 560 -> 454 us at k = 1024, 443 -> 211 us at k = 64.
 //
-// Kernel roles (one CTA of 384 threads per SM, persistent over 128-sample
-// tiles; 12 warps leave 168 registers per thread, so nothing spills):
+// Kernel roles (one CTA of 320 threads per SM, persistent over 128-sample
+// tiles; 10 warps leave up to 204 registers per thread):
 //   warp 0      bulk copies: the centroid image once, X tiles into a 2-4 stage ring
 //   warp 1      TMEM allocation; one thread issues tcgen05.mma (M=128, N=256,
 //               K=16) into two 256-column TMEM accumulators
-//   warps 2-9   epilogue: tcgen05.ld of score pairs, P1/P2, certification, labels
-//   warps 10-11 update: w*x of certified samples into cluster-major sums.
-//               d > 32: fire-and-forget red.global.add.v4.f32 into the
-//               private copy of this CTA (copy blockIdx % n_copies), summed in
-//               copy order afterwards.  d <= 32: integer (fixed-point) sums
-//               in shared memory from terms packed once per fit, added at the
-//               end into order-independent integer totals (fixed_sums_role);
-//               when those sums do not fit shared memory,
-//               red.global.add.f64 per feature into the CTA's copy
-// Samples that fail certification are accumulated by the recheck kernel.
-// Waits poll mbarrier.test_wait.
+//   warps 2-9   epilogue: tcgen05.ld of scores, P1/P2, certification, labels
+// The recheck kernel labels the samples that were not certified; the cluster
+// sums are a pass of their own over the labels (sum_sorted_kernel).
+// A pass without sums over 4M x 64 (two update warps in the kernel before):
+// 454 -> 416 us at k = 1024, 217 -> 177 us at k = 256, 211 -> 159 us at k = 64.
 //
 // Every wait is bounded.  A wait that runs out raises the CTA's error flag;
 // the other roles see it and stop, the producer and the MMA issuer then wait
@@ -94,10 +88,7 @@ constexpr int kTileM = 128;
 constexpr int kChunkN = 256;
 constexpr uint32_t kNormRowBytes = 32;  // K=16 block holding the half-norm parts
 constexpr int kEpiWarps = 8;
-constexpr int kUpdWarps = 2;
-constexpr int kUpdThreads = 32 * kUpdWarps;  // each handles rows u and u + 64 of a tile
-constexpr int kThreadsMixed = 32 * (2 + kEpiWarps + kUpdWarps);
-constexpr int kMaxChunks = 4;   // 256-column chunks per pass (k <= 1024)
+constexpr int kThreadsMixed = 32 * (2 + kEpiWarps);
 constexpr uint32_t kTileBytes = kTileM * 128;  // one 64-wide K block of a tile
 constexpr size_t kSmemLimit = 232448;
 
@@ -121,57 +112,18 @@ struct MixedConsts {
 };
 
 // Order-independent totals of the fixed-point sums (d <= 32): element e
-// (cluster-major [k][d4] sums, then the k sizes) of copy c is
-// hi[c stride + e] 2^32 + lo[c stride + e]; contributions q are added as
-// (q >> 32) into hi and (q mod 2^32) into lo with 64-bit integer atomics (the
-// copies, CTA b into copy b mod copies, spread the contention), and the copies
-// are added as integers, so every order gives the same bits.  xq: the packed
-// terms ([n][d4 + 4]); null when not in use.
+// (cluster-major [k][d4] sums, then the k sizes) of copy c is sum[c stride + e];
+// CTA b adds into copy b mod copies, which spreads the contention, and the
+// scale keeps every copy below 2^61.  The copies are added as integers too, so
+// every order gives the same bits.  xq: the packed terms ([n][d4 + 4]); null
+// when not in use.
 struct FxAcc {
     const int *xq;
-    long long *hi;
-    unsigned long long *lo;
+    unsigned long long *sum;
     int64_t stride;  // elements per copy
     int copies;
     int *dirty;      // set when a term went to the float64 copies instead
-    // the copy of block b
-    __device__ __forceinline__ FxAcc copy_of(unsigned b) const {
-        FxAcc r = *this;
-        if (hi != nullptr) {
-            const int64_t o = (int64_t)(b % (unsigned)copies) * stride;
-            r.hi += o;
-            r.lo += o;
-        }
-        return r;
-    }
 };
-
-__device__ __forceinline__ void fx_add(const FxAcc &fx, int64_t e, long long q) {
-    atomicAdd(reinterpret_cast<unsigned long long *>(fx.hi + e), (unsigned long long)(q >> 32));
-    atomicAdd(fx.lo + e, (unsigned long long)(q & 0xffffffffll));
-}
-
-// Sample i (label c) into the integer totals of fx (this block's copy): its
-// packed terms w x_j (j < d4) and w; a flagged term (not representable) goes
-// as its exact float value into the float64 copy acc64 ([k_pad][d4] sums,
-// then k_pad sizes).
-__device__ __forceinline__ void add_packed_row(const FxAcc &fx, double *acc64, int64_t k_pad,
-                                               int64_t k, int64_t d4, const float *xrow,
-                                               const float *w, int64_t i, int64_t c) {
-    const int64_t ds = d4 + 4;
-    const float wv = w[i];
-    for (int64_t j = 0; j <= d4; ++j) {
-        const int pk = fx.xq[i * ds + j];
-        if (pk == 1) {
-            const float v = j < d4 ? __fmul_rn(xrow[i * d4 + j], wv) : wv;
-            *reinterpret_cast<volatile int *>(fx.dirty) = 1;
-            atomicAdd(j < d4 ? acc64 + c * d4 + j : acc64 + k_pad * d4 + c, (double)v);
-        } else if (pk != 0) {
-            fx_add(fx, j < d4 ? c * d4 + j : k * d4 + c,
-                   (long long)(pk >> 6) * (1ll << ((pk >> 1) & 31)));
-        }
-    }
-}
 
 struct MixedArgs {
     const uint8_t *ximg;
@@ -179,25 +131,14 @@ struct MixedArgs {
     const float *nx;
     const float *ndx;   // ||operand rounding error of x_i|| / sigma, rounded up
     const MixedConsts *consts;
-    const float *X;
-    const float *w;
     void *labels;
-    // Cluster sums in n_copies private copies ([copy][k_pad*d4 + k_pad]:
-    // cluster-major sums, then sizes; CTA b uses copy b % n_copies), reduced
-    // in a fixed order afterwards.
-    float *sums32;     // fp32 copies (vector-red path)
-    double *acc64;     // fp64 copies (acc_f64 path)
-    int n_copies;
-    const float *xrow; // [n][d4] row-major fp32 copy of X (update and recheck)
     uint4 *cand;
     int *flagged;
     int *n_flagged;
     int *err_global;
     const LoopState *guard;
-    int64_t n, d, k, k_pad, d4;
-    int update;
+    int64_t n;
     int label64;
-    int acc_f64;       // red.global.add.f64 per feature (else red.global.add.v4.f32)
     int stages;        // depth of the X-tile ring
     long long wait_limit;  // SM clocks after which a wait gives up
     int stall;         // test of the timeout path: the epilogue first waits on a
@@ -205,34 +146,16 @@ struct MixedArgs {
     LoopState *state;  // receives the error bit and stops the loop (nullable)
     // Column passes (n_clusters beyond what one launch holds in shared
     // memory): this launch covers columns col0 .. col0 + NCH*256 - 1 of a
-    // global centroid image of k_img rows.  With multi set it writes, per
+    // global centroid image of k_img rows.  With column passes it writes, per
     // sample, its best score of the pass (pmax) and full candidate masks of
     // the pass (cand) instead of labels; a combine kernel decides.
     int64_t k_img, col0;
-    int multi;
     float *pmax;
-    // > 0: the sums of own_k clusters are accumulated per CTA in shared memory
-    // (fixed point), own_f packed columns per update thread
-    int64_t own_k;
-    int own_f;
-    const int *xq;  // [n][d4 + 4] packed fixed-point terms (w x, then w, 0, 0, 0)
-    FxAcc fx;       // their order-independent totals
 };
-
-// Fixed-point sums: each of the 64 update threads adds own_f consecutive
-// columns of its rows, w columns / own_f threads per row, so the rows are
-// split into (and the sums kept in) this many groups.
-__host__ __device__ constexpr int fx_copies(int64_t w, int own_f) {
-    return (int)(kUpdThreads / (w / own_f));
-}
 
 struct SmemLayout {
-    size_t c, hnb, aon, x, xch, lab, bar, p1, osum, ostage, ocode, ow, total;
+    size_t c, hnb, aon, x, xch, bar, total;
 };
-
-// Sub-chunk maxima stay in registers up to two chunks; beyond that they go
-// to shared memory (registers would spill).
-__host__ __device__ constexpr bool p1_in_smem(int64_t nch) { return nch >= 3; }
 
 // c:    centroid image, NKB blocks of k_pad x 128 bytes (128-byte swizzle)
 // hnb:  half-norm parts, k_pad x 32 bytes (32-byte swizzle); c and hnb are
@@ -240,15 +163,7 @@ __host__ __device__ constexpr bool p1_in_smem(int64_t nch) { return nch >= 3; }
 // aon:  constant A block (128 x 32 bytes): columns 0..2 = -2^10, -1, -2^-10
 // x:    X-tile ring (stages x NKB x 16 KB)
 // xch:  per-row maxima of the two column halves (two tiles in flight)
-// lab:  labels / recheck slots handed to the update warps (two tiles)
-// p1:   sub-chunk maxima, [sub-chunk][256 epilogue threads] (3+ chunks)
-// osum: the CTA's fixed-point cluster sums and sizes, R copies of
-//       [own_k + 1][d4 + 4] (int64), R = fx_copies(d4 + 4, own_f); ostage /
-//       ocode: a tile's packed rows and labels handed between the two update
-//       warps (fixed-point sums only)
-__host__ __device__ inline SmemLayout smem_layout(int nkb, int64_t k_pad, int64_t d4,
-                                                  int stages, int64_t own_k = 0,
-                                                  int own_f = 1) {
+__host__ __device__ inline SmemLayout smem_layout(int nkb, int64_t k_pad, int stages) {
     SmemLayout L;
     size_t off = 0;
     L.c = off;
@@ -263,28 +178,8 @@ __host__ __device__ inline SmemLayout smem_layout(int nkb, int64_t k_pad, int64_
     off += (size_t)stages * nkb * kTileBytes;
     L.xch = off;
     off += sizeof(float) * 2 * 2 * kTileM;
-    L.lab = off;
-    off += sizeof(int) * 2 * kTileM;
-    off = (off + 15) & ~size_t(15);
     L.bar = off;
-    off += 8 * 19 + 16;
-    off = (off + 15) & ~size_t(15);
-    L.p1 = off;
-    if (p1_in_smem(k_pad / kChunkN)) off += sizeof(float) * 32 * kEpiWarps * (size_t)(k_pad / 64);
-    off = (off + 15) & ~size_t(15);
-    L.osum = off;
-    L.ostage = L.ocode = L.ow = off;
-    if (own_k > 0) {
-        // R copies of [own_k + 1][d4 + 4] (the last cluster row takes rows
-        // without a certified label)
-        off += sizeof(long long) * (size_t)fx_copies(d4 + 4, own_f) * (size_t)(own_k + 1) *
-               (size_t)(d4 + 4);
-        L.ostage = off;
-        off += sizeof(int) * kTileM * (size_t)(d4 + 4);
-        L.ocode = off;
-        off += sizeof(int) * kTileM;
-        L.ow = off;
-    }
+    off += 8 * 15 + 8;
     L.total = off + 1024;  // slack for aligning the dynamic shared memory base
     return L;
 }
@@ -305,12 +200,15 @@ __device__ __forceinline__ float u2f(uint32_t v) { return __uint_as_float(v); }
 // tcgen05.ld writes its registers asynchronously; after tcgen05.wait::ld the
 // empty asm statements (ordered after the wait like every volatile asm) make
 // each later use of the registers depend on the wait.
-__device__ __forceinline__ void tmem_ld_wait_regs(uint32_t (&r0)[32], uint32_t (&r1)[32], uint32_t &m0,
-                                                  uint32_t &m1) {
+__device__ __forceinline__ void tmem_ld_wait_regs(uint32_t (&r0)[32], uint32_t (&r1)[32],
+                                                  uint32_t (&r2)[32], uint32_t (&r3)[32],
+                                                  uint32_t (&m)[4]) {
     tmem_ld_wait();
-    asm volatile("" : "+r"(m0), "+r"(m1));
 #pragma unroll
-    for (int t = 0; t < 32; ++t) asm volatile("" : "+r"(r0[t]), "+r"(r1[t]));
+    for (int t = 0; t < 4; ++t) asm volatile("" : "+r"(m[t]));
+#pragma unroll
+    for (int t = 0; t < 32; ++t)
+        asm volatile("" : "+r"(r0[t]), "+r"(r1[t]), "+r"(r2[t]), "+r"(r3[t]));
 }
 
 // The test v >= thr as a fused multiply-add with saturation, which runs on
@@ -359,24 +257,6 @@ __device__ __forceinline__ bool pair_any(bool v, int q) {
     return r != 0;
 }
 
-// Barrier of the two update warps (named barrier 12, 64 threads); upd_any
-// also returns the OR of v over them.
-__device__ __forceinline__ void upd_sync() {
-    asm volatile("bar.sync 12, 64;" ::: "memory");
-}
-__device__ __forceinline__ bool upd_any(bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.red.or.pred q, 12, 64, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)v)
-        : "memory");
-    return r != 0;
-}
-
 // 2^e as a float (e in [-126, 127]).
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }
 
@@ -395,177 +275,6 @@ __host__ __device__ inline int pack_fixed(float v, int emin) {
     const int m = (int)((b & 0x7fffffu) | 0x800000u);
     const int ms = (b >> 31) ? -m : m;
     return (int)(((uint32_t)ms << 6) | (sh << 1));
-}
-
-// sum += the integer a packed term stands for (one 32 x 32 -> 64-bit
-// multiply-add).
-__device__ __forceinline__ void add_packed(unsigned long long &sum, int p) {
-    const int ms = p >> 6;
-    const int pw = 1 << ((p >> 1) & 31);
-    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(sum) : "r"(ms), "r"(pw));
-}
-
-// own_f (2 or 4) consecutive 64-bit sums at a 16-byte aligned shared-window
-// address (volatile: kept in program order with each other).
-template <int F>
-__device__ __forceinline__ void lds_sums(uint32_t addr, unsigned long long (&q)[F]) {
-    static_assert(F == 2 || F == 4, "two or four columns per thread");
-#pragma unroll
-    for (int j = 0; j < F; j += 2)
-        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(q[j]), "=l"(q[j + 1]) : "r"(addr + 8u * j));
-}
-template <int F>
-__device__ __forceinline__ void sts_sums(uint32_t addr, const unsigned long long (&q)[F]) {
-    static_assert(F == 2 || F == 4, "two or four columns per thread");
-#pragma unroll
-    for (int j = 0; j < F; j += 2)
-        asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr + 8u * j), "l"(q[j]), "l"(q[j + 1]));
-}
-
-// Second pass over a tile's terms that the fixed-point sums cannot hold
-// (flag 1: below the scale's resolution, or NaN): their exact float values
-// straight into the float64 sums.  Kept out of line so that no float64
-// instruction enters the first pass.  Columns c0 .. c0 + nc - 1 of rows
-// grp, grp + R, ... of the tile whose first sample is i0.
-__device__ __noinline__ void rare_terms(const MixedArgs &a, double *acc64, int64_t ks, int64_t i0,
-                                        const int *code, const int *stage, int grp, int R, int c0,
-                                        int nc) {
-    const int64_t d4 = a.d4, ds = d4 + 4;
-    for (int r = grp; r < kTileM; r += R) {
-        const int c = code[r];
-        if (c < 0 || c >= a.k) continue;
-        for (int j = c0; j < c0 + nc; ++j) {
-            if (stage[r * ds + j] != 1) continue;
-            const float w = a.w[i0 + r];
-            *reinterpret_cast<volatile int *>(a.fx.dirty) = 1;
-            if (j < d4) {
-                const float v = __fmul_rn(a.xrow[(i0 + r) * d4 + j], w);
-                if (v != 0.f) atomicAdd(acc64 + (int64_t)c * d4 + j, (double)v);
-            } else if (j == d4) {
-                atomicAdd(acc64 + ks * d4 + c, (double)w);
-            }
-        }
-    }
-}
-
-// The update role of the tensor-core kernel with fixed-point sums (d <= 32,
-// one column pass): the CTA adds the features and weights of its certified
-// rows into integer sums in shared memory and adds them to the fit's
-// order-independent integer totals (FxAcc) once at the end.  Every term w x (and w) is prepared once per
-// fit as the packed integer w x 2^fx_shift (the shift keeps every CTA's sums
-// below 2^61), so a term costs one multiply-add on the integer pipe per
-// iteration.  No float64 instruction runs per tile: on this part even a
-// predicated-off float64 conversion costs the issue slots of a whole row.
-// Terms below the scale's resolution, and NaNs, are rare: a tile that has
-// some adds them to the float64 copy in a second pass.
-//
-// Rows are d4 + 4 packed columns (w x_0 .. w x_{d4-1}, w, 0, 0, 0).  Thread
-// u adds columns j0 .. j0 + F - 1, j0 = F (u mod T), T = (d4 + 4) / F, of
-// rows r = g (mod R), g = u / T, R = fx_copies(d4 + 4, F), into its group's
-// copy [g][cluster][column]; rows without a certified label go to the spare
-// cluster row own_k.  The two update warps copy each tile's packed rows and
-// labels into shared memory (named barrier 12) and load the next tile's rows
-// while they add this one's.
-template <int F>
-__device__ __forceinline__ void fixed_sums_role(const MixedArgs &a, const MixedConsts &cst,
-                                                uint8_t *smem, const SmemLayout &L, int *lab_s,
-                                                uint64_t *ufull, uint64_t *uempty, volatile int *err,
-                                                long long lim, double *acc64, int64_t ks) {
-    const int u = threadIdx.x - 32 * (2 + kEpiWarps);
-    const int64_t n = a.n, k = a.k, d4 = a.d4, ok = a.own_k;
-    const int ds = (int)d4 + 4, dq = ds / 4;  // packed columns, uint4 per row
-    const int64_t ntiles = ceil_div<int64_t>(n, kTileM);
-    const int T = ds / F, R = fx_copies(ds, F);
-    const int grp = u / T, j0 = F * (u - grp * T);
-    long long *osum = reinterpret_cast<long long *>(smem + L.osum);
-    int *ostage = reinterpret_cast<int *>(smem + L.ostage);
-    int *ocode = reinterpret_cast<int *>(smem + L.ocode);
-    const uint32_t mine = smem_u32(osum + (int64_t)grp * (ok + 1) * ds + j0);
-    const uint32_t cstride = 8u * (uint32_t)ds;
-
-    for (int64_t e = u; e < (int64_t)R * (ok + 1) * ds; e += kUpdThreads) osum[e] = 0;
-    // rows u and u + 64 of a tile, loaded one tile ahead
-    uint4 ra[9], rb[9];
-    auto load_rows = [&](int64_t tile) {
-        const int64_t i0 = tile * kTileM + u, i1 = i0 + 64;
-        const uint4 *pa = reinterpret_cast<const uint4 *>(a.xq + i0 * ds);
-        const uint4 *pb = reinterpret_cast<const uint4 *>(a.xq + i1 * ds);
-#pragma unroll
-        for (int g = 0; g < 9; ++g) {
-            const bool in = g < dq && tile < ntiles;
-            ra[g] = (in && i0 < n) ? __ldg(pa + g) : make_uint4(0u, 0u, 0u, 0u);
-            rb[g] = (in && i1 < n) ? __ldg(pb + g) : make_uint4(0u, 0u, 0u, 0u);
-        }
-    };
-    load_rows(blockIdx.x);
-    int tl = 0;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tl) {
-        const int tb = tl & 1;
-        const bool got = mbar_wait(&ufull[tb], ((uint32_t)tl >> 1) & 1u, err, lim);
-        int c0 = -1, c1 = -1;
-        if (got) {
-            c0 = lab_s[tb * kTileM + u];
-            c1 = lab_s[tb * kTileM + u + 64];
-            mbar_arrive(&uempty[tb]);
-        }
-        // both warps stop together (this barrier also orders the previous
-        // tile's reads of the stage before the writes below)
-        if (upd_any(!got)) break;
-        uint4 *sa = reinterpret_cast<uint4 *>(ostage + u * ds);
-        uint4 *sb = reinterpret_cast<uint4 *>(ostage + (u + 64) * ds);
-#pragma unroll
-        for (int g = 0; g < 9; ++g)
-            if (g < dq) {
-                sa[g] = ra[g];
-                sb[g] = rb[g];
-            }
-        // labels of rows the kernel did not certify (and padding) go to the
-        // spare cluster row
-        ocode[u] = (c0 >= 0 && c0 < k) ? c0 : (int)ok;
-        ocode[u + 64] = (c1 >= 0 && c1 < k) ? c1 : (int)ok;
-        upd_sync();
-        load_rows(tile + gridDim.x);
-        if (grp < R) {
-            int flags = 0;
-            for (int r = grp; r < kTileM; r += R) {
-                const int c = ocode[r];
-                const int *t = ostage + r * ds + j0;
-                int v[F];
-                if constexpr (F == 4) {
-                    const int4 q = *reinterpret_cast<const int4 *>(t);
-                    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-                } else {
-                    const int2 q = *reinterpret_cast<const int2 *>(t);
-                    v[0] = q.x, v[1] = q.y;
-                }
-                const uint32_t addr = mine + (uint32_t)c * cstride;
-                unsigned long long sum[F];
-                lds_sums<F>(addr, sum);
-                int rf = 0;
-#pragma unroll
-                for (int j = 0; j < F; ++j) {
-                    add_packed(sum[j], v[j]);
-                    rf |= v[j];
-                }
-                sts_sums<F>(addr, sum);
-                // flagged terms of the spare row never count
-                flags |= c != (int)ok ? rf : 0;
-            }
-            if (flags & 1)
-                rare_terms(a, acc64, ks, tile * kTileM, ocode, ostage, grp, R, j0, F);
-        }
-    }
-    upd_sync();
-    // this CTA's sums (its R copies added exactly) into the order-independent
-    // integer totals
-    const FxAcc fxc = a.fx.copy_of(blockIdx.x);
-    for (int64_t e = u; e < ok * (d4 + 1); e += kUpdThreads) {
-        const int64_t c = e < ok * d4 ? e / d4 : e - ok * d4;
-        const int64_t j = e < ok * d4 ? e - c * d4 : d4;
-        long long q = 0;
-        for (int g = 0; g < R; ++g) q += osum[((int64_t)g * (ok + 1) + c) * ds + j];
-        if (q != 0) fx_add(fxc, e, q);
-    }
 }
 
 // Packed fixed-point terms of every sample: w x_j for j < d4 (rounded
@@ -613,22 +322,20 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int64_t k_pad = (int64_t)NCH * kChunkN;
     const int stages = a.stages;
-    const SmemLayout L = smem_layout(NKB, k_pad, a.d4, stages, a.own_k, a.own_f);
+    const SmemLayout L = smem_layout(NKB, k_pad, stages);
     uint8_t *cimg_s = smem + L.c;
     uint8_t *aon_s = smem + L.aon;
     uint8_t *xring = smem + L.x;
     float *xch = reinterpret_cast<float *>(smem + L.xch);
-    int *lab_s = reinterpret_cast<int *>(smem + L.lab);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bar);
     uint64_t *full = bars, *empty = bars + 4, *tfull = bars + 8, *tempty = bars + 10;
-    uint64_t *ufull = bars + 12, *uempty = bars + 14, *cbar = bars + 16, *tdone = bars + 17;
-    uint64_t *never = bars + 18;  // completed by no role (timeout test only)
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 19);
+    uint64_t *cbar = bars + 12, *tdone = bars + 13;
+    uint64_t *never = bars + 14;  // completed by no role (timeout test only)
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
     volatile int *err = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // k: columns from this pass's first on (the padding beyond never wins)
-    const int64_t n = a.n, k = a.k - a.col0;
+    const int64_t n = a.n;
     const long long lim = a.wait_limit;
     const int64_t ntiles = ceil_div<int64_t>(n, kTileM);
     const uint32_t cbytes = (uint32_t)cimg_bytes(NKB, k_pad);
@@ -641,8 +348,6 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
             mbar_init(&tempty[b], 32 * kEpiWarps);
-            mbar_init(&ufull[b], kTileM);
-            mbar_init(&uempty[b], kUpdThreads);
         }
         mbar_init(cbar, 1);
         mbar_init(tdone, 1);
@@ -756,17 +461,14 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
             mbar_wait_drain(tdone, 0, err);
         }
         __syncwarp();
-    } else if (warp < 2 + kEpiWarps) {
+    } else {
         // ------------------------------ epilogue ------------------------------
         // Thread (row, h) scans columns h*128 .. h*128+127 of every chunk for
         // tile row `row`: P2[t] = max over its columns j = t (mod 32), P1[s] =
         // max over its 32-column sub-chunk s (4 per chunk).
         constexpr int kSub = 4 * NCH;
         constexpr uint32_t kAll1 = (kSub == 32) ? ~0u : ((1u << kSub) - 1u);
-        constexpr bool kP1s = p1_in_smem(NCH);
-        constexpr int kChunkUnroll = kP1s ? 1 : NCH;
         const int ew = warp - 2;
-        float *my_p1 = reinterpret_cast<float *>(smem + L.p1) + (ew * 32 + lane);
         const int q = warp & 3;   // TMEM lane quadrant accessible to this warp
         const int h = ew >> 2;    // column half of each 256-wide chunk
         const int row = 32 * q + lane;
@@ -798,21 +500,12 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                     dx_next = a.ndx[inext];
                 }
             }
-            float P2[32], P1[kP1s ? 1 : kSub];
+            float P2[32], P1[kSub];
             float Mh = -pos_inf<float>();
-            // sub-chunk maximum m of sub-chunk sc (register or shared copy)
-            auto put = [&](int sc, float m) {
-                Mh = fmaxf(Mh, m);
-                if constexpr (kP1s)
-                    my_p1[sc * 32 * kEpiWarps] = m;
-                else
-                    P1[sc] = m;
-            };
 #pragma unroll
             for (int t = 0; t < 32; ++t) P2[t] = -pos_inf<float>();
             bool bad = false;
-            // unrolled when the maxima live in registers (static indices)
-#pragma unroll kChunkUnroll
+#pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 const uint32_t b = cnt & 1u, bph = (cnt >> 1) & 1u;
                 if (!mbar_wait(&tfull[b], bph, err, lim)) bad = true;
@@ -823,28 +516,24 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                 }
                 tc_fence_after();
                 const uint32_t cb = tmem + lane_addr + b * kChunkN + h * 128;
-                uint32_t ra[32], rb[32], m0, m1;
-                // sub-chunks 0 and 1
-                tmem_ld32_max(cb, ra, m0);
-                tmem_ld32_max(cb + 32, rb, m1);
-                tmem_ld_wait_regs(ra, rb, m0, m1);
-#pragma unroll
-                for (int t = 0; t < 32; ++t) P2[t] = max3f(P2[t], u2f(ra[t]), u2f(rb[t]));
-                // the loads below reuse ra / rb: finish every read of them first
-#pragma unroll
-                for (int t = 0; t < 32; ++t) asm volatile("" : "+f"(P2[t]));
-                put(4 * c, u2f(m0));
-                put(4 * c + 1, u2f(m1));
-                // sub-chunks 2 and 3
-                tmem_ld32_max(cb + 64, ra, m0);
-                tmem_ld32_max(cb + 96, rb, m1);
-                tmem_ld_wait_regs(ra, rb, m0, m1);
+                // all 128 columns into registers, so that the accumulator is free
+                // again before they are looked at
+                uint32_t ra[32], rb[32], rc[32], rd[32], m[4];
+                tmem_ld32_max(cb, ra, m[0]);
+                tmem_ld32_max(cb + 32, rb, m[1]);
+                tmem_ld32_max(cb + 64, rc, m[2]);
+                tmem_ld32_max(cb + 96, rd, m[3]);
+                tmem_ld_wait_regs(ra, rb, rc, rd, m);
                 tc_fence_before();
                 mbar_arrive(&tempty[b]);  // the accumulator may be overwritten now
 #pragma unroll
-                for (int t = 0; t < 32; ++t) P2[t] = max3f(P2[t], u2f(ra[t]), u2f(rb[t]));
-                put(4 * c + 2, u2f(m0));
-                put(4 * c + 3, u2f(m1));
+                for (int t = 0; t < 32; ++t)
+                    P2[t] = max3f(max3f(P2[t], u2f(ra[t]), u2f(rb[t])), u2f(rc[t]), u2f(rd[t]));
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    P1[4 * c + t] = u2f(m[t]);
+                    Mh = fmaxf(Mh, u2f(m[t]));
+                }
                 ++cnt;
             }
 
@@ -862,8 +551,7 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
             // sub-chunk lie in distinct classes).
             const float thr = fmaxf(Mh, Mo) - E2;
             // exactly one of the pair wins, whatever the maxima (a NaN loses
-            // every comparison: the first half then wins); only the winner
-            // hands the row over, and ufull counts one arrival per row
+            // every comparison: the first half then wins)
             const bool win = (Mh > Mo) || (h == 0 && !(Mo > Mh));
             uint32_t hot1 = 0u, hot2 = 0u;
             const HotTest ht = hot_test(thr);
@@ -873,7 +561,7 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                 float l1 = 0.f, l2 = 0.f, h2 = 0.f;
 #pragma unroll
                 for (int t = 0; t < kSub; ++t) {
-                    const float m = kP1s ? my_p1[t * 32 * kEpiWarps] : P1[kP1s ? 0 : t];
+                    const float m = P1[t];
                     l1 = fmaf(ht.hot(m), (float)(1u << t), l1);
                 }
 #pragma unroll
@@ -886,7 +574,7 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
             } else {
 #pragma unroll
                 for (int t = 0; t < kSub; ++t) {
-                    const float m = kP1s ? my_p1[t * 32 * kEpiWarps] : P1[kP1s ? 0 : t];
+                    const float m = P1[t];
                     hot1 |= (m >= thr) ? (1u << t) : 0u;
                 }
 #pragma unroll
@@ -898,7 +586,6 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                 hot2 = ~0u;
                 loser_hot = true;
             }
-            int code = -1;  // handoff to the update warps: >= 0 label, <= -2 recheck slot
             if (MULTI && i < n) {
                 // column pass: the pass's best score and both halves' masks
                 // (single bits for a unique winner), decided by the combine
@@ -920,7 +607,7 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                 if (win) {
                     if (!loser_hot && __popc(hot1) == 1 && __popc(hot2) == 1) {
                         const int sc = __ffs(hot1) - 1, t = __ffs(hot2) - 1;
-                        code = (sc >> 2) * kChunkN + h * 128 + (sc & 3) * 32 + t;
+                        const int code = (sc >> 2) * kChunkN + h * 128 + (sc & 3) * 32 + t;
                         if (a.label64)
                             reinterpret_cast<int64_t *>(a.labels)[i] = code;
                         else
@@ -933,110 +620,13 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                             cw[2 + (h ^ 1)] = 0u;
                         }
                         const int pos = atomicAdd(a.n_flagged, 1);
-                        if (pos >= 0 && pos < n) {
-                            a.flagged[pos] = (int)i;
-                            code = -2 - pos;
-                        }
+                        if (pos >= 0 && pos < n) a.flagged[pos] = (int)i;
                     }
                 } else if (loser_hot) {
                     cw[h] = hot1;
                     cw[2 + h] = hot2;
                 }
             }
-            const int tb = tl & 1;
-            // Only the thread that hands the row over waits: its own arrival is
-            // part of the next phase, so the phase it waits for cannot be
-            // overtaken.  A loser's arrival is not: one that polled late saw
-            // the barrier two phases on, with the parity of the phase it
-            // waited for, and never passed.
-            if (win && mbar_wait(&uempty[tb], (((uint32_t)tl >> 1) & 1u) ^ 1u, err, lim)) {
-                lab_s[tb * kTileM + row] = code;
-                mbar_arrive(&ufull[tb]);
-            }
-        }
-    } else {
-        // ------------------------------ update --------------------------------
-        // Thread u handles rows u and u + 64 of every tile.  The rows (from
-        // the row-major fp32 copy of X) and weights are loaded before their
-        // labels are known, so the loads overlap the epilogue of the tile.
-        // Uncertified rows are left to the recheck kernel.
-        const int u = threadIdx.x - 32 * (2 + kEpiWarps);
-        const int64_t d4 = a.d4;
-        const int64_t ks = MULTI ? a.k_img : k_pad;  // rows of the cluster sums (all columns)
-        const int64_t cstride = ks * d4 + ks;
-        float *sums32 = a.sums32 + (int64_t)(blockIdx.x % (unsigned)a.n_copies) * cstride;
-        double *acc64 = a.acc64 + (int64_t)(blockIdx.x % (unsigned)a.n_copies) * cstride;
-        auto consume = [&](int code, const float4 (&xv)[16], float wv, int pass) {
-            if (code < 0 || code >= k || !a.update) return;
-            if (a.acc_f64) {
-                // small d: float64 sums keep the trajectory on the reference's
-                double *dst = acc64 + (int64_t)code * d4 + pass * 64;
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    if ((int64_t)pass * 64 + 4 * g < d4) {
-                        atomicAdd(dst + 4 * g + 0, (double)__fmul_rn(xv[g].x, wv));
-                        atomicAdd(dst + 4 * g + 1, (double)__fmul_rn(xv[g].y, wv));
-                        atomicAdd(dst + 4 * g + 2, (double)__fmul_rn(xv[g].z, wv));
-                        atomicAdd(dst + 4 * g + 3, (double)__fmul_rn(xv[g].w, wv));
-                    }
-                }
-                if (pass == 0) atomicAdd(acc64 + ks * d4 + code, (double)wv);
-            } else {
-                float4 *dst = reinterpret_cast<float4 *>(sums32 + (int64_t)code * d4 + pass * 64);
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    if ((int64_t)pass * 64 + 4 * g < d4) {
-                        float4 v;
-                        v.x = __fmul_rn(xv[g].x, wv);
-                        v.y = __fmul_rn(xv[g].y, wv);
-                        v.z = __fmul_rn(xv[g].z, wv);
-                        v.w = __fmul_rn(xv[g].w, wv);
-                        atomicAdd(dst + g, v);
-                    }
-                }
-                if (pass == 0) atomicAdd(sums32 + ks * d4 + code, wv);
-            }
-        };
-        bool owned_done = false;
-        if constexpr (NKB == 1 && !MULTI) {
-            if (a.update && a.own_k > 0 && cst.fx_ok) {
-                if (a.own_f == 4)
-                    fixed_sums_role<4>(a, cst, smem, L, lab_s, ufull, uempty, err, lim, acc64, ks);
-                else
-                    fixed_sums_role<2>(a, cst, smem, L, lab_s, ufull, uempty, err, lim, acc64, ks);
-                owned_done = true;
-            }
-        }
-        int tl = 0;
-        for (int64_t tile = blockIdx.x; !owned_done && tile < ntiles; tile += gridDim.x, ++tl) {
-            const int tb = tl & 1;
-            const int64_t i0 = tile * kTileM + u, i1 = i0 + 64;
-            const float w0 = (a.update && i0 < n) ? __ldg(a.w + i0) : 0.f;
-            const float w1 = (a.update && i1 < n) ? __ldg(a.w + i1) : 0.f;
-            int c0 = -1, c1 = -1;
-            bool have_code = false;
-#pragma unroll 1
-            for (int pass = 0; pass < NKB; ++pass) {
-                float4 xa[16], xb[16];
-                const float4 *ra = reinterpret_cast<const float4 *>(a.xrow + i0 * d4 + pass * 64);
-                const float4 *rb = reinterpret_cast<const float4 *>(a.xrow + i1 * d4 + pass * 64);
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    const bool in = (int64_t)pass * 64 + 4 * g < d4;
-                    xa[g] = (a.update && in && i0 < n) ? __ldg(ra + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    xb[g] = (a.update && in && i1 < n) ? __ldg(rb + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                if (!have_code) {
-                    if (!mbar_wait(&ufull[tb], ((uint32_t)tl >> 1) & 1u, err, lim)) break;
-                    c0 = lab_s[tb * kTileM + u];
-                    c1 = lab_s[tb * kTileM + u + 64];
-                    mbar_arrive(&uempty[tb]);
-                    have_code = true;
-                }
-                consume(c0, xa, w0, pass);
-                consume(c1, xb, w1, pass);
-            }
-            if (!have_code) break;
         }
     }
 
@@ -1088,7 +678,7 @@ __global__ void sigma_kernel(MixedConsts *c, int bf16, int64_t d) {
     c->overflow = 0;
 }
 
-// Shift of the fixed-point cluster sums: a CTA adds at most `rows` (>= 128)
+// Shift of the fixed-point cluster sums: a copy adds up at most `rows` (>= 128)
 // values w x per feature (|w x| <= max|x| max|w|) and `rows` weights, so with
 // bound = rows max(max|x| max|w|, max|w|) < 2^e the shift 61 - e keeps every
 // sum below 2^61 and every term below 2^54 (all-zero data gives 0).
@@ -1397,11 +987,9 @@ __device__ __forceinline__ int pass_count(const uint4 &m) {
 }
 
 __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
-    const float *xrow, const float *ct, const float *hn, const float *w, const uint4 *cand,
-    const int *flagged, const int *n_flagged, int64_t n, int64_t d, int64_t k, int64_t d4,
-    void *labels, int label64, int update, int acc_f64, float *sums32, double *acc64,
-    int64_t k_pad, int n_copies, const LoopState *guard, int passes, int64_t pass_cols, FxAcc fx,
-    const MixedConsts *consts, long long *stats) {
+    const float *xrow, const float *ct, const float *hn, const uint4 *cand, const int *flagged,
+    const int *n_flagged, int64_t n, int64_t d, int64_t k, int64_t d4, void *labels, int label64,
+    const LoopState *guard, int passes, int64_t pass_cols, long long *stats) {
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the fit's statistics: samples rechecked in this pass, and in total
@@ -1409,18 +997,10 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
         stats[1] += *n_flagged;
     }
     constexpr int kWarps = kRecheckThreads / 32;
-    const bool use_fx = fx.xq != nullptr && consts->fx_ok;
-    fx = fx.copy_of(blockIdx.x);
     __shared__ unsigned long long key_s[kWarps][32];
     __shared__ int incl_s[kWarps][32];
     __shared__ int row_s[kWarps][32];
     __shared__ uint4 cm_s[kWarps][32];
-    {
-        // this block's share of the per-CTA copies of the cluster sums
-        const int64_t copy = (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
-        sums32 += copy;
-        acc64 += copy;
-    }
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
     const int64_t nf = (int64_t)*n_flagged;
     const int64_t total = nf < n ? nf : n;
@@ -1513,31 +1093,6 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
                 reinterpret_cast<int64_t *>(labels)[i] = bj;
             else
                 reinterpret_cast<int32_t *>(labels)[i] = bj;
-            if (update && use_fx) {
-                add_packed_row(fx, acc64, k_pad, k, d4, xrow, w, i, bj);
-            } else if (update) {
-                const float4 *xr = reinterpret_cast<const float4 *>(xrow + i * d4);
-                const float wv = w[i];
-                if (acc_f64) {
-                    double *dst = acc64 + (int64_t)bj * d4;
-                    for (int64_t g = 0; g < g4; ++g) {
-                        const float4 xv = __ldg(xr + g);
-                        atomicAdd(dst + 4 * g + 0, (double)__fmul_rn(xv.x, wv));
-                        atomicAdd(dst + 4 * g + 1, (double)__fmul_rn(xv.y, wv));
-                        atomicAdd(dst + 4 * g + 2, (double)__fmul_rn(xv.z, wv));
-                        atomicAdd(dst + 4 * g + 3, (double)__fmul_rn(xv.w, wv));
-                    }
-                    atomicAdd(acc64 + k_pad * d4 + bj, (double)wv);
-                } else {
-                    float4 *dst = reinterpret_cast<float4 *>(sums32 + (int64_t)bj * d4);
-                    for (int64_t g = 0; g < g4; ++g) {
-                        const float4 xv = __ldg(xr + g);
-                        atomicAdd(dst + g, make_float4(__fmul_rn(xv.x, wv), __fmul_rn(xv.y, wv),
-                                                       __fmul_rn(xv.z, wv), __fmul_rn(xv.w, wv)));
-                    }
-                    atomicAdd(sums32 + k_pad * d4 + bj, wv);
-                }
-            }
         }
         __syncwarp();  // this batch's keys and masks are read before the next batch
     }
@@ -1555,23 +1110,15 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
 // sample goes to the recheck list.
 __global__ void __launch_bounds__(256) combine_kernel(
     const float *pmax, uint4 *cand, int passes, int64_t pass_cols, const float *nx,
-    const float *ndx, const MixedConsts *consts, const float *xrow, const float *w, void *labels,
-    int label64, int update, int acc_f64, float *sums32, double *acc64, int64_t k_pad,
-    int64_t d4, int n_copies, int *flagged, int *n_flagged, int64_t n, int64_t k,
-    const LoopState *guard, FxAcc fx) {
+    const float *ndx, const MixedConsts *consts, void *labels, int label64, int *flagged,
+    int *n_flagged, int64_t n, int64_t k, const LoopState *guard) {
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     const MixedConsts cst = *consts;
-    const bool use_fx = fx.xq != nullptr && cst.fx_ok;
-    fx = fx.copy_of(blockIdx.x);
-    {
-        const int64_t copy = (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
-        sums32 += copy;
-        acc64 += copy;
-    }
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const float e = fmaf(nx[i], cst.alpha, fmaf(ndx[i], cst.beta1, cst.beta0));
         const float E2 = 2.f * e * 1.000001f;
+        int64_t label = -1;
         float M = -pos_inf<float>();
         bool nan = false;
         for (int p = 0; p < passes; ++p) {
@@ -1587,7 +1134,6 @@ __global__ void __launch_bounds__(256) combine_kernel(
                 ++hot;
                 ph = p;
             }
-        int64_t label = -1;
         if (!nan && hot == 1) {
             const uint4 m = cand[(int64_t)ph * n + i];
             const bool a0 = (m.x | m.z) != 0u, a1 = (m.y | m.w) != 0u;
@@ -1607,31 +1153,6 @@ __global__ void __launch_bounds__(256) combine_kernel(
                 reinterpret_cast<int64_t *>(labels)[i] = label;
             else
                 reinterpret_cast<int32_t *>(labels)[i] = (int32_t)label;
-            if (update && use_fx) {
-                add_packed_row(fx, acc64, k_pad, k, d4, xrow, w, i, label);
-            } else if (update) {
-                const float4 *xr = reinterpret_cast<const float4 *>(xrow + i * d4);
-                const float wv = w[i];
-                if (acc_f64) {
-                    double *dst = acc64 + label * d4;
-                    for (int64_t g = 0; g < d4 / 4; ++g) {
-                        const float4 xv = __ldg(xr + g);
-                        atomicAdd(dst + 4 * g + 0, (double)__fmul_rn(xv.x, wv));
-                        atomicAdd(dst + 4 * g + 1, (double)__fmul_rn(xv.y, wv));
-                        atomicAdd(dst + 4 * g + 2, (double)__fmul_rn(xv.z, wv));
-                        atomicAdd(dst + 4 * g + 3, (double)__fmul_rn(xv.w, wv));
-                    }
-                    atomicAdd(acc64 + k_pad * d4 + label, (double)wv);
-                } else {
-                    float4 *dst = reinterpret_cast<float4 *>(sums32 + label * d4);
-                    for (int64_t g = 0; g < d4 / 4; ++g) {
-                        const float4 xv = __ldg(xr + g);
-                        atomicAdd(dst + g, make_float4(__fmul_rn(xv.x, wv), __fmul_rn(xv.y, wv),
-                                                       __fmul_rn(xv.z, wv), __fmul_rn(xv.w, wv)));
-                    }
-                    atomicAdd(sums32 + k_pad * d4 + label, wv);
-                }
-            }
         } else {
             if (!nan)
                 for (int p = 0; p < passes; ++p)
@@ -1643,15 +1164,333 @@ __global__ void __launch_bounds__(256) combine_kernel(
     }
 }
 
+// ---------------------------------------------------------------------------
+// Cluster sums of an iteration, from the labels that the kernels above wrote.
+//
+// Their own pass over the samples: inside the assignment kernel, few warps had
+// to load each tile's rows, wait for its labels and reduce them, and those
+// chains, not the tensor cores, set its pace (4M x 64, k = 64: 665 us with the
+// sums, 167 us without).  Here every SM is full of warps that do nothing else.
+// A warp takes 32 samples; their rows are one contiguous run of the row-major
+// copy, which its lanes walk together, so that a load or reduction touches one
+// or a few rows.  The reductions' rate bounds it (26 clocks per warp and SM of
+// red.v4.f32, 13 of red.u64).
+// ---------------------------------------------------------------------------
+constexpr int kSumThreads = 256;
+
+// Predicated read-only loads (0 when not in).  Volatile: plain loads would be
+// moved into the branch of the reduction that uses them, one latency each.
+__device__ __forceinline__ float4 load_f4_if(const float4 *p, bool in) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %5, 0;\n\t"
+        "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+        "@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+        : "l"(p), "r"((uint32_t)in));
+    return v;
+}
+__device__ __forceinline__ int load_i_if(const int *p, bool in) {
+    int v;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %2, 0;\n\t"
+        "mov.s32 %0, 0;\n\t"
+        "@p ld.global.nc.s32 %0, [%1];\n\t}"
+        : "=&r"(v)
+        : "l"(p), "r"((uint32_t)in));
+    return v;
+}
+
+template <typename I>
+__device__ __forceinline__ int label_of(const I *labels, int64_t i, int64_t n, int64_t k) {
+    if (i >= n) return -1;
+    const I c = labels[i];
+    return c >= 0 && c < k ? (int)c : -1;
+}
+
+// Beyond 32 features: float32 sums in copies of [k_pad][d4] and k_pad sizes
+// (CTA b adds into copy b mod n_copies).
+template <typename I>
+__global__ void __launch_bounds__(kSumThreads) sum_rows_kernel(
+    const float *xrow, const float *w, const I *labels, int64_t n, int64_t d4, int64_t k,
+    int64_t k_pad, float *sums, int n_copies, const LoopState *guard) {
+    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
+    constexpr int kBatch = 4;
+    const int lane = threadIdx.x & 31, g4 = (int)(d4 / 4);
+    const int step_r = 32 / g4, step_m = 32 % g4;
+    sums += (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
+    for (int64_t base = (int64_t)blockIdx.x * kSumThreads + (threadIdx.x & ~31); base < n;
+         base += (int64_t)gridDim.x * kSumThreads) {
+        const int c = label_of(labels, base + lane, n, k);
+        const float wv = base + lane < n ? w[base + lane] : 0.f;
+        const float4 *src = reinterpret_cast<const float4 *>(xrow) + base * g4 + lane;
+        int r = lane / g4, m = lane - r * g4;
+        for (int t0 = 0; t0 < g4; t0 += kBatch) {
+            float4 v[kBatch];
+            float wr[kBatch];
+            int64_t e[kBatch];
+#pragma unroll
+            for (int t = 0; t < kBatch; ++t) {
+                // r < 32 while t0 + t < g4
+                const int cr = __shfl_sync(0xffffffffu, c, r & 31);
+                wr[t] = __shfl_sync(0xffffffffu, wv, r & 31);
+                e[t] = cr >= 0 && t0 + t < g4 ? (int64_t)cr * g4 + m : -1;
+                v[t] = load_f4_if(src + 32 * (t0 + t), e[t] >= 0);
+                r += step_r;
+                m += step_m;
+                if (m >= g4) {
+                    m -= g4;
+                    ++r;
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < kBatch; ++t)
+                if (e[t] >= 0)
+                    atomicAdd(reinterpret_cast<float4 *>(sums) + e[t],
+                              make_float4(__fmul_rn(v[t].x, wr[t]), __fmul_rn(v[t].y, wr[t]),
+                                          __fmul_rn(v[t].z, wr[t]), __fmul_rn(v[t].w, wr[t])));
+        }
+        if (c >= 0) atomicAdd(sums + k_pad * d4 + c, wv);
+    }
+}
+
+// Columns 4 l .. 4 l + 3 of sample i (label c) into the float64 copies, out of
+// line: those whose packed terms are flagged (packed null: all of them).
+__device__ __noinline__ void add_columns_f64(const float *xrow, const float *w, const int *packed,
+                                             int64_t i, int c, int l, int64_t d4, int64_t k_pad,
+                                             double *acc, int *dirty) {
+    const float wv = w[i];
+    *reinterpret_cast<volatile int *>(dirty) = 1;
+    for (int64_t j = 4 * l; j < 4 * l + 4 && j <= d4; ++j) {
+        if (packed != nullptr && packed[j] != 1) continue;
+        const float v = j < d4 ? __fmul_rn(xrow[i * d4 + j], wv) : wv;
+        atomicAdd(j < d4 ? acc + c * d4 + j : acc + k_pad * d4 + c, (double)v);
+    }
+}
+
+// Up to 32 features: the packed terms (w x_j, then w) into the integer copies,
+// one 64-bit reduction per term that is not zero; F terms of a lane in flight.
+// No float64 instruction on the main path: on this part even a predicated-off
+// float64 conversion costs the issue slots of a whole row.
+template <typename I, int F>
+__global__ void __launch_bounds__(kSumThreads) sum_terms_kernel(
+    const float *xrow, const float *w, const I *labels, int64_t n, int64_t d4, int64_t k,
+    int64_t k_pad, FxAcc fx, double *acc, int n_copies, const MixedConsts *consts,
+    const LoopState *guard) {
+    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
+    const int lane = threadIdx.x & 31, w1 = (int)d4 + 1, ds = (int)d4 + 4;
+    const int step_r = 32 / w1, step_m = 32 % w1;
+    const bool fx_ok = consts->fx_ok;
+    unsigned long long *sum = fx.sum + (int64_t)(blockIdx.x % (unsigned)fx.copies) * fx.stride;
+    acc += (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
+    for (int64_t base = (int64_t)blockIdx.x * kSumThreads + (threadIdx.x & ~31); base < n;
+         base += (int64_t)gridDim.x * kSumThreads) {
+        const int c = label_of(labels, base + lane, n, k);
+        if (!fx_ok) {
+            for (int l = 0; c >= 0 && l <= (int)d4 / 4; ++l)
+                add_columns_f64(xrow, w, nullptr, base + lane, c, l, d4, k_pad, acc, fx.dirty);
+            continue;
+        }
+        const int *src = fx.xq + base * ds;
+        int r = lane / w1, m = lane - r * w1, flags = 0;
+        for (int t0 = 0; t0 < w1; t0 += F) {
+            int v[F];
+            int64_t e[F];
+#pragma unroll
+            for (int t = 0; t < F; ++t) {
+                // r < 32 while t0 + t < w1
+                const int cr = __shfl_sync(0xffffffffu, c, r & 31);
+                const bool in = cr >= 0 && t0 + t < w1;
+                e[t] = m < (int)d4 ? cr * d4 + m : k * d4 + cr;
+                v[t] = load_i_if(src + r * ds + m, in);
+                r += step_r;
+                m += step_m;
+                if (m >= w1) {
+                    m -= w1;
+                    ++r;
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < F; ++t) {
+                flags |= v[t];
+                // not zero, not flagged
+                if ((unsigned)v[t] > 1u)
+                    atomicAdd(sum + e[t], (unsigned long long)((long long)(v[t] >> 6) *
+                                                               (1 << ((v[t] >> 1) & 31))));
+            }
+        }
+        if (__any_sync(0xffffffffu, (flags & 1) != 0))
+            for (int l = 0; c >= 0 && l <= (int)d4 / 4; ++l)
+                add_columns_f64(xrow, w, src + lane * ds, base + lane, c, l, d4, k_pad, acc, fx.dirty);
+    }
+}
+
+// Up to kSortClusters clusters: a CTA sorts a tile of samples by label first
+// (counting sort in shared memory), then groups of lanes walk runs of the sorted
+// samples, one lane per 16 bytes of a row, sum equal labels in registers and
+// reduce once per run of a label.  F = 0: float32 rows and weights, four rows of
+// a group in flight; F = 2, 4: packed terms, F rows in flight.
+// 4M samples, direct kernel -> sorted: 64 features, k = 64: 299 -> 172 us (5.9
+// TB/s), k = 1024: 285 -> 194; packed, 16 features, k = 100: 199 -> 113; 32 and
+// 256: 350 -> 195 (2M, 32 and 1000: 195 -> 160).  The larger the tile, the fewer
+// runs: k = 1024 takes 219 us with 2048 samples.  Bound by memory for few
+// clusters, by the runs' reductions for many; with more clusters than
+// kSortClusters most runs are single samples and the sort only costs.
+constexpr int kSortTile = 4096, kSortClusters = 2048;
+constexpr int kSortCtas = 4;  // resident per SM (64 registers)
+
+inline size_t sort_smem(int tile, int64_t k) {
+    return (sizeof(int2) + sizeof(float)) * (size_t)tile + sizeof(int) * (size_t)(k + 1);
+}
+
+template <typename I, int F>
+__global__ void __launch_bounds__(kSumThreads, kSortCtas) sum_sorted_kernel(
+    const float *xrow, const float *w, const I *labels, int64_t n, int64_t d4, int64_t k,
+    int64_t k_pad, int tile_rows, float *sums, FxAcc fx, double *acc, int n_copies,
+    const MixedConsts *consts, const LoopState *guard) {
+    if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
+    constexpr bool FX = F != 0;
+    constexpr int kPer = kSortTile / kSumThreads, kWarps = kSumThreads / 32, kBatch = FX ? F : 4;
+    extern __shared__ __align__(16) uint8_t sort_raw[];
+    int2 *key = reinterpret_cast<int2 *>(sort_raw);  // (label, row of the tile) by label
+    float *ws = reinterpret_cast<float *>(key + tile_rows);  // weights, same order
+    int *hist = reinterpret_cast<int *>(ws + tile_rows);     // counts, then first positions
+    __shared__ int warp_sum[kWarps];
+    const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
+    const int vecs = FX ? (int)d4 / 4 + 1 : (int)d4 / 4;  // 16-byte vectors of a row
+    unsigned long long *isum = nullptr;
+    if (FX) {
+        isum = fx.sum + (int64_t)(blockIdx.x % (unsigned)fx.copies) * fx.stride;
+        acc += (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
+    } else {
+        sums += (int64_t)(blockIdx.x % (unsigned)n_copies) * (k_pad * d4 + k_pad);
+    }
+    const bool fx_ok = !FX || consts->fx_ok;
+    for (int64_t i0 = (int64_t)blockIdx.x * tile_rows; i0 < n; i0 += (int64_t)gridDim.x * tile_rows) {
+        const int rows = (int)(n - i0 < tile_rows ? n - i0 : tile_rows);
+        __syncthreads();  // every read of the previous tile's order
+        for (int64_t j = tid; j <= k; j += kSumThreads) hist[j] = 0;
+        int c[kPer], rank[kPer];
+#pragma unroll
+        for (int t = 0; t < kPer; ++t)
+            c[t] = tid + kSumThreads * t < rows ? label_of(labels, i0 + tid + kSumThreads * t, n, k) : -1;
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kPer; ++t)
+            if (c[t] >= 0) rank[t] = atomicAdd(hist + c[t], 1);
+        __syncthreads();
+        // exclusive sums of the counts, a run of them per thread
+        const int per = ((int)k + kSumThreads) / kSumThreads, j0 = tid * per;
+        int total = 0;
+        for (int j = j0; j < j0 + per && j <= k; ++j) total += hist[j];
+        int incl = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) warp_sum[wq] = incl;
+        __syncthreads();
+        int first = incl - total;
+        for (int q = 0; q < wq; ++q) first += warp_sum[q];
+        for (int j = j0; j < j0 + per && j <= k; ++j) {
+            const int v = hist[j];
+            hist[j] = first;
+            first += v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kPer; ++t)
+            if (c[t] >= 0) {
+                const int row = tid + kSumThreads * t, pos = hist[c[t]] + rank[t];
+                key[pos] = make_int2(c[t], row);
+                ws[pos] = FX ? 0.f : w[i0 + row];
+            }
+        __syncthreads();
+        const int valid = hist[k];  // samples with a label (all of them)
+        for (int v0 = 0; v0 < vecs; v0 += 32) {
+            const int L = vecs - v0 < 32 ? vecs - v0 : 32, per_warp = 32 / L;
+            const int grp = lane / L, l = v0 + lane - grp * L;
+            if (grp >= per_warp) continue;
+            const int groups = kWarps * per_warp, id = wq * per_warp + grp;
+            const int a = valid * id / groups, b = valid * (id + 1) / groups;
+            int cur = -1;
+            float4 fs = make_float4(0.f, 0.f, 0.f, 0.f);
+            float fw = 0.f;
+            long long qs[4] = {0, 0, 0, 0};
+            auto flush = [&]() {
+                if (cur < 0) return;
+                if constexpr (FX) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int64_t j = 4 * l + q;
+                        if (j <= d4 && qs[q] != 0)
+                            atomicAdd(isum + (j < d4 ? cur * d4 + j : k * d4 + cur),
+                                      (unsigned long long)qs[q]);
+                        qs[q] = 0;
+                    }
+                } else {
+                    atomicAdd(reinterpret_cast<float4 *>(sums + cur * d4) + l, fs);
+                    if (l == 0) atomicAdd(sums + k_pad * d4 + cur, fw);
+                    fs = make_float4(0.f, 0.f, 0.f, 0.f);
+                    fw = 0.f;
+                }
+            };
+            for (int p0 = a; p0 < b; p0 += kBatch) {
+                int2 kk[kBatch];
+                float4 x[kBatch];
+#pragma unroll
+                for (int t = 0; t < kBatch; ++t) {
+                    const bool in = p0 + t < b;
+                    kk[t] = key[in ? p0 + t : a];
+                    const float *src = FX ? reinterpret_cast<const float *>(fx.xq) + (i0 + kk[t].y) * (d4 + 4)
+                                          : xrow + (i0 + kk[t].y) * d4;
+                    x[t] = load_f4_if(reinterpret_cast<const float4 *>(src) + l, in);
+                    if (!in) kk[t].x = -1;
+                }
+#pragma unroll
+                for (int t = 0; t < kBatch; ++t) {
+                    if (kk[t].x < 0) continue;
+                    if (kk[t].x != cur) {
+                        flush();
+                        cur = kk[t].x;
+                    }
+                    if constexpr (FX) {
+                        const int v[4] = {__float_as_int(x[t].x), __float_as_int(x[t].y),
+                                          __float_as_int(x[t].z), __float_as_int(x[t].w)};
+                        if (!fx_ok || ((v[0] | v[1] | v[2] | v[3]) & 1))
+                            add_columns_f64(xrow, w,
+                                            fx_ok ? fx.xq + (i0 + kk[t].y) * (d4 + 4) : nullptr,
+                                            i0 + kk[t].y, cur, l, d4, k_pad, acc, fx.dirty);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            qs[q] += (long long)(v[q] >> 6) * (1 << ((v[q] >> 1) & 31));
+                    } else {
+                        const float wv = ws[p0 + t];
+                        fs.x += __fmul_rn(x[t].x, wv);
+                        fs.y += __fmul_rn(x[t].y, wv);
+                        fs.z += __fmul_rn(x[t].z, wv);
+                        fs.w += __fmul_rn(x[t].w, wv);
+                        fw += wv;
+                    }
+                }
+            }
+            flush();
+        }
+    }
+}
+
 // The sums of an iteration (km_step.cuh): the fixed-point totals (exact to one
 // rounding), then the cluster-major float copies ([copy][k_pad d4 + k_pad]),
 // each copy zeroed once read.  With fixed-point totals the float64 copies hold
-// anything only when a kernel set acc_dirty (`always`: the assignment's own
-// float64 reductions use them).
+// anything only when a kernel set acc_dirty.
 template <typename A>
 struct MixedSums {
     A *copies;
-    int n_copies, always;
+    int n_copies;
     int64_t k, k_pad, d4;
     FxAcc fx;
     MixedConsts *consts;
@@ -1663,7 +1502,8 @@ struct MixedSums {
     // cluster-major, the sizes last
     __device__ __forceinline__ void at(int64_t e, int64_t d, int64_t *f, int64_t *j) const {
         if (e < k * d) {
-            *j = e / d;
+            // a 64-bit division is a hundred instructions
+            *j = e <= 0xffffffffll ? (int64_t)((uint32_t)e / (uint32_t)d) : e / d;
             *f = e - *j * d;
         } else {
             *f = d;
@@ -1672,30 +1512,24 @@ struct MixedSums {
     }
     __device__ __forceinline__ Part load(int64_t f, int64_t j, int64_t d, int g, int groups) const {
         Part p = zero();
-        const bool use_fx = fx.hi != nullptr && consts->fx_ok;
+        const bool use_fx = fx.sum != nullptr && consts->fx_ok;
         if (use_fx) {
             const int64_t e = f < d ? j * d4 + f : k * d4 + j;
-            for (int c = g; c < fx.copies; c += 4 * groups) {
-                long long h[4];
-                unsigned long long l[4];
+            for (int c = g; c < fx.copies; c += 8 * groups) {
+                unsigned long long l[8];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool in = c + u * groups < fx.copies;
-                    h[u] = in ? fx.hi[(c + u * groups) * fx.stride + e] : 0;
-                    l[u] = in ? fx.lo[(c + u * groups) * fx.stride + e] : 0ull;
-                }
+                for (int u = 0; u < 8; ++u)
+                    l[u] = c + u * groups < fx.copies ? fx.sum[(c + u * groups) * fx.stride + e] : 0ull;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (c + u * groups < fx.copies) {
-                        fx.hi[(c + u * groups) * fx.stride + e] = 0;
-                        fx.lo[(c + u * groups) * fx.stride + e] = 0ull;
-                    }
-                    p.hi += h[u];
-                    p.lo += l[u];
+                for (int u = 0; u < 8; ++u) {
+                    if (c + u * groups < fx.copies) fx.sum[(c + u * groups) * fx.stride + e] = 0ull;
+                    // copies below 2^61 in two parts: no overflow for any count
+                    p.hi += (long long)l[u] >> 32;
+                    p.lo += l[u] & 0xffffffffull;
                 }
             }
         }
-        if (!use_fx || always || consts->acc_dirty) {
+        if (!use_fx || consts->acc_dirty) {
             A *q = copies + (f < d ? j * d4 + f : k_pad * d4 + j);
             const int64_t stride = k_pad * d4 + k_pad;
             for (int c = g; c < n_copies; c += 8 * groups) {
@@ -1720,7 +1554,7 @@ struct MixedSums {
         a.lo += b.lo;
     }
     __device__ __forceinline__ double value(const Part &p) const {
-        if (fx.hi == nullptr || !consts->fx_ok) return p.v;
+        if (fx.sum == nullptr || !consts->fx_ok) return p.v;
         return ((double)p.hi * 4294967296.0 + (double)p.lo) *
                    (1.0 / (double)pow2f(consts->fx_shift)) + p.v;
     }
@@ -1762,14 +1596,14 @@ MixedKernel pick_kernel(int bf16, int nkb, int nch, bool multi = false) {
 constexpr int kMaxFeatureBlocks = 4;
 
 // Column chunks per pass and X-ring depth for nkb feature blocks: the widest
-// pass (at most kMaxChunks chunks, and no wider than needed for kp columns)
+// pass (no wider than needed for kp columns)
 // that fits shared memory with a ring of at least two stages, else one stage.
-bool pass_plan(int nkb, int64_t kp, int64_t d4, int *nch_out, int *stages_out) {
+bool pass_plan(int nkb, int64_t kp, int *nch_out, int *stages_out) {
     const int want = (int)std::min<int64_t>(max_chunks(nkb), kp / kChunkN);
     for (int nch = want; nch >= 1; --nch) {
         if (pick_kernel(0, nkb, nch) == nullptr) continue;
         for (int st = 4; st >= 1; --st)
-            if (smem_layout(nkb, (int64_t)nch * kChunkN, d4, st).total <= kSmemLimit) {
+            if (smem_layout(nkb, (int64_t)nch * kChunkN, st).total <= kSmemLimit) {
                 if (st == 1 && nch > 1) break;  // a narrower pass keeps a two-stage ring
                 *nch_out = nch;
                 *stages_out = st;
@@ -1812,10 +1646,8 @@ int make_mixed_fit_impl(const FitParams<float, I> &p, int form, std::unique_ptr<
 // Times each candidate variant on a synthetic fit (Gaussian blobs of d
 // features, k clusters) for four iterations after one warm-up, and caches the
 // fastest per (d, k, form, size class).  Fits of at least 32 tiles per SM
-// ("large") are timed with 48 tiles per SM, smaller ones with 8: the
-// per-CTA costs of the fixed-point sums (zeroing and adding the shared-memory
-// copies) weigh on few tiles, not on many.  KMC_TUNE=0 keeps the default (the
-// first candidate).
+// ("large") are timed with 48 tiles per SM, smaller ones with 8.  KMC_TUNE=0 keeps
+// the default (the first candidate).
 int tune_mixed_variant(int64_t d, int64_t k, int form, bool large, const std::vector<int> &cand,
                        cudaStream_t s, int *code) {
     Range range("kmc.tune_mixed_variant");
@@ -1910,7 +1742,7 @@ struct MixedFit : PlainFit<float, I> {
     float *nx = nullptr, *ndx = nullptr, *ct = nullptr, *xrow = nullptr;
     float *sums32 = nullptr;
     double *acc64 = nullptr;
-    int n_copies = 1;  // private copies of the cluster sums (one per CTA)
+    int n_copies = 1;  // private copies of the cluster sums
     MixedConsts *consts = nullptr;
     uint4 *cand = nullptr;
     int *flagged = nullptr, *n_flagged = nullptr, *err_dev = nullptr;
@@ -1937,29 +1769,22 @@ struct MixedFit : PlainFit<float, I> {
     int nch = 1;     // 256-column chunks per pass
     int passes = 1;  // column passes per assignment (n_clusters beyond one pass)
     float *pmax = nullptr;
-    int variant = 0;    // 10 stages + fixed-point columns per thread (0: none)
-    int64_t own_k = 0;  // > 0: fixed-point sums accumulated per CTA in shared memory
-    int own_f = 1;      // packed columns per update thread in those sums
+    int variant = 0;  // 10 stages + packed rows in flight per lane of the sums (0: no such sums)
     int *xq = nullptr;  // [n][d4 + 4] packed fixed-point terms
-    long long *fxhi = nullptr;           // their integer totals (high words)
-    unsigned long long *fxlo = nullptr;  // (low words)
-    // Up to 32 features (fits with weights): packed terms and integer totals
-    // for every accumulating kernel -- the assignment's fixed-point sums when
-    // its variant has them, the recheck and the column passes' combine.
+    unsigned long long *fxsum = nullptr;  // their integer totals
+    // Up to 32 features (fits with weights): packed terms, integer totals
     bool fx_on = false;
     FxAcc fx_acc() const {
-        return fx_on ? FxAcc{xq, fxhi, fxlo, this->prm.k * d4 + this->prm.k, n_copies,
-                             &consts->acc_dirty}
-                     : FxAcc{nullptr, nullptr, nullptr, 0, 1, &consts->acc_dirty};
+        return fx_on ? FxAcc{xq, fxsum, this->prm.k * d4 + this->prm.k, n_copies, &consts->acc_dirty}
+                     : FxAcc{nullptr, nullptr, 0, 1, &consts->acc_dirty};
     }
 
     static bool supported(int64_t d, int64_t k) {
         const int nk = (int)ceil_div<int64_t>(std::max<int64_t>(d, 1), 64);
         if (nk > kMaxFeatureBlocks || k < 1) return false;
         const int64_t kp = ceil_div<int64_t>(k, kChunkN) * kChunkN;
-        const int64_t dd = ceil_div<int64_t>(std::max<int64_t>(d, 1), 4) * 4;
         int c = 0, st = 0;
-        return pass_plan(nk, kp, dd, &c, &st);
+        return pass_plan(nk, kp, &c, &st);
     }
 
     int init_mixed(int form) {
@@ -1969,44 +1794,36 @@ struct MixedFit : PlainFit<float, I> {
         nkb = (int)ceil_div<int64_t>(std::max<int64_t>(p.d, 1), 64);
         d4 = ceil_div<int64_t>(std::max<int64_t>(p.d, 1), 4) * 4;
         ntiles = ceil_div<int64_t>(p.n, kTileM);
-        if (!pass_plan(nkb, ceil_div<int64_t>(p.k, kChunkN) * kChunkN, d4, &nch, &stages)) {
+        if (!pass_plan(nkb, ceil_div<int64_t>(p.k, kChunkN) * kChunkN, &nch, &stages)) {
             set_error("mixed form: operands do not fit in shared memory");
             return KMC_ERR_UNSUPPORTED;
         }
         // the centroid image has whole passes of rows (zero padding)
         passes = (int)ceil_div<int64_t>(p.k, (int64_t)nch * kChunkN);
         k_pad = (int64_t)passes * nch * kChunkN;
-        // Cluster sums: up to 32 features, float64 reductions per feature
-        // (a few per sample; they keep the trajectory on the float64
-        // reference's), beyond that float32 four-wide reductions.
+        // Cluster sums: up to 32 features, exact integer sums of packed terms
+        // (float64 for terms that do not fit; they keep the trajectory on the
+        // float64 reference's), beyond that float32 four-wide reductions.
         acc_f64 = d4 <= 32 ? 1 : 0;
-        // float64 sums that fit shared memory next to the operands (keeping a
-        // ring of at least two stages) are formed per CTA in fixed point: the
-        // deepest ring that fits, then as many columns per update thread as
-        // fit beside it.  One column per thread leaves a single copy, whose
-        // read-modify-write chain (one row after another) is slower than the
-        // float64 reductions.  Fits only: a prediction has no weights and no
-        // sums.
-        //
-        // The choice (ring depth, and for these sums fixed point with 4 or 2
-        // columns per thread or float64 reductions) is a variant code
-        // 10 stages + f (f = 0: no fixed point).  The autotuner times the
-        // variants that fit on a synthetic fit once per (d, power-of-two
-        // bucket of k, form, size class) and caches the fastest; the rule
-        // above is the default when tuning is off.
+        // Ring depth and, for the integer sums, the rows (or terms) a lane has
+        // in flight: a variant code 10 stages + f (f = 4 or 2; 0: other sums).
+        // The autotuner times the variants that fit on a synthetic fit once
+        // per (d, power-of-two bucket of k, form, size class) and caches the
+        // fastest; the deepest ring with f = 2 is the default when tuning is
+        // off.
         {
             std::vector<int> cand;
             const int64_t kb = std::min<int64_t>(k_pad, std::max<int64_t>(pow2_at_least(p.k), 1));
-            const bool fx_shape = acc_f64 && passes == 1 && p.w != nullptr;
-            for (int st = stages; st >= 2; --st) {
-                if (fx_shape)
-                    for (int f : {4, 2})
-                        if (smem_layout(nkb, k_pad, d4, st, kb, f).total <= kSmemLimit)
-                            cand.push_back(10 * st + f);
-                if (smem_layout(nkb, k_pad, d4, st).total <= kSmemLimit) cand.push_back(10 * st);
-            }
+            const bool fx_shape = acc_f64 && p.w != nullptr;
+            for (int st = stages; st >= std::min(stages, 2); --st)
+                if (fx_shape) {
+                    cand.push_back(10 * st + 2);
+                    cand.push_back(10 * st + 4);
+                } else {
+                    cand.push_back(10 * st);
+                }
             if (cand.empty()) cand.push_back(10 * stages);
-            int code = cand.front();  // deepest ring, widest fixed-point sums
+            int code = cand.front();
             const int forced = forced_variant();
             if (forced >= 0) {
                 if (std::find(cand.begin(), cand.end(), forced) == cand.end()) {
@@ -2023,10 +1840,6 @@ struct MixedFit : PlainFit<float, I> {
             }
             variant = code;
             stages = code / 10;
-            if (code % 10 != 0) {
-                own_k = p.k;
-                own_f = code % 10;
-            }
         }
         size_t off = 0;
         auto take = [&](size_t bytes) {
@@ -2039,25 +1852,27 @@ struct MixedFit : PlainFit<float, I> {
         const size_t o_ct = take(sizeof(float) * k_pad * d4);
         const size_t o_nx = take(sizeof(float) * p.n);
         const size_t o_ndx = take(sizeof(float) * p.n);
-        // Small sums get private copies, one per CTA of the assignment for
-        // large n: their few addresses would otherwise serialise the
-        // reductions of all SMs.  Every iteration reduces every copy, so
-        // small fits get one copy per eight tiles instead (a 50K-sample fit
-        // spent more time there than in its assignment).
-        // Large sums (c3-sized, 266 KB) stay single: per-CTA copies would
-        // crowd L2 for less contention than they remove.
-        n_copies = (k_pad * d4 <= 32768)
-                       ? (int)std::max<int64_t>(1, std::min<int64_t>(ntiles / 8, num_sms()))
-                       : 1;
+        // Private copies of the sums, CTA b of their kernel into copy b mod
+        // n_copies: with few clusters their few addresses would serialise the
+        // reductions of all SMs (4M x 64 alone: k = 100 and 1 copy 502 us, 16
+        // copies 260, 152 copies 231; k = 1024 and 1 copy 272, 4 copies 227).
+        // Every iteration reads every copy, so the float32 sums get 4096 / k,
+        // and small fits one per eight tiles.  A copy of the integer sums also
+        // bounds the rows it adds up, which the scale pays for in bits: one
+        // per SM, as far as they fit 64 MB.
+        {
+            const int64_t most = std::min<int64_t>(ntiles / 8, num_sms());
+            const int64_t want = std::max<int64_t>(4096 / p.k, acc_f64 ? 16 : 4);
+            n_copies = (int)std::max<int64_t>(1, std::min(most, want));
+        }
         const int64_t csz = (int64_t)n_copies * (k_pad * d4 + k_pad);
         const size_t o_s32 = take(acc_f64 ? 16 : sizeof(float) * csz);
         const size_t o_a64 = take(acc_f64 ? sizeof(double) * csz : 16);
         const size_t o_xf = take(sizeof(float) * std::max<int64_t>(p.n, 1) * d4);
         fx_on = acc_f64 && p.w != nullptr;
         const size_t o_xq = take(fx_on ? sizeof(int) * std::max<int64_t>(p.n, 1) * (d4 + 4) : 16);
-        const size_t o_fx = take(fx_on ? 2 * sizeof(long long) * (size_t)n_copies *
-                                                 (size_t)(p.k * d4 + p.k)
-                                           : 16);
+        const size_t o_fx = take(fx_on ? sizeof(long long) * (size_t)n_copies * (size_t)(p.k * d4 + p.k)
+                                       : 16);
         const size_t o_cst = take(sizeof(MixedConsts));
         // candidate masks (and best scores) of every column pass
         const size_t o_cand = take(sizeof(uint4) * (size_t)p.n * passes);
@@ -2076,10 +1891,7 @@ struct MixedFit : PlainFit<float, I> {
         acc64 = reinterpret_cast<double *>(b + o_a64);
         xrow = reinterpret_cast<float *>(b + o_xf);
         xq = reinterpret_cast<int *>(b + o_xq);
-        if (fx_on) {
-            fxhi = reinterpret_cast<long long *>(b + o_fx);
-            fxlo = reinterpret_cast<unsigned long long *>(fxhi + n_copies * (p.k * d4 + p.k));
-        }
+        fxsum = reinterpret_cast<unsigned long long *>(b + o_fx);
         consts = reinterpret_cast<MixedConsts *>(b + o_cst);
         cand = reinterpret_cast<uint4 *>(b + o_cand);
         pmax = reinterpret_cast<float *>(b + o_pmax);
@@ -2104,9 +1916,10 @@ struct MixedFit : PlainFit<float, I> {
         if (fx_on) {
             absmax_kernel<<<grid1d(p.n, 256, 4096), 256, 0, s>>>(p.w, p.n, &consts->wmax_bits);
             KMC_TRY(check_launch("absmax_w"));
-            // rows one CTA of the assignment handles at most
-            const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(ntiles, num_sms()));
-            const double rows = (double)ceil_div<int64_t>(std::max<int64_t>(ntiles, 1), grid) * kTileM;
+            // rows that one copy of the sums adds up at most
+            const int64_t g = sum_grid(), tile = sum_tile();
+            const int64_t cta = ceil_div<int64_t>(p.n, g * tile) * tile;
+            const double rows = (double)std::max<int64_t>(kTileM, std::min(p.n, ceil_div<int64_t>(g, n_copies) * cta));
             fixed_scale_kernel<<<1, 1, 0, s>>>(consts, rows);
             KMC_TRY(check_launch("fixed_scale"));
             this->launches += 2;
@@ -2152,7 +1965,14 @@ struct MixedFit : PlainFit<float, I> {
         return check_launch("mixed_prep");
     }
 
-    int assign_pass(const float *cur, int update, const LoopState *guard) {
+    // enough CTAs for every sample flagged (8 warps of 32 per CTA round), at
+    // most 8 per SM
+    int64_t recheck_grid() const {
+        return std::max<int64_t>(1, std::min<int64_t>((int64_t)num_sms() * 8,
+                                                      ceil_div<int64_t>(this->prm.n, kRecheckThreads)));
+    }
+
+    int assign_pass(const float *cur, const LoopState *guard) {
         const FitParams<float, I> &p = this->prm;
         cudaStream_t s = p.stream;
         KMC_TRY(centroid_prep(cur, guard));
@@ -2162,46 +1982,23 @@ struct MixedFit : PlainFit<float, I> {
         a.nx = nx;
         a.ndx = ndx;
         a.consts = consts;
-        a.X = p.X;
-        a.w = p.w;
         a.labels = p.labels;
-        a.sums32 = sums32;
-        a.acc64 = acc64;
-        a.n_copies = n_copies;
-        a.xrow = xrow;
-        a.cand = cand;
         a.flagged = flagged;
         a.n_flagged = n_flagged;
         a.err_global = err_dev;
         a.guard = guard;
         a.n = p.n;
-        a.d = p.d;
-        a.k = p.k;
-        a.k_pad = k_pad;
-        a.d4 = d4;
-        a.update = update;
         a.label64 = sizeof(I) == 8 ? 1 : 0;
-        a.acc_f64 = acc_f64;
         a.stages = stages;
         a.wait_limit = wait_limit;
         a.stall = stall_once;
         a.state = this->state;
         stall_once = 0;
         const int64_t pass_cols = (int64_t)nch * kChunkN;
-        a.k_pad = pass_cols;
         a.k_img = k_pad;
-        a.multi = passes > 1 ? 1 : 0;
-        if (a.multi) a.update = 0;  // the combine accumulates the certified samples
-        a.own_k = a.multi ? 0 : own_k;
-        a.own_f = own_f;
-        a.xq = xq;
-        a.fx = fx_acc();
-        const SmemLayout L = smem_layout(nkb, pass_cols, d4, stages, a.own_k, a.own_f);
-        if ((L.ostage & 15) != 0 || (L.osum & 15) != 0) {
-            set_error("mixed form: misaligned shared-memory sums layout");
-            return KMC_ERR_CUDA;
-        }
-        auto kern = pick_kernel(bf16, nkb, nch, a.multi != 0);
+        const bool multi = passes > 1;
+        const SmemLayout L = smem_layout(nkb, pass_cols, stages);
+        auto kern = pick_kernel(bf16, nkb, nch, multi);
         if (kern == nullptr) {
             set_error("mixed form: no kernel for %d feature blocks and %d chunks", nkb, nch);
             return KMC_ERR_UNSUPPORTED;
@@ -2213,52 +2010,86 @@ struct MixedFit : PlainFit<float, I> {
             for (int ps = 0; ps < passes; ++ps) {
                 a.col0 = (int64_t)ps * pass_cols;
                 a.cand = cand + (int64_t)ps * p.n;
-                a.pmax = pmax + (a.multi ? (int64_t)ps * p.n : 0);
+                a.pmax = pmax + (multi ? (int64_t)ps * p.n : 0);
                 kern<<<(unsigned)grid, kThreadsMixed, L.total, s>>>(a);
                 KMC_TRY(check_launch("mixed_assign"));
                 a.stall = 0;
             }
-            if (a.multi) {
+            if (multi) {
                 combine_kernel<<<grid1d(p.n, 256, num_sms() * 8), 256, 0, s>>>(
-                    pmax, cand, passes, pass_cols, nx, ndx, consts, xrow, p.w, p.labels, a.label64,
-                    update, acc_f64, sums32, acc64, k_pad, d4, n_copies, flagged, n_flagged, p.n,
-                    p.k, guard, fx_acc());
+                    pmax, cand, passes, pass_cols, nx, ndx, consts, p.labels, a.label64, flagged,
+                    n_flagged, p.n, p.k, guard);
                 KMC_TRY(check_launch("mixed_combine"));
             }
         }
-        // enough CTAs for every sample flagged (8 warps of 32 per CTA round),
-        // at most 8 per SM
-        const int64_t rgrid = std::max<int64_t>(
-            1, std::min<int64_t>((int64_t)num_sms() * 8, ceil_div<int64_t>(p.n, kRecheckThreads)));
-        recheck_kernel<<<(unsigned)rgrid, kRecheckThreads, 0, s>>>(
-            xrow, ct, this->hn, p.w, cand, flagged, n_flagged, p.n, p.d, p.k, d4, p.labels,
-            a.label64, update, acc_f64, sums32, acc64, k_pad, n_copies, guard, passes, pass_cols,
-            fx_acc(), consts, stats);
+        recheck_kernel<<<(unsigned)recheck_grid(), kRecheckThreads, 0, s>>>(
+            xrow, ct, this->hn, cand, flagged, n_flagged, p.n, p.d, p.k, d4, p.labels, a.label64,
+            guard, passes, pass_cols, stats);
         return check_launch("mixed_recheck");
     }
 
+    // The sums' kernel: CTAs, samples of a CTA's tile, rounds of tiles.  The
+    // sorted one has all of its CTAs resident and gives them equal rounds.
+    bool sums_sorted() const { return this->prm.k <= kSortClusters; }
+    int64_t sum_grid() const {
+        const int64_t n = std::max<int64_t>(this->prm.n, 1);
+        const int64_t most = (int64_t)num_sms() * (sums_sorted() ? kSortCtas : 8);
+        return std::min(most, ceil_div<int64_t>(n, kSumThreads));
+    }
+    int sum_tile() const {
+        if (!sums_sorted()) return kSumThreads;
+        const int64_t n = std::max<int64_t>(this->prm.n, 1), g = sum_grid();
+        const int64_t rounds = ceil_div<int64_t>(n, g * kSortTile);
+        return (int)(ceil_div<int64_t>(n, g * rounds * 32) * 32);
+    }
+
+    int sum_pass(const LoopState *guard) {
+        const FitParams<float, I> &p = this->prm;
+        if (sums_sorted()) {
+            const int tile = sum_tile();
+            auto kern = !acc_f64 ? sum_sorted_kernel<I, 0>
+                                 : (variant % 10 == 2 ? sum_sorted_kernel<I, 2> : sum_sorted_kernel<I, 4>);
+            const size_t smem = sort_smem(tile, p.k);
+            if (smem > 48 * 1024)
+                KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)smem));
+            kern<<<(unsigned)sum_grid(), kSumThreads, smem, p.stream>>>(
+                xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32, fx_acc(), acc64, n_copies,
+                consts, guard);
+            return check_launch("mixed_sums");
+        }
+        const unsigned grid = (unsigned)sum_grid();
+        if (acc_f64) {
+            auto kern = variant % 10 == 2 ? sum_terms_kernel<I, 2> : sum_terms_kernel<I, 4>;
+            kern<<<grid, kSumThreads, 0, p.stream>>>(xrow, p.w, p.labels, p.n, d4, p.k, k_pad, fx_acc(),
+                                                     acc64, n_copies, consts, guard);
+        } else {
+            sum_rows_kernel<I><<<grid, kSumThreads, 0, p.stream>>>(xrow, p.w, p.labels, p.n, d4, p.k,
+                                                                   k_pad, sums32, n_copies, guard);
+        }
+        return check_launch("mixed_sums");
+    }
+
     int step_assign_and_accumulate(const float *cur, int64_t *n_launches) override {
-        *n_launches = 3 + (passes > 1 ? passes : 0);
-        return assign_pass(cur, 1, this->state);
+        *n_launches = 4 + (passes > 1 ? passes : 0);
+        KMC_TRY(assign_pass(cur, this->state));
+        return sum_pass(this->state);
     }
 
     int finish_step(int64_t *n_launches) override {
         const FitParams<float, I> &p = this->prm;
         if (acc_f64) {
-            // the assignment of a one-pass fit without shared-memory sums
-            // reduces into the float64 copies itself
-            const MixedSums<double> src{acc64, n_copies, passes == 1 && own_k == 0 ? 1 : 0,
-                                        p.k, k_pad, d4, fx_acc(), consts};
+            const MixedSums<double> src{acc64, n_copies, p.k, k_pad, d4, fx_acc(), consts};
             return launch_reduce_and_finish<float>(src, n_copies, this->finish_args(), n_launches,
                                                    p.stream);
         }
-        const MixedSums<float> src{sums32, n_copies, 1, p.k, k_pad, d4,
-                                   FxAcc{nullptr, nullptr, nullptr, 0, 1, nullptr}, consts};
+        const MixedSums<float> src{sums32, n_copies, p.k, k_pad, d4,
+                                   FxAcc{nullptr, nullptr, 0, 1, nullptr}, consts};
         return launch_reduce_and_finish<float>(src, n_copies, this->finish_args(), n_launches,
                                                p.stream);
     }
 
-    int final_assignment() override { return assign_pass(this->prm.centroids, 0, nullptr); }
+    int final_assignment() override { return assign_pass(this->prm.centroids, nullptr); }
 
     int counters(int64_t *last, int64_t *total, int *device_error) override {
         long long h[2] = {0, 0};

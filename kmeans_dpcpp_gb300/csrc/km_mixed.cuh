@@ -56,6 +56,20 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
+// The same, suspending the thread for a short, bounded time while the phase is
+// open, so that waiting warps leave the issue slots to the working ones.
+__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
+        : "memory");
+    return ok != 0;
+}
+
 // Waits for the phase with the given parity.  Returns false (and raises the
 // CTA error flag) after `limit` SM clocks, or as soon as another role has
 // raised the flag.  A thread may wait only for a phase that cannot be followed by
@@ -66,7 +80,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     if (mbar_test(bar, parity)) return true;
     const long long t0 = clock64();
     while (true) {
-        if (mbar_test(bar, parity)) return true;
+        if (mbar_try(bar, parity)) return true;
         if (*err) return false;
         if (clock64() - t0 > limit) {
             *err = 1;

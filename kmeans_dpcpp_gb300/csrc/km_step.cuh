@@ -111,36 +111,41 @@ struct ReducedSums {
     }
 };
 
-// Private copies -> sums and sizes.  A CTA takes 32 consecutive elements; 16
-// threads share an element's copies (g, g + 16, ..., then the 16 partial sums
-// in order: a fixed order, so float64 fits stay reproducible).  One thread per
-// element walked 304 copies as a chain of memory latencies: 46 us for 240
-// elements, 5 us now.
+// Private copies -> sums and sizes.  G threads share an element's copies (g, g +
+// G, ..., then the G partial sums in order: a fixed order, so float64 fits stay
+// reproducible); a CTA takes kReduceThreads / G consecutive elements.  One
+// thread per element walked 304 copies as a chain of memory latencies: 46 us
+// for 240 elements, 5 us with 16.  Up to kFewCopies copies four threads do, and
+// the grid is a quarter (4 copies of 132,096 elements: 39 -> 23 us).
 constexpr int kReduceLanes = 32, kReduceGroups = 16;
+constexpr int kReduceThreads = kReduceLanes * kReduceGroups, kFewCopies = 8;
 
-template <typename T, typename Src>
-__global__ void __launch_bounds__(kReduceLanes * kReduceGroups)
+template <typename T, typename Src, int G>
+__global__ void __launch_bounds__(kReduceThreads)
     reduce_sums_kernel(Src src, T *sums, T *sizes, int64_t d, int64_t k, const LoopState *state) {
     if (*reinterpret_cast<const volatile int *>(&state->done)) return;
-    __shared__ typename Src::Part red[kReduceGroups][kReduceLanes];
-    const int el = threadIdx.x % kReduceLanes, g = threadIdx.x / kReduceLanes;
-    const int64_t e = blockIdx.x * (int64_t)kReduceLanes + el;
+    constexpr int kLanes = kReduceThreads / G;
+    __shared__ typename Src::Part red[G][kLanes];
+    const int el = threadIdx.x % kLanes, g = threadIdx.x / kLanes;
+    const int64_t e = blockIdx.x * (int64_t)kLanes + el;
     int64_t f = 0, j = 0;
     typename Src::Part p = Src::zero();
     if (e < (d + 1) * k) {
         src.at(e, d, &f, &j);
-        p = src.load(f, j, d, g, kReduceGroups);
+        p = src.load(f, j, d, g, G);
     }
     red[g][el] = p;
     __syncthreads();
-    if (g < 4) {
-        p = red[4 * g][el];
+    if constexpr (G > 4) {
+        if (g < 4) {
+            p = red[G / 4 * g][el];
 #pragma unroll
-        for (int q = 1; q < 4; ++q) Src::add(p, red[4 * g + q][el]);
+            for (int q = 1; q < G / 4; ++q) Src::add(p, red[G / 4 * g + q][el]);
+        }
+        __syncthreads();
+        if (g < 4) red[g][el] = p;
+        __syncthreads();
     }
-    __syncthreads();
-    if (g < 4) red[g][el] = p;
-    __syncthreads();
     if (g == 0 && e < (d + 1) * k) {
 #pragma unroll
         for (int q = 1; q < 4; ++q) Src::add(p, red[q][el]);
@@ -302,9 +307,10 @@ int launch_reduce_and_finish(const Src &src, int64_t copies, const FinishArgs<T>
     *n_launches = 1;
     if (copies <= kDirectCopies) return launch_finish<T>(src, a, s);
     *n_launches = 2;
-    const int64_t grid = ceil_div<int64_t>((a.d + 1) * a.k, kReduceLanes);
-    reduce_sums_kernel<T, Src><<<(unsigned)grid, kReduceLanes * kReduceGroups, 0, s>>>(
-        src, a.sums, a.sizes, a.d, a.k, a.state);
+    const bool few = copies <= kFewCopies;
+    const int64_t grid = ceil_div<int64_t>((a.d + 1) * a.k, kReduceThreads / (few ? 4 : kReduceGroups));
+    auto kern = few ? reduce_sums_kernel<T, Src, 4> : reduce_sums_kernel<T, Src, kReduceGroups>;
+    kern<<<(unsigned)grid, kReduceThreads, 0, s>>>(src, a.sums, a.sizes, a.d, a.k, a.state);
     KMC_TRY(check_launch("reduce_sums"));
     return launch_finish<T>(ReducedSums<T>{a.sums, a.sizes, a.k}, a, s);
 }
