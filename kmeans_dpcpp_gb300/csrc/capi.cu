@@ -68,6 +68,7 @@ cudaMemPool_t scratch_pool() {
 }
 
 int trim_pools() {
+    release_host_slots();
     std::lock_guard<std::mutex> lk(g_pool_mu);
     for (int d = 0; d < 64; ++d)
         if (g_pools[d] != nullptr) KMC_CUDA_TRY(cudaMemPoolTrimTo(g_pools[d], 0));

@@ -20,12 +20,81 @@
 #include <algorithm>
 #include <cstdarg>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "km_kernels.cuh"
 #include "km_fit.cuh"
 
 namespace kmc {
+
+namespace {
+struct KeptSlot {
+    HostSlot *p;
+    cudaEvent_t ev[2];
+    int device;
+};
+std::mutex g_slots_mutex;
+std::vector<KeptSlot> g_slots;
+
+void free_slot(const KeptSlot &k) {
+    for (cudaEvent_t e : k.ev)
+        if (e != nullptr) cudaEventDestroy(e);
+    if (k.p != nullptr) cudaFreeHost(k.p);
+}
+}  // namespace
+
+HostSlotRef::HostSlotRef() {
+    if (cudaGetDevice(&device) != cudaSuccess) return;
+    {
+        std::lock_guard<std::mutex> lock(g_slots_mutex);
+        for (size_t q = 0; q < g_slots.size(); ++q)
+            if (g_slots[q].device == device) {
+                p = g_slots[q].p;
+                ev[0] = g_slots[q].ev[0];
+                ev[1] = g_slots[q].ev[1];
+                g_slots.erase(g_slots.begin() + (long)q);
+                return;
+            }
+    }
+    KeptSlot k{nullptr, {nullptr, nullptr}, device};
+    void *mem = nullptr;
+    if (cudaHostAlloc(&mem, sizeof(HostSlot), cudaHostAllocDefault) == cudaSuccess)
+        k.p = static_cast<HostSlot *>(mem);
+    bool ok = k.p != nullptr;
+    for (cudaEvent_t &e : k.ev)
+        ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {
+        free_slot(k);
+        cudaGetLastError();  // the caller goes on without
+        return;
+    }
+    p = k.p;
+    ev[0] = k.ev[0];
+    ev[1] = k.ev[1];
+}
+
+HostSlotRef::~HostSlotRef() {
+    if (p == nullptr) return;
+    const KeptSlot k{p, {ev[0], ev[1]}, device};
+    {
+        std::lock_guard<std::mutex> lock(g_slots_mutex);
+        if (g_slots.size() < (size_t)kKeptHostSlots) {
+            g_slots.push_back(k);
+            return;
+        }
+    }
+    free_slot(k);
+}
+
+void release_host_slots() {
+    std::vector<KeptSlot> drop;
+    {
+        std::lock_guard<std::mutex> lock(g_slots_mutex);
+        drop.swap(g_slots);
+    }
+    for (const KeptSlot &k : drop) free_slot(k);
+}
 
 template <typename T, typename I>
 int PlainFit<T, I>::init(const FitParams<T, I> &p) {
@@ -199,9 +268,88 @@ int PlainFit<T, I>::read_state(LoopState &out) {
     return check_device_error(out);
 }
 
+// Two batches of iterations are in flight: while one runs, the host waits for
+// the loop state at the end of the one before, so the device never waits for
+// the host (reading the state after each of batches of 1, 2, 4, ... iterations
+// left it idle for 15 to 30 us each; 50,000 x 14, 20 iterations: 742 -> 706 us,
+// 300,000 x 100 bf16, 6 iterations: 1357 -> 1311).  Batches stay small: what is enqueued
+// behind the end of the loop, or behind a pause, still costs a few launches
+// that return at once.
+template <typename T, typename I>
+int PlainFit<T, I>::run_pipelined(HostSlotRef &slot) {
+    constexpr int64_t kMaxBatch = 4;
+    const FitParams<T, I> &p = prm;
+    LoopState h{};
+    if (issued == 0) {
+        h.done = host_done;  // nothing has run: as init left it
+    } else {
+        KMC_TRY(read_state(h));
+    }
+    // iterations of the batches in flight, oldest first
+    int64_t in_flight[2] = {0, 0};
+    int first = 0, flying = 0;
+    auto send = [&](int64_t m) -> int {
+        for (int64_t t = 0; t < m; ++t) KMC_TRY(enqueue_iteration(false));
+        const int q = (first + flying) & 1;
+        KMC_CUDA_TRY(cudaMemcpyAsync(&slot.p->st[q], state, sizeof(LoopState),
+                                     cudaMemcpyDeviceToHost, p.stream));
+        ++flying;  // a copy into the slot is under way, whatever follows
+        in_flight[q] = m;
+        KMC_CUDA_TRY(cudaEventRecord(slot.ev[q], p.stream));
+        return KMC_OK;
+    };
+    auto receive = [&]() -> int {
+        KMC_CUDA_TRY(cudaEventSynchronize(slot.ev[first]));
+        h = slot.p->st[first];
+        first ^= 1;
+        --flying;
+        return KMC_OK;
+    };
+    auto loop = [&]() -> int {
+        int64_t batch = 1;
+        if (h.done == kPaused) {
+            KMC_TRY(enqueue_relocation());
+            KMC_TRY(send(0));
+            KMC_TRY(receive());
+            KMC_TRY(check_device_error(h));
+        }
+        while (true) {
+            while (flying < 2 && !h.done) {
+                int64_t ahead = h.n_iter;
+                for (int q = 0; q < flying; ++q) ahead += in_flight[(first + q) & 1];
+                const int64_t m = std::min(batch, p.max_iter - ahead);
+                if (m <= 0) break;
+                KMC_TRY(send(m));
+                batch = std::min(2 * batch, kMaxBatch);
+            }
+            if (flying == 0) return KMC_OK;
+            KMC_TRY(receive());
+            KMC_TRY(check_device_error(h));
+            if (h.done == 0) continue;
+            // nothing behind the end or the pause did anything
+            while (flying > 0) KMC_TRY(receive());
+            if (h.done != kPaused) return check_device_error(h);
+            KMC_TRY(enqueue_relocation());  // ends the paused iteration
+            ++h.n_iter;
+            h.done = 0;
+            batch = 1;
+            if (h.n_iter >= p.max_iter) KMC_TRY(send(0));
+        }
+    };
+    const int rc = loop();
+    host_done = h.done;
+    // no copy into the slot outlives this call
+    if (flying > 0) cudaStreamSynchronize(p.stream);
+    return rc;
+}
+
 template <typename T, typename I>
 int PlainFit<T, I>::run(int64_t max_batch) {
     const FitParams<T, I> &p = prm;
+    if (!p.verbose && max_batch <= 0) {
+        HostSlotRef slot;
+        if (slot.p != nullptr) return run_pipelined(slot);
+    }
     LoopState h{};
     KMC_TRY(read_state(h));
     int64_t batch = 1;
@@ -261,8 +409,16 @@ template <typename T, typename I>
 int PlainFit<T, I>::finalize(int64_t *n_iter_out, double *inertia_out) {
     LoopState h{};
     double tot = 0.0;
-    KMC_TRY(finalize_enqueue(&h, &tot));
-    KMC_CUDA_TRY(cudaStreamSynchronize(prm.stream));
+    {
+        HostSlotRef slot;  // pinned, so that the second copy does not wait for the first
+        LoopState *hs = slot.p != nullptr ? &slot.p->st[0] : &h;
+        double *ts = slot.p != nullptr ? &slot.p->inertia : &tot;
+        const int rc = finalize_enqueue(hs, ts);
+        KMC_CUDA_TRY(cudaStreamSynchronize(prm.stream));
+        KMC_TRY(rc);
+        h = *hs;
+        tot = *ts;
+    }
     host_done = h.done;
     KMC_TRY(check_device_error(h));
     if (n_iter_out) *n_iter_out = h.n_iter;

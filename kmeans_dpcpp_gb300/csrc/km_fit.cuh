@@ -92,6 +92,27 @@ struct FitBase {
     }
 };
 
+// Pinned host memory for a fit's loop state (two reads in flight) and inertia,
+// with the events that mark the reads.  Allocating pinned memory costs more
+// than a small fit, so freed slots are kept: at most kKeptHostSlots, given back
+// by trim_pools().  Any thread may take and return them; a slot belongs to the
+// device that was current when it was made.
+struct HostSlot {
+    LoopState st[2];
+    double inertia;
+};
+constexpr int kKeptHostSlots = 16;
+struct HostSlotRef {
+    HostSlot *p = nullptr;  // null: no pinned memory was to be had
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    int device = -1;
+    HostSlotRef();
+    ~HostSlotRef();
+    HostSlotRef(const HostSlotRef &) = delete;
+    HostSlotRef &operator=(const HostSlotRef &) = delete;
+};
+void release_host_slots();
+
 template <typename T, typename I>
 struct PlainFit : FitBase {
     FitParams<T, I> prm;
@@ -120,6 +141,7 @@ struct PlainFit : FitBase {
     int enqueue_relocation() override;
     int read_state(LoopState &out) override;
     int run(int64_t max_batch) override;
+    int run_pipelined(HostSlotRef &slot);
     int finalize(int64_t *n_iter_out, double *inertia_out) override;
     int finalize_enqueue(LoopState *state_out, double *inertia_out) override;
     const LoopState *device_state() const override { return state; }
