@@ -74,6 +74,7 @@
 #include <vector>
 
 #include "km_batch.cuh"
+#include "km_dist.cuh"
 #include "km_fit.cuh"
 #include "km_mixed.cuh"
 #include "km_step.cuh"
@@ -275,25 +276,6 @@ __host__ __device__ inline int pack_fixed(float v, int emin) {
     const int m = (int)((b & 0x7fffffu) | 0x800000u);
     const int ms = (b >> 31) ? -m : m;
     return (int)(((uint32_t)ms << 6) | (sh << 1));
-}
-
-// Packed fixed-point terms of every sample: w x_j for j < d4 (rounded
-// products, as the reference forms them), then w, 0, 0, 0.
-__global__ void fx_pack_kernel(const float *xrow, const float *w, int64_t n, int64_t d4,
-                               const MixedConsts *c, int *xq) {
-    const int64_t ds = d4 + 4;
-    const int emin = 150 - c->fx_shift;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * ds;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = e / ds, j = e - i * ds;
-        const float wi = w[i];
-        float v = 0.f;
-        if (j < d4)
-            v = __fmul_rn(xrow[i * d4 + j], wi);
-        else if (j == d4)
-            v = wi;
-        xq[e] = pack_fixed(v, emin);
-    }
 }
 
 template <int BF16>
@@ -649,13 +631,38 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
 // ---------------------------------------------------------------------------
 // preparation kernels
 // ---------------------------------------------------------------------------
-__global__ void absmax_kernel(const float *X, int64_t count, unsigned int *out_bits) {
+// max |X[e]| (NaNs lose).  One atomic per CTA: one per warp of 4096 CTAs took 27
+// us whatever the size (1M floats now 3 us; 640M floats 440 -> 367 us, 7.0 TB/s).
+constexpr int kAbsmaxThreads = 256;
+__global__ void __launch_bounds__(kAbsmaxThreads)
+    absmax_kernel(const float *X, int64_t count, unsigned int *out_bits) {
+    __shared__ float red[kAbsmaxThreads / 32];
+    constexpr int kBatch = 4;
+    const int64_t tid = blockIdx.x * (int64_t)kAbsmaxThreads + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kAbsmaxThreads;
     float m = 0.f;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count;
-         e += (int64_t)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(X[e]));
+    // whole float4s from the first 16-byte boundary on, the rest one by one
+    const int64_t head = min(count, (int64_t)((16u - ((uint32_t)reinterpret_cast<uintptr_t>(X) & 15u)) & 15u) / 4);
+    const int64_t vecs = (count - head) / 4;
+    const float4 *V = reinterpret_cast<const float4 *>(X + head);
+    for (int64_t e = tid; e < vecs; e += kBatch * step) {
+        float4 v[kBatch];
+#pragma unroll
+        for (int t = 0; t < kBatch; ++t) v[t] = load_f4_if(V + e + t * step, e + t * step < vecs);
+#pragma unroll
+        for (int t = 0; t < kBatch; ++t)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[t].x), fabsf(v[t].y)), fmaxf(fabsf(v[t].z), fabsf(v[t].w))));
+    }
+    if (tid < head) m = fmaxf(m, fabsf(X[tid]));
+    const int64_t rest = head + 4 * vecs + tid;
+    if (rest < count) m = fmaxf(m, fabsf(X[rest]));
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m == m) atomicMax(out_bits, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < kAbsmaxThreads / 32; ++q) m = fmaxf(m, red[q]);
+        atomicMax(out_bits, __float_as_uint(m));
+    }
 }
 
 // fp16 operands: sigma is the largest power of two in [2^-60, 2^60] with
@@ -709,14 +716,19 @@ __device__ __forceinline__ float round16(float v) {
     return __half2float(__float2half_rn(v));
 }
 
-// One CTA per 128-sample tile (including the zero rows that pad the last
+// One-time conversion of X.  A CTA takes one 128-sample tile at a time (the image
+// holds K blocks of 64 features, zero-padded, for every 128-sample
 // tile): the tile's features are staged in shared memory (coalesced reads of
 // each feature's 128 samples from a feature-major X, or of each sample's d
 // features from a row-major one), then written out as the 128-byte-swizzled
 // K-major image of (x * sigma) and the row-major fp32 copy of x (features
 // d..d4-1 zero), both as contiguous 16-byte chunks, and per sample ||x|| and
 // the norm of the image's rounding error ||round16(x sigma) - x sigma|| /
-// sigma, both rounded up.
+// sigma, both rounded up; with xq also the packed fixed-point terms (w x_j
+// rounded as the reference forms it, then w, 0, 0, 0).
+// Bound by memory.  10M x 64: 1.41 -> 1.29 ms (the norms had a loop of their own in
+// half of the threads); 1M x 16 with packed terms, which had a kernel of their
+// own: 139 -> 89 us.
 constexpr int kXImageThreads = 256;
 constexpr int kXsPitch = kTileM + 1;  // floats per staged feature (bank offset)
 
@@ -727,68 +739,115 @@ __host__ __device__ inline size_t x_image_smem(int nkb) {
 template <int BF16>
 __global__ void __launch_bounds__(kXImageThreads) x_image_kernel(
     const float *X, int64_t n, int64_t d, int64_t d4, int nkb, int64_t ntiles,
-    const MixedConsts *c, uint8_t *img, float *xrow, float *nx, float *ndx, int rowmajor) {
+    const MixedConsts *c, uint8_t *img, float *xrow, float *nx, float *ndx, int rowmajor,
+    const float *w, int *xq) {
     extern __shared__ float xs[];  // [feature][kXsPitch]
+    constexpr int kBatch = 8;
+    constexpr int kRows = 4;  // rows of a thread in each feature block
+    static_assert(kRows * kXImageThreads == kTileM * 8, "eight lanes per row");
     const float sigma = c->sigma;
-    const int F = nkb * 64;
-    const int g4 = (int)(d4 / 4);
+    const int F = nkb * 64, tid = threadIdx.x;
+    const int g4 = (int)(d4 / 4), emin = 150 - c->fx_shift;
+    // the padding features stay zero
+    for (int e = (int)d * kXsPitch + tid; e < F * kXsPitch; e += kXImageThreads) xs[e] = 0.f;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t i0 = tile * kTileM;
-        if (rowmajor) {
-            for (int e = threadIdx.x; e < F * kTileM; e += kXImageThreads) {
-                const int r = e / F, f = e - r * F;
-                const int64_t i = i0 + r;
-                xs[f * kXsPitch + r] = (f < d && i < n) ? X[i * d + f] : 0.f;
+        const int rows_here = (n - i0 < (int64_t)kTileM) ? (int)(n - i0) : kTileM;
+        const int total = (int)d * kTileM;
+        for (int e0 = tid; e0 < total; e0 += kBatch * kXImageThreads) {
+            float v[kBatch];
+            int o[kBatch];
+#pragma unroll
+            for (int t = 0; t < kBatch; ++t) {
+                const int e = e0 + t * kXImageThreads;
+                int f, r;
+                if (rowmajor) {
+                    r = e / (int)d;
+                    f = e - r * (int)d;
+                } else {
+                    f = e >> 7;
+                    r = e & (kTileM - 1);
+                }
+                o[t] = e < total ? f * kXsPitch + r : -1;
+                const float *src = rowmajor ? X + (i0 + r) * d + f : X + (int64_t)f * n + i0 + r;
+                v[t] = load_f_if(src, e < total && r < rows_here);
             }
-        } else {
-            for (int e = threadIdx.x; e < F * kTileM; e += kXImageThreads) {
-                const int f = e >> 7, r = e & (kTileM - 1);
-                const int64_t i = i0 + r;
-                xs[f * kXsPitch + r] = (f < d && i < n) ? X[(int64_t)f * n + i] : 0.f;
-            }
+#pragma unroll
+            for (int t = 0; t < kBatch; ++t)
+                if (o[t] >= 0) xs[o[t]] = v[t];
         }
         __syncthreads();
         // image: 16-byte chunk q of feature block kb holds row r, features
-        // 8 ch .. 8 ch + 7 with ch = (q mod 8) xor (r mod 8) (128-byte swizzle)
-        for (int q = threadIdx.x; q < nkb * 1024; q += kXImageThreads) {
-            const int kb = q >> 10, qq = q & 1023;
+        // 8 ch .. 8 ch + 7 with ch = (q mod 8) xor (r mod 8) (128-byte swizzle);
+        // the eight lanes of a row also sum its squares.  (An upper bound of
+        // the norms needs no order: see below.)
+        float s2[kRows] = {0.f, 0.f, 0.f, 0.f}, sd[kRows] = {0.f, 0.f, 0.f, 0.f};
+        for (int kb = 0; kb < nkb; ++kb) {
+#pragma unroll
+            for (int t = 0; t < kRows; ++t) {
+                const int qq = tid + t * kXImageThreads;
+                const int r = (qq >> 6) * 8 + ((qq >> 3) & 7);
+                const int ch = (qq & 7) ^ (r & 7);
+                const float *src = xs + (kb * 64 + ch * 8) * kXsPitch + r;
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float x = src[e * kXsPitch];
+                    s2[t] = __fmaf_rn(x, x, s2[t]);
+                    v[e] = x * sigma;
+                    const float dv = round16<BF16>(v[e]) - v[e];  // exact
+                    sd[t] = __fmaf_rn(dv, dv, sd[t]);
+                }
+                uint4 pk;
+                pk.x = pack2<BF16>(v[0], v[1]);
+                pk.y = pack2<BF16>(v[2], v[3]);
+                pk.z = pack2<BF16>(v[4], v[5]);
+                pk.w = pack2<BF16>(v[6], v[7]);
+                *reinterpret_cast<uint4 *>(img + ((size_t)tile * nkb + kb) * kTileBytes +
+                                           (size_t)qq * 16) = pk;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kRows; ++t) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                s2[t] += __shfl_xor_sync(0xffffffffu, s2[t], o);
+                sd[t] += __shfl_xor_sync(0xffffffffu, sd[t], o);
+            }
+            const int qq = tid + t * kXImageThreads;
             const int r = (qq >> 6) * 8 + ((qq >> 3) & 7);
-            const int ch = (qq & 7) ^ (r & 7);
-            const float *src = xs + (kb * 64 + ch * 8) * kXsPitch + r;
-            uint4 pk;
-            pk.x = pack2<BF16>(src[0 * kXsPitch] * sigma, src[1 * kXsPitch] * sigma);
-            pk.y = pack2<BF16>(src[2 * kXsPitch] * sigma, src[3 * kXsPitch] * sigma);
-            pk.z = pack2<BF16>(src[4 * kXsPitch] * sigma, src[5 * kXsPitch] * sigma);
-            pk.w = pack2<BF16>(src[6 * kXsPitch] * sigma, src[7 * kXsPitch] * sigma);
-            *reinterpret_cast<uint4 *>(img + ((size_t)tile * nkb + kb) * kTileBytes +
-                                       (size_t)qq * 16) = pk;
+            if ((tid & 7) == 0 && r < rows_here) {
+                // A float32 sum of m non-negative terms, in any order, is at
+                // least (1 - 2^-24)^m times the exact sum (each term passes at
+                // most m roundings); m <= 256 here, so the factor 1 + (m + 2)
+                // 2^-23 applied with upward rounding (and an upward square
+                // root) gives upper bounds of both norms (1 / sigma is a power
+                // of two).
+                const float grow = 1.f + (float)(nkb * 64 + 2) * 0x1p-23f;
+                nx[i0 + r] = __fsqrt_ru(__fmul_ru(s2[t], grow));
+                ndx[i0 + r] = __fmul_ru(__fsqrt_ru(__fmul_ru(sd[t], grow)), 1.f / sigma);
+            }
         }
         // row-major fp32 rows: the tile's block of xrow is contiguous
-        const int rows_here = (n - i0 < (int64_t)kTileM) ? (int)(n - i0) : kTileM;
-        for (int e = threadIdx.x; e < rows_here * g4; e += kXImageThreads) {
+        for (int e = tid; e < rows_here * g4; e += kXImageThreads) {
             const int r = e / g4, g = e - r * g4;
             const float *src = xs + (4 * g) * kXsPitch + r;
-            reinterpret_cast<float4 *>(xrow + (i0 + r) * d4)[g] =
+            reinterpret_cast<float4 *>(xrow + i0 * d4)[e] =
                 make_float4(src[0], src[kXsPitch], src[2 * kXsPitch], src[3 * kXsPitch]);
         }
-        if (threadIdx.x < kTileM && threadIdx.x < rows_here) {
-            const int r = threadIdx.x;
-            float s2 = 0.f, sd = 0.f;  // float32 sums, bounded from above below
-            for (int f = 0; f < F; ++f) {
-                const float x = xs[f * kXsPitch + r];
-                s2 = __fmaf_rn(x, x, s2);
-                const float v = x * sigma;
-                const float dv = round16<BF16>(v) - v;  // exact
-                sd = __fmaf_rn(dv, dv, sd);
+        if (xq != nullptr) {
+            for (int e = tid; e < rows_here * (g4 + 1); e += kXImageThreads) {
+                const int r = e / (g4 + 1), g = e - r * (g4 + 1);
+                const float wi = w[i0 + r];
+                const float *src = xs + (4 * g) * kXsPitch + r;
+                int4 q = make_int4(pack_fixed(wi, emin), 0, 0, 0);
+                if (g < g4)
+                    q = make_int4(pack_fixed(__fmul_rn(src[0], wi), emin),
+                                  pack_fixed(__fmul_rn(src[kXsPitch], wi), emin),
+                                  pack_fixed(__fmul_rn(src[2 * kXsPitch], wi), emin),
+                                  pack_fixed(__fmul_rn(src[3 * kXsPitch], wi), emin));
+                reinterpret_cast<int4 *>(xq + i0 * (d4 + 4))[e] = q;
             }
-            // A float32 sum of m non-negative terms (each rounded once) is at
-            // least (1 - 2^-24)^m times the exact sum; m <= 128 here, so the
-            // factor 1 + (m + 2) 2^-23 applied with upward rounding (and an
-            // upward square root) gives upper bounds of both norms (1 / sigma
-            // is a power of two).
-            const float grow = 1.f + (float)(nkb * 64 + 2) * 0x1p-23f;
-            nx[i0 + r] = __fsqrt_ru(__fmul_ru(s2, grow));
-            ndx[i0 + r] = __fmul_ru(__fsqrt_ru(__fmul_ru(sd, grow)), 1.f / sigma);
         }
         __syncthreads();
     }
@@ -1177,32 +1236,6 @@ __global__ void __launch_bounds__(256) combine_kernel(
 // red.v4.f32, 13 of red.u64).
 // ---------------------------------------------------------------------------
 constexpr int kSumThreads = 256;
-
-// Predicated read-only loads (0 when not in).  Volatile: plain loads would be
-// moved into the branch of the reduction that uses them, one latency each.
-__device__ __forceinline__ float4 load_f4_if(const float4 *p, bool in) {
-    float4 v;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.u32 p, %5, 0;\n\t"
-        "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
-        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-        "@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-        : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
-        : "l"(p), "r"((uint32_t)in));
-    return v;
-}
-__device__ __forceinline__ int load_i_if(const int *p, bool in) {
-    int v;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.u32 p, %2, 0;\n\t"
-        "mov.s32 %0, 0;\n\t"
-        "@p ld.global.nc.s32 %0, [%1];\n\t}"
-        : "=&r"(v)
-        : "l"(p), "r"((uint32_t)in));
-    return v;
-}
 
 template <typename I>
 __device__ __forceinline__ int label_of(const I *labels, int64_t i, int64_t n, int64_t k) {
@@ -1613,6 +1646,12 @@ bool pass_plan(int nkb, int64_t kp, int *nch_out, int *stages_out) {
     return false;
 }
 
+// Four float4s per thread and round, at most eight CTAs per SM.
+unsigned absmax_grid(int64_t count) {
+    return (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>(ceil_div<int64_t>(count, 16 * kAbsmaxThreads), (int64_t)num_sms() * 8));
+}
+
 unsigned grid1d(int64_t work, int block, int cap = 8192) {
     int64_t g = ceil_div<int64_t>(work, block);
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(g, cap));
@@ -1908,13 +1947,13 @@ struct MixedFit : PlainFit<float, I> {
         KMC_CUDA_TRY(cudaMemsetAsync(n_flagged, 0, sizeof(int) * 4, s));
         KMC_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(long long) * 2, s));
         // one-time conversion of X (charged to the fit, reported separately)
-        absmax_kernel<<<grid1d(p.n * p.d, 256, 4096), 256, 0, s>>>(p.X, p.n * p.d,
-                                                                    &consts->xmax_bits);
+        absmax_kernel<<<absmax_grid(p.n * p.d), kAbsmaxThreads, 0, s>>>(p.X, p.n * p.d,
+                                                                       &consts->xmax_bits);
         KMC_TRY(check_launch("absmax"));
         sigma_kernel<<<1, 1, 0, s>>>(consts, bf16, p.d);
         KMC_TRY(check_launch("sigma"));
         if (fx_on) {
-            absmax_kernel<<<grid1d(p.n, 256, 4096), 256, 0, s>>>(p.w, p.n, &consts->wmax_bits);
+            absmax_kernel<<<absmax_grid(p.n), kAbsmaxThreads, 0, s>>>(p.w, p.n, &consts->wmax_bits);
             KMC_TRY(check_launch("absmax_w"));
             // rows that one copy of the sums adds up at most
             const int64_t g = sum_grid(), tile = sum_tile();
@@ -1932,16 +1971,11 @@ struct MixedFit : PlainFit<float, I> {
                                                   (int)xsm));
             const int64_t xg = std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)num_sms() * 8));
             xk<<<(unsigned)xg, kXImageThreads, xsm, s>>>(p.X, p.n, p.d, d4, nkb, ntiles, consts,
-                                                         ximg, xrow, nx, ndx, p.x_rowmajor);
+                                                         ximg, xrow, nx, ndx, p.x_rowmajor, p.w,
+                                                         fx_on ? xq : nullptr);
         }
         KMC_TRY(check_launch("x_image"));
         this->launches += 3;
-        if (fx_on) {
-            fx_pack_kernel<<<grid1d(p.n * (d4 + 4), 256, 8192), 256, 0, s>>>(xrow, p.w, p.n, d4,
-                                                                           consts, xq);
-            KMC_TRY(check_launch("fx_pack"));
-            this->launches += 1;
-        }
         return KMC_OK;
     }
 
