@@ -88,8 +88,18 @@ __device__ __forceinline__ double fma_k(double a, double b, double c) { return _
 // sequentially, from shared memory, otherwise.  Updating, summing and picking
 // in one launch leaves one pass over X_t per centre.  A whole estimator fit of
 // 200,003 x 32, 64 centres, 20 iterations: 70.8 -> 7.8 ms, labels unchanged.
-constexpr int kPPThreads = 512;
+//
+// A block is split into kPPParts parts, a CTA's work at a time, so that few
+// samples still fill the SMs (a CTA per block: 49 CTAs and 42 us per centre at
+// 200,003 x 32, now 15 us).  The CTA that finishes a block's last part forms the
+// block's sum, and the one that finishes the last block draws; the parts' sums
+// also narrow the draw to one part, which a single warp searches.
+constexpr int kPPThreads = 256;
 constexpr int kPPOwn = kPPBlock / kPPThreads;  // samples per thread and block
+constexpr int kPPParts = 8;
+constexpr int kPPPart = kPPBlock / kPPParts;
+constexpr int kPPMine = kPPPart / kPPThreads;  // samples per thread and part
+constexpr int kPPWarpBlocks = 1024;  // block sums that one warp draws from
 constexpr int kPPWarps = kPPThreads / 32;
 constexpr int kKeyNone = 1 << 20, kKeyFail = -(1 << 20);
 
@@ -108,11 +118,57 @@ __device__ __forceinline__ int exponent_field(double v) {
     return (int)((__double_as_longlong(v) >> 52) & 0x7ff);
 }
 
+// Sums whose terms are all multiples of L = 2^(key - 1075) and stay below
+// 2^53 L are formed in units of L with 64-bit integers: float64 operations run
+// at 2 per clock and SM with 60 clocks of latency (the draw took 19 K of a
+// centre's 33 K clocks with them).
+
+// v / L; v a non-negative multiple of L.  ok is cleared at 2^53 and above.
+__device__ __forceinline__ long long units_of(double v, int key, bool &ok) {
+    const long long b = __double_as_longlong(v);
+    if (b == 0) return 0;
+    const int s = exponent_field(v) - key;
+    if (s > 0) {
+        ok = false;
+        return 0;
+    }
+    return s < -52 ? 0 : ((b & 0xfffffffffffffll) | 0x10000000000000ll) >> -s;
+}
+// units L as a float64; exact below 2^53.
+__device__ __forceinline__ double from_units(long long units, int key) {
+    return units == 0 ? 0.0 : ldexp((double)units, key - 1075);
+}
+
+// w m = p 2^(e - 1075) of two floats, p < 2^48 exact; false when negative,
+// infinite or NaN.
+__device__ __forceinline__ bool float_term(float w, float m, unsigned long long &p, int &e) {
+    const unsigned a = __float_as_uint(w), b = __float_as_uint(m);
+    const unsigned ea = (a >> 23) & 0xffu, eb = (b >> 23) & 0xffu;
+    const unsigned ma = (a & 0x7fffffu) | (ea != 0u ? 0x800000u : 0u);
+    const unsigned mb = (b & 0x7fffffu) | (eb != 0u ? 0x800000u : 0u);
+    p = (unsigned long long)ma * mb;
+    e = (int)(max(ea, 1u) + max(eb, 1u)) - 300 + 1075;
+    return ea != 255u && eb != 255u && (p == 0 || (a | b) >> 31 == 0u);
+}
+__device__ __forceinline__ int term_key(unsigned long long p, int e) {
+    return p == 0 ? kKeyNone : e + __ffsll((long long)p) - 1;
+}
+__device__ __forceinline__ long long term_units(unsigned long long p, int e, int key, bool &ok) {
+    if (p == 0) return 0;
+    const int s = e - key;
+    if (64 - __clzll((long long)p) + s > 53) {
+        ok = false;
+        return 0;
+    }
+    return (long long)(s >= 0 ? p << s : p >> -s);
+}
+
 // Block-wide sum (tree) and minimum key; valid in every thread.
 struct PPShared {
     double v[kPPBlock];
     double wsum[kPPWarps];
     int wkey[kPPWarps];
+    long long usum[kPPWarps];
     double scalar;
     int first, last;
     int flag;
@@ -130,12 +186,23 @@ __device__ __forceinline__ void pp_block_sum(PPShared &sh, double &sum, int &key
         sh.wkey[wid] = key;
     }
     __syncthreads();
-    sum = (lane < kPPWarps) ? sh.wsum[lane] : 0.0;
-    key = (lane < kPPWarps) ? sh.wkey[lane] : kKeyNone;
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        key = min(key, __shfl_xor_sync(0xffffffffu, key, o));
+    if (wid == 0) {
+        // float64 additions share 2 lanes per clock: by one warp only
+        sum = lane < kPPWarps ? sh.wsum[lane] : 0.0;
+        key = lane < kPPWarps ? sh.wkey[lane] : kKeyNone;
+        for (int o = kPPWarps / 2; o > 0; o >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            key = min(key, __shfl_xor_sync(0xffffffffu, key, o));
+        }
+        __syncwarp();
+        if (lane == 0) {
+            sh.wsum[0] = sum;
+            sh.wkey[0] = key;
+        }
     }
+    __syncthreads();
+    sum = sh.wsum[0];
+    key = sh.wkey[0];
 }
 
 // Sum of sh.v[0..count) added to `run` one after another (thread 0), each
@@ -178,46 +245,177 @@ __device__ __forceinline__ double pp_exclusive(PPShared &sh, double x) {
     return before + exc;
 }
 
+// v of sample i.
+template <typename T>
+__device__ __forceinline__ double pp_value(const T *w, const T *min_d2, int64_t i, int t) {
+    const double v = w ? (double)w[i] : 1.0;
+    return t > 0 ? __dmul_rn(v, (double)__ldcg(min_d2 + i)) : v;
+}
+
+// The draw among exact sums, by one warp and in units of their common L: the
+// block, its part, the sample.  Returns -1 when some sum's order matters (or
+// none exceeds the target).
+template <typename T>
+__device__ __forceinline__ int64_t pp_draw_exact(const T *w, const T *min_d2, int64_t n, int64_t nb,
+                                                 int t, double u, const double *partials,
+                                                 const int *keys, const double *parts) {
+    const int lane = threadIdx.x & 31;
+    const int per = (int)((nb + 31) / 32);
+    const int b0 = min(lane * per, (int)nb), b1 = min(b0 + per, (int)nb);
+    auto scan = [&](long long x) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        return x;
+    };
+    auto least = [&](int x) { return __reduce_min_sync(0xffffffffu, x); };
+    bool ok = true;
+    int key = kKeyNone;
+    for (int q = b0; q < b1; ++q) key = min(key, __ldcg(keys + q));
+    key = least(key);
+    if (key == kKeyNone || key < 0) return -1;  // nothing to draw, or an order that matters
+    long long own = 0;
+    for (int q = b0; q < b1; ++q) own += units_of(__ldcg(partials + q), key, ok);
+    const long long incl = scan(own), total = __shfl_sync(0xffffffffu, incl, 31);
+    if (__any_sync(0xffffffffu, !ok) || total >= (1ll << 53)) return -1;
+    // a running sum exceeds the target when its units exceed the target's floor
+    const double target = u * from_units(total, key);
+    bool fits = true;
+    long long goal = 0;
+    {
+        const int s = exponent_field(target) - key;
+        if (target > 0.0 && exponent_field(target) > 0 && s > -53)
+            goal = units_of(target, key, fits);
+    }
+    if (!fits) return -1;
+    long long run = incl - own, before = 0;
+    int mine = (int)nb;
+    for (int q = b0; q < b1 && mine == (int)nb; ++q) {
+        before = run;
+        run += units_of(__ldcg(partials + q), key, ok);
+        if (run > goal) mine = q;
+    }
+    const int b = least(mine);
+    if (b >= (int)nb) return -1;
+    before = __shfl_sync(0xffffffffu, before, __ffs(__ballot_sync(0xffffffffu, mine == b)) - 1);
+    // the part
+    const long long part =
+        lane < kPPParts && (int64_t)b * kPPBlock + (int64_t)lane * kPPPart < n
+            ? units_of(__ldcg(parts + (int64_t)b * kPPParts + lane), key, ok)
+            : 0;
+    const long long pincl = before + scan(part);
+    const unsigned past = __ballot_sync(0xffffffffu, lane < kPPParts && pincl > goal);
+    if (past == 0u) return -1;
+    const int p = __ffs(past) - 1;
+    before = __shfl_sync(0xffffffffu, pincl - part, p);
+    // the sample: consecutive ones per lane, their loads unconditional and in
+    // flight together
+    constexpr int kOwn = kPPPart / 32;
+    const int64_t i0 = (int64_t)b * kPPBlock + p * kPPPart + lane * kOwn;
+    long long v[kOwn], sum = 0;
+    {
+        T m[kOwn], wv[kOwn];
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r) m[r] = t > 0 ? __ldcg(min_d2 + min(i0 + r, n - 1)) : T(1);
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r) wv[r] = w ? w[min(i0 + r, n - 1)] : T(1);
+#pragma unroll
+        for (int r = 0; r < kOwn; ++r) {
+            if constexpr (sizeof(T) == 4) {
+                unsigned long long q;
+                int e;
+                ok = float_term(wv[r], m[r], q, e) && ok;
+                v[r] = term_units(q, e, key, ok);
+            } else {
+                v[r] = units_of(__dmul_rn((double)wv[r], (double)m[r]), key, ok);
+            }
+            if (i0 + r >= n) v[r] = 0;
+            sum += v[r];
+        }
+    }
+    long long x = before + scan(sum) - sum;
+    int hit = kPPPart;
+#pragma unroll
+    for (int r = 0; r < kOwn; ++r) {
+        x += v[r];
+        if (hit == kPPPart && v[r] > 0 && x > goal) hit = lane * kOwn + r;
+    }
+    hit = least(hit);
+    return hit < kPPPart ? (int64_t)b * kPPBlock + p * kPPPart + hit : -1;
+}
+
+// Sum of one part's v and its key (kKeyFail: the order matters), valid in every
+// thread; float data in units of L.
+__device__ __forceinline__ void pp_part_sum(PPShared &sh, const unsigned long long (&p)[kPPMine],
+                                            const int (&e)[kPPMine], bool valid, double &sum,
+                                            int &key) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    key = kKeyNone;
+#pragma unroll
+    for (int r = 0; r < kPPMine; ++r) key = min(key, term_key(p[r], e[r]));
+    key = __reduce_min_sync(0xffffffffu, valid ? key : kKeyFail);
+    if (lane == 0) sh.wkey[wid] = key;
+    __syncthreads();
+    key = kKeyNone;
+#pragma unroll
+    for (int q = 0; q < kPPWarps; ++q) key = min(key, sh.wkey[q]);
+    long long units = 0;
+    bool ok = key >= 0;
+    if (ok) {
+#pragma unroll
+        for (int r = 0; r < kPPMine; ++r) units += term_units(p[r], e[r], key, ok);
+    }
+    for (int o = 16; o > 0; o >>= 1) units += __shfl_xor_sync(0xffffffffu, units, o);
+    if (lane == 0) sh.usum[wid] = units;
+    ok = !__syncthreads_or(!ok);
+    units = 0;
+#pragma unroll
+    for (int q = 0; q < kPPWarps; ++q) units += sh.usum[q];
+    if (!ok || units >= (1ll << 53)) key = kKeyFail;
+    sum = key == kKeyFail || key == kKeyNone ? 0.0 : from_units(units, key);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
     const T *__restrict__ Xt, const T *__restrict__ w, T *min_d2, int64_t n, int64_t d, int64_t k,
-    int t, uint64_t seed, double *partials, double *prefix, int *keys, int32_t *chosen, T *Ct,
-    unsigned *ticket) {
+    int t, uint64_t seed, double *partials, double *prefix, int *keys, double *parts, int *part_keys,
+    unsigned *arrived, int32_t *chosen, T *Ct, unsigned *ticket) {
     __shared__ PPShared sh;
     __shared__ T centre[kPPThreads];
     const int tid = threadIdx.x;
-    const int64_t nb = (n + kPPBlock - 1) / kPPBlock;
-    const int64_t c = t > 0 ? (int64_t)chosen[t - 1] : 0;
+    const int64_t nb = (n + kPPBlock - 1) / kPPBlock, items = (n + kPPPart - 1) / kPPPart;
+    bool last_of_all = false;
 
-    for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
-        const int64_t i0 = b * kPPBlock;
-        T acc[kPPOwn];
+    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const int64_t i0 = item * kPPPart;
+        T acc[kPPMine];
 #pragma unroll
-        for (int r = 0; r < kPPOwn; ++r) acc[r] = T(0);
+        for (int r = 0; r < kPPMine; ++r) acc[r] = T(0);
         for (int64_t f0 = 0; t > 0 && f0 < d; f0 += kPPThreads) {
             __syncthreads();
-            if (f0 + tid < d) centre[tid] = Xt[(f0 + tid) * n + c];
+            // the previous centre
+            if (f0 + tid < d) centre[tid] = Ct[(f0 + tid) * k + t - 1];
             __syncthreads();
             const int fn = (int)(d - f0 < kPPThreads ? d - f0 : kPPThreads);
-            if (i0 + kPPBlock <= n) {
-#pragma unroll 2
+            const T *row = Xt + f0 * n + i0 + tid;
+            if (i0 + kPPPart <= n) {
+#pragma unroll 8
                 for (int f = 0; f < fn; ++f) {
-                    const T *row = Xt + (f0 + f) * n + i0 + tid;
                     const T cf = centre[f];
 #pragma unroll
-                    for (int r = 0; r < kPPOwn; ++r) {
-                        const T diff = row[r * kPPThreads] - cf;
+                    for (int r = 0; r < kPPMine; ++r) {
+                        const T diff = row[f * n + r * kPPThreads] - cf;
                         acc[r] = fma_k(diff, diff, acc[r]);
                     }
                 }
             } else {
                 for (int f = 0; f < fn; ++f) {
-                    const T *row = Xt + (f0 + f) * n + i0 + tid;
                     const T cf = centre[f];
 #pragma unroll
-                    for (int r = 0; r < kPPOwn; ++r) {
+                    for (int r = 0; r < kPPMine; ++r) {
                         if (i0 + tid + r * kPPThreads < n) {
-                            const T diff = row[r * kPPThreads] - cf;
+                            const T diff = row[f * n + r * kPPThreads] - cf;
                             acc[r] = fma_k(diff, diff, acc[r]);
                         }
                     }
@@ -226,43 +424,108 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
         }
         double sum = 0.0;
         int key = kKeyNone;
+        T old[kPPMine], wv[kPPMine], m[kPPMine];
 #pragma unroll
-        for (int r = 0; r < kPPOwn; ++r) {
+        for (int r = 0; r < kPPMine; ++r) {
+            const int64_t i = min(i0 + tid + r * kPPThreads, n - 1);
+            old[r] = t > 1 ? min_d2[i] : T(0);
+            wv[r] = w ? w[i] : T(1);
+        }
+#pragma unroll
+        for (int r = 0; r < kPPMine; ++r) {
             const int64_t i = i0 + tid + r * kPPThreads;
-            double v = 0.0;
-            if (i < n) {
-                v = w ? (double)w[i] : 1.0;
-                if (t > 0) {
-                    T m = acc[r];
-                    if (t > 1) {
-                        const T old = min_d2[i];
-                        m = (m < old) ? m : old;
-                    }
-                    min_d2[i] = m;
-                    v = __dmul_rn(v, (double)m);
-                }
+            m[r] = T(1);
+            if (t > 0) {
+                m[r] = acc[r];
+                if (t > 1) m[r] = (m[r] < old[r]) ? m[r] : old[r];
+                if (i < n) min_d2[i] = m[r];
             }
-            sh.v[tid + r * kPPThreads] = v;
-            sum += v;
-            key = min(key, exact_key(v));
+            if (i >= n) wv[r] = m[r] = T(0);
         }
-        pp_block_sum(sh, sum, key);
-        const bool exact = key >= exponent_field(sum);
+        if constexpr (sizeof(T) == 4) {
+            unsigned long long p[kPPMine];
+            int e[kPPMine];
+            bool valid = true;
+#pragma unroll
+            for (int r = 0; r < kPPMine; ++r) valid = float_term(wv[r], m[r], p[r], e[r]) && valid;
+            pp_part_sum(sh, p, e, valid, sum, key);
+        } else {
+#pragma unroll
+            for (int r = 0; r < kPPMine; ++r) {
+                const double v = __dmul_rn((double)wv[r], (double)m[r]);
+                sum += v;
+                key = min(key, exact_key(v));
+            }
+            pp_block_sum(sh, sum, key);
+        }
+        // the CTA that finishes the block's last part sums the block
+        const int64_t b = item / kPPParts;
+        const int have = (int)(items - b * kPPParts < kPPParts ? items - b * kPPParts : kPPParts);
         if (tid == 0) {
-            const int count = (int)(n - i0 < kPPBlock ? n - i0 : kPPBlock);
-            partials[b] = exact ? sum : pp_sequential(sh, 0.0, count, false);
-            keys[b] = exact ? key : kKeyFail;
+            parts[item] = sum;
+            part_keys[item] = key;
+            __threadfence();
+            sh.flag = atomicAdd(arrived + b, 1u) == (unsigned)have - 1u;
         }
-        __syncthreads();  // sh.v is rewritten by the next block
+        __syncthreads();
+        if (!sh.flag) continue;
+        __threadfence();
+        if (tid < 32) {
+            double all = tid < have ? __ldcg(parts + b * kPPParts + tid) : 0.0;
+            int least = tid < have ? __ldcg(part_keys + b * kPPParts + tid) : kKeyNone;
+            for (int o = kPPParts / 2; o > 0; o >>= 1) {
+                all += __shfl_xor_sync(0xffffffffu, all, o);
+                least = min(least, __shfl_xor_sync(0xffffffffu, least, o));
+            }
+            if (tid == 0) {
+                sh.scalar = all;
+                sh.first = least >= exponent_field(all) ? least : kKeyFail;
+            }
+        }
+        __syncthreads();
+        double block_sum = sh.scalar;
+        const int block_key = sh.first;
+        if (block_key == kKeyFail) {
+            const int64_t j0 = b * kPPBlock;
+            const int count = (int)(n - j0 < kPPBlock ? n - j0 : kPPBlock);
+            for (int q = tid; q < count; q += kPPThreads) sh.v[q] = pp_value(w, min_d2, j0 + q, t);
+            __syncthreads();
+            if (tid == 0) block_sum = pp_sequential(sh, 0.0, count, false);
+        }
+        if (tid == 0) {
+            partials[b] = block_sum;
+            keys[b] = block_key;
+            arrived[b] = 0u;  // for the next centre's launch
+            __threadfence();
+            sh.flag = atomicAdd(ticket, 1u) == (unsigned)nb - 1u;
+        }
+        __syncthreads();
+        // the last block: nothing is left for any CTA
+        last_of_all = sh.flag;
+        __syncthreads();  // sh.flag is rewritten by the next part
     }
+    if (!last_of_all) return;
+    __threadfence();
 
-    // the last CTA to finish draws the sample
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) sh.flag = atomicAdd(ticket, 1u) == gridDim.x - 1u;
-    __syncthreads();
-    if (!sh.flag) return;
-    __threadfence();
+    // the CTA that finished the last block draws the sample
+    const double u = (double)(splitmix64(seed ^ splitmix64((uint64_t)t)) >> 11) * 0x1p-53;
+    if (nb <= kPPWarpBlocks) {
+        if (tid < 32) {
+            const int64_t hit = pp_draw_exact(w, min_d2, n, nb, t, u, partials, keys, parts);
+            if (tid == 0) sh.first = (int)hit;  // n < 2^31
+        }
+        __syncthreads();
+        const int64_t hit = sh.first;
+        if (hit >= 0) {
+            if (tid == 0) {
+                chosen[t] = (int32_t)hit;
+                *ticket = 0u;  // for the next centre's launch
+            }
+            for (int64_t f = tid; f < d; f += kPPThreads) Ct[f * k + t] = Xt[f * n + hit];
+            return;
+        }
+        __syncthreads();
+    }
 
     // total of the block sums, and the running sums when their order matters
     const int64_t per = (nb + kPPThreads - 1) / kPPThreads;
@@ -295,7 +558,6 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
     }
     int64_t sel = -1;
     if (total > 0.0) {
-        const double u = (double)(splitmix64(seed ^ splitmix64((uint64_t)t)) >> 11) * 0x1p-53;
         const double target = u * total;
         // first block whose running sum exceeds the target
         if (tid == 0) sh.first = (int)nb;
@@ -330,12 +592,7 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
         // its samples, each thread kPPOwn consecutive ones
         __syncthreads();
         for (int q = tid; q < kPPBlock; q += kPPThreads) {
-            double v = 0.0;
-            if (q < count) {
-                v = w ? (double)w[i0 + q] : 1.0;
-                if (t > 0) v = __dmul_rn(v, (double)__ldcg(min_d2 + i0 + q));
-            }
-            sh.v[q] = v;
+            sh.v[q] = q < count ? pp_value(w, min_d2, i0 + q, t) : 0.0;
         }
         if (tid == 0) {
             sh.first = kPPBlock;
@@ -501,19 +758,26 @@ int kmeanspp(const T *Xt, const T *w, int64_t n, int64_t d, int64_t k, uint64_t 
     const int64_t nb = ceil_div<int64_t>(n, kPPBlock);
     Scratch mem;
     const size_t o_p = align256(sizeof(T) * n), o_f = o_p + align256(sizeof(double) * nb);
-    const size_t o_k = o_f + align256(sizeof(double) * nb), o_t = o_k + align256(sizeof(int) * nb);
-    KMC_TRY(mem.alloc(o_t + sizeof(unsigned), s));
+    const size_t o_k = o_f + align256(sizeof(double) * nb), o_s = o_k + align256(sizeof(int) * nb);
+    const size_t o_sk = o_s + align256(sizeof(double) * nb * kPPParts);
+    const size_t o_t = o_sk + align256(sizeof(int) * nb * kPPParts);
+    KMC_TRY(mem.alloc(o_t + sizeof(unsigned) * (nb + 1), s));
     char *b = mem.as<char>();
     T *min_d2 = reinterpret_cast<T *>(b);
     double *partials = reinterpret_cast<double *>(b + o_p);
     double *prefix = reinterpret_cast<double *>(b + o_f);
     int *keys = reinterpret_cast<int *>(b + o_k);
     unsigned *ticket = reinterpret_cast<unsigned *>(b + o_t);
-    KMC_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
-    const unsigned grid = (unsigned)std::min<int64_t>(nb, 3 * (int64_t)num_sms());
+    double *parts = reinterpret_cast<double *>(b + o_s);
+    int *part_keys = reinterpret_cast<int *>(b + o_sk);
+    KMC_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned) * (nb + 1), s));
+    // four CTAs fit an SM
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(n, kPPPart),
+                                                      4 * (int64_t)num_sms());
     for (int64_t t = 0; t < k; ++t) {
         pp_step_kernel<T><<<grid, kPPThreads, 0, s>>>(Xt, w, min_d2, n, d, k, (int)t, seed,
-                                                      partials, prefix, keys, chosen, Ct, ticket);
+                                                      partials, prefix, keys, parts, part_keys,
+                                                      ticket + 1, chosen, Ct, ticket);
         KMC_TRY(check_launch("kmeanspp_step"));
     }
     KMC_CUDA_TRY(cudaStreamSynchronize(s));

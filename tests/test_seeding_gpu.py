@@ -68,3 +68,23 @@ def test_variance_of_split_features(n, d):
                                                         torch.cuda.current_stream().cuda_stream))
     # two passes in float64: the mean's error enters squared
     np.testing.assert_allclose(out.value, np.mean(np.var(X, axis=1)), rtol=1e-12, atol=1e-28)
+
+
+@pytest.mark.parametrize("n,k,weights", [(511, 30, "none"), (512, 30, "random"), (513, 30, "powers"),
+                                         (4096 + 513, 40, "mostly_zero"), (4096 * 1024 + 5, 3, "none"),
+                                         (4096 * 1024 - 5, 3, "powers")])
+@pytest.mark.parametrize("data", ["normal", "grid", "range"])
+def test_rows_at_the_edges_of_a_blocks_parts(oracle, n, k, weights, data):
+    import torch
+
+    from kmeans_dpcpp_gb300 import capi
+
+    rng = np.random.default_rng(n + k)
+    X, w = _samples(data, n, 2, rng), _weights(weights, n, rng)
+    rows_o, _ = oracle.kmeans_plusplus(X, k, 11, w)
+    Xg, wg = torch.from_numpy(X).cuda(), None if w is None else torch.from_numpy(w).cuda()
+    C, rows = torch.zeros((2, k), device="cuda"), torch.full((k,), -1, dtype=torch.int32, device="cuda")
+    capi.check(capi.lib().kmc_kmeans_plusplus_f32(Xg.data_ptr(), None if wg is None else wg.data_ptr(), n, 2, k, 11,
+                                                  C.data_ptr(), rows.data_ptr(),
+                                                  torch.cuda.current_stream().cuda_stream))
+    np.testing.assert_array_equal(rows.cpu().numpy(), rows_o)
