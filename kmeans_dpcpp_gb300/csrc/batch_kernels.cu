@@ -11,7 +11,7 @@
 //                 over f = 0..d-1, D = hn - dot, strict < over ascending j
 //                 (src/device_functions.hpp:106-162) -- so labels equal a
 //                 single fit's bit for bit.  Fitting instances add w*x into
-//                 float64 copies of the sums.  Three kernels differ in the
+//                 float64 copies of the sums.  Three variants differ in the
 //                 centroids per thread (16, 32 or 64 columns per step); the
 //                 autotuner picks one per (d, k)
 //   batch_assign  the same for instances of more features than a panel takes,
@@ -45,6 +45,7 @@ constexpr int kBK = 16;
 constexpr int kTM = 8;
 constexpr size_t kPrivBytes = 72 * 1024;  // with the tiles: two CTAs per SM
 constexpr int kSumCopies = 48;            // global copies of small instances' sums
+constexpr int kFewSumCopies = 8;          // and of larger ones'
 
 constexpr int kPrepThreads = 128;
 
@@ -125,7 +126,6 @@ __global__ void __launch_bounds__(kThreadsB, 2)
         if (it >= n_items) break;
         const BItem item = items[it];
         const BInst &in = tab[item.inst];
-        if (panel::fits(in.d, DIST ? panel::MODE_DIST : panel::MODE_LABELS)) continue;
         const float *X = in.X, *C = in.C, *hn = in.hn, *w = in.w;
         int32_t *labels = in.labels;
         const int64_t n = in.n;
@@ -303,9 +303,11 @@ __global__ void __launch_bounds__(kThreadsB, 2)
 }
 
 // The same items for instances whose samples fit panels (km_panel.cuh): the
-// CTA takes an item, its warps the item's panels of 32 samples; TN centroids
-// per thread, so 8 TN columns per step.
-template <int TN, int DIST>
+// CTA takes an item, its warps the item's panels of 32 samples; the instance's
+// variant chooses the centroids per thread (2, 4 or 8, so 16, 32 or 64 columns
+// per step).  One kernel and one queue for all variants: a kernel per variant
+// ran one after another, each with its own tail.
+template <int DIST>
 __global__ void __launch_bounds__(32 * panel::kMaxWarps, 1)
     batch_panel_kernel(const BInst *tab, const BItem *items, int n_items, int *counter) {
     extern __shared__ __align__(16) float psmem[];
@@ -320,8 +322,8 @@ __global__ void __launch_bounds__(32 * panel::kMaxWarps, 1)
         const BItem item = items[it];
         const BInst &in = tab[item.inst];
         const int warps = panel::warps_for(in.d, mode);
-        if (warps == 0) continue;  // batch_assign_kernel takes it
-        const int64_t copy = DIST ? 0 : (int64_t)(blockIdx.x % (unsigned)in.copies);
+        const int64_t copy =
+            DIST ? 0 : (int64_t)((blockIdx.x * panel::kMaxWarps + (threadIdx.x >> 5)) % (unsigned)in.copies);
         const int64_t dk = (int64_t)in.d * in.k;
         // the copies lie one after another, each with its sizes
         double *sums = in.mode == B_FIT ? in.sums + copy * (dk + in.k) : nullptr;
@@ -330,12 +332,22 @@ __global__ void __launch_bounds__(32 * panel::kMaxWarps, 1)
         if constexpr (DIST) {
             const panel::Args<float, float> a{in.X, nullptr, in.C, nullptr, nullptr, 0, nullptr,
                                               nullptr, in.dist, in.n, in.d, in.k, 1, nullptr};
-            panel::run_panels<TN, mode, float, float>(a, warps, first, end, warps, 0, psmem);
+            if (in.variant == 0)
+                panel::run_panels<2, mode, float, float>(a, warps, first, end, warps, 0, psmem);
+            else if (in.variant == 1)
+                panel::run_panels<4, mode, float, float>(a, warps, first, end, warps, 0, psmem);
+            else
+                panel::run_panels<8, mode, float, float>(a, warps, first, end, warps, 0, psmem);
         } else {
             const panel::Args<float, double> a{in.X, in.w, in.C, in.hn, in.labels, 0, sums,
                                                sums ? sums + dk : nullptr, nullptr, in.n, in.d,
                                                in.k, 1, nullptr};
-            panel::run_panels<TN, mode, float, double>(a, warps, first, end, warps, 0, psmem);
+            if (in.variant == 0)
+                panel::run_panels<2, mode, float, double>(a, warps, first, end, warps, 0, psmem);
+            else if (in.variant == 1)
+                panel::run_panels<4, mode, float, double>(a, warps, first, end, warps, 0, psmem);
+            else
+                panel::run_panels<8, mode, float, double>(a, warps, first, end, warps, 0, psmem);
         }
     }
 }
@@ -370,11 +382,21 @@ __global__ void __launch_bounds__(kBatchReduceThreads)
     const int d = in.d, k = in.k;
     const int64_t dk = (int64_t)d * k, total = dk + k;
     const int el = threadIdx.x % kReduceLanes, g = threadIdx.x / kReduceLanes;
-    if (in.copies == 1) {
+    if (in.copies <= kFewSumCopies) {
+        // a thread per element, its copies' loads in flight together
         for (int64_t e = blockIdx.x * (int64_t)kBatchReduceThreads + threadIdx.x; e < total;
              e += (int64_t)gridDim.x * kBatchReduceThreads) {
-            const float v = (float)in.sums[e];
-            in.sums[e] = 0.0;
+            double x[kFewSumCopies], acc = 0.0;
+#pragma unroll
+            for (int c = 0; c < kFewSumCopies; ++c)
+                x[c] = in.sums[(c < in.copies ? c : 0) * total + e];
+#pragma unroll
+            for (int c = 0; c < kFewSumCopies; ++c)
+                if (c < in.copies) {
+                    in.sums[c * total + e] = 0.0;
+                    acc += x[c];
+                }
+            const float v = (float)acc;
             if (e < dk)
                 in.Cn[e] = v;
             else
@@ -579,19 +601,19 @@ int launch_assign_v(int variant, const BInst *tab, const BItem *items, int n_ite
     return check_launch("batch_assign");
 }
 
-template <int TN, int DIST>
+template <int DIST>
 int prepare_panels() {
-    KMC_CUDA_TRY(cudaFuncSetAttribute(batch_panel_kernel<TN, DIST>,
+    KMC_CUDA_TRY(cudaFuncSetAttribute(batch_panel_kernel<DIST>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)panel::kSmemBytes));
     return KMC_OK;
 }
 
-template <int TN, int DIST>
+template <int DIST>
 int launch_panels(const BInst *tab, const BItem *items, int n_items, int *counter,
                   cudaStream_t s) {
     const int grid = std::min(n_items, num_sms());
-    batch_panel_kernel<TN, DIST><<<grid, 32 * panel::kMaxWarps, panel::kSmemBytes, s>>>(
+    batch_panel_kernel<DIST><<<grid, 32 * panel::kMaxWarps, panel::kSmemBytes, s>>>(
         tab, items, n_items, counter);
     return check_launch("batch_panel");
 }
@@ -646,8 +668,17 @@ void tune_store(int64_t d, int64_t k, const std::string &tag, int v) {
 
 }  // namespace
 
-int batch_sum_copies(int64_t d, int64_t k) {
-    return ((d + 1) * k * (int64_t)sizeof(double) <= (int64_t)kPrivBytes) ? kSumCopies : 1;
+int batch_sum_copies(int64_t n, int64_t d, int64_t k) {
+    // larger sums: a few copies (24 fits of 2,000 to 500,000 samples, d = 8 to
+    // 128, k = 4 to 512, 10 iterations: 10.3 -> 10.0 ms)
+    const int64_t elems = (d + 1) * k;
+    if (elems * (int64_t)sizeof(double) <= (int64_t)kPrivBytes) {
+        // few clusters: more copies (207,209 x 32, k = 4 alone: 48 copies 141 us,
+        // 404 89)
+        const int64_t c = std::min<int64_t>(608, 4864 / std::max<int64_t>(k, 1));
+        return (int)std::max<int64_t>(kSumCopies, std::min<int64_t>(c, n / 512));
+    }
+    return elems <= 65536 ? kFewSumCopies : elems <= 524288 ? 4 : 1;
 }
 
 int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int *counters,
@@ -666,31 +697,29 @@ int prepare_batch_assign() {
     KMC_TRY((assign_shape<2, 1>(0, &sh)));
     KMC_TRY((assign_shape<4, 1>(1, &sh)));
     KMC_TRY((assign_shape<8, 1>(2, &sh)));
-    KMC_TRY((prepare_panels<2, 0>()));
-    KMC_TRY((prepare_panels<4, 0>()));
-    KMC_TRY((prepare_panels<8, 0>()));
-    KMC_TRY((prepare_panels<2, 1>()));
-    KMC_TRY((prepare_panels<4, 1>()));
-    return prepare_panels<8, 1>();
+    KMC_TRY((prepare_panels<0>()));
+    return prepare_panels<1>();
 }
 
 bool batch_in_panels(int64_t d, int dist) {
     return panel::fits(d, dist ? panel::MODE_DIST : panel::MODE_LABELS);
 }
 
-int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, const BItem *items,
-                        int n_items, int *counter, cudaStream_t s) {
+int batch_panel_round(int64_t d, int dist) {
+    return panel::warps_for(d, dist ? panel::MODE_DIST : panel::MODE_LABELS) * panel::kRows /
+           kBatchTileM;
+}
+
+int launch_batch_panels(int dist, const BInst *tab, const BItem *items, int n_items, int *counter,
+                        cudaStream_t s) {
     if (n_items <= 0) return KMC_OK;
-    if (panels) {
-        if (dist) {
-            if (variant == 0) return launch_panels<2, 1>(tab, items, n_items, counter, s);
-            if (variant == 1) return launch_panels<4, 1>(tab, items, n_items, counter, s);
-            return launch_panels<8, 1>(tab, items, n_items, counter, s);
-        }
-        if (variant == 0) return launch_panels<2, 0>(tab, items, n_items, counter, s);
-        if (variant == 1) return launch_panels<4, 0>(tab, items, n_items, counter, s);
-        return launch_panels<8, 0>(tab, items, n_items, counter, s);
-    }
+    return dist ? launch_panels<1>(tab, items, n_items, counter, s)
+                : launch_panels<0>(tab, items, n_items, counter, s);
+}
+
+int launch_batch_assign(int variant, int dist, const BInst *tab, const BItem *items, int n_items,
+                        int *counter, cudaStream_t s) {
+    if (n_items <= 0) return KMC_OK;
     if (dist) {
         if (variant == 0) return launch_assign_v<2, 1>(0, tab, items, n_items, counter, s);
         if (variant == 1) return launch_assign_v<4, 1>(1, tab, items, n_items, counter, s);
@@ -824,7 +853,6 @@ int tune_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
     BInst *tab = reinterpret_cast<BInst *>(b + off_tab);
     BItem *items = reinterpret_cast<BItem *>(b + off_item);
     int *cnt = reinterpret_cast<int *>(b + off_cnt);
-    KMC_CUDA_TRY(cudaMemcpyAsync(tab, &h, sizeof(h), cudaMemcpyHostToDevice, s));
     KMC_CUDA_TRY(cudaMemcpyAsync(items, hi, sizeof(hi), cudaMemcpyHostToDevice, s));
     cudaEvent_t e0, e1;
     KMC_CUDA_TRY(cudaEventCreate(&e0));
@@ -833,10 +861,15 @@ int tune_variant(int64_t d, int64_t k_in, cudaStream_t s, int *variant) {
     int best = 2;
     for (int v = 0; v < kBatchVariants; ++v) {
         float tot = 0.f;
+        h.variant = v;
+        KMC_CUDA_TRY(cudaMemcpyAsync(tab, &h, sizeof(h), cudaMemcpyHostToDevice, s));
         for (int rep = 0; rep < 3; ++rep) {
             KMC_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), s));
             KMC_CUDA_TRY(cudaEventRecord(e0, s));
-            KMC_TRY(launch_batch_assign(v, 0, batch_in_panels(d, 0), tab, items, 64, cnt, s));
+            if (batch_in_panels(d, 0))
+                KMC_TRY(launch_batch_panels(0, tab, items, 64, cnt, s));
+            else
+                KMC_TRY(launch_batch_assign(v, 0, tab, items, 64, cnt, s));
             KMC_CUDA_TRY(cudaEventRecord(e1, s));
             KMC_CUDA_TRY(cudaEventSynchronize(e1));
             float ms = 0.f;

@@ -32,7 +32,7 @@ struct BInst {
     int d, k;
     int mode;              // B_FIT or B_ASSIGN
     int variant;           // centroid columns per step: 0 -> 16, 1 -> 32, 2 -> 64 (panels)
-    int copies;            // private copies of sums (CTA b adds into copy b % copies)
+    int copies;            // private copies of sums (a warp or CTA adds into one of them)
     int n_empty;           // empty clusters of this step
     unsigned tickets[2];   // CTAs of batch_reduce / batch_update that are through
     LoopState st;          // done / n_iter / max_iter / tol / last_shift
@@ -52,7 +52,7 @@ constexpr int kBatchCounters = 4 * kBatchVariants;
 
 // Private global copies of an instance's float64 sums: small sums get several
 // (their few addresses would serialise the reductions of many CTAs).
-int batch_sum_copies(int64_t d, int64_t k);
+int batch_sum_copies(int64_t n, int64_t d, int64_t k);
 
 // ---- launchers (batch.cu) ----
 int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int *counters,
@@ -60,11 +60,15 @@ int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int 
 // Sets the assign kernels' shared-memory attributes (outside graph capture).
 int prepare_batch_assign();
 // dist != 0: the transform kernel (items of B_TRANSFORM instances only).
-// panels: the kernel for instances whose features fit panels (it skips the
-// other items, as the other kernel skips these).
+// Instances whose features fit panels, every variant in one launch:
 bool batch_in_panels(int64_t d, int dist);
-int launch_batch_assign(int variant, int dist, bool panels, const BInst *tab, const BItem *items,
-                        int n_items, int *counter, cudaStream_t s);
+int launch_batch_panels(int dist, const BInst *tab, const BItem *items, int n_items, int *counter,
+                        cudaStream_t s);
+// 128-sample tiles that a CTA's warps take at once there.
+int batch_panel_round(int64_t d, int dist);
+// The others, by variant:
+int launch_batch_assign(int variant, int dist, const BInst *tab, const BItem *items, int n_items,
+                        int *counter, cudaStream_t s);
 // Copies -> sums, sizes and empty-cluster lists of the fits idx; max_elems,
 // max_k: the largest (d + 1) k and k among them.
 int launch_batch_reduce(BInst *tab, const int *idx, int count, int64_t max_elems,

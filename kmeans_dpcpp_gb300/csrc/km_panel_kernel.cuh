@@ -518,7 +518,9 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) panel_kernel(Args<T, A> a) 
     const int warps = blockDim.x >> 5;
     run_panels<TN, MODE, T, A>(a, warps, (int64_t)blockIdx.x * warps,
                                ceil_div<int64_t>(a.n, kRows), (int64_t)gridDim.x * warps,
-                               (int64_t)blockIdx.x % a.P, smem);
+                               (a.P > (int64_t)gridDim.x ? (int64_t)blockIdx.x * warps + (threadIdx.x >> 5)
+                                         : (int64_t)blockIdx.x) % a.P,
+               smem);
 }
 
 template <int TN, int MODE, typename T, typename A>

@@ -315,8 +315,9 @@ __global__ void __launch_bounds__(max_threads(DP), 1) reg_kernel(Args<T, A> a) {
         }
         if constexpr (!kF64) {
             if (a.sums != nullptr) {
-                // w x into this CTA's copy with fire-and-forget reductions
-                const int64_t copy = (int64_t)blockIdx.x % a.P;
+                // w x into this CTA's copy (this warp's, where there are more
+                // copies than CTAs) with fire-and-forget reductions
+                const int64_t copy = (a.P > (int64_t)gridDim.x ? wfirst : (int64_t)blockIdx.x) % a.P;
                 A *sums = a.sums + copy * (int64_t)d * k, *sizes = a.sizes + copy * k;
 #pragma unroll
                 for (int s = 0; s < S; ++s) {

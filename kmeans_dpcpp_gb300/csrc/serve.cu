@@ -47,6 +47,45 @@ void append_items(int q, int64_t n, int mode, int variant,
             BItem{q, (int)std::min<int64_t>(kItemTiles, tiles - t), (long long)t});
 }
 
+// Work items of the instances whose samples are taken in panels, one list per
+// kind, the most expensive first (the CTAs pull them in order).  An item holds
+// whole rounds of its CTA's warps, as few as keep it near a quarter of an SM's
+// share of all work: with 1024 samples per item 47 SMs shared the heaviest
+// instance of a batch while the others waited.
+struct PanelJob {
+    int q;
+    int64_t n, d, k;
+};
+
+void plan_panels(const std::vector<PanelJob> &jobs, int dist, std::vector<BItem> *out) {
+    // Cost in products (128 per clock and SM): besides its k products, a
+    // feature of a sample costs a load and a reduction (half a clock), and each
+    // round of a CTA about 5 us of latencies.
+    auto cost = [&](const PanelJob &j, int64_t rows) {
+        const double rounds =
+            (double)ceil_div<int64_t>(rows, std::max(1, batch_panel_round(j.d, dist)) * kBatchTileM);
+        return (double)rows * (double)j.d * (double)(j.k + 100) + 1e6 * rounds;
+    };
+    double all = 0.0;
+    for (const PanelJob &j : jobs) all += cost(j, j.n);
+    const double share = all / (4.0 * num_sms());
+    std::vector<std::pair<double, BItem>> items;
+    for (const PanelJob &j : jobs) {
+        const int round = std::max(1, batch_panel_round(j.d, dist));
+        const double one = cost(j, (int64_t)round * kBatchTileM);
+        const int64_t per = round * std::max<int64_t>(1, std::min<int64_t>(64, (int64_t)(share / one)));
+        const int64_t tiles = ceil_div<int64_t>(j.n, kBatchTileM);
+        for (int64_t t = 0; t < tiles; t += per) {
+            const int64_t m = std::min<int64_t>(per, tiles - t);
+            items.emplace_back(cost(j, m * kBatchTileM), BItem{j.q, (int)m, (long long)t});
+        }
+    }
+    std::stable_sort(items.begin(), items.end(),
+                     [](const auto &a, const auto &b) { return a.first > b.first; });
+    out->clear();
+    for (const auto &it : items) out->push_back(it.second);
+}
+
 // Engine-owned device memory of one instance.
 struct SlotMem {
     Scratch mem;
@@ -59,7 +98,7 @@ struct SlotMem {
 size_t slot_bytes(int mode, int64_t n, int64_t d, int64_t k) {
     size_t b = align256(sizeof(float) * d * k) + 2 * align256(sizeof(float) * k);
     if (mode == B_FIT) {
-        b += align256(sizeof(double) * (d * k + k) * batch_sum_copies(d, k)) +
+        b += align256(sizeof(double) * (d * k + k) * batch_sum_copies(n, d, k)) +
              align256(sizeof(int32_t) * (k + 1)) +
              align256(sizeof(float) * n) + align256(sizeof(int32_t) * (n + 2)) +
              align256(sizeof(float)) + align256(threshold_scratch_bytes()) +
@@ -82,7 +121,7 @@ int alloc_slot(SlotMem &m, int mode, int64_t n, int64_t d, int64_t k, cudaStream
     m.hn = reinterpret_cast<float *>(take(sizeof(float) * k));
     m.sizes = reinterpret_cast<float *>(take(sizeof(float) * k));
     if (mode == B_FIT) {
-        m.sums = reinterpret_cast<double *>(take(sizeof(double) * (d * k + k) * batch_sum_copies(d, k)));
+        m.sums = reinterpret_cast<double *>(take(sizeof(double) * (d * k + k) * batch_sum_copies(n, d, k)));
         m.empty_list = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (k + 1)));
         m.sq_dist = reinterpret_cast<float *>(take(sizeof(float) * n));
         m.selected = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (n + 2)));
@@ -133,9 +172,10 @@ struct BatchEngine {
     std::vector<double> res_inertia;
     // current step plan
     std::vector<int> all, fits;
-    // [0][v]: assignment items of variant v, [1][v]: transform items
-    int n_items[2][kBatchVariants] = {{0, 0, 0}, {0, 0, 0}};
-    int64_t item_off[2][kBatchVariants] = {{0, 0, 0}, {0, 0, 0}};
+    // [0][v]: assignment items of variant v, [1][v]: transform items; v =
+    // kBatchVariants: those in panels
+    int n_items[2][kBatchVariants + 1] = {};
+    int64_t item_off[2][kBatchVariants + 1] = {};
     bool dirty = true;
     GraphExec graph;
     int64_t max_k = 1, max_elems = 1;  // over the fitting instances
@@ -251,7 +291,7 @@ struct BatchEngine {
         h.hn = m->hn;
         h.sizes = m->sizes;
         h.sums = m->sums;
-        h.copies = mode == B_FIT ? batch_sum_copies(d, k) : 1;
+        h.copies = mode == B_FIT ? batch_sum_copies(n, d, k) : 1;
         // each step's reduction leaves the sums at zero again
         if (mode == B_FIT)
             KMC_CUDA_TRY(cudaMemsetAsync(m->sums, 0, sizeof(double) * (d * k + k) * h.copies, s));
@@ -302,8 +342,8 @@ struct BatchEngine {
         fits.clear();
         max_k = max_elems = 1;
         int64_t all_k = 1;
-        std::vector<BItem> items[2][kBatchVariants];
-        bool use[2][2][kBatchVariants] = {};  // [panels][kind][variant]
+        std::vector<BItem> items[2][kBatchVariants], panel_items[2];
+        std::vector<PanelJob> jobs[2];
         for (int64_t q = 0; q < cap; ++q) {
             if (state[(size_t)q] != RUNNING) continue;
             const BInst &h = tab[(size_t)q];
@@ -314,15 +354,21 @@ struct BatchEngine {
                 max_k = std::max<int64_t>(max_k, h.k);
                 max_elems = std::max<int64_t>(max_elems, ((int64_t)h.d + 1) * h.k);
             }
-            append_items((int)q, h.n, h.mode, h.variant, items);
             const int kind = h.mode == B_TRANSFORM ? 1 : 0;
-            use[batch_in_panels(h.d, kind) ? 1 : 0][kind][h.variant] = true;
+            if (batch_in_panels(h.d, kind))
+                jobs[kind].push_back(PanelJob{(int)q, h.n, h.d, h.k});
+            else
+                append_items((int)q, h.n, h.mode, h.variant, items);
         }
+        for (int kind = 0; kind < 2; ++kind) plan_panels(jobs[kind], kind, &panel_items[kind]);
+        auto list = [&](int kind, int v) -> const std::vector<BItem> & {
+            return v < kBatchVariants ? items[kind][v] : panel_items[kind];
+        };
         int64_t total = 0;
         for (int kind = 0; kind < 2; ++kind)
-            for (int v = 0; v < kBatchVariants; ++v) {
+            for (int v = 0; v <= kBatchVariants; ++v) {
                 item_off[kind][v] = total;
-                n_items[kind][v] = (int)items[kind][v].size();
+                n_items[kind][v] = (int)list(kind, v).size();
                 total += n_items[kind][v];
             }
         if (total > items_cap) {
@@ -331,10 +377,10 @@ struct BatchEngine {
             items_d = items_mem.as<BItem>();
         }
         for (int kind = 0; kind < 2; ++kind)
-            for (int v = 0; v < kBatchVariants; ++v)
+            for (int v = 0; v <= kBatchVariants; ++v)
                 if (n_items[kind][v] > 0)
                     KMC_CUDA_TRY(cudaMemcpyAsync(items_d + item_off[kind][v],
-                                                 items[kind][v].data(),
+                                                 list(kind, v).data(),
                                                  sizeof(BItem) * n_items[kind][v],
                                                  cudaMemcpyHostToDevice, s));
         if (!all.empty())
@@ -349,18 +395,19 @@ struct BatchEngine {
         KMC_TRY(capture(&graph, [&]() -> int {
             KMC_TRY(launch_batch_prep(tab_d, all_d, (int)all.size(), all_k, counters_d, s));
             KMC_CUDA_TRY(cudaEventRecord(ev_fork, s));
-            // one branch per centroid-window variant: its assignment items,
-            // then its transform items
+            // the instances in panels, then one branch per centroid-window
+            // variant: its assignment items, then its transform items
+            for (int kind = 0; kind < 2; ++kind)
+                KMC_TRY(launch_batch_panels(kind, tab_d, items_d + item_off[kind][kBatchVariants],
+                                            n_items[kind][kBatchVariants],
+                                            counters_d + (2 + kind) * kBatchVariants, s));
             for (int v = 0; v < kBatchVariants; ++v) {
                 if (n_items[0][v] + n_items[1][v] == 0) continue;
                 KMC_CUDA_TRY(cudaStreamWaitEvent(side[v], ev_fork, 0));
                 for (int kind = 0; kind < 2; ++kind)
-                    for (int pn = 1; pn >= 0; --pn)
-                        if (use[pn][kind][v])
-                            KMC_TRY(launch_batch_assign(
-                                v, kind, pn != 0, tab_d, items_d + item_off[kind][v],
-                                n_items[kind][v],
-                                counters_d + (2 * pn + kind) * kBatchVariants + v, side[v]));
+                    KMC_TRY(launch_batch_assign(v, kind, tab_d, items_d + item_off[kind][v],
+                                                n_items[kind][v],
+                                                counters_d + kind * kBatchVariants + v, side[v]));
                 KMC_CUDA_TRY(cudaEventRecord(ev_join[v], side[v]));
                 KMC_CUDA_TRY(cudaStreamWaitEvent(s, ev_join[v], 0));
             }

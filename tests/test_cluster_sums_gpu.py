@@ -1,5 +1,6 @@
 """Cluster sums of the tensor-core forms (sorted by label, or sample by sample
-beyond 2048 clusters).
+beyond 2048 clusters) and of the plain form (float64 copies whose number follows
+the sizes).
 
 One iteration from given centroids: the next centroids are the weighted means of
 the samples by their exact float32 labels.  Up to 32 features the sums are exact
@@ -29,9 +30,22 @@ SHAPES = [
 ]
 
 
+# plain: copies per warp (few clusters), 16 copies, 4 copies, one
+PLAIN = [(700_001, 4, 3), (400_003, 40, 5), (100_001, 64, 300), (70_000, 128, 700), (9_000, 140, 4000)]
+
+
+@pytest.mark.parametrize("n,d,k", PLAIN)
+def test_plain_sums_with_any_number_of_copies(oracle, n, d, k):
+    _one_iteration(oracle, n, d, k, "plain", np.int32)
+
+
 @pytest.mark.parametrize("n,d,k", SHAPES)
 @pytest.mark.parametrize("form,labels", [("mixed-fp16", np.int32), ("mixed-bf16", np.int64)])
 def test_one_iteration_gives_the_weighted_means(oracle, n, d, k, form, labels):
+    _one_iteration(oracle, n, d, k, form, labels)
+
+
+def _one_iteration(oracle, n, d, k, form, labels):
     import torch
 
     import kmeans_dpcpp_gb300 as kdp
@@ -57,7 +71,7 @@ def test_one_iteration_gives_the_weighted_means(oracle, n, d, k, form, labels):
                             1, 8, 128, 0.7, None, form=form)
     got = res.cpu().numpy().astype(np.float64)
     u = 2.0 ** -24
-    # packed: products, sum, size and quotient are rounded once each
-    terms = 4 if d <= 32 else 2 * m[None, :] + 4
+    # packed or float64: products, sum, size and quotient are rounded once each
+    terms = 4 if d <= 32 or form == "plain" else 2 * m[None, :] + 4
     assert np.all(np.abs(got - mean) <= terms * u * mag * 1.01 + 1e-37)
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.assignment(X, res.cpu().numpy()))
