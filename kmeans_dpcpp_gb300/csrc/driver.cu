@@ -230,6 +230,7 @@ int PlainFit<T, I>::enqueue_iteration(bool relocate) {
         KMC_TRY(launch_sum_f64<T>(sq_dist, n, partials, dsum, s));
         launches += 3;
     }
+    hn_current = true;
     if (relocate) KMC_TRY(enqueue_relocation());
     ++issued;
     return KMC_OK;
@@ -247,6 +248,7 @@ int PlainFit<T, I>::enqueue_relocation() {
                              reloc, reloc + p.k, reloc + 2 * p.k, xv, p.w, p.labels, sq_dist, p.n,
                              p.d, p.k, xfs, xss, cr, crs, wait_clocks(), state, ctl};
     KMC_TRY((launch_relocation<T, I>(ra, p.stream)));
+    hn_current = false;
     ++launches;
     return KMC_OK;
 }
@@ -355,6 +357,7 @@ int PlainFit<T, I>::run_pipelined(HostSlotRef &slot) {
 template <typename T, typename I>
 int PlainFit<T, I>::run(int64_t max_batch) {
     const FitParams<T, I> &p = prm;
+    hn_current = false;
     if (!p.verbose && max_batch <= 0) {
         HostSlotRef slot;
         if (slot.p != nullptr) return run_pipelined(slot);

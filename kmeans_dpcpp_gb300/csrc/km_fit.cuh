@@ -126,6 +126,10 @@ struct PlainFit : FitBase {
     double *partials = nullptr, *dsum = nullptr;
     int64_t issued = 0;
     int host_done = 0;
+    // hn holds the half norms of the centroids as the enqueued work leaves
+    // them (plain forms; not after a relocation, nor across run() calls, between
+    // which the caller may change its centroids)
+    bool hn_current = false;
     bool split64 = false;  // float64 samples: labels, then sums (sums64.cu)
     int tile_variant = 0;  // autotuned centroid-tile width of the plain kernels
     Scratch xt;  // feature-major copy of a row-major X (forms that need one)
@@ -154,15 +158,16 @@ struct PlainFit : FitBase {
     virtual int finish_step(int64_t *n_launches);
     FinishArgs<T> finish_args() const {
         const FitParams<T, I> &p = prm;
-        return FinishArgs<T>{p.centroids, p.new_centroids, prev, sums, sizes, shifts, empty_list,
-                             p.d, p.k, 1, state, ctl};
+        return FinishArgs<T>{p.centroids, p.new_centroids, prev, sums, sizes, shifts,
+                             uses_private_copies() ? hn : nullptr, empty_list, p.d, p.k, 1, state, ctl};
     }
     // Limit (SM clocks) of the waits of a relocation's grid barriers.
     virtual long long wait_clocks() const { return 4000000000LL; }
-    // Half norms of the current centroids, where the form's own preparation
-    // does not make them.
+    // Half norms of the current centroids, where neither the form's own
+    // preparation nor the end of the iteration before made them.
     virtual int begin_step(int64_t *n_launches) {
-        *n_launches = 1;
+        *n_launches = hn_current ? 0 : 1;
+        if (hn_current) return KMC_OK;
         return launch_half_norm<T>(prm.centroids, hn, prm.d, prm.k, prm.stream, state);
     }
     // Whether the step accumulates into the driver's float64 private copies

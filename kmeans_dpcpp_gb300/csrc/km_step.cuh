@@ -52,6 +52,7 @@ struct FinishArgs {
     T *sums;            // (d, k) cluster sums, kept for a relocation
     T *sizes;           // (k)
     T *shifts;          // (k)
+    T *hn;              // (k) half norms of the new centroids, or null
     int64_t *empty_list;  // (k), ascending
     int64_t d, k;
     int jc;             // clusters per CTA
@@ -195,13 +196,14 @@ __device__ __forceinline__ float fma_step(float a, float b, float c) { return __
 __device__ __forceinline__ double fma_step(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // Division, each cluster's shift (features in order, as the reference adds
-// them) and, in the last CTA, the stop rule or the empty-cluster list.  A CTA
+// them), the plain forms' half norms for the next iteration (a launch of their
+// own before: 50,000 x 14, k = 16, 20 iterations 707 -> 629 us) and, in the last CTA, the stop rule or the empty-cluster list.  A CTA
 // takes jc clusters.  Latency-bound: all loads of a round are issued together
 // (sums, previous centroids, sizes), and the CTAs meet once, at the ticket.
 template <typename T, typename Src>
 __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishArgs<T> a) {
     if (*reinterpret_cast<const volatile int *>(&a.state->done)) return;
-    __shared__ T diff_sh[kFinishElems];
+    __shared__ T diff_sh[kFinishElems], new_sh[kFinishElems];
     __shared__ T size_sh[32];
     __shared__ double sh[32];
     __shared__ int warp_counts[kFinishThreads / 32];
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
     const int64_t d = a.d, k = a.k, j0 = (int64_t)blockIdx.x * a.jc;
     const int jn = (int)(k - j0 < a.jc ? k - j0 : a.jc);
     const int64_t fc = kFinishElems / a.jc;  // features per round
-    T shift = T(0);
+    T shift = T(0), norm = T(0);
     for (int64_t f0 = 0; f0 == 0 || f0 < d; f0 += fc) {
         const int nf = (int)(d - f0 < fc ? d - f0 : fc), cnt = nf * jn;
         T s[kFinishOwn], old[kFinishOwn];
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
                 a.cur[at] = c;
                 a.nxt[at] = c;
                 diff_sh[e] = old[u] - c;
+                new_sh[e] = c;
             }
         }
         __syncthreads();
@@ -250,9 +253,17 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
                 const T diff = diff_sh[f * jn + tid];
                 shift = fma_step(diff, diff, shift);
             }
+        } else if (tid >= 32 && tid < 32 + jn) {
+            // the next iteration's half norms, by another warp
+#pragma unroll 4
+            for (int f = 0; f < nf; ++f) {
+                const T c = new_sh[f * jn + tid - 32];
+                norm = fma_step(c, c, norm);
+            }
         }
         __syncthreads();
     }
+    if (a.hn != nullptr && tid >= 32 && tid < 32 + jn) a.hn[j0 + tid - 32] = norm / T(2);
     if (tid < 32) {
         const bool empty = tid < jn && size_sh[tid] == T(0);
         if (tid < jn) a.shifts[j0 + tid] = shift;
