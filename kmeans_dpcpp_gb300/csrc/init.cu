@@ -381,6 +381,8 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
     const T *__restrict__ Xt, const T *__restrict__ w, T *min_d2, int64_t n, int64_t d, int64_t k,
     int t, uint64_t seed, double *partials, double *prefix, int *keys, double *parts, int *part_keys,
     unsigned *arrived, int32_t *chosen, T *Ct, unsigned *ticket) {
+    wait_for_previous();
+    allow_next();
     __shared__ PPShared sh;
     __shared__ T centre[kPPThreads];
     const int tid = threadIdx.x;
@@ -775,10 +777,9 @@ int kmeanspp(const T *Xt, const T *w, int64_t n, int64_t d, int64_t k, uint64_t 
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(n, kPPPart),
                                                       4 * (int64_t)num_sms());
     for (int64_t t = 0; t < k; ++t) {
-        pp_step_kernel<T><<<grid, kPPThreads, 0, s>>>(Xt, w, min_d2, n, d, k, (int)t, seed,
-                                                      partials, prefix, keys, parts, part_keys,
-                                                      ticket + 1, chosen, Ct, ticket);
-        KMC_TRY(check_launch("kmeanspp_step"));
+        KMC_TRY(launch_chained("kmeanspp_step", pp_step_kernel<T>, dim3(grid), dim3(kPPThreads), 0, s, Xt, w,
+                               min_d2, n, d, k, (int)t, seed, partials, prefix, keys, parts, part_keys,
+                               ticket + 1, chosen, Ct, ticket));
     }
     KMC_CUDA_TRY(cudaStreamSynchronize(s));
     return KMC_OK;

@@ -297,6 +297,7 @@ __host__ __device__ constexpr float norm_coef(int bf16, int part) {
 
 template <int BF16, int NKB, int NCH, bool MULTI>
 __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArgs a) {
+    wait_for_previous();
     if (a.guard != nullptr && *reinterpret_cast<const volatile int *>(&a.guard->done)) return;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // the swizzles are functions of absolute shared-memory address bits, so
@@ -883,6 +884,8 @@ template <int BF16>
 __global__ void __launch_bounds__(256) mixed_prep_kernel(
     const float *C, int64_t d, int64_t k, int64_t k_pad, int nkb, MixedConsts *c, uint8_t *img,
     float *hn, float *ct, int64_t d4, int *n_flagged, const LoopState *guard) {
+    wait_for_previous();
+    allow_next();
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     __shared__ float cs[64 * 4 * (kPrepRows + 1)];
     __shared__ double q_sh[2][kPrepRows];
@@ -1049,6 +1052,7 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
     const float *xrow, const float *ct, const float *hn, const uint4 *cand, const int *flagged,
     const int *n_flagged, int64_t n, int64_t d, int64_t k, int64_t d4, void *labels, int label64,
     const LoopState *guard, int passes, int64_t pass_cols, long long *stats) {
+    wait_for_previous();
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the fit's statistics: samples rechecked in this pass, and in total
@@ -1384,6 +1388,7 @@ __global__ void __launch_bounds__(kSumThreads, kSortCtas) sum_sorted_kernel(
     const float *xrow, const float *w, const I *labels, int64_t n, int64_t d4, int64_t k,
     int64_t k_pad, int tile_rows, float *sums, FxAcc fx, double *acc, int n_copies,
     const MixedConsts *consts, const LoopState *guard) {
+    wait_for_previous();
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     constexpr bool FX = F != 0;
     constexpr int kPer = kSortTile / kSumThreads, kWarps = kSumThreads / 32, kBatch = FX ? F : 4;
@@ -1994,9 +1999,9 @@ struct MixedFit : PlainFit<float, I> {
         const FitParams<float, I> &p = this->prm;
         const int lanes = nkb <= 1 ? 8 : (nkb == 2 ? 16 : 32);
         auto kern = bf16 ? mixed_prep_kernel<1> : mixed_prep_kernel<0>;
-        kern<<<(unsigned)(k_pad / kPrepRows), lanes * kPrepRows, 0, p.stream>>>(
-            cur, p.d, p.k, k_pad, nkb, consts, cimg, this->hn, ct, d4, n_flagged, guard);
-        return check_launch("mixed_prep");
+        return launch_chained("mixed_prep", kern, dim3((unsigned)(k_pad / kPrepRows)),
+                              dim3((unsigned)(lanes * kPrepRows)), 0, p.stream, cur, p.d, p.k, k_pad,
+                              nkb, consts, cimg, this->hn, ct, d4, n_flagged, guard);
     }
 
     // enough CTAs for every sample flagged (8 warps of 32 per CTA round), at
@@ -2045,8 +2050,8 @@ struct MixedFit : PlainFit<float, I> {
                 a.col0 = (int64_t)ps * pass_cols;
                 a.cand = cand + (int64_t)ps * p.n;
                 a.pmax = pmax + (multi ? (int64_t)ps * p.n : 0);
-                kern<<<(unsigned)grid, kThreadsMixed, L.total, s>>>(a);
-                KMC_TRY(check_launch("mixed_assign"));
+                KMC_TRY(launch_chained("mixed_assign", kern, dim3((unsigned)grid), dim3(kThreadsMixed),
+                                       L.total, s, a));
                 a.stall = 0;
             }
             if (multi) {
@@ -2056,10 +2061,10 @@ struct MixedFit : PlainFit<float, I> {
                 KMC_TRY(check_launch("mixed_combine"));
             }
         }
-        recheck_kernel<<<(unsigned)recheck_grid(), kRecheckThreads, 0, s>>>(
-            xrow, ct, this->hn, cand, flagged, n_flagged, p.n, p.d, p.k, d4, p.labels, a.label64,
-            guard, passes, pass_cols, stats);
-        return check_launch("mixed_recheck");
+        return launch_chained("mixed_recheck", recheck_kernel, dim3((unsigned)recheck_grid()),
+                              dim3(kRecheckThreads), 0, s, xrow, ct, this->hn, cand, flagged,
+                              n_flagged, p.n, p.d, p.k, d4, p.labels, a.label64, guard, passes,
+                              pass_cols, stats);
     }
 
     // The sums' kernel: CTAs, samples of a CTA's tile, rounds of tiles.  The
@@ -2087,10 +2092,9 @@ struct MixedFit : PlainFit<float, I> {
             if (smem > 48 * 1024)
                 KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)smem));
-            kern<<<(unsigned)sum_grid(), kSumThreads, smem, p.stream>>>(
-                xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32, fx_acc(), acc64, n_copies,
-                consts, guard);
-            return check_launch("mixed_sums");
+            return launch_chained("mixed_sums", kern, dim3((unsigned)sum_grid()), dim3(kSumThreads), smem,
+                                  p.stream, xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32,
+                                  fx_acc(), acc64, n_copies, consts, guard);
         }
         const unsigned grid = (unsigned)sum_grid();
         if (acc_f64) {

@@ -513,6 +513,7 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
 
 template <int TN, int MODE, typename T, typename A>
 __global__ void __launch_bounds__(32 * kMaxWarps, 1) panel_kernel(Args<T, A> a) {
+    wait_for_previous();
     if (a.guard != nullptr && *reinterpret_cast<const volatile int *>(&a.guard->done)) return;
     extern __shared__ __align__(16) float smem[];
     const int warps = blockDim.x >> 5;
@@ -535,8 +536,7 @@ int launch_width(const Args<T, A> &a, cudaStream_t s) {
     KMC_CUDA_TRY(
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t grid = std::min<int64_t>(num_sms(), ceil_div<int64_t>(wtiles, warps));
-    kern<<<(unsigned)grid, (unsigned)(32 * warps), smem, s>>>(a);
-    return check_launch("panel");
+    return launch_chained("panel", kern, dim3((unsigned)grid), dim3((unsigned)(32 * warps)), smem, s, a);
 }
 
 // Columns of a step: 64, 32 or 16, whichever pads k least for its rate (the

@@ -55,6 +55,7 @@ struct Bound {
 
 template <int DP, int MODE, typename T, typename A>
 __global__ void __launch_bounds__(max_threads(DP), 1) reg_kernel(Args<T, A> a) {
+    wait_for_previous();
     if (a.guard != nullptr && *reinterpret_cast<const volatile int *>(&a.guard->done)) return;
     constexpr bool kF64 = sizeof(T) == 8;  // float64 samples: certified labels
     constexpr bool kPair = paired(DP, MODE), kDist = MODE == MODE_DIST;
@@ -369,8 +370,7 @@ int launch_class(const Args<T, A> &a, cudaStream_t s) {
     const int64_t warps = std::max<int64_t>(
         1, std::min<int64_t>(max_threads(DP) / 32, ceil_div<int64_t>(wtiles, num_sms())));
     const int64_t grid = std::min<int64_t>(num_sms(), ceil_div<int64_t>(wtiles, warps));
-    kern<<<(unsigned)grid, (unsigned)(32 * warps), smem, s>>>(a);
-    return check_launch("reg_kernel");
+    return launch_chained("reg_kernel", kern, dim3((unsigned)grid), dim3((unsigned)(32 * warps)), smem, s, a);
 }
 
 template <int MODE, typename T, typename A>

@@ -124,6 +124,8 @@ constexpr int kReduceThreads = kReduceLanes * kReduceGroups, kFewCopies = 8;
 template <typename T, typename Src, int G>
 __global__ void __launch_bounds__(kReduceThreads)
     reduce_sums_kernel(Src src, T *sums, T *sizes, int64_t d, int64_t k, const LoopState *state) {
+    wait_for_previous();
+    allow_next();
     if (*reinterpret_cast<const volatile int *>(&state->done)) return;
     constexpr int kLanes = kReduceThreads / G;
     __shared__ typename Src::Part red[G][kLanes];
@@ -202,6 +204,8 @@ __device__ __forceinline__ double fma_step(double a, double b, double c) { retur
 // (sums, previous centroids, sizes), and the CTAs meet once, at the ticket.
 template <typename T, typename Src>
 __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishArgs<T> a) {
+    wait_for_previous();
+    allow_next();
     if (*reinterpret_cast<const volatile int *>(&a.state->done)) return;
     __shared__ T diff_sh[kFinishElems], new_sh[kFinishElems];
     __shared__ T size_sh[32];
@@ -304,8 +308,8 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
 template <typename T, typename Src>
 int launch_finish(const Src &src, FinishArgs<T> a, cudaStream_t s) {
     a.jc = (int)std::min<int64_t>(32, ceil_div<int64_t>(a.k, 128));
-    finish_kernel<T, Src><<<(unsigned)ceil_div<int64_t>(a.k, a.jc), kFinishThreads, 0, s>>>(src, a);
-    return check_launch("finish");
+    return launch_chained("finish", finish_kernel<T, Src>, dim3((unsigned)ceil_div<int64_t>(a.k, a.jc)),
+                          dim3(kFinishThreads), 0, s, src, a);
 }
 
 // Up to this many private copies finish_kernel reads them itself.
@@ -321,8 +325,8 @@ int launch_reduce_and_finish(const Src &src, int64_t copies, const FinishArgs<T>
     const bool few = copies <= kFewCopies;
     const int64_t grid = ceil_div<int64_t>((a.d + 1) * a.k, kReduceThreads / (few ? 4 : kReduceGroups));
     auto kern = few ? reduce_sums_kernel<T, Src, 4> : reduce_sums_kernel<T, Src, kReduceGroups>;
-    kern<<<(unsigned)grid, kReduceThreads, 0, s>>>(src, a.sums, a.sizes, a.d, a.k, a.state);
-    KMC_TRY(check_launch("reduce_sums"));
+    KMC_TRY(launch_chained("reduce_sums", kern, dim3((unsigned)grid), dim3(kReduceThreads), 0, s, src,
+                           a.sums, a.sizes, a.d, a.k, (const LoopState *)a.state));
     return launch_finish<T>(ReducedSums<T>{a.sums, a.sizes, a.k}, a, s);
 }
 

@@ -645,6 +645,7 @@ constexpr int kItersPerVisit = 4;
 int capture_iteration(Active &a) {
     cudaGraph_t g = nullptr;
     KMC_CUDA_TRY(cudaStreamBeginCapture(a.st, cudaStreamCaptureModeRelaxed));
+    const UnchainedLaunches unchained;
     int rc = a.fit->enqueue_iteration(false);
     if (rc == KMC_OK) {
         const cudaError_t e = cudaMemcpyAsync(a.hstate, a.fit->device_state(), sizeof(LoopState),
@@ -1025,6 +1026,7 @@ struct Server {
             }
             // a paused loop relocates its empty clusters and goes on
             const bool paused = hs->done == kPaused;
+            const UnchainedLaunches unchained;
             if (paused) KMC_TRY(a.fit->enqueue_relocation());
             if (a.iter_graph == nullptr || (hs->done && !paused)) {
                 KMC_TRY(a.fit->finalize_enqueue(a.hstate, a.hinertia));

@@ -55,6 +55,7 @@ template <typename I, bool HALF>
 __global__ void __launch_bounds__(32 * kSumsWarps, 1)
     sums64_kernel(const double *X, const double *w, const I *labels, double *out, double *out_sizes,
                   int64_t n, int d, int64_t k, const LoopState *guard) {
+    wait_for_previous();
     if (guard != nullptr && *reinterpret_cast<const volatile int *>(&guard->done)) return;
     extern __shared__ __align__(16) double sh[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
@@ -155,8 +156,8 @@ int launch_sums64(const double *X, const double *w, const I *labels, double *sum
     if (smem > 48 * 1024)
         KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    kern<<<(unsigned)copies, 32 * warps, smem, s>>>(X, w, labels, sums, sizes, n, (int)d, k, guard);
-    return check_launch("sums64");
+    return launch_chained("sums64", kern, dim3((unsigned)copies), dim3((unsigned)(32 * warps)), smem, s, X,
+                          w, labels, sums, sizes, n, (int)d, k, guard);
 }
 
 template int launch_sums64<int32_t>(const double *, const double *, const int32_t *, double *,
