@@ -413,21 +413,23 @@ def _roofline(workload, form, n, d, k, kern_ms, clocks, sm_count, f64=False):
         r = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
              "peak_source": "nominal dense FP64 rate of a GB300 (no measured FP64 peak); the "
                             "plain float64 form runs on the FP64 pipe",
-             "kernel": "tile_kernel (exact fused assignment + accumulation, float64)"}
+             "kernel": "panel_kernel + sums64_kernel (float64 labels certified by float32 scores, "
+                       "ordered float64 sums)"}
     elif form == "plain":
         clk_mhz = (clocks or {}).get("sm_max_mhz") or 2070.0
         peak = sm_count * 128 * 2 * clk_mhz * 1e6 / 1e12
         r = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
              "peak_source": f"nominal FP32 FFMA rate ({sm_count} SMs x 128 lanes x 2 flop x "
                             f"{clk_mhz:.0f} MHz); the plain form runs on the FP32 pipe",
-             "kernel": "tile_kernel (exact fused assignment + accumulation)"}
+             "kernel": "panel_kernel (exact fused assignment + accumulation)"}
     else:
         # the timed region is tens of milliseconds: the burst figure applies
         peak = peaks.get("bf16_tflops", 1900.0)
         r = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
              "peak_source": f"bf16_tflops (burst) of MEASURED_PEAKS.json ({peak_src}); the "
                             "fp16 dense tensor rate equals the bf16 one",
-             "kernel": "mixed_assign_kernel + recheck_kernel (tcgen05 assignment + accumulation)"}
+             "kernel": "mixed_assign_kernel + recheck_kernel + sum_sorted_kernel (tcgen05 "
+                       "assignment, then accumulation)"}
     per_sample = TRAFFIC_PER_SAMPLE.get((workload, form))
     r.update({"frac": achieved / peak, "traffic": per_sample * n if per_sample else None,
               "traffic_source": ("ncu capture at n=1M of this shape, scaled by n" if per_sample
