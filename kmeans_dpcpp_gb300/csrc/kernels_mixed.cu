@@ -152,6 +152,7 @@ struct MixedArgs {
     // the pass (cand) instead of labels; a combine kernel decides.
     int64_t k_img, col0;
     float *pmax;
+    int last_k;  // 16-feature steps of the last feature block (the rest is zero)
 };
 
 struct SmemLayout {
@@ -330,7 +331,8 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], 32 * kEpiWarps);
+            // one chunk: an accumulator belongs to a group of four warps
+            mbar_init(&tempty[b], NCH == 1 ? 16 * kEpiWarps : 32 * kEpiWarps);
         }
         mbar_init(cbar, 1);
         mbar_init(tdone, 1);
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
             const uint32_t cbase = smem_u32(cimg_s);
             const uint32_t hbase = cbase + (uint32_t)(NKB * k_pad * 128);
             const uint64_t adesc_norm = desc_sw32(smem_u32(aon_s));
+            const int last_k = a.last_k;
             bool ok = mbar_wait(cbar, 0, err, lim);
             int s = 0;
             uint32_t ph = 0, cnt = 0;
@@ -421,6 +424,9 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
                     for (int kb = 0; kb < NKB; ++kb)
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
+                            // steps of padding would add zeros (2M x 32, k = 1000:
+                            // 216 -> 200 us; 4M x 16, 100: 153 -> 144)
+                            if (kb == NKB - 1 && kk > 0 && kk >= last_k) continue;
                             const uint64_t ad = desc_sw128(xbase + kb * kTileBytes + kk * 32);
                             const uint64_t bd = desc_sw128(cbase + (uint32_t)(kb * k_pad * 128) +
                                                            (uint32_t)(c * kChunkN * 128) + kk * 32);
@@ -444,6 +450,122 @@ __global__ void __launch_bounds__(kThreadsMixed, 1) mixed_assign_kernel(MixedArg
             mbar_wait_drain(tdone, 0, err);
         }
         __syncwarp();
+    } else if constexpr (NCH == 1) {
+        // ---------------------- epilogue, one chunk per tile -------------------
+        // Two groups of four warps take tiles in turn, each with an accumulator
+        // of its own; a thread scans a whole row, so nothing is exchanged, and
+        // one group's loads and masks run beside the other's (a chunk's chain of
+        // load, exchange, masks and labels bounded the tile: 4M x 64, k = 64
+        // 159 -> 144 us, k = 256 177 -> 153; 16 and 100 163 -> 153).  With more chunks the scans are as
+        // long as the tensor cores' work and two accumulators per tile hide
+        // more.
+        constexpr int kSub = 8;
+        const int ew = warp - 2, g = ew >> 2;
+        const int q = warp & 3;   // TMEM lane quadrant accessible to this warp
+        const int row = 32 * q + lane;
+        const uint32_t cb = tmem + ((uint32_t)(32 * q) << 16) + g * kChunkN;
+        // test of the timeout path: this wait runs out after `lim` clocks
+        if (a.stall) mbar_wait(never, 0, err, lim);
+        const int64_t step = 2 * (int64_t)gridDim.x;
+        // per-sample norms of the next tile are loaded one tile ahead
+        float nx_next = 0.f, dx_next = 0.f;
+        auto load_norms = [&](int64_t tile) {
+            const int64_t i = tile * kTileM + row;
+            if (i < n) {
+                nx_next = a.nx[i];
+                dx_next = a.ndx[i];
+            }
+        };
+        const int64_t first = blockIdx.x + (int64_t)g * gridDim.x;
+        load_norms(first);
+        uint32_t phase = 0;
+        for (int64_t tile = first; tile < ntiles; tile += step, phase ^= 1u) {
+            const int64_t i = tile * kTileM + row;
+            const float e = fmaf(nx_next, cst.alpha, fmaf(dx_next, cst.beta1, cst.beta0));
+            const float E2 = i < n ? 2.f * e * 1.000001f : 0.f;
+            load_norms(tile + step);
+            const bool bad = !mbar_wait(&tfull[g], phase, err, lim);
+            // tcgen05.ld is warp-collective: re-converge after the wait
+            if (__any_sync(0xffffffffu, bad || *err != 0)) break;
+            tc_fence_after();
+            float P2[32], P1[kSub];
+            {
+                uint32_t ra[32], rb[32], rc[32], rd[32], m[4];
+                tmem_ld32_max(cb, ra, m[0]);
+                tmem_ld32_max(cb + 32, rb, m[1]);
+                tmem_ld32_max(cb + 64, rc, m[2]);
+                tmem_ld32_max(cb + 96, rd, m[3]);
+                tmem_ld_wait_regs(ra, rb, rc, rd, m);
+#pragma unroll
+                for (int t = 0; t < 32; ++t)
+                    P2[t] = max3f(fmaxf(u2f(ra[t]), u2f(rb[t])), u2f(rc[t]), u2f(rd[t]));
+#pragma unroll
+                for (int t = 0; t < 4; ++t) P1[t] = u2f(m[t]);
+                // the loads below reuse the registers: finish every read first
+#pragma unroll
+                for (int t = 0; t < 32; ++t) asm volatile("" : "+f"(P2[t]));
+                tmem_ld32_max(cb + 128, ra, m[0]);
+                tmem_ld32_max(cb + 160, rb, m[1]);
+                tmem_ld32_max(cb + 192, rc, m[2]);
+                tmem_ld32_max(cb + 224, rd, m[3]);
+                tmem_ld_wait_regs(ra, rb, rc, rd, m);
+                tc_fence_before();
+                mbar_arrive(&tempty[g]);  // the accumulator may be overwritten now
+#pragma unroll
+                for (int t = 0; t < 32; ++t)
+                    P2[t] = max3f(max3f(P2[t], u2f(ra[t]), u2f(rb[t])), u2f(rc[t]), u2f(rd[t]));
+#pragma unroll
+                for (int t = 0; t < 4; ++t) P1[4 + t] = u2f(m[t]);
+            }
+            float M = -pos_inf<float>();
+#pragma unroll
+            for (int t = 0; t < kSub; ++t) M = fmaxf(M, P1[t]);
+            // as in the other form: columns that reach thr can win; two distinct
+            // ones differ in their sub-chunk or in their class
+            const float thr = M - E2;
+            uint32_t hot1 = 0u, hot2 = 0u;
+            const HotTest ht = hot_test(thr);
+            if (ht.ok) {
+                float l1 = 0.f, l2 = 0.f, h2 = 0.f;
+#pragma unroll
+                for (int t = 0; t < kSub; ++t) l1 = fmaf(ht.hot(P1[t]), (float)(1u << t), l1);
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    l2 = fmaf(ht.hot(P2[t]), (float)(1u << t), l2);
+                    h2 = fmaf(ht.hot(P2[16 + t]), (float)(1u << t), h2);
+                }
+                hot1 = __float2uint_rz(l1);
+                hot2 = __float2uint_rz(l2) | (__float2uint_rz(h2) << 16);
+            } else {
+#pragma unroll
+                for (int t = 0; t < kSub; ++t) hot1 |= (P1[t] >= thr) ? (1u << t) : 0u;
+#pragma unroll
+                for (int t = 0; t < 32; ++t) hot2 |= (P2[t] >= thr) ? (1u << t) : 0u;
+            }
+            if (!(thr == thr)) {  // cannot happen with finite operands; recheck all
+                hot1 = 0xffu;
+                hot2 = ~0u;
+            }
+            if (i >= n) continue;
+            const bool sure = __popc(hot1) == 1 && __popc(hot2) == 1;
+            if (MULTI || !sure) {
+                // by column halves, the classes of a row in both
+                const uint32_t lo = hot1 & 15u, hi = hot1 >> 4;
+                a.cand[i] = make_uint4(lo, hi, lo ? hot2 : 0u, hi ? hot2 : 0u);
+            }
+            if (MULTI) {
+                a.pmax[i] = M;  // decided by the combine
+            } else if (sure) {
+                const int code = (__ffs(hot1) - 1) * 32 + __ffs(hot2) - 1;
+                if (a.label64)
+                    reinterpret_cast<int64_t *>(a.labels)[i] = code;
+                else
+                    reinterpret_cast<int32_t *>(a.labels)[i] = code;
+            } else {
+                const int pos = atomicAdd(a.n_flagged, 1);
+                if (pos >= 0 && pos < n) a.flagged[pos] = (int)i;
+            }
+        }
     } else {
         // ------------------------------ epilogue ------------------------------
         // Thread (row, h) scans columns h*128 .. h*128+127 of every chunk for
@@ -2035,6 +2157,7 @@ struct MixedFit : PlainFit<float, I> {
         stall_once = 0;
         const int64_t pass_cols = (int64_t)nch * kChunkN;
         a.k_img = k_pad;
+        a.last_k = (int)ceil_div<int64_t>(std::max<int64_t>(p.d, 1) - 64 * (nkb - 1), 16);
         const bool multi = passes > 1;
         const SmemLayout L = smem_layout(nkb, pass_cols, stages);
         auto kern = pick_kernel(bf16, nkb, nch, multi);
