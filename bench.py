@@ -84,11 +84,11 @@ FP64_NOMINAL_TFLOPS = 1.25
 FORMS = {"plain": 0, "mixed-bf16": 1, "mixed-fp16": 2}
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of
-# the dominant kernel per sample, from one ncu capture at n=1,000,000 of the
+# the dominant kernels per sample, from one ncu capture at n=1,000,000 of the
 # workload's shape (profiles/mixed_assign_c3_n1M.txt and
-# profiles/tile_kernel_plain_c3_n1M.txt); the kernels stream every sample
+# profiles/panel_kernel_plain_c3_n1M.txt); the kernels stream every sample
 # once, so a launch's traffic scales with n.
-TRAFFIC_PER_SAMPLE = {("c3", "mixed-fp16"): 404.9, ("c3", "plain"): 267.6}
+TRAFFIC_PER_SAMPLE = {("c3", "mixed-fp16"): 415.2, ("c3", "plain"): 269.9}
 
 
 # ---------------------------------------------------------------------------
