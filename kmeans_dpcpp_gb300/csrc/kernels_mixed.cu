@@ -49,15 +49,17 @@
 // sums over 4M x 64: 560 -> 454 us at k = 1024, 443 -> 211 us at k = 64.
 //
 // Kernel roles (one CTA of 320 threads per SM, persistent over 128-sample
-// tiles; 10 warps leave up to 204 registers per thread):
+// tiles, 168 registers per thread at most):
 //   warp 0      bulk copies: the centroid image once, X tiles into a 2-4 stage ring
 //   warp 1      TMEM allocation; one thread issues tcgen05.mma (M=128, N=256,
 //               K=16) into two 256-column TMEM accumulators
-//   warps 2-9   epilogue: tcgen05.ld of scores, P1/P2, certification, labels
+//   warps 2-9   epilogue: tcgen05.ld of scores, P1/P2, certification, labels (two
+//               threads per row; tiles of one chunk: two groups, a thread per row)
 // The recheck kernel labels the samples that were not certified; the cluster
 // sums are a pass of their own over the labels (sum_sorted_kernel).
 // A pass without sums over 4M x 64 (two update warps in the kernel before):
-// 454 -> 416 us at k = 1024, 217 -> 177 us at k = 256, 211 -> 159 us at k = 64.
+// 454 -> 416 us at k = 1024, 217 -> 177 us at k = 256, 211 -> 159 us at k = 64
+// (146 and 145 with the two groups).
 //
 // Every wait is bounded.  A wait that runs out raises the CTA's error flag;
 // the other roles see it and stop, the producer and the MMA issuer then wait
