@@ -378,10 +378,7 @@ int launch_tile(TileArgs<T, I, A> args, cudaStream_t s) {
     size_t smem = TileSmem<T, TN>::base_bytes;
     if (MODE == MODE_FUSED && args.priv) smem += sizeof(A) * (size_t)(args.d * args.k + args.k);
     auto kern = tile_kernel<T, I, MODE, A, TN>;
-    if (smem > 48 * 1024) {
-        KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-    }
+    if (smem > 48 * 1024) KMC_TRY(allow_smem(kern, TileSmem<T, TN>::base_bytes + kPrivMaxBytes));
     int per_sm = 0;
     KMC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     if (per_sm < 1) per_sm = 1;

@@ -2100,9 +2100,7 @@ struct MixedFit : PlainFit<float, I> {
         {
             auto xk = bf16 ? x_image_kernel<1> : x_image_kernel<0>;
             const size_t xsm = x_image_smem(nkb);
-            if (xsm > 48 * 1024)
-                KMC_CUDA_TRY(cudaFuncSetAttribute(xk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)xsm));
+            if (xsm > 48 * 1024) KMC_TRY(allow_smem(xk, x_image_smem(kMaxFeatureBlocks)));
             const int64_t xg = std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)num_sms() * 8));
             xk<<<(unsigned)xg, kXImageThreads, xsm, s>>>(p.X, p.n, p.d, d4, nkb, ntiles, consts,
                                                          ximg, xrow, nx, ndx, p.x_rowmajor, p.w,
@@ -2172,8 +2170,7 @@ struct MixedFit : PlainFit<float, I> {
             set_error("mixed form: no kernel for %d feature blocks and %d chunks", nkb, nch);
             return KMC_ERR_UNSUPPORTED;
         }
-        KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)L.total));
+        KMC_TRY(allow_smem(kern, kSmemLimit));
         const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(ntiles, num_sms()));
         if (p.n > 0) {
             for (int ps = 0; ps < passes; ++ps) {
@@ -2219,9 +2216,7 @@ struct MixedFit : PlainFit<float, I> {
             auto kern = !acc_f64 ? sum_sorted_kernel<I, 0>
                                  : (variant % 10 == 2 ? sum_sorted_kernel<I, 2> : sum_sorted_kernel<I, 4>);
             const size_t smem = sort_smem(tile, p.k);
-            if (smem > 48 * 1024)
-                KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)smem));
+            if (smem > 48 * 1024) KMC_TRY(allow_smem(kern, sort_smem(kSortTile, kSortClusters)));
             return launch_chained("mixed_sums", kern, dim3((unsigned)sum_grid()), dim3(kSumThreads), smem,
                                   p.stream, xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32,
                                   fx_acc(), acc64, n_copies, consts, guard);

@@ -383,8 +383,7 @@ int launch_relocation(const RelocArgs<T, I> &a, cudaStream_t s) {
                             ? sizeof(float) * kDistTile * (kRelocThreads / 32)
                             : 0;
     auto kern = relocate_kernel<T, I>;
-    if (smem > 0)
-        KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 0) KMC_TRY(allow_smem(kern, smem));
     RelocArgs<T, I> args = a;
     void *params[] = {&args};
     KMC_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(grid),

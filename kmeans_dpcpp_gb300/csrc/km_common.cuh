@@ -83,6 +83,17 @@ inline int check_launch(const char *what) {
     return KMC_OK;
 }
 
+// Lets launches of a kernel take up to `most` bytes of dynamic shared memory.  The
+// limit belongs to the function, not to a launch, so `most` is what the largest
+// shape takes, the same in every call for a kernel: with a launch's own size, a
+// call of another host thread could narrow the limit in front of that launch.
+// Set in front of every launch that may need it, which holds after a device reset too.
+template <typename... K>
+int allow_smem(void (*kern)(K...), size_t most) {
+    KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return KMC_OK;
+}
+
 // Launches of a chain of dependent kernels on a stream (programmatic dependent
 // launch): the kernel may be set up while the one before still runs, and waits
 // in wait_for_previous(), its first instruction, until that one is complete and

@@ -533,8 +533,7 @@ int launch_width(const Args<T, A> &a, cudaStream_t s) {
     const int warps = (int)std::max<int64_t>(
         1, std::min<int64_t>(warps_for(a.d, MODE), ceil_div<int64_t>(wtiles, num_sms())));
     const size_t smem = sizeof(float) * shape(a.d, a.k, TN, MODE, warps).total;
-    KMC_CUDA_TRY(
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KMC_TRY(allow_smem(kern, kSmemBytes));
     const int64_t grid = std::min<int64_t>(num_sms(), ceil_div<int64_t>(wtiles, warps));
     return launch_chained("panel", kern, dim3((unsigned)grid), dim3((unsigned)(32 * warps)), smem, s, a);
 }

@@ -174,9 +174,7 @@ int launch_sums64(const double *X, const double *w, const I *labels, double *sum
     const int warps = warps_for(d, k);
     const size_t smem = warp_bytes(d, k) * (size_t)warps;
     auto kern = half_warps(d) ? sums64_kernel<I, true> : sums64_kernel<I, false>;
-    if (smem > 48 * 1024)
-        KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    if (smem > 48 * 1024) KMC_TRY(allow_smem(kern, kSumsSmem));
     return launch_chained("sums64", kern, dim3((unsigned)copies), dim3((unsigned)(32 * warps)), smem, s, X,
                           w, labels, sums, sizes, n, (int)d, k, guard);
 }
