@@ -1507,6 +1507,7 @@ __global__ void __launch_bounds__(kSumThreads) sum_terms_kernel(
 // kSortClusters most runs are single samples and the sort only costs.
 constexpr int kSortTile = 4096, kSortClusters = 2048;
 constexpr int kSortCtas = 4;  // resident per SM (64 registers)
+constexpr size_t kSortStatic = 1024;  // more than the kernel's static shared memory
 
 inline size_t sort_smem(int tile, int64_t k) {
     return (sizeof(int2) + sizeof(float)) * (size_t)tile + sizeof(int) * (size_t)(k + 1);
@@ -2216,7 +2217,9 @@ struct MixedFit : PlainFit<float, I> {
             auto kern = !acc_f64 ? sum_sorted_kernel<I, 0>
                                  : (variant % 10 == 2 ? sum_sorted_kernel<I, 2> : sum_sorted_kernel<I, 4>);
             const size_t smem = sort_smem(tile, p.k);
-            if (smem > 48 * 1024) KMC_TRY(allow_smem(kern, sort_smem(kSortTile, kSortClusters)));
+            // the kernel's own arrays count towards the 48 KB too
+            if (smem + kSortStatic > 48 * 1024)
+                KMC_TRY(allow_smem(kern, sort_smem(kSortTile, kSortClusters)));
             return launch_chained("mixed_sums", kern, dim3((unsigned)sum_grid()), dim3(kSumThreads), smem,
                                   p.stream, xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32,
                                   fx_acc(), acc64, n_copies, consts, guard);
