@@ -681,12 +681,29 @@ int batch_sum_copies(int64_t n, int64_t d, int64_t k) {
     return elems <= 65536 ? kFewSumCopies : elems <= 524288 ? 4 : 1;
 }
 
+namespace {
+// Instances of a launch: its grid counts them along y, whose extent is limited.
+// (Along x, with an instance's CTAs far apart, 24 fits ran 1 % slower.)
+constexpr int kSliceInstances = 65535;
+
+// launch(first, instances) for slices of `count` instances, at least once.
+template <typename F>
+int in_slices(int count, const char *what, F launch) {
+    for (int first = 0; first == 0 || first < count; first += kSliceInstances) {
+        launch(first, std::min(count - first, kSliceInstances));
+        KMC_TRY(check_launch(what));
+    }
+    return KMC_OK;
+}
+}  // namespace
+
 int launch_batch_prep(BInst *tab, const int *idx, int count, int64_t max_k, int *counters,
                       cudaStream_t s) {
-    const dim3 grid((unsigned)std::max<int64_t>(1, ceil_div<int64_t>(max_k, kPrepThreads)),
-                    (unsigned)std::max(count, 1));
-    batch_prep_kernel<<<grid, kPrepThreads, 0, s>>>(tab, idx, count, counters);
-    return check_launch("batch_prep");
+    const unsigned parts = (unsigned)std::max<int64_t>(1, ceil_div<int64_t>(max_k, kPrepThreads));
+    return in_slices(count, "batch_prep", [&](int first, int m) {
+        const dim3 grid(parts, (unsigned)std::max(m, 1));
+        batch_prep_kernel<<<grid, kPrepThreads, 0, s>>>(tab, idx + first, m, counters);
+    });
 }
 
 int prepare_batch_assign() {
@@ -740,19 +757,21 @@ unsigned ctas_per_instance(int64_t most, int count) {
 int launch_batch_reduce(BInst *tab, const int *idx, int count, int64_t max_elems,
                         int *n_empty_out, cudaStream_t s) {
     if (count <= 0) return KMC_OK;
-    const dim3 grid(ctas_per_instance(ceil_div<int64_t>(max_elems, 2 * kReduceLanes), count),
-                    (unsigned)count);
-    batch_reduce_kernel<<<grid, kBatchReduceThreads, 0, s>>>(tab, idx, count, n_empty_out);
-    return check_launch("batch_reduce");
+    const unsigned parts = ctas_per_instance(ceil_div<int64_t>(max_elems, 2 * kReduceLanes), count);
+    return in_slices(count, "batch_reduce", [&](int first, int m) {
+        batch_reduce_kernel<<<dim3(parts, (unsigned)m), kBatchReduceThreads, 0, s>>>(
+            tab, idx + first, m, n_empty_out + first);
+    });
 }
 
 int launch_batch_update(BInst *tab, const int *idx, int count, int64_t max_k, int *done_out,
                         bool relocated, cudaStream_t s) {
     if (count <= 0) return KMC_OK;
-    const dim3 grid(ctas_per_instance(ceil_div<int64_t>(max_k, 32), count), (unsigned)count);
-    batch_update_kernel<<<grid, kFinishThreads, 0, s>>>(tab, idx, count, done_out,
-                                                        relocated ? 1 : 0);
-    return check_launch("batch_update");
+    const unsigned parts = ctas_per_instance(ceil_div<int64_t>(max_k, 32), count);
+    return in_slices(count, "batch_update", [&](int first, int m) {
+        batch_update_kernel<<<dim3(parts, (unsigned)m), kFinishThreads, 0, s>>>(
+            tab, idx + first, m, done_out + first, relocated ? 1 : 0);
+    });
 }
 
 int launch_blobs(float *X, int64_t n, int64_t d, int64_t n_centers, float box_lo,
