@@ -484,20 +484,22 @@ int kmc_fit_set_profiling(kmc_fit_t fit, int enable);
 int kmc_fit_phase_time(kmc_fit_t fit, int phase, double *total_ms_out, int64_t *count_out);
 /* Mixed forms: samples whose tensor-core margin did not certify their label
  * and were re-evaluated in exact float32 (last pass and running total), and
- * the device-side error flag of the tensor-core kernel (1 after a bounded
- * wait timed out).  Plain form: zeros.  Blocking. */
+ * the device-side error flag (1 after a bounded wait timed out).  The plain
+ * form rechecks nothing (zeros).  Blocking. */
 int kmc_fit_rechecked(kmc_fit_t fit, int64_t *last_out, int64_t *total_out, int *device_error_out);
 /* No counterpart in the reference.  Limit, in SM clocks, of every
- * device-side wait of the tensor-core kernels of a mixed-form session
- * (clocks <= 0 restores the default, 4e9 clocks or about two seconds).  A
- * wait that runs out makes the kernel wind down (it waits for the copies and
- * tensor-core operations it issued, frees its tensor memory) and stops the
- * loop; the next blocking call (kmc_fit_run, kmc_fit_status,
- * kmc_fit_finalize) returns KMC_ERR_DEVICE_TIMEOUT and kmc_fit_rechecked
- * reports device_error = 1.  stall_once = 1 makes the next assignment pass
- * first wait on a barrier that nothing completes, so that this wait runs out
- * after `clocks`: a test of the timeout path that faults and hangs nothing.
- * The plain form has no device-side waits and ignores both. */
+ * device-side wait of a session: those of the mixed forms' tensor-core kernels
+ * and, in every form, the grid barriers of the kernel that relocates empty
+ * clusters (clocks <= 0 restores the default, 4e9 clocks or about two
+ * seconds).  A wait that runs out makes the kernel wind down (a tensor-core
+ * kernel waits for the copies and tensor-core operations it issued and frees
+ * its tensor memory) and stops the loop; the next blocking call (kmc_fit_run,
+ * kmc_fit_status, kmc_fit_finalize) returns KMC_ERR_DEVICE_TIMEOUT and
+ * kmc_fit_rechecked reports device_error = 1.  The limit holds for what is
+ * enqueued afterwards.  stall_once = 1 makes the next assignment pass of a
+ * mixed form first wait on a barrier that nothing completes, so that this wait
+ * runs out after `clocks`: a test of the timeout path that faults and hangs
+ * nothing (the plain form ignores it). */
 int kmc_fit_set_wait_limit(kmc_fit_t fit, int64_t clocks, int stall_once);
 /* No counterpart in the reference (whose kernels take a window height and a
  * work-group size as arguments).  The plain form's kernels choose their

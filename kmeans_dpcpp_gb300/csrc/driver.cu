@@ -246,7 +246,7 @@ int PlainFit<T, I>::enqueue_relocation() {
     const T *cr = c_rows(&crs);
     const RelocArgs<T, I> ra{p.centroids, p.new_centroids, prev, sums, sizes, shifts, empty_list,
                              reloc, reloc + p.k, reloc + 2 * p.k, xv, p.w, p.labels, sq_dist, p.n,
-                             p.d, p.k, xfs, xss, cr, crs, wait_clocks(), state, ctl};
+                             p.d, p.k, xfs, xss, cr, crs, wait_limit, state, ctl};
     KMC_TRY((launch_relocation<T, I>(ra, p.stream)));
     hn_current = false;
     ++launches;
@@ -277,6 +277,17 @@ int PlainFit<T, I>::read_state(LoopState &out) {
     KMC_CUDA_TRY(cudaStreamSynchronize(prm.stream));
     host_done = out.done;
     return check_device_error(out);
+}
+
+template <typename T, typename I>
+int PlainFit<T, I>::counters(int64_t *last, int64_t *total, int *device_error) {
+    LoopState h{};
+    KMC_CUDA_TRY(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, prm.stream));
+    KMC_CUDA_TRY(cudaStreamSynchronize(prm.stream));
+    if (last) *last = 0;
+    if (total) *total = 0;
+    if (device_error) *device_error = h.err != 0;
+    return KMC_OK;
 }
 
 // Two batches of iterations are in flight: while one runs, the host waits for

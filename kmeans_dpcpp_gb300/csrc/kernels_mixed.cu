@@ -1921,13 +1921,11 @@ struct MixedFit : PlainFit<float, I> {
     uint4 *cand = nullptr;
     int *flagged = nullptr, *n_flagged = nullptr, *err_dev = nullptr;
     long long *stats = nullptr;  // [0] last pass, [1] total
-    long long wait_limit = kWaitClocks;
     int stall_once = 0;
 
     int set_wait_limit(long long clocks, int stall) override {
-        wait_limit = clocks > 0 ? clocks : kWaitClocks;
         stall_once = stall != 0;
-        return KMC_OK;
+        return Base::set_wait_limit(clocks, stall);
     }
 
     // The one-time conversion reads X in either layout; afterwards every
@@ -2117,7 +2115,6 @@ struct MixedFit : PlainFit<float, I> {
         *n_launches = 0;
         return KMC_OK;
     }
-    long long wait_clocks() const override { return wait_limit; }
     const float *c_rows(int64_t *stride) const override {
         *stride = d4;
         return ct;
@@ -2157,7 +2154,7 @@ struct MixedFit : PlainFit<float, I> {
         a.n = p.n;
         a.label64 = sizeof(I) == 8 ? 1 : 0;
         a.stages = stages;
-        a.wait_limit = wait_limit;
+        a.wait_limit = this->wait_limit;
         a.stall = stall_once;
         a.state = this->state;
         stall_once = 0;
@@ -2265,9 +2262,11 @@ struct MixedFit : PlainFit<float, I> {
         KMC_CUDA_TRY(cudaMemcpyAsync(&e, err_dev, sizeof(int), cudaMemcpyDeviceToHost,
                                      this->prm.stream));
         KMC_CUDA_TRY(cudaStreamSynchronize(this->prm.stream));
+        int reloc = 0;  // a relocation's wait
+        KMC_TRY(Base::counters(nullptr, nullptr, &reloc));
         if (last) *last = h[0];
         if (total) *total = h[1];
-        if (device_error) *device_error = e;
+        if (device_error) *device_error = e != 0 || reloc != 0;
         return KMC_OK;
     }
 };

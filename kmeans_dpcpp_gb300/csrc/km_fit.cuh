@@ -68,28 +68,20 @@ struct FitBase {
     // inertia total land in *state_out and *inertia_out (pinned host memory)
     // once the fit's stream reaches this point.
     virtual int finalize_enqueue(LoopState *state_out, double *inertia_out) = 0;
-    // Limit (SM clocks) of the device-side waits of the tensor-core kernels;
-    // with `stall`, the next assignment pass first waits on a barrier that
+    // Limit (SM clocks; <= 0: the default) of the device-side waits: of the
+    // tensor-core kernels and of a relocation's grid barriers.  With `stall`,
+    // the next tensor-core assignment pass first waits on a barrier that
     // nothing completes, so that wait runs out (test of the timeout path).
-    // The plain form has no device-side waits and ignores both.
-    virtual int set_wait_limit(long long clocks, int stall) {
-        (void)clocks;
-        (void)stall;
-        return KMC_OK;
-    }
+    virtual int set_wait_limit(long long clocks, int stall) = 0;
     // Centroid-tile variant of the plain form's kernels (the autotuner's
     // choice unless set here); the mixed forms ignore it.
     virtual int set_tile_variant(int v) {
         (void)v;
         return KMC_OK;
     }
-    // Samples re-evaluated in exact arithmetic (mixed form): last pass and total.
-    virtual int counters(int64_t *last, int64_t *total, int *device_error) {
-        if (last) *last = 0;
-        if (total) *total = 0;
-        if (device_error) *device_error = 0;
-        return KMC_OK;
-    }
+    // Samples re-evaluated in exact arithmetic (mixed form): last pass and
+    // total; and whether a device-side wait ran out.
+    virtual int counters(int64_t *last, int64_t *total, int *device_error) = 0;
 };
 
 // Pinned host memory for a fit's loop state (two reads in flight) and inertia,
@@ -133,7 +125,15 @@ struct PlainFit : FitBase {
     bool split64 = false;  // float64 samples: labels, then sums (sums64.cu)
     int tile_variant = 0;  // autotuned centroid-tile width of the plain kernels
     Scratch xt;  // feature-major copy of a row-major X (forms that need one)
+    static constexpr long long kWaitClocks = 4000000000LL;  // about two seconds
+    long long wait_limit = kWaitClocks;
 
+    int set_wait_limit(long long clocks, int stall) override {
+        (void)stall;
+        wait_limit = clocks > 0 ? clocks : kWaitClocks;
+        return KMC_OK;
+    }
+    int counters(int64_t *last, int64_t *total, int *device_error) override;
     int set_tile_variant(int v) override {
         KMC_CHECK_ARG(v >= 0 && v <= 2, "tile variant must be 0, 1 or 2");
         tile_variant = v;
@@ -161,8 +161,6 @@ struct PlainFit : FitBase {
         return FinishArgs<T>{p.centroids, p.new_centroids, prev, sums, sizes, shifts,
                              uses_private_copies() ? hn : nullptr, empty_list, p.d, p.k, 1, state, ctl};
     }
-    // Limit (SM clocks) of the waits of a relocation's grid barriers.
-    virtual long long wait_clocks() const { return 4000000000LL; }
     // Half norms of the current centroids, where neither the form's own
     // preparation nor the end of the iteration before made them.
     virtual int begin_step(int64_t *n_launches) {
