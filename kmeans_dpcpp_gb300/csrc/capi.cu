@@ -158,11 +158,11 @@ int relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *
     T *thr = reinterpret_cast<T *>(b + o_thr);
     I *cnt = reinterpret_cast<I *>(b + o_cnt);
     I *sel = reinterpret_cast<I *>(b + o_sel);
-    KMC_TRY(launch_threshold<T>(sq_dist, n, n_empty, thr, b + o_tsc, s));
+    KMC_TRY(launch_threshold<T>(sq_dist, n, n_empty, thr, b + o_tsc, s, true));
     KMC_TRY(launch_fill<I>(cnt, I(0), 1, s));
     KMC_TRY(launch_fill<I>(cnt + 1, I(1), 1, s));
     KMC_TRY(launch_select<T, I>(n_empty, sq_dist, thr, sel, cnt, cnt + 1, n, b + o_ssc, s));
-    return launch_relocate<T, I>(n_empty, X, w, labels, sel, cnt, list, C, sizes,
+    return launch_relocate<T, I>(n_empty, X, w, labels, sel, cnt, cnt + 1, list, C, sizes,
                                  inertia, n, d, k, s);
 }
 

@@ -52,6 +52,12 @@ struct KeyOf<double> {
     }
 };
 
+// NaN as a relocation ranks it: below every distance.
+template <typename T>
+__device__ __forceinline__ T nan_last(T v) {
+    return v == v ? v : -pos_inf<T>();
+}
+
 // Radix-select scratch (device memory).
 struct SelectState {
     unsigned long long hist[256];
@@ -73,7 +79,8 @@ __global__ void threshold_init_kernel(SelectState *st, int64_t topk, int64_t n) 
 }
 
 template <typename T>
-__global__ void threshold_hist_kernel(const T *data, int64_t n, SelectState *st, int pass) {
+__global__ void threshold_hist_kernel(const T *data, int64_t n, SelectState *st, int pass,
+                                      int low_nan) {
     using K = KeyOf<T>;
     using U = typename K::U;
     if (st->active == 0) return;
@@ -86,7 +93,8 @@ __global__ void threshold_hist_kernel(const T *data, int64_t n, SelectState *st,
     const U hi_mask = (pass == 0) ? (U)0 : (U)(~(U)0) << (kBits - 8 * pass);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        U key = K::key(data[i]);
+        const T v = data[i];
+        const U key = K::key(low_nan ? nan_last(v) : v);
         if ((key & hi_mask) == prefix) atomicAdd(&h[(unsigned)(key >> shift) & 0xffu], 1u);
     }
     __syncthreads();
@@ -410,14 +418,19 @@ __global__ void select_place_kernel(SelLayout L, I *selected) {
     }
 }
 
-// relocate_empty_clusters_kernel, src/util_kernels.hpp:302-390.
+// relocate_empty_clusters_kernel, src/util_kernels.hpp:302-390.  n_gt, n_eq: the
+// selection's counters, started at 0 and 1.
 template <typename T, typename I>
 __global__ void relocate_kernel(int64_t n_empty, const T *X, const T *w, const I *labels,
-                                const I *selected, const I *n_gt, const I *empty_list, T *sums,
-                                T *sizes, T *inertia, int64_t n, int64_t d, int64_t k) {
+                                const I *selected, const I *n_gt, const I *n_eq,
+                                const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
+                                int64_t d, int64_t k) {
     const int64_t gt = (int64_t)*n_gt;
-    // Samples available: the gt ones plus the eq ones written at the back.
-    if (n_empty > n) n_empty = n;
+    // Samples available: the gt ones plus the eq ones written at the back; fewer
+    // than n_empty where the distances of the others are NaN (the last empty
+    // clusters then get none).
+    const int64_t available = gt + (int64_t)*n_eq - 1;
+    if (n_empty > available) n_empty = available;
     int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (f >= d) return;
     for (int64_t r = 0; r < n_empty; ++r) {
@@ -447,14 +460,14 @@ size_t threshold_scratch_bytes() { return align256(sizeof(SelectState)); }
 
 template <typename T>
 int launch_threshold(const T *data, int64_t n, int64_t topk, T *threshold, void *scratch,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool low_nan) {
     SelectState *st = static_cast<SelectState *>(scratch);
     threshold_init_kernel<<<1, 256, 0, s>>>(st, topk, n);
     KMC_TRY(check_launch("threshold_init"));
     int64_t g = ceil_div<int64_t>(n, 1024);
     int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, (int64_t)num_sms() * 4));
     for (int pass = 0; pass < KeyOf<T>::kPasses; ++pass) {
-        threshold_hist_kernel<T><<<grid, 1024, 0, s>>>(data, n, st, pass);
+        threshold_hist_kernel<T><<<grid, 1024, 0, s>>>(data, n, st, pass, low_nan ? 1 : 0);
         KMC_TRY(check_launch("threshold_hist"));
         threshold_digit_kernel<T><<<1, 256, 0, s>>>(st, pass, threshold);
         KMC_TRY(check_launch("threshold_digit"));
@@ -496,24 +509,24 @@ int launch_select(int64_t max_selected, const T *dist, const T *threshold, I *se
 
 template <typename T, typename I>
 int launch_relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *selected,
-                    const I *n_gt, const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
-                    int64_t d, int64_t k, cudaStream_t s) {
+                    const I *n_gt, const I *n_eq, const I *empty_list, T *sums, T *sizes,
+                    T *inertia, int64_t n, int64_t d, int64_t k, cudaStream_t s) {
     int grid = (int)ceil_div<int64_t>(std::max<int64_t>(d, 1), 128);
-    relocate_kernel<T, I><<<grid, 128, 0, s>>>(n_empty, X, w, labels, selected, n_gt, empty_list,
-                                               sums, sizes, inertia, n, d, k);
+    relocate_kernel<T, I><<<grid, 128, 0, s>>>(n_empty, X, w, labels, selected, n_gt, n_eq,
+                                               empty_list, sums, sizes, inertia, n, d, k);
     return check_launch("relocate");
 }
 
 template int launch_threshold<float>(const float *, int64_t, int64_t, float *, void *,
-                                     cudaStream_t);
+                                     cudaStream_t, bool);
 template int launch_threshold<double>(const double *, int64_t, int64_t, double *, void *,
-                                      cudaStream_t);
+                                      cudaStream_t, bool);
 #define KMC_INST_RELOC(T, I)                                                                  \
     template int launch_select<T, I>(int64_t, const T *, const T *, I *, I *, I *, int64_t,   \
                                      void *, cudaStream_t);                                   \
     template int launch_relocate<T, I>(int64_t, const T *, const T *, const I *, const I *,   \
-                                       const I *, const I *, T *, T *, T *, int64_t, int64_t, \
-                                       int64_t, cudaStream_t);
+                                       const I *, const I *, const I *, T *, T *, T *,        \
+                                       int64_t, int64_t, int64_t, cudaStream_t);
 KMC_INST_RELOC(float, int32_t)
 KMC_INST_RELOC(float, int64_t)
 KMC_INST_RELOC(double, int32_t)

@@ -7,6 +7,8 @@ namespace kmc {
 namespace {
 
 // Order-preserving unsigned keys (larger value -> larger key) and their digits.
+// Not of NaN, whose bits are the compiler's to choose: its key could differ
+// between the histograms of one selection.
 __device__ __forceinline__ unsigned long long order_of(float v) {
     const unsigned b = __float_as_uint(v);
     return (b & 0x80000000u) ? (unsigned)~b : (b | 0x80000000u);
@@ -84,7 +86,9 @@ constexpr int64_t kRankAll = 4096;  // ranked by counting all pairs; beyond, by 
 
 // The relocation of src/util_kernels.hpp:163-476: the r-th empty cluster (in
 // ascending order) takes the r-th farthest sample (ties: the lower index); the
-// threshold is found by a radix select over 8-bit digits.  Every CTA of the
+// threshold is found by a radix select over 8-bit digits.  Samples whose distance
+// is NaN rank last and stay; where too few others are left, the last empty
+// clusters get none.  Every CTA of the
 // grid works on its range of samples, with a grid barrier between the phases.
 // Bounded by the pass over X for the distances; the selection reads 4 bytes a
 // sample and pass from L2.
@@ -128,6 +132,7 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
         } else if (ok) {
             v = sq_dist_cols<T>(a.X, a.fs, a.ss, a.prev, d, k, i, c);
         }
+        if (!(v == v)) v = -pos_inf<T>();  // no distance
         if (i < b1) a.sq_dist[i] = v;
         // the leading digits of similar distances are the same few: lanes that
         // share the first lane's digit count once
@@ -206,10 +211,11 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
     if (!grid_barrier(ctl, round, a.wait_limit)) return false;
     const bool any = pick[0] != 0ull;  // of this CTA's samples
     // samples of the CTAs before this one, and of all CTAs
-    long long pg = 0, pe = 0, tg = 0;
+    long long pg = 0, pe = 0, tg = 0, te = 0;
     for (int b = tid; b < (int)gridDim.x; b += kRelocThreads) {
         const long long g = __ldcg(&ctl->counts[b]), e = __ldcg(&ctl->counts[kMaxRelocCtas + b]);
         tg += g;
+        te += e;
         if (b < (int)blockIdx.x) {
             pg += g;
             pe += e;
@@ -219,20 +225,25 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
         pg += __shfl_down_sync(0xffffffffu, pg, o);
         pe += __shfl_down_sync(0xffffffffu, pe, o);
         tg += __shfl_down_sync(0xffffffffu, tg, o);
+        te += __shfl_down_sync(0xffffffffu, te, o);
     }
     if (lane == 0) {
         wsum[0][wid] = pg;
         wsum[1][wid] = pe;
         h[wid] = (unsigned long long)tg;
+        h[kRelocThreads / 32 + wid] = (unsigned long long)te;
     }
     __syncthreads();
-    pg = pe = tg = 0;
+    pg = pe = tg = te = 0;
     for (int q = 0; q < kRelocThreads / 32; ++q) {
         pg += wsum[0][q];
         pe += wsum[1][q];
         tg += (long long)h[q];
+        te += (long long)h[kRelocThreads / 32 + q];
     }
-    const long long need = m - tg;  // at the threshold (fewer than m lie beyond it)
+    // at the threshold (fewer than m lie beyond it; none when only samples
+    // without a distance are left)
+    const long long need = thr == -pos_inf<T>() ? 0 : (m - tg < te ? m - tg : te);
     __syncthreads();
     for (int64_t i0 = b0; any && i0 < b1; i0 += kRelocThreads) {
         const int64_t i = i0 + tid;

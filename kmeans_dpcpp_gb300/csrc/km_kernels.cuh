@@ -145,9 +145,10 @@ int launch_distances(const T *X, const T *C, T *out, int64_t n, int64_t d, int64
 // relocate in kernels_step.cu) ----
 // Scratch bytes needed by launch_threshold for n samples.
 size_t threshold_scratch_bytes();
+// NaN ranks above every number, with low_nan (relocations) below.
 template <typename T>
 int launch_threshold(const T *data, int64_t n, int64_t topk, T *threshold, void *scratch,
-                     cudaStream_t s);
+                     cudaStream_t s, bool low_nan = false);
 // Scratch for launch_select of n_selected samples.
 size_t select_scratch_bytes(int64_t n_selected);
 template <typename T, typename I>
@@ -155,7 +156,7 @@ int launch_select(int64_t n_selected, const T *dist, const T *threshold, I *sele
                   I *n_eq, int64_t n, void *scratch, cudaStream_t s);
 template <typename T, typename I>
 int launch_relocate(int64_t n_empty, const T *X, const T *w, const I *labels, const I *selected,
-                    const I *n_gt, const I *empty_list, T *sums, T *sizes, T *inertia, int64_t n,
-                    int64_t d, int64_t k, cudaStream_t s);
+                    const I *n_gt, const I *n_eq, const I *empty_list, T *sums, T *sizes,
+                    T *inertia, int64_t n, int64_t d, int64_t k, cudaStream_t s);
 
 }  // namespace kmc

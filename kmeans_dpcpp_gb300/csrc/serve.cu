@@ -444,14 +444,14 @@ struct BatchEngine {
         int32_t *counters = sm.selected + h.n;
         KMC_TRY(launch_inertia<float, int32_t>(h.X, nullptr, h.C, h.labels, sm.sq_dist, h.n, h.d,
                                                h.k, s));
-        KMC_TRY(launch_threshold<float>(sm.sq_dist, h.n, m, sm.thr, sm.thr_scratch, s));
+        KMC_TRY(launch_threshold<float>(sm.sq_dist, h.n, m, sm.thr, sm.thr_scratch, s, true));
         KMC_TRY(launch_fill<int32_t>(counters, 0, 1, s));
         KMC_TRY(launch_fill<int32_t>(counters + 1, 1, 1, s));
         KMC_TRY(launch_select<float, int32_t>(m, sm.sq_dist, sm.thr, sm.selected, counters,
                                               counters + 1, h.n, sm.sel_scratch, s));
         KMC_TRY(launch_relocate<float, int32_t>(m, h.X, h.w, h.labels, sm.selected,
-                                                counters, sm.empty_list, sm.Cn, sm.sizes,
-                                                sm.sq_dist, h.n, h.d, h.k, s));
+                                                counters, counters + 1, sm.empty_list, sm.Cn,
+                                                sm.sizes, sm.sq_dist, h.n, h.d, h.k, s));
         ++relocations;
         return KMC_OK;
     }
