@@ -151,7 +151,8 @@ int PlainFit<T, I>::init(const FitParams<T, I> &p) {
     const size_t o_dsum = take(sizeof(double) * 2);
     KMC_TRY(ws.alloc(off, p.stream));
     // the tile kernels' width for this (d, k, dtype), where they are used
-    if (uses_private_copies() && !panel::fits(d)) KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
+    if (uses_private_copies() && (!panel::fits(d) || (sizeof(T) == 8 && !split64)))
+        KMC_TRY(tune_fit_variant<T>(d, k, p.stream, &tile_variant));
     if (p.x_rowmajor && !reads_rowmajor()) {
         KMC_TRY(xt.alloc(sizeof(T) * (size_t)n * (size_t)d, p.stream));
         if (sizeof(T) == 4)
