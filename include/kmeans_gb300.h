@@ -621,7 +621,8 @@ int kmc_generate_blobs_f32(float *X_t, int64_t n_samples, int64_t n_features,
                            float std_hi, uint64_t seed, kmc_stream_t stream);
 /* Seeded distinct row indices for random-row initialisation (host). */
 int kmc_seeded_rows(int64_t n_samples, int64_t n_clusters, uint64_t seed, int32_t *rows_out);
-/* The batched engine's work items for instances of n_samples[q] samples, mode
+/* The batched engine's work items for instances with more features than a
+ * panel takes (148, transforms 126), of n_samples[q] samples, mode
  * modes[q] (0 fit, 1 assign, 2 transform) and tile variant variants[q] (host
  * planning only, for tests): runs of at most 8 128-sample tiles, listed by
  * group (kind * 3 + variant; kind 1 = transforms) in instance order.  Writes up
@@ -630,6 +631,16 @@ int kmc_debug_batch_items(int64_t count, const int64_t *n_samples, const int *mo
                           const int *variants, int64_t capacity, int32_t *instance_out,
                           int32_t *tiles_out, int64_t *first_tile_out, int32_t *group_out,
                           int64_t *n_items_out);
+/* The same for the other instances, which are taken in panels: one list of runs
+ * of 128-sample tiles for the fits and assignments, one for the transforms
+ * (transform != 0), the most expensive first, on a device of `sms` SMs.  An item
+ * holds whole rounds of a CTA's warps (512 samples, fewer for many features),
+ * the last of an instance the rest.  No reference counterpart. */
+int kmc_debug_batch_panel_items(int64_t count, const int64_t *n_samples,
+                                const int64_t *n_features, const int64_t *n_clusters,
+                                int transform, int sms, int64_t capacity, int32_t *instance_out,
+                                int32_t *tiles_out, int64_t *first_tile_out,
+                                int64_t *n_items_out);
 
 /* ---- serving loop ------------------------------------------------------------------
  * No counterpart in the reference.  Replays a stream of fit and predict

@@ -33,7 +33,8 @@ namespace {
 
 constexpr int kItemTiles = 8;  // 128-sample tiles per work item
 
-// Work items of one instance: runs of at most kItemTiles 128-sample tiles,
+// Work items of one instance with more features than a panel takes: runs of at
+// most kItemTiles 128-sample tiles,
 // appended to the list of its (kind, tile variant); kind 1 = distance
 // (transform) instances, 0 = the rest.  The persistent assign kernels take
 // items from a device counter (atomicAdd), so every tile is handled by one
@@ -57,7 +58,7 @@ struct PanelJob {
     int64_t n, d, k;
 };
 
-void plan_panels(const std::vector<PanelJob> &jobs, int dist, std::vector<BItem> *out) {
+void plan_panels(const std::vector<PanelJob> &jobs, int dist, int sms, std::vector<BItem> *out) {
     // Cost in products (128 per clock and SM): besides its k products, a
     // feature of a sample costs a load and a reduction (half a clock), and each
     // round of a CTA about 5 us of latencies.
@@ -68,7 +69,7 @@ void plan_panels(const std::vector<PanelJob> &jobs, int dist, std::vector<BItem>
     };
     double all = 0.0;
     for (const PanelJob &j : jobs) all += cost(j, j.n);
-    const double share = all / (4.0 * num_sms());
+    const double share = all / (4.0 * sms);
     std::vector<std::pair<double, BItem>> items;
     for (const PanelJob &j : jobs) {
         const int round = std::max(1, batch_panel_round(j.d, dist));
@@ -360,7 +361,7 @@ struct BatchEngine {
             else
                 append_items((int)q, h.n, h.mode, h.variant, items);
         }
-        for (int kind = 0; kind < 2; ++kind) plan_panels(jobs[kind], kind, &panel_items[kind]);
+        for (int kind = 0; kind < 2; ++kind) plan_panels(jobs[kind], kind, num_sms(), &panel_items[kind]);
         auto list = [&](int kind, int v) -> const std::vector<BItem> & {
             return v < kBatchVariants ? items[kind][v] : panel_items[kind];
         };
@@ -1349,6 +1350,30 @@ int kmc_debug_batch_items(int64_t count, const int64_t *n_samples, const int *mo
             }
         }
     *n_items_out = total;
+    return KMC_OK;
+}
+
+int kmc_debug_batch_panel_items(int64_t count, const int64_t *n_samples, const int64_t *n_features,
+                                const int64_t *n_clusters, int transform, int sms,
+                                int64_t capacity, int32_t *instance_out, int32_t *tiles_out,
+                                int64_t *first_tile_out, int64_t *n_items_out) {
+    KMC_CHECK_ARG(count >= 0 && sms >= 1 && n_items_out != nullptr, "invalid arguments");
+    KMC_CHECK_ARG(count == 0 || (n_samples && n_features && n_clusters), "null input");
+    std::vector<kmc::PanelJob> jobs;
+    for (int64_t q = 0; q < count; ++q) {
+        KMC_CHECK_ARG(n_samples[q] >= 0 && n_clusters[q] >= 1 &&
+                          kmc::batch_in_panels(n_features[q], transform),
+                      "instance %lld is not taken in panels", (long long)q);
+        jobs.push_back(kmc::PanelJob{(int)q, n_samples[q], n_features[q], n_clusters[q]});
+    }
+    std::vector<kmc::BItem> items;
+    kmc::plan_panels(jobs, transform, sms, &items);
+    for (size_t t = 0; t < items.size() && (int64_t)t < capacity; ++t) {
+        instance_out[t] = items[t].inst;
+        tiles_out[t] = items[t].ntiles;
+        first_tile_out[t] = items[t].tile0;
+    }
+    *n_items_out = (int64_t)items.size();
     return KMC_OK;
 }
 
