@@ -1507,11 +1507,24 @@ __global__ void __launch_bounds__(kSumThreads) sum_terms_kernel(
 // kSortClusters most runs are single samples and the sort only costs.
 constexpr int kSortTile = 4096, kSortClusters = 2048;
 constexpr int kSortCtas = 4;  // resident per SM (64 registers)
-constexpr size_t kSortStatic = 1024;  // more than the kernel's static shared memory
 
-inline size_t sort_smem(int tile, int64_t k) {
-    return (sizeof(int2) + sizeof(float)) * (size_t)tile + sizeof(int) * (size_t)(k + 1);
+// Shared memory of a CTA.  All of it is dynamic: beside the 1024-byte aligned
+// image of the assignment kernel, a static array would take 1 KB.
+constexpr size_t kSortRowBytes = sizeof(int2) + sizeof(float);
+constexpr size_t sort_smem(int tile, int64_t k) {
+    return kSortRowBytes * (size_t)tile + sizeof(int) * (size_t)(k + 1 + kSumThreads / 32);
 }
+// The most rows of a tile, so that kSortCtas CTAs fit an SM (228 KB, 1 KB of a
+// CTA reserved): 4096 up to 2031 clusters, 4064 beyond.
+constexpr size_t kSortSmem = 228 * 1024 / kSortCtas - 1024;
+constexpr int sort_rows(int64_t k) {
+    const int64_t fit = (int64_t)((kSortSmem - sort_smem(0, k)) / kSortRowBytes) / 32 * 32;
+    return fit < kSortTile ? (int)fit : kSortTile;
+}
+static_assert(sort_rows(1) == kSortTile && sort_rows(2031) == kSortTile &&
+                  sort_rows(kSortClusters) == 4064 &&
+                  sort_smem(sort_rows(kSortClusters), kSortClusters) <= kSortSmem,
+              "tiles of the sorted sums");
 
 template <typename I, int F>
 __global__ void __launch_bounds__(kSumThreads, kSortCtas) sum_sorted_kernel(
@@ -1526,7 +1539,7 @@ __global__ void __launch_bounds__(kSumThreads, kSortCtas) sum_sorted_kernel(
     int2 *key = reinterpret_cast<int2 *>(sort_raw);  // (label, row of the tile) by label
     float *ws = reinterpret_cast<float *>(key + tile_rows);  // weights, same order
     int *hist = reinterpret_cast<int *>(ws + tile_rows);     // counts, then first positions
-    __shared__ int warp_sum[kWarps];
+    int *warp_sum = hist + k + 1;
     const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
     const int vecs = FX ? (int)d4 / 4 + 1 : (int)d4 / 4;  // 16-byte vectors of a row
     unsigned long long *isum = nullptr;
@@ -2203,7 +2216,7 @@ struct MixedFit : PlainFit<float, I> {
     int sum_tile() const {
         if (!sums_sorted()) return kSumThreads;
         const int64_t n = std::max<int64_t>(this->prm.n, 1), g = sum_grid();
-        const int64_t rounds = ceil_div<int64_t>(n, g * kSortTile);
+        const int64_t rounds = ceil_div<int64_t>(n, g * sort_rows(this->prm.k));
         return (int)(ceil_div<int64_t>(n, g * rounds * 32) * 32);
     }
 
@@ -2214,9 +2227,7 @@ struct MixedFit : PlainFit<float, I> {
             auto kern = !acc_f64 ? sum_sorted_kernel<I, 0>
                                  : (variant % 10 == 2 ? sum_sorted_kernel<I, 2> : sum_sorted_kernel<I, 4>);
             const size_t smem = sort_smem(tile, p.k);
-            // the kernel's own arrays count towards the 48 KB too
-            if (smem + kSortStatic > 48 * 1024)
-                KMC_TRY(allow_smem(kern, sort_smem(kSortTile, kSortClusters)));
+            if (smem > 48 * 1024) KMC_TRY(allow_smem(kern, kSortSmem));
             return launch_chained("mixed_sums", kern, dim3((unsigned)sum_grid()), dim3(kSumThreads), smem,
                                   p.stream, xrow, p.w, p.labels, p.n, d4, p.k, k_pad, tile, sums32,
                                   fx_acc(), acc64, n_copies, consts, guard);
