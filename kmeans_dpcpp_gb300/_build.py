@@ -58,7 +58,7 @@ CU_SOURCES = [
     "init.cu",
 ]
 HEADERS = ["km_common.cuh", "km_kernels.cuh", "km_fit.cuh", "km_mixed.cuh", "km_batch.cuh",
-           "km_step.cuh", "km_dist.cuh", "km_reg.cuh",
+           "km_step.cuh", "km_dist.cuh", "km_pair.cuh", "km_reg.cuh",
            "km_reg_kernel.cuh", "km_panel.cuh", "km_panel_kernel.cuh"]
 
 

@@ -66,12 +66,6 @@ __global__ void gather_kernel(const T *Xt, int64_t n, int64_t d, const int32_t *
     }
 }
 
-template <typename T>
-__device__ __forceinline__ T fma_k(T a, T b, T c);
-template <>
-__device__ __forceinline__ float fma_k(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-template <>
-__device__ __forceinline__ double fma_k(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // k-means++ draw, one launch per centre.  Each CTA takes blocks of kPPBlock
 // samples: it lowers the samples' min_d2 by the distance to the previous
@@ -408,7 +402,7 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
 #pragma unroll
                     for (int r = 0; r < kPPMine; ++r) {
                         const T diff = row[f * n + r * kPPThreads] - cf;
-                        acc[r] = fma_k(diff, diff, acc[r]);
+                        acc[r] = fma_rn(diff, diff, acc[r]);
                     }
                 }
             } else {
@@ -418,7 +412,7 @@ __global__ void __launch_bounds__(kPPThreads) pp_step_kernel(
                     for (int r = 0; r < kPPMine; ++r) {
                         if (i0 + tid + r * kPPThreads < n) {
                             const T diff = row[f * n + r * kPPThreads] - cf;
-                            acc[r] = fma_k(diff, diff, acc[r]);
+                            acc[r] = fma_rn(diff, diff, acc[r]);
                         }
                     }
                 }

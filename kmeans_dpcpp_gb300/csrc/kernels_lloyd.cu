@@ -66,10 +66,6 @@ constexpr int kThreads = 256;
 constexpr int MODE_ASSIGN = 0, MODE_FUSED = 1, MODE_DIST = 2;
 constexpr size_t kPrivMaxBytes = 64 * 1024;
 
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float sqrt_t(float a) { return __fsqrt_rn(a); }
 __device__ __forceinline__ double sqrt_t(double a) { return __dsqrt_rn(a); }
 
@@ -243,9 +239,9 @@ __global__ void __launch_bounds__(kThreads, 2) tile_kernel(TileArgs<T, I, A> a) 
                         for (int q = 0; q < TN; ++q) {
                             if (MODE == MODE_DIST) {
                                 T diff = cv[q] - xv[m];
-                                acc[m][q] = fma_t(diff, diff, acc[m][q]);
+                                acc[m][q] = fma_rn(diff, diff, acc[m][q]);
                             } else {
-                                acc[m][q] = fma_t(xv[m], cv[q], acc[m][q]);
+                                acc[m][q] = fma_rn(xv[m], cv[q], acc[m][q]);
                             }
                         }
                 }

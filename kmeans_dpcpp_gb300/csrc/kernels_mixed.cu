@@ -1739,7 +1739,6 @@ struct MixedSums {
         return ((double)p.hi * 4294967296.0 + (double)p.lo) *
                    (1.0 / (double)pow2f(consts->fx_shift)) + p.v;
     }
-    __device__ __forceinline__ void done() const {}
 };
 
 using MixedKernel = void (*)(MixedArgs);

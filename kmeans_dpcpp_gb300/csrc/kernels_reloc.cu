@@ -19,8 +19,6 @@ namespace kmc {
 
 namespace {
 
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 // Order-preserving unsigned keys (larger value -> larger key).
 template <typename T>

@@ -26,8 +26,6 @@ __device__ __forceinline__ double value_of(unsigned long long k, double) {
         (long long)((k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
-__device__ __forceinline__ float mul_step(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_step(double a, double b) { return __dmul_rn(a, b); }
 
 // Barrier over the (cooperatively launched) grid, number `*round` so far.  A
 // wait that runs out fails the fit: every CTA then leaves.
@@ -327,7 +325,7 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
             if (old < 0 || old >= k || cl < 0 || cl >= k) continue;
             const T wv = a.w[s];
             if (f < d) {
-                const T xw = mul_step(a.X[f * a.fs + s * a.ss], wv);  // rounded, as the reference
+                const T xw = mul_rn(a.X[f * a.fs + s * a.ss], wv);  // rounded, as the reference
                 a.sums[f * k + old] -= xw;
                 a.sums[f * k + cl] = xw;
             }
@@ -358,7 +356,7 @@ __global__ void __launch_bounds__(kRelocThreads, 2) relocate_kernel(RelocArgs<T,
                 const T diff = a.prev[at] - c;
                 a.nxt[at] = c;
                 a.cur[at] = c;
-                shift = fma_step(diff, diff, shift);
+                shift = fma_rn(diff, diff, shift);
             }
             a.shifts[j] = shift;
         }

@@ -12,10 +12,6 @@ namespace kmc {
 
 namespace {
 
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 __device__ __forceinline__ bool stopped(const LoopState *g) {
     return g != nullptr && *reinterpret_cast<const volatile int *>(&g->done) != 0;
@@ -47,11 +43,11 @@ __global__ void half_norm_kernel(const T *C, T *out, int64_t d, int64_t k,
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = C[(f + u) * k + j];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc = fma_t(v[u], v[u], acc);
+        for (int u = 0; u < 8; ++u) acc = fma_rn(v[u], v[u], acc);
     }
     for (; f < d; ++f) {
         const T v = C[f * k + j];
-        acc = fma_t(v, v, acc);
+        acc = fma_rn(v, v, acc);
     }
     out[j] = acc / T(2);
 }
@@ -146,7 +142,7 @@ __global__ void shifts_kernel(const T *old_c, const T *new_c, T *out, int64_t d,
     T acc = T(0);
     for (int64_t f = 0; f < d; ++f) {
         T diff = old_c[f * k + j] - new_c[f * k + j];
-        acc = fma_t(diff, diff, acc);
+        acc = fma_rn(diff, diff, acc);
     }
     out[j] = acc;
 }

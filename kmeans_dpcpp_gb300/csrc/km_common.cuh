@@ -138,6 +138,12 @@ int launch_chained(const char *what, void (*kern)(K...), dim3 grid, dim3 block, 
     return check_launch(what);
 }
 
+// Products and fused multiply-adds rounded as the reference's, never contracted.
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 // quotient_ceil of src/quotients_utils.hpp:5-6
 template <typename T>
 __host__ __device__ constexpr T ceil_div(T a, T b) { return (a + b - 1) / b; }

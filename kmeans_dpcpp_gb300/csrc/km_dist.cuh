@@ -7,8 +7,6 @@
 
 namespace kmc {
 
-__device__ __forceinline__ float fma_dist(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_dist(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // Predicated read-only loads (0 when not in).  Volatile: plain loads would be
 // moved into a branch that uses them, one latency each.
@@ -60,11 +58,11 @@ __device__ __forceinline__ T sq_dist_cols(const T *X, int64_t fs, int64_t ss, co
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = x[(f + u) * fs] - q[(f + u) * k];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc = fma_dist(v[u], v[u], acc);
+        for (int u = 0; u < 8; ++u) acc = fma_rn(v[u], v[u], acc);
     }
     for (; f < d; ++f) {
         const T diff = x[f * fs] - q[f * k];
-        acc = fma_dist(diff, diff, acc);
+        acc = fma_rn(diff, diff, acc);
     }
     return acc;
 }

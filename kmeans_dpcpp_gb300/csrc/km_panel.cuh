@@ -38,8 +38,6 @@
 namespace kmc {
 namespace panel {
 
-using u64 = unsigned long long;
-
 constexpr int MODE_LABELS = 0, MODE_DIST = 1;
 constexpr int kMaxWarps = 16;
 constexpr int kRows = 32;  // samples of a panel
@@ -92,10 +90,9 @@ __host__ __device__ inline int warps_for(int64_t d, int mode) {
 __host__ __device__ inline bool fits(int64_t d, int mode = MODE_LABELS) { return d >= 1 && warps_for(d, mode) > 0; }
 
 // T float with A float or double sums, and T = A = double (labels only).
-// tn: centroids per thread (8, 4 or 2; 0: the launcher's rule).
 template <typename T, typename A>
-int launch_labels(const Args<T, A> &a, cudaStream_t s, int tn = 0);
-int launch_dist(const Args<float, float> &a, cudaStream_t s, int tn = 0);
+int launch_labels(const Args<T, A> &a, cudaStream_t s);
+int launch_dist(const Args<float, float> &a, cudaStream_t s);
 
 }  // namespace panel
 }  // namespace kmc

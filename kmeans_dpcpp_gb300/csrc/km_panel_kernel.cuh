@@ -1,39 +1,17 @@
 // The kernel of km_panel.cuh (included by the panel_*.cu translation units).
 #pragma once
 
+#include "km_pair.cuh"
 #include "km_panel.cuh"
 
 namespace kmc {
 namespace panel {
 
-__device__ __forceinline__ u64 pack(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack(u64 v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 // The micro-tile's own: volatile keeps the order below, in which consecutive
 // instructions share an operand (the register file delivers two of the three
 // 64-bit operands per issue; 10M x 64 against 256 ran 13 % slower reordered).
 __device__ __forceinline__ void fma2_acc(u64 &acc, u64 a, u64 b) {
     asm volatile("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
-// float -> double.  The conversion instruction shares the float64 unit (2 per
-// clock and SM); a normal float is widened with integer operations instead.
-__device__ __forceinline__ double widen(float v) {
-    const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
-    if (e - 1u < 254u)
-        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
-                                (int)(b << 29));
-    return (double)v;
 }
 
 __device__ __forceinline__ void copy_async4(float *dst, const float *src, bool in) {
@@ -452,28 +430,8 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
                 // one undecided sample at a time, the warp's lanes over its centroids
                 const int src = __ffs(todo) - 1;
                 todo &= todo - 1u;
-                const T *xc = a.X + i0 + __shfl_sync(0xffffffffu, row, src);
-                T bv = pos_inf<T>();
-                int bj = 0;
-                for (int64_t j = lane; j < k; j += 32) {
-                    T dot = T(0);
-#pragma unroll 4
-                    for (int f = 0; f < d; ++f)
-                        dot = __fma_rn(xc[(int64_t)f * n], a.C[(int64_t)f * k + j], dot);
-                    const T e = a.hn[j] - dot;
-                    if (e < bv) {
-                        bv = e;
-                        bj = (int)j;
-                    }
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    const T ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                    const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-                    if (ov < bv || (ov == bv && oj < bj)) {
-                        bv = ov;
-                        bj = oj;
-                    }
-                }
+                const T *x = a.X + i0 + __shfl_sync(0xffffffffu, row, src);
+                const int bj = exact_label(x, n, a.C, a.hn, d, k);
                 if (lane == src) bidx[0] = bj;
             }
             labs[row] = bidx[0];
@@ -556,8 +514,8 @@ inline int columns_per_thread(int64_t k) {
 }
 
 template <int MODE, typename T, typename A>
-int launch_any(const Args<T, A> &a, cudaStream_t s, int tn) {
-    if (tn == 0) tn = columns_per_thread(a.k);
+int launch_any(const Args<T, A> &a, cudaStream_t s) {
+    const int tn = columns_per_thread(a.k);
     if (tn == 8) return launch_width<8, MODE, T, A>(a, s);
     if (tn == 4) return launch_width<4, MODE, T, A>(a, s);
     return launch_width<2, MODE, T, A>(a, s);

@@ -67,9 +67,9 @@ int launch_labels(const Args<T, A> &a, cudaStream_t s);
 int launch_dist(const Args<float, float> &a, cudaStream_t s);
 
 // Up to this many centroids the registers are used for labels / distances.
-constexpr int64_t kFewLabels = 64, kFewDist = 32;
+constexpr int64_t most_centroids(int mode) { return mode == MODE_DIST ? 32 : 64; }
 inline bool fits(int64_t d, int64_t k, int mode) {
-    return d >= 1 && d <= kMaxFeatures && k <= (mode == MODE_DIST ? kFewDist : kFewLabels);
+    return d >= 1 && d <= kMaxFeatures && k <= most_centroids(mode);
 }
 
 }  // namespace reg

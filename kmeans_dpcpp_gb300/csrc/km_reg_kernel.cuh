@@ -4,41 +4,11 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "km_pair.cuh"
 #include "km_reg.cuh"
 
 namespace kmc {
 namespace reg {
-
-using u64 = unsigned long long;
-
-__device__ __forceinline__ u64 pack(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack(u64 v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// float -> double.  The conversion instruction shares the float64 unit (2 per
-// clock and SM); a normal float is widened with integer operations instead.
-__device__ __forceinline__ double widen(float v) {
-    const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
-    if (e - 1u < 254u)
-        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
-                                (int)(b << 29));
-    return (double)v;
-}
 
 // Certification of float64 labels by float32 scores.  In units scaled by the
 // power of two sigma (largest |centroid coordinate| about 2^10), with u = 2^-24,
@@ -67,6 +37,10 @@ __global__ void __launch_bounds__(max_threads(DP), 1) reg_kernel(Args<T, A> a) {
     const int d = (int)a.d;
     const int kc = (int)(k < KC ? k : KC);
     float *cs = smem, *hs = smem + (size_t)kc * RS;
+    // Always so: fits() admits fewer centroids.  Written as a choice because the
+    // compiler schedules the float32 loops worse without the streamed form (1M x
+    // 32, k = 64: 111 us with it, 120 to 135 without, in five ways of writing the
+    // loop; a whole 200,003 x 32 estimator fit 2601 / 2735).
     const bool resident = k <= KC;
 
     float sigma = 1.f;
@@ -279,27 +253,7 @@ __global__ void __launch_bounds__(max_threads(DP), 1) reg_kernel(Args<T, A> a) {
                     const int src = __ffs(todo) - 1;
                     todo &= todo - 1u;
                     const T *xc = a.X + (i0 - lane + src + 32 * s);
-                    T bv = pos_inf<T>();
-                    int bj = 0;
-                    for (int64_t j = lane; j < k; j += 32) {
-                        T dot = T(0);
-#pragma unroll 4
-                        for (int f = 0; f < d; ++f)
-                            dot = __fma_rn(xc[(int64_t)f * n], a.C[(int64_t)f * k + j], dot);
-                        const T e = a.hn[j] - dot;
-                        if (e < bv) {
-                            bv = e;
-                            bj = (int)j;
-                        }
-                    }
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const T ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                        const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-                        if (ov < bv || (ov == bv && oj < bj)) {
-                            bv = ov;
-                            bj = oj;
-                        }
-                    }
+                    const int bj = exact_label(xc, n, a.C, a.hn, d, k);
                     if (lane == src) idx[s] = bj;
                 }
             }
@@ -362,9 +316,8 @@ int launch_class(const Args<T, A> &a, cudaStream_t s) {
     auto kern = reg_kernel<DP, MODE, T, A>;
     const int64_t rows = std::min<int64_t>(a.k, chunk_rows(DP, MODE));
     const size_t smem = sizeof(float) * (size_t)rows * (row_floats(DP, MODE) + 1);
-    if (smem > 48 * 1024)
-        KMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    static_assert(sizeof(float) * most_centroids(MODE) * (row_floats(DP, MODE) + 1) <= 47 * 1024,
+                  "the centroids fit the shared memory that needs no opt-in");
     // one CTA per SM; few samples are spread over all SMs in smaller CTAs
     const int64_t wtiles = ceil_div<int64_t>(a.n, 32 * samples_per_thread(DP));
     const int64_t warps = std::max<int64_t>(

@@ -75,7 +75,6 @@ struct PlainSums {
     static __device__ __forceinline__ Part zero() { return Part{0.0}; }
     static __device__ __forceinline__ void add(Part &a, const Part &b) { a.v += b.v; }
     __device__ __forceinline__ double value(const Part &p) const { return p.v; }
-    __device__ __forceinline__ void done() const {}
     // Copies g, g + groups, ... in order, zeroed once read; eight loads in flight.
     __device__ __forceinline__ Part load(int64_t f, int64_t j, int64_t d, int g, int groups) const {
         double *p = f < d ? sums + f * k + j : sizes + j;
@@ -106,7 +105,6 @@ struct ReducedSums {
         T v;
     };
     __device__ __forceinline__ T value(const Part &p) const { return p.v; }
-    __device__ __forceinline__ void done() const {}
     __device__ __forceinline__ Part load(int64_t f, int64_t j, int64_t d, int, int) const {
         return Part{f < d ? sums[f * k + j] : sizes[j]};
     }
@@ -194,8 +192,6 @@ __device__ __forceinline__ bool last_cta(unsigned *ticket) {
     return last_sh != 0;
 }
 
-__device__ __forceinline__ float fma_step(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_step(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // Division, each cluster's shift (features in order, as the reference adds
 // them), the plain forms' half norms for the next iteration (a launch of their
@@ -255,14 +251,14 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
 #pragma unroll 4
             for (int f = 0; f < nf; ++f) {
                 const T diff = diff_sh[f * jn + tid];
-                shift = fma_step(diff, diff, shift);
+                shift = fma_rn(diff, diff, shift);
             }
         } else if (tid >= 32 && tid < 32 + jn) {
             // the next iteration's half norms, by another warp
 #pragma unroll 4
             for (int f = 0; f < nf; ++f) {
                 const T c = new_sh[f * jn + tid - 32];
-                norm = fma_step(c, c, norm);
+                norm = fma_rn(c, c, norm);
             }
         }
         __syncthreads();
@@ -275,7 +271,6 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(Src src, FinishA
         if (tid == 0 && m != 0u) atomicAdd(&a.ctl->n_empty, __popc(m));
     }
     if (!last_cta(&a.ctl->finish_ticket)) return;
-    src.done();
     const int n_empty = *reinterpret_cast<volatile int *>(&a.ctl->n_empty);
     if (n_empty == 0) {
         stop_rule<T>(a.shifts, k, a.state, sh);

@@ -3,8 +3,8 @@
 
 namespace kmc {
 namespace panel {
-int launch_dist(const Args<float, float> &a, cudaStream_t s, int tn) {
-    return launch_any<MODE_DIST, float, float>(a, s, tn);
+int launch_dist(const Args<float, float> &a, cudaStream_t s) {
+    return launch_any<MODE_DIST, float, float>(a, s);
 }
 }  // namespace panel
 }  // namespace kmc

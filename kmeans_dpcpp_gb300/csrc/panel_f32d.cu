@@ -4,8 +4,8 @@
 namespace kmc {
 namespace panel {
 template <>
-int launch_labels<float, double>(const Args<float, double> &a, cudaStream_t s, int tn) {
-    return launch_any<MODE_LABELS, float, double>(a, s, tn);
+int launch_labels<float, double>(const Args<float, double> &a, cudaStream_t s) {
+    return launch_any<MODE_LABELS, float, double>(a, s);
 }
 }  // namespace panel
 }  // namespace kmc

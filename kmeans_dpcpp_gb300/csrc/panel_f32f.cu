@@ -4,8 +4,8 @@
 namespace kmc {
 namespace panel {
 template <>
-int launch_labels<float, float>(const Args<float, float> &a, cudaStream_t s, int tn) {
-    return launch_any<MODE_LABELS, float, float>(a, s, tn);
+int launch_labels<float, float>(const Args<float, float> &a, cudaStream_t s) {
+    return launch_any<MODE_LABELS, float, float>(a, s);
 }
 }  // namespace panel
 }  // namespace kmc

@@ -4,8 +4,8 @@
 namespace kmc {
 namespace panel {
 template <>
-int launch_labels<double, double>(const Args<double, double> &a, cudaStream_t s, int tn) {
-    return launch_any<MODE_LABELS, double, double>(a, s, tn);
+int launch_labels<double, double>(const Args<double, double> &a, cudaStream_t s) {
+    return launch_any<MODE_LABELS, double, double>(a, s);
 }
 }  // namespace panel
 }  // namespace kmc
