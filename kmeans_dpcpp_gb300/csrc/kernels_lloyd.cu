@@ -396,7 +396,7 @@ namespace {
 // shape (the tiles of this file do).
 template <typename T, typename A>
 bool launch_warp_labels(const reg::Args<T, A> &r, cudaStream_t s, int *rc) {
-    if (reg::fits(r.d, r.k, reg::MODE_LABELS))
+    if (reg::fits(r.d, r.k, reg::MODE_LABELS) && !reg::few_samples(r.n, r.d, r.k, sizeof(T) == 8))
         *rc = reg::launch_labels<T, A>(r, s);
     else if (panel::fits(r.d))
         *rc = panel::launch_labels<T, A>(r, s);
@@ -468,7 +468,8 @@ int launch_distances(const T *X, const T *C, T *out, int64_t n, int64_t d, int64
     if constexpr (sizeof(T) == 4) {
         const reg::Args<float, float> r{X, nullptr, C, nullptr, nullptr, 0, nullptr, nullptr, out,
                                         n, d, k, 1, nullptr};
-        if (reg::fits(d, k, reg::MODE_DIST)) return reg::launch_dist(r, s);
+        if (reg::fits(d, k, reg::MODE_DIST) && !reg::few_samples(n, d, k, false))
+            return reg::launch_dist(r, s);
         if (panel::fits(d, panel::MODE_DIST)) return panel::launch_dist(r, s);
     }
     TileArgs<T, int32_t> a{X, nullptr, C, nullptr, nullptr, nullptr, nullptr, out,

@@ -470,11 +470,10 @@ __device__ __forceinline__ void run_panels(const Args<T, A> &a, int warps, int64
 }
 
 template <int TN, int MODE, typename T, typename A>
-__global__ void __launch_bounds__(32 * kMaxWarps, 1) panel_kernel(Args<T, A> a) {
+__global__ void __launch_bounds__(32 * kMaxWarps, 1) panel_kernel(Args<T, A> a, int warps) {
     wait_for_previous();
     if (a.guard != nullptr && *reinterpret_cast<const volatile int *>(&a.guard->done)) return;
     extern __shared__ __align__(16) float smem[];
-    const int warps = blockDim.x >> 5;
     run_panels<TN, MODE, T, A>(a, warps, (int64_t)blockIdx.x * warps,
                                ceil_div<int64_t>(a.n, kRows), (int64_t)gridDim.x * warps,
                                (a.P > (int64_t)gridDim.x ? (int64_t)blockIdx.x * warps + (threadIdx.x >> 5)
@@ -486,14 +485,23 @@ template <int TN, int MODE, typename T, typename A>
 int launch_width(const Args<T, A> &a, cudaStream_t s) {
     if (a.n == 0) return KMC_OK;
     auto kern = panel_kernel<TN, MODE, T, A>;
-    // one CTA per SM; few samples are spread over all SMs in smaller CTAs
-    const int64_t wtiles = ceil_div<int64_t>(a.n, kRows);
-    const int warps = (int)std::max<int64_t>(
-        1, std::min<int64_t>(warps_for(a.d, MODE), ceil_div<int64_t>(wtiles, num_sms())));
+    // One CTA per SM.  Warps without samples help to load the centroids (2000 x
+    // 64 against 1000: 171 us without them, 66 with).  Up to three rounds are
+    // made equal: with all warps in the first and few samples left for the last,
+    // 80,000 x 64 against 600 took 232 us instead of 180 (with more rounds the
+    // last counts less than warps left out: distances of 400,003 x 30 to 250,
+    // six rounds of 16 warps 289 us, of 14 295).  Not for float64, whose undecided
+    // samples want all warps (80,000 x 64 against 600: 321 us, in equal rounds 441).
+    const int64_t wtiles = ceil_div<int64_t>(a.n, kRows), sms = num_sms();
+    const int all = warps_for(a.d, MODE);
+    int64_t rounds = ceil_div<int64_t>(wtiles, sms * all);
+    if (sizeof(T) == 8 || rounds > 3) rounds = 1;
+    const int warps = (int)std::min<int64_t>(all, ceil_div<int64_t>(wtiles, sms * rounds));
     const size_t smem = sizeof(float) * shape(a.d, a.k, TN, MODE, warps).total;
     KMC_TRY(allow_smem(kern, kSmemBytes));
     const int64_t grid = std::min<int64_t>(num_sms(), ceil_div<int64_t>(wtiles, warps));
-    return launch_chained("panel", kern, dim3((unsigned)grid), dim3((unsigned)(32 * warps)), smem, s, a);
+    return launch_chained("panel", kern, dim3((unsigned)grid), dim3((unsigned)(32 * all)), smem, s, a,
+                          warps);
 }
 
 // Columns of a step: 64, 32 or 16, whichever pads k least for its rate (the

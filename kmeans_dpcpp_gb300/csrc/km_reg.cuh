@@ -71,6 +71,15 @@ constexpr int64_t most_centroids(int mode) { return mode == MODE_DIST ? 32 : 64;
 inline bool fits(int64_t d, int64_t k, int mode) {
     return d >= 1 && d <= kMaxFeatures && k <= most_centroids(mode);
 }
+// With less than two warps per SM, a thread's own chain over all centroids bounds
+// the call, and the panels, which share it among eight lanes, are faster (labels of
+// 2000 samples, registers against panels, float32: 14 features and 64 centroids
+// 13.1 / 4.0 us, 32 and 16 8.5 / 3.9, 64 and 64 36 / 7.3; but 32 and 4 at 32,000
+// 4.4 / 4.8; float64: 32 and 64 49 / 16, but 4 and 53 7.5 / 8.6).
+inline bool few_samples(int64_t n, int64_t d, int64_t k, bool f64) {
+    const int64_t two_warps = 2 * 32 * (int64_t)num_sms() * samples_per_thread((int)d);
+    return n < two_warps && k >= 12 && k * d >= (f64 ? 500 : 200);
+}
 
 }  // namespace reg
 
