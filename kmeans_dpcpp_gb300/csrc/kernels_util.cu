@@ -5,6 +5,8 @@
 // Arithmetic order follows the SYCL kernels cited on each function: sums over
 // features run sequentially f = 0..d-1 with a fused multiply-add, exactly as
 // `acc += a * b` is contracted by the reference's device compiler.
+#include <algorithm>
+
 #include "km_dist.cuh"
 #include "km_kernels.cuh"
 
@@ -84,10 +86,8 @@ __global__ void __launch_bounds__(kCopyLanes * G)
                     if (p + u * G < P) s += v[u];
             }
         }
-        if (G > 1) {
-            red[g][el] = s;
-            __syncthreads();
-        }
+        red[g][el] = s;
+        __syncthreads();
         if (g == 0 && e < dk + k) {
 #pragma unroll
             for (int q = 1; q < G; ++q) s += red[q][el];
@@ -96,8 +96,75 @@ __global__ void __launch_bounds__(kCopyLanes * G)
             else
                 out_sizes[e - dk] = s;
         }
-        if (G > 1) __syncthreads();
+        __syncthreads();
     }
+}
+
+// The same sums, bit for bit, by one thread per element that holds the G partial
+// sums.  With enough elements (wide_sums) there are threads enough, and whole
+// warps read consecutive ones.  float64 additions bound the float64 form, so its
+// CTAs are small, for equal shares of the SMs.  137,004 elements: 16 copies 23.6 ->
+// 9.3 us (float64 48 -> 17), 152 copies 38 -> 15 (90 -> 64); 4 copies 11.3 -> 9.3.
+template <typename T>
+constexpr int kWideThreads = sizeof(T) == 8 ? 64 : 256;
+
+// 16 threads per element are as fast below (21,000 elements of 304 float copies
+// 13.4 us, by one thread 15.4; 31,000: 15.4, 15.4; 16,000 of 64: 11.3, 9.3;
+// float64 41,000 of 304: 49, 60; 61,000: 68, 66).
+template <typename T>
+bool wide_sums(int64_t elems, int64_t P) {
+    return elems >= std::max<int64_t>(16384, (sizeof(T) == 8 ? 200 : 100) * P);
+}
+
+// Loads that stay in front of the additions (the compiler keeps fewer in flight).
+__device__ __forceinline__ float load_in_order(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double load_in_order(const double *p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+template <typename T, int G>
+__global__ void __launch_bounds__(kWideThreads<T>)
+    reduce_copies_wide_kernel(const T *sizes_cp, const T *cent_cp, T *out_sizes, T *out_cent,
+                              int64_t P, int64_t d, int64_t k) {
+    const int64_t dk = d * k, e = blockIdx.x * (int64_t)kWideThreads<T> + threadIdx.x;
+    if (e >= dk + k) return;
+    const T *src = (e < dk) ? cent_cp + e : sizes_cp + (e - dk);
+    const int64_t stride = (e < dk) ? dk : k;
+    constexpr int kBatch = G > 1 ? G : 4;
+    T s[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) s[g] = T(0);
+    int64_t p = 0;
+    for (; p + kBatch <= P; p += kBatch) {
+        T v[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) v[u] = load_in_order(src + (p + u) * stride);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) s[u % G] += v[u];
+    }
+    if constexpr (G == 1) {
+        for (; p < P; ++p) s[0] += src[p * stride];
+    } else if (p < P) {
+        T v[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+            v[u] = load_in_order(src + (p + u < P ? p + u : p) * stride);
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+            if (p + u < P) s[u] += v[u];
+    }
+#pragma unroll
+    for (int g = 1; g < G; ++g) s[0] += s[g];
+    if (e < dk)
+        out_cent[e] = s[0];
+    else
+        out_sizes[e - dk] = s[0];
 }
 
 // Part 2: empty-cluster list.  The reference appends through an atomic
@@ -264,13 +331,16 @@ int launch_reduce_centroids(const T *sizes_cp, const T *cent_cp, T *out_sizes, T
                             I *empty_list, I *n_empty, int64_t P, int64_t d, int64_t k,
                             cudaStream_t s) {
     if (k == 0) return KMC_OK;
-    // up to 8 copies one thread has all its loads in flight at once
-    const unsigned grid = grid_for(d * k + k, kCopyLanes, 16384);
+    const int64_t elems = d * k + k;
+    const unsigned wide = (unsigned)ceil_div<int64_t>(elems, kWideThreads<T>);
     if (P <= 8)
-        reduce_copies_kernel<T, 1><<<grid, kCopyLanes, 0, s>>>(sizes_cp, cent_cp, out_sizes,
-                                                               out_cent, P, d, k);
+        reduce_copies_wide_kernel<T, 1><<<wide, kWideThreads<T>, 0, s>>>(
+            sizes_cp, cent_cp, out_sizes, out_cent, P, d, k);
+    else if (wide_sums<T>(elems, P))
+        reduce_copies_wide_kernel<T, 16><<<wide, kWideThreads<T>, 0, s>>>(
+            sizes_cp, cent_cp, out_sizes, out_cent, P, d, k);
     else
-        reduce_copies_kernel<T, 16><<<grid, kCopyLanes * 16, 0, s>>>(
+        reduce_copies_kernel<T, 16><<<grid_for(elems, kCopyLanes, 16384), kCopyLanes * 16, 0, s>>>(
             sizes_cp, cent_cp, out_sizes, out_cent, P, d, k);
     KMC_TRY(check_launch("reduce_centroids_data"));
     empty_list_kernel<T, I><<<1, 1024, 0, s>>>(out_sizes, empty_list, n_empty, k);
