@@ -116,18 +116,6 @@ bool wide_sums(int64_t elems, int64_t P) {
     return elems >= std::max<int64_t>(16384, (sizeof(T) == 8 ? 200 : 100) * P);
 }
 
-// Loads that stay in front of the additions (the compiler keeps fewer in flight).
-__device__ __forceinline__ float load_in_order(const float *p) {
-    float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double load_in_order(const double *p) {
-    double v;
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-
 template <typename T, int G>
 __global__ void __launch_bounds__(kWideThreads<T>)
     reduce_copies_wide_kernel(const T *sizes_cp, const T *cent_cp, T *out_sizes, T *out_cent,

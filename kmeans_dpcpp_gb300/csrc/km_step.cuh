@@ -82,9 +82,11 @@ struct PlainSums {
         double acc = 0.0;
         for (int64_t c = g; c < copies; c += 8 * groups) {
             double v[8];
+            // unconditional (the first again in the place of those past the last
+            // copy): a load behind a condition waits for the one before it
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                v[u] = c + u * groups < copies ? p[(c + u * groups) * stride] : 0.0;
+                v[u] = load_in_order(p + (c + u * groups < copies ? c + u * groups : c) * stride);
 #pragma unroll
             for (int u = 0; u < 8; ++u)
                 if (c + u * groups < copies) p[(c + u * groups) * stride] = 0.0;
