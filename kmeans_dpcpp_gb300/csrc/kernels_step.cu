@@ -276,14 +276,19 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
     const int64_t gid = blockIdx.x * (int64_t)kRelocThreads + tid;
     const int64_t gstride = (int64_t)gridDim.x * kRelocThreads;
     if (total <= kRankAll) {
-        for (int64_t e = gid; e < total; e += gstride) {
+        // a warp per entry, its lanes over the others (a thread per entry waited
+        // for each of them in turn: 2 ms for 3000)
+        const int64_t warps = (int64_t)gridDim.x * (kRelocThreads / 32);
+        for (int64_t e = (int64_t)wid * gridDim.x + blockIdx.x; e < total; e += warps) {
             const int64_t ie = __ldcg(a.gt_list + e);
-            int64_t r = 0;
-            for (int64_t q = 0; q < total; ++q) {
+            int r = 0;
+#pragma unroll 4
+            for (int64_t q = lane; q < total; q += 32) {
                 const int64_t iq = __ldcg(a.gt_list + q);
                 r += iq != ie && farther(a.sq_dist, iq, ie);
             }
-            a.far[r] = ie;
+            r = __reduce_add_sync(0xffffffffu, r);
+            if (lane == 0) a.far[r] = ie;
         }
     } else {
         // merge sort: an entry's place is its place in its own run plus the
@@ -315,26 +320,47 @@ __device__ __noinline__ bool relocate(const RelocArgs<T, I> &a, unsigned *round)
     }
     if (!grid_barrier(ctl, round, a.wait_limit)) return false;
 
-    // move the samples, one thread per feature, empty clusters in order
-    for (int64_t f = gid; f < d || f == 0; f += gstride) {
-        for (int64_t r = 0; r < m; ++r) {
-            if (r >= tg + need) break;
-            const int64_t s = __ldcg(a.far + r), cl = __ldcg(a.empty_list + r);
-            if (s < 0 || s >= n) continue;
-            const int64_t old = (int64_t)a.labels[s];
-            if (old < 0 || old >= k || cl < 0 || cl >= k) continue;
-            const T wv = a.w[s];
-            if (f < d) {
-                const T xw = mul_rn(a.X[f * a.fs + s * a.ss], wv);  // rounded, as the reference
-                a.sums[f * k + old] -= xw;
-                a.sums[f * k + cl] = xw;
+    // move the samples, one thread per feature (one more for the sizes), empty
+    // clusters in order; the loads of eight moves in flight
+    constexpr int kMoves = 8;
+    const int64_t moves = m < tg + need ? m : tg + need;
+    for (int64_t f = gid; f <= d; f += gstride) {
+        T *const row = f < d ? a.sums + f * k : a.sizes;
+        for (int64_t r0 = 0; r0 < moves; r0 += kMoves) {
+            int64_t s[kMoves], from[kMoves], to[kMoves];
+            T xw[kMoves], left[kMoves];
+#pragma unroll
+            for (int u = 0; u < kMoves; ++u) {
+                const int64_t r = r0 + u < moves ? r0 + u : r0;
+                s[u] = __ldcg(a.far + r);
+                to[u] = __ldcg(a.empty_list + r);
+                if (r0 + u >= moves || s[u] < 0 || s[u] >= n) s[u] = -1;
             }
-            if (f == 0) {
-                a.sizes[old] -= wv;
-                a.sizes[cl] = wv;
+#pragma unroll
+            for (int u = 0; u < kMoves; ++u) {
+                const int64_t i = s[u] < 0 ? 0 : s[u];
+                from[u] = (int64_t)a.labels[i];
+                if (s[u] < 0 || from[u] < 0 || from[u] >= k || to[u] < 0 || to[u] >= k)
+                    from[u] = to[u] = -1;
+                xw[u] = a.w[i];
+                if (f < d) xw[u] = mul_rn(a.X[f * a.fs + i * a.ss], xw[u]);  // rounded, as the reference
+            }
+#pragma unroll
+            for (int u = 0; u < kMoves; ++u) left[u] = row[from[u] < 0 ? 0 : from[u]];
+#pragma unroll
+            for (int u = 0; u < kMoves; ++u) {
+                // what the moves before it, loaded with it, made of that sum
+#pragma unroll
+                for (int v = 0; v < u; ++v) {
+                    if (from[v] == from[u]) left[u] = left[v];
+                    if (to[v] == from[u]) left[u] = xw[v];
+                }
+                left[u] -= xw[u];
+                if (from[u] < 0) continue;
+                row[from[u]] = left[u];
+                row[to[u]] = xw[u];
             }
         }
-        if (f >= d) break;
     }
     return grid_barrier(ctl, round, a.wait_limit);
 }
@@ -346,17 +372,32 @@ __global__ void __launch_bounds__(kRelocThreads, 2) relocate_kernel(RelocArgs<T,
     StepCtl *ctl = a.ctl;
     unsigned round = 0;
     if (relocate<T, I>(a, &round)) {
-        const int64_t gid = blockIdx.x * (int64_t)kRelocThreads + threadIdx.x;
-        for (int64_t j = gid; j < a.k; j += (int64_t)gridDim.x * kRelocThreads) {
+        // 32 clusters to a warp, the warps of all CTAs in turn: the divisions,
+        // float64 ones above all, want every SM
+        constexpr int kBatch = 4;
+        const int64_t warps = (int64_t)gridDim.x * (kRelocThreads / 32);
+        for (int64_t g = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; g * 32 < a.k; g += warps) {
+            const int64_t j = g * 32 + (threadIdx.x & 31);
+            if (j >= a.k) continue;
             const T size = __ldcg(a.sizes + j);
             T shift = T(0);
-            for (int64_t f = 0; f < a.d; ++f) {
-                const int64_t at = f * a.k + j;
-                const T c = __ldcg(a.sums + at) / size;
-                const T diff = a.prev[at] - c;
-                a.nxt[at] = c;
-                a.cur[at] = c;
-                shift = fma_rn(diff, diff, shift);
+            for (int64_t f0 = 0; f0 < a.d; f0 += kBatch) {
+                T sum[kBatch], old[kBatch];
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const int64_t at = (f0 + u < a.d ? f0 + u : f0) * a.k + j;
+                    sum[u] = __ldcg(a.sums + at);
+                    old[u] = a.prev[at];
+                }
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    if (f0 + u >= a.d) break;
+                    const int64_t at = (f0 + u) * a.k + j;
+                    const T c = sum[u] / size, diff = old[u] - c;
+                    a.nxt[at] = c;
+                    a.cur[at] = c;
+                    shift = fma_rn(diff, diff, shift);
+                }
             }
             a.shifts[j] = shift;
         }
@@ -383,9 +424,10 @@ __global__ void __launch_bounds__(kRelocThreads, 2) relocate_kernel(RelocArgs<T,
 
 template <typename T, typename I>
 int launch_relocation(const RelocArgs<T, I> &a, cudaStream_t s) {
-    // enough CTAs for the distances; two per SM are resident together (a
-    // cooperative launch)
-    const int64_t want = ceil_div<int64_t>(a.n, 4 * kRelocThreads);
+    // enough CTAs for the distances, and for the divisions; two per SM are resident
+    // together (a cooperative launch)
+    const int64_t want = std::max(ceil_div<int64_t>(a.n, 4 * kRelocThreads),
+                                  std::min(ceil_div<int64_t>(a.k, 32), a.d * a.k / 4096));
     const int64_t most = std::min<int64_t>(2 * (int64_t)num_sms(), kMaxRelocCtas);
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, most));
     const size_t smem = sizeof(T) == 4 && a.c_rows != nullptr && a.d > kRowVec
