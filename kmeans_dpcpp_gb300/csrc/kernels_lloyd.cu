@@ -1,5 +1,10 @@
-// Exact SIMT (FP32 / FP64) distance tiles: the fused Lloyd step, the
-// assignment kernel and the centroid-to-sample distance matrix.
+// Labels, the fused Lloyd step and the centroid-to-sample distance matrix in
+// exact FP32 / FP64 arithmetic: the choice among the register kernel
+// (km_reg.cuh), the panels (km_panel.cuh) and the tiles, which are below.  The
+// tiles take what the other two do not: more than 148 features (126 for
+// distances), float64 distances, the float64 step with its sums in one kernel
+// (the API's, and a fit's whose ordered sums do not fit, sums64.cu), and
+// float32 steps into fewer copies than SMs.
 //
 // Semantics (per sample i, centroid j), following the reference:
 //   dot_j  = sum_f x[f] * c[f, j]   accumulated f = 0..d-1 with one fused
@@ -10,7 +15,7 @@
 // The fused step then adds w*x into the centroid sums of `label` and w into
 // its size (src/lloyd_single_step.hpp:169-203).
 //
-// GB300 design: a 256-thread CTA owns a tile of BM samples and sweeps the
+// The tiles: a 256-thread CTA owns a tile of BM samples and sweeps the
 // centroids in tiles of BN; each thread keeps a TM x TN register micro-tile
 // of dot products (outer products over the feature axis from shared memory),
 // so every x and c element fetched from shared memory feeds TM or TN fused

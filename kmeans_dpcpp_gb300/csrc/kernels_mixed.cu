@@ -1149,8 +1149,8 @@ __global__ void __launch_bounds__(256) mixed_prep_kernel(
 // Exact fp32 re-evaluation of samples whose margin did not certify them: the
 // reference's arithmetic (sequential fma dot over f = 0..d-1, hn - dot,
 // strict < with the lowest index on ties) over the candidate set (hot
-// sub-chunks x hot classes of each column half).  A warp takes 32 flagged
-// samples and spreads their (sample, candidate) pairs evenly over its lanes,
+// sub-chunks x hot classes of each column half).  A warp takes its share of the
+// flagged samples, up to 32 at a time, and spreads their (sample, candidate) pairs evenly over its lanes,
 // so one sample with many candidates does not hold its warp back; each pair's
 // result goes into the sample's 64-bit (distance, index) key with a
 // shared-memory atomic minimum, which is exactly the lexicographic minimum a
@@ -1297,9 +1297,8 @@ __global__ void __launch_bounds__(kRecheckThreads) recheck_kernel(
 // best score minus E2, which is at most thr, so a hot pass's masks hold a
 // superset of its candidates.  The sample is certified when exactly one pass
 // reaches thr and that pass has a unique winner (single bits in one half,
-// nothing in the other): its label is written and w x added to its cluster's
-// sums.  Otherwise the masks of the passes below thr are cleared and the
-// sample goes to the recheck list.
+// nothing in the other): its label is written.  Otherwise the masks of the
+// passes below thr are cleared and the sample goes to the recheck list.
 __global__ void __launch_bounds__(256) combine_kernel(
     const float *pmax, uint4 *cand, int passes, int64_t pass_cols, const float *nx,
     const float *ndx, const MixedConsts *consts, void *labels, int label64, int *flagged,
@@ -2040,10 +2039,9 @@ struct MixedFit : PlainFit<float, I> {
         // n_copies: with few clusters their few addresses would serialise the
         // reductions of all SMs (4M x 64 alone: k = 100 and 1 copy 502 us, 16
         // copies 260, 152 copies 231; k = 1024 and 1 copy 272, 4 copies 227).
-        // Every iteration reads every copy, so the float32 sums get 4096 / k,
-        // and small fits one per eight tiles.  A copy of the integer sums also
-        // bounds the rows it adds up, which the scale pays for in bits: one
-        // per SM, as far as they fit 64 MB.
+        // Every iteration reads and clears every copy, so there are 4096 / k of
+        // them (at least 4, of the integer sums 16, since the rows that a copy
+        // adds up cost the scale bits), at most one per SM and per eight tiles.
         {
             const int64_t most = std::min<int64_t>(ntiles / 8, num_sms());
             const int64_t want = std::max<int64_t>(4096 / p.k, acc_f64 ? 16 : 4);
@@ -2205,7 +2203,9 @@ struct MixedFit : PlainFit<float, I> {
     }
 
     // The sums' kernel: CTAs, samples of a CTA's tile, rounds of tiles.  The
-    // sorted one has all of its CTAs resident and gives them equal rounds.
+    // sorted one has all of its CTAs resident (kSortCtas per SM, whose shared
+    // memory sort_rows keeps within an SM's) and gives them equal rounds; the
+    // direct ones, beyond kSortClusters, take 256 samples at a time.
     bool sums_sorted() const { return this->prm.k <= kSortClusters; }
     int64_t sum_grid() const {
         const int64_t n = std::max<int64_t>(this->prm.n, 1);

@@ -73,8 +73,8 @@ struct FitBase {
     // the next tensor-core assignment pass first waits on a barrier that
     // nothing completes, so that wait runs out (test of the timeout path).
     virtual int set_wait_limit(long long clocks, int stall) = 0;
-    // Centroid-tile variant of the plain form's kernels (the autotuner's
-    // choice unless set here); the mixed forms ignore it.
+    // Centroid-tile variant of a plain fit whose iterations run in the tiles
+    // (the autotuner's choice unless set here); other fits ignore it.
     virtual int set_tile_variant(int v) {
         (void)v;
         return KMC_OK;
@@ -123,7 +123,7 @@ struct PlainFit : FitBase {
     // which the caller may change its centroids)
     bool hn_current = false;
     bool split64 = false;  // float64 samples: labels, then sums (sums64.cu)
-    int tile_variant = 0;  // autotuned centroid-tile width of the plain kernels
+    int tile_variant = 0;  // autotuned centroid-tile width (fits that run in the tiles)
     Scratch xt;  // feature-major copy of a row-major X (forms that need one)
     static constexpr long long kWaitClocks = 4000000000LL;  // about two seconds
     long long wait_limit = kWaitClocks;
