@@ -66,7 +66,6 @@ __global__ void gather_kernel(const T *Xt, int64_t n, int64_t d, const int32_t *
     }
 }
 
-
 // k-means++ draw, one launch per centre.  Each CTA takes blocks of kPPBlock
 // samples: it lowers the samples' min_d2 by the distance to the previous
 // centre (one fused multiply-add per feature, f = 0..d-1) and forms the

@@ -574,7 +574,6 @@ template int tune_fit_variant<double>(int64_t, int64_t, cudaStream_t, int *);
                                             T *, T *, int64_t, int64_t, int64_t, int64_t,     \
                                             cudaStream_t, const LoopState *, int);            \
 
-
 template int launch_fused_step<float, int32_t, double>(const float *, const float *,
                                                        const float *, const float *, int32_t *,
                                                        double *, double *, int64_t, int64_t,

@@ -57,8 +57,8 @@
 //               threads per row; tiles of one chunk: two groups, a thread per row)
 // The recheck kernel labels the samples that were not certified; the cluster
 // sums are a pass of their own over the labels (sum_sorted_kernel).
-// A pass without sums over 4M x 64 (two update warps in the kernel before):
-// 454 -> 416 us at k = 1024, 217 -> 177 us at k = 256, 211 -> 159 us at k = 64
+// A pass without sums over 4M x 64 (before, two warps that added the sums ran
+// beside the epilogue): 454 -> 416 us at k = 1024, 217 -> 177 us at k = 256, 211 -> 159 us at k = 64
 // (146 and 145 with the two groups).
 //
 // Every wait is bounded.  A wait that runs out raises the CTA's error flag;
@@ -1829,8 +1829,9 @@ template <typename I>
 int make_mixed_fit_impl(const FitParams<float, I> &p, int form, std::unique_ptr<FitBase> *out);
 
 // Times each candidate variant on a synthetic fit (Gaussian blobs of d
-// features, k clusters) for four iterations after one warm-up, and caches the
-// fastest per (d, k, form, size class).  Fits of at least 32 tiles per SM
+// features, k clusters) for four iterations after one warm-up, and keeps the
+// fastest per (d, k, form, size class) in memory (the file's reader takes tile
+// widths only, so every process times these anew).  Fits of at least 32 tiles per SM
 // ("large") are timed with 48 tiles per SM, smaller ones with 8.  KMC_TUNE=0 keeps
 // the default (the first candidate).
 int tune_mixed_variant(int64_t d, int64_t k, int form, bool large, const std::vector<int> &cand,
@@ -1991,7 +1992,7 @@ struct MixedFit : PlainFit<float, I> {
         // Ring depth and, for the integer sums, the rows (or terms) a lane has
         // in flight: a variant code 10 stages + f (f = 4 or 2; 0: other sums).
         // The autotuner times the variants that fit on a synthetic fit once
-        // per (d, power-of-two bucket of k, form, size class) and caches the
+        // per (d, power-of-two bucket of k, form, size class) and keeps the
         // fastest; the deepest ring with f = 2 is the default when tuning is
         // off.
         {

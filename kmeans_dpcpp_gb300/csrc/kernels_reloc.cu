@@ -19,7 +19,6 @@ namespace kmc {
 
 namespace {
 
-
 // Order-preserving unsigned keys (larger value -> larger key).
 template <typename T>
 struct KeyOf;

@@ -26,7 +26,6 @@ __device__ __forceinline__ double value_of(unsigned long long k, double) {
         (long long)((k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
-
 // Barrier over the (cooperatively launched) grid, number `*round` so far.  A
 // wait that runs out fails the fit: every CTA then leaves.
 __device__ __forceinline__ bool grid_barrier(StepCtl *ctl, unsigned *round, long long limit) {

@@ -14,7 +14,6 @@ namespace kmc {
 
 namespace {
 
-
 __device__ __forceinline__ bool stopped(const LoopState *g) {
     return g != nullptr && *reinterpret_cast<const volatile int *>(&g->done) != 0;
 }

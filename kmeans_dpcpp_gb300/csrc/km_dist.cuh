@@ -7,7 +7,6 @@
 
 namespace kmc {
 
-
 // Predicated read-only loads (0 when not in).  Volatile: plain loads would be
 // moved into a branch that uses them, one latency each.
 __device__ __forceinline__ float4 load_f4_if(const float4 *p, bool in) {

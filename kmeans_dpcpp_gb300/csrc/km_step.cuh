@@ -194,7 +194,6 @@ __device__ __forceinline__ bool last_cta(unsigned *ticket) {
     return last_sh != 0;
 }
 
-
 // Division, each cluster's shift (features in order, as the reference adds
 // them), the plain forms' half norms for the next iteration (a launch of their
 // own before: 50,000 x 14, k = 16, 20 iterations 707 -> 629 us) and, in the last CTA, the stop rule or the empty-cluster list.  A CTA

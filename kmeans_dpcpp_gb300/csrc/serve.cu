@@ -668,7 +668,6 @@ int capture_iteration(Active &a) {
     return KMC_OK;
 }
 
-
 // A request server: fits, predictions and transforms of different sizes on
 // caller buffers, admitted in submission order while the HBM budget and the
 // number of running requests allow; predictions wait (without blocking the
@@ -1088,7 +1087,6 @@ struct Server {
     }
 };
 
-
 // Shapes a form can serve: the batched engine takes d <= 1024 and k <= 4096;
 // the tensor-core sessions take what the mixed fit supports.
 int check_shape(int form, int64_t d, int64_t k) {
@@ -1209,7 +1207,6 @@ int serve_run(const kmc_serve_request_t *rq, int64_t n_req, int form, int64_t bu
 }
 
 }  // namespace serving
-
 
 }  // namespace kmc
 

@@ -1,6 +1,5 @@
-"""The autotuner's cache file: which fits are tuned, and which lines of an
-existing file are believed.  Each case runs in a process of its own, because the
-file is read once per process."""
+"""The autotuner's cache file: which fits are tuned.  Each case runs in a process
+of its own, because the file is read once per process."""
 import os
 import subprocess
 import sys
